@@ -118,7 +118,9 @@ struct psb_ctx {
     float2* rpc = nullptr;
     float* rho_x = nullptr;
     unsigned long long* err_hist = nullptr;
-    int* flags = nullptr;     // [0] overflow [1] max count [2..3] pair total [4] clamped
+    int* flags = nullptr;     // [0] overflow [1] max count [2..3] pair total [4] clamped [5] wall list length
+    int* wall_list = nullptr;         // config-profile SPH: slots near the box faces (Params::wall_list)
+    uint32_t* wall_bits = nullptr;
     void* stage = nullptr;    // device staging for uploads/downloads
     // learned warm start
     float* feats = nullptr;   // n_max x 8
@@ -326,6 +328,7 @@ void free_all(psb_ctx* c) {
     cudaFree(c->hist); cudaFree(c->cell_start); cudaFree(c->cell_end); cudaFree(c->nbr_count);
     cudaFree(c->nbr_list); cudaFree(c->fnp); cudaFree(c->vs); cudaFree(c->rpc); cudaFree(c->rho_x);
     cudaFree(c->err_hist); cudaFree(c->flags); cudaFree(c->stage);
+    cudaFree(c->wall_list); cudaFree(c->wall_bits);
     cudaFree(c->bnd_vel); cudaFree(c->bnd_fext); cudaFree(c->bnd_pred); cudaFree(c->bnd_react);
     cudaFree(c->feats); cudaFree(c->mlp_w); cudaFree(c->mlp_m1); cudaFree(c->mlp_m2); cudaFree(c->mlp_grad); cudaFree(c->mlp_part);
     cudaFree(c->mlp_loss); cudaFree(c->mlp_wbf); cudaFree(c->ds_X); cudaFree(c->ds_T); cudaFree(c->sel);
@@ -580,12 +583,12 @@ int build(psb_ctx* c, bool keep_p = false, bool features = false) {
     const bool split = capturing(st) ? c->capture_split : c->in_pending;
     if (split) {
         timed(c, "reorder_pos", [&] {
-            psb::launch_reorder_pos(st, n, c->keys[res], c->vals[res], c->pos[os], c->ids[orr], c->pos[ns], c->ids[nr],
+            psb::launch_reorder_pos(st, P, c->keys[res], c->vals[res], c->pos[os], c->ids[orr], c->pos[ns], c->ids[nr],
                                     c->cell_start, c->cell_end);
         });
     } else {
         timed(c, "reorder", [&] {
-            psb::launch_reorder(st, n, c->keys[res], c->vals[res], c->pos[os], c->vel[os], c->vap[os], c->rp[orr],
+            psb::launch_reorder(st, P, c->keys[res], c->vals[res], c->pos[os], c->vel[os], c->vap[os], c->rp[orr],
                                 c->ids[orr], c->pos[ns], c->vel[ns], c->vap[ns], c->rp[nr], c->ids[nr], c->cell_start,
                                 c->cell_end);
         });
@@ -1041,6 +1044,13 @@ int create_impl(const psb_scene* scene, size_t ncells, psb_ctx** out) {
     if (!rc) rc = dalloc(c, &c->rho_x, n);
     if (!rc) rc = dalloc(c, &c->err_hist, PSB_MAX_ITERS + 1);
     if (!rc) rc = dalloc(c, &c->flags, 8);
+    if (!c->P.ref && !c->P.dem) {       // the profile with wall ghosts
+        if (!rc) rc = dalloc(c, &c->wall_list, n);
+        if (!rc) rc = dalloc(c, &c->wall_bits, (n + 31) / 32);
+        c->P.wall_list = c->wall_list;
+        c->P.wall_bits = c->wall_bits;
+        c->P.wall_count = c->flags + 5;
+    }
     // uploads and downloads stage every array at once: 3 x 12 + 2 x 4 bytes
     if (!rc) rc = dalloc(c, (char**)&c->stage, n * 48);
     if (!rc) rc = dalloc(c, &c->feats, n * 8);

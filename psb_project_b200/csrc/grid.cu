@@ -170,18 +170,51 @@ __global__ void __launch_bounds__(kBlock) k_radix_scatter(int n, int shift, int 
     }
 }
 
+// Lists slot t (position x) in P.wall_list when it lies near a box face, and
+// writes the warp's flag word; every lane of the warp calls it. One atomic
+// add per warp that has such a particle; the list's order is left open.
+template <bool BATCH>
+__device__ __forceinline__ void list_near_walls(const Params& P, int t, float4 x) {
+    if (!P.wall_list || P.n < kWallListMin) return;
+    bool near = false;
+    if (t < P.n) {
+        const float reach = kWallReach * P.hf;
+        float lo_x = P.bx0, lo_y = P.by0, lo_z = P.bz0, hi_x = P.bx1, hi_y = P.by1, hi_z = P.bz1;
+        if (BATCH) {
+            const SceneGeom* G = P.scenes + P.slot_scene[t];
+            lo_x = G->bx0; lo_y = G->by0; lo_z = G->bz0; hi_x = G->bx1; hi_y = G->by1; hi_z = G->bz1;
+        }
+        near = x.x - lo_x < reach || hi_x - x.x < reach || x.y - lo_y < reach || hi_y - x.y < reach ||
+               x.z - lo_z < reach || hi_z - x.z < reach;
+    }
+    const unsigned word = __ballot_sync(0xffffffffu, near);
+    const int lane = threadIdx.x & 31;
+    int base = 0;
+    if (lane == 0) {
+        if (t < P.n) P.wall_bits[t >> 5] = word;
+        if (word) base = atomicAdd(P.wall_count, __popc(word));
+    }
+    if (!word) return;
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (near) P.wall_list[base + __popc(word & ((1u << lane) - 1u))] = t;
+}
+
 // Gathers the particle state into sorted order and records each occupied
 // cell's [start, end) slot range.
-__global__ void k_reorder(int n, const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals,
+template <bool BATCH>
+__global__ void k_reorder(Params P, const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals,
                           const float4* __restrict__ pos, const float4* __restrict__ vel,
                           const float4* __restrict__ vap, const float2* __restrict__ rp, const int* __restrict__ ids,
                           float4* __restrict__ pos2, float4* __restrict__ vel2, float4* __restrict__ vap2,
                           float2* __restrict__ rp2, int* __restrict__ ids2, uint32_t* __restrict__ cell_start,
                           uint32_t* __restrict__ cell_end) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int n = P.n;
+    const uint32_t s = t < n ? vals[t] : 0u;
+    const float4 x = t < n ? pos[s] : make_float4(0.f, 0.f, 0.f, 0.f);
+    list_near_walls<BATCH>(P, t, x);
     if (t >= n) return;
-    const uint32_t s = vals[t];
-    pos2[t] = pos[s];
+    pos2[t] = x;
     vel2[t] = vel[s];
     vap2[t] = vap[s];
     rp2[t] = rp[s];
@@ -194,14 +227,18 @@ __global__ void k_reorder(int n, const uint32_t* __restrict__ keys, const uint32
 // The same in two launches, for the first step after an upload: positions,
 // ids and cell ranges (all that the neighbour build reads) here, the rest
 // in k_reorder_state once the upload's copies of it are in.
-__global__ void k_reorder_pos(int n, const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals,
+template <bool BATCH>
+__global__ void k_reorder_pos(Params P, const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals,
                               const float4* __restrict__ pos, const int* __restrict__ ids, float4* __restrict__ pos2,
                               int* __restrict__ ids2, uint32_t* __restrict__ cell_start,
                               uint32_t* __restrict__ cell_end) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int n = P.n;
+    const uint32_t s = t < n ? vals[t] : 0u;
+    const float4 x = t < n ? pos[s] : make_float4(0.f, 0.f, 0.f, 0.f);
+    list_near_walls<BATCH>(P, t, x);
     if (t >= n) return;
-    const uint32_t s = vals[t];
-    pos2[t] = pos[s];
+    pos2[t] = x;
     ids2[t] = ids[s];
     const uint32_t k = keys[t];
     if (t == 0 || keys[t - 1] != k) cell_start[k] = (uint32_t)t;
@@ -383,18 +420,20 @@ int radix_sort(cudaStream_t st, int n, int bits, uint32_t* keys[2], uint32_t* va
     return cur;
 }
 
-void launch_reorder(cudaStream_t st, int n, const uint32_t* keys, const uint32_t* vals, const float4* pos,
+void launch_reorder(cudaStream_t st, const Params& P, const uint32_t* keys, const uint32_t* vals, const float4* pos,
                     const float4* vel, const float4* vap, const float2* rp, const int* ids, float4* pos2, float4* vel2,
                     float4* vap2, float2* rp2, int* ids2, uint32_t* cell_start, uint32_t* cell_end) {
-    if (n > 0)
-        k_reorder<<<grid_of(n), kBlock, 0, st>>>(n, keys, vals, pos, vel, vap, rp, ids, pos2, vel2, vap2, rp2, ids2,
-                                                 cell_start, cell_end);
+    if (P.n <= 0) return;
+    auto kernel = P.scenes ? k_reorder<true> : k_reorder<false>;
+    kernel<<<grid_of(P.n), kBlock, 0, st>>>(P, keys, vals, pos, vel, vap, rp, ids, pos2, vel2, vap2, rp2, ids2,
+                                            cell_start, cell_end);
 }
 
-void launch_reorder_pos(cudaStream_t st, int n, const uint32_t* keys, const uint32_t* vals, const float4* pos,
+void launch_reorder_pos(cudaStream_t st, const Params& P, const uint32_t* keys, const uint32_t* vals, const float4* pos,
                         const int* ids, float4* pos2, int* ids2, uint32_t* cell_start, uint32_t* cell_end) {
-    if (n > 0)
-        k_reorder_pos<<<grid_of(n), kBlock, 0, st>>>(n, keys, vals, pos, ids, pos2, ids2, cell_start, cell_end);
+    if (P.n <= 0) return;
+    auto kernel = P.scenes ? k_reorder_pos<true> : k_reorder_pos<false>;
+    kernel<<<grid_of(P.n), kBlock, 0, st>>>(P, keys, vals, pos, ids, pos2, ids2, cell_start, cell_end);
 }
 
 void launch_reorder_state(cudaStream_t st, int n, const uint32_t* vals, const float4* vel, const float4* vap,

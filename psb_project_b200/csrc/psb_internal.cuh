@@ -118,7 +118,23 @@ struct Params {
     // (colliders.cuh); n_coll == 0: none. Single-scene contexts only.
     const Collider* coll;
     int n_coll;
+    // Particles near the box faces (config-profile SPH; sph.cu): their slots
+    // in any order, how many, and a flag bit per slot, all written by the
+    // step's reorder. wall_list == nullptr: none. wall_blocks: the blocks of
+    // a launch that take the list (set per launch).
+    int* wall_list;
+    int* wall_count;
+    uint32_t* wall_bits;
+    int wall_blocks;
 };
+
+// Distance to a face, in h, up to which the reorder lists a particle: past
+// the h within which a face has ghosts, so that the corrector's predictions
+// (a CFL step moves a particle well under 0.1 h) rarely bring an unlisted
+// particle into range. The list is used from kWallListMin particles on
+// (sph.cu gives both sides' times).
+constexpr float kWallReach = 1.1f;
+constexpr int kWallListMin = 131072;
 
 // Runs f(std::integral_constant<int, B>) with B the tuned block size.
 template <class F>
@@ -250,10 +266,11 @@ int radix_blocks(int n);
 // The whole state into sorted order, with the cell ranges; or in two
 // launches: positions, ids and cell ranges (what the neighbour build reads),
 // then the rest.
-void launch_reorder(cudaStream_t st, int n, const uint32_t* keys, const uint32_t* vals, const float4* pos,
+// Both also list the particles near the box faces (P.wall_list).
+void launch_reorder(cudaStream_t st, const Params& P, const uint32_t* keys, const uint32_t* vals, const float4* pos,
                     const float4* vel, const float4* vap, const float2* rp, const int* ids, float4* pos2, float4* vel2,
                     float4* vap2, float2* rp2, int* ids2, uint32_t* cell_start, uint32_t* cell_end);
-void launch_reorder_pos(cudaStream_t st, int n, const uint32_t* keys, const uint32_t* vals, const float4* pos,
+void launch_reorder_pos(cudaStream_t st, const Params& P, const uint32_t* keys, const uint32_t* vals, const float4* pos,
                         const int* ids, float4* pos2, int* ids2, uint32_t* cell_start, uint32_t* cell_end);
 void launch_reorder_state(cudaStream_t st, int n, const uint32_t* vals, const float4* vel, const float4* vap,
                           const float2* rp, float4* vel2, float4* vap2, float2* rp2);

@@ -142,95 +142,100 @@ __device__ __forceinline__ float3 wall_accel(const Params& P, int t, float4 x, f
 // the neighbour list yields all of them. Ghosts carry j's pressure continued
 // hydrostatically across the faces, p_j + rho0 (-g . n) 2 d_j, so a resting
 // column is held by its bottom layer as by any interior layer.
-// The faces near a particle, packed in one word: bits 0-1 hold their count
-// n (at most one face per axis), and face k takes 3 bits at 2 + 3k: its axis
-// (2 bits) and whether it is the lower face (inward normal +1).
+//
+// The ghost walk is the longest chain of a sweep: every sweep takes at least
+// as long as one corner particle's. With per-face loops over packed face
+// words and every set's distance formed, that was 75-80 us at any size
+// (density at x at 16,384 particles: 80 us). With the faces in registers, the
+// sets unrolled and most neighbours left out by one compare per axis it is
+// 20 us there, and 24 against 86 us for the density pass at 97,000.
+//
+// The faces near a particle at x_i, one per axis at most: inward normal
+// (+1 lower, -1 upper), plane and x_i's distance inside it, clamped at 0 so
+// that a particle pushed through the face still sees its ghosts on the wall
+// side (unclamped, its own ghost would push it further out). An axis with no
+// near face has its plane at -infinity: every distance from it is infinite,
+// so no ghost across it passes the range tests below.
+struct NearFaces {
+    float nrm[3], plane[3], di[3];
+};
+
 __device__ __forceinline__ float comp(float4 v, int a) { return a == 0 ? v.x : (a == 1 ? v.y : v.z); }
-__device__ __forceinline__ float gcomp(const Params& P, int a) { return a == 0 ? P.gx : (a == 1 ? P.gy : P.gz); }
 
+// Fills W for x; whether any face is within h.
 template <class F_>
-__device__ __forceinline__ unsigned near_walls(const Params& P, const F_& F, float4 x) {
-    unsigned w = 0u, n = 0u;
-    auto push = [&](unsigned axis, unsigned lower) { w |= (axis | (lower << 2)) << (2u + 3u * n); ++n; };
-    if (x.x - F.x0() < P.hf) push(0u, 1u);
-    else if (F.x1() - x.x < P.hf) push(0u, 0u);
-    if (x.y - F.y0() < P.hf) push(1u, 1u);
-    else if (F.y1() - x.y < P.hf) push(1u, 0u);
-    if (x.z - F.z0() < P.hf) push(2u, 1u);
-    else if (F.z1() - x.z < P.hf) push(2u, 0u);
-    return w | n;
-}
-
-// Reflects the offset across face k of w: with d = nrm (x - plane) the
-// distances on the box side, component a of r becomes nrm (d_i + d_j), both
-// clamped at 0 so that a particle pushed through the face still sees its
-// ghosts on the wall side (unclamped, its own ghost would push it further
-// out). False if x_j is h or more inside.
-template <class F_>
-__device__ __forceinline__ bool reflect(const Params& P, const F_& F, unsigned w, int k, float4 xi, float4 xj,
-                                        float3& r, float& dp) {
-    const unsigned f = (w >> (2 + 3 * k)) & 7u;
-    const int a = (int)(f & 3u);
-    const bool lower = (f >> 2) != 0u;
-    const float plane = lower ? (a == 0 ? F.x0() : (a == 1 ? F.y0() : F.z0()))
-                              : (a == 0 ? F.x1() : (a == 1 ? F.y1() : F.z1()));
-    const float nrm = lower ? 1.f : -1.f;
-    const float dj = fmaxf(__fmul_rn(nrm, __fsub_rn(comp(xj, a), plane)), 0.f);
-    if (dj >= P.hf) return false;
-    const float di = fmaxf(__fmul_rn(nrm, __fsub_rn(comp(xi, a), plane)), 0.f);
-    const float v = __fmul_rn(nrm, __fadd_rn(di, dj));
-    if (a == 0) r.x = v; else if (a == 1) r.y = v; else r.z = v;
-    dp = __fmaf_rn(__fmul_rn(__fmul_rn(P.rho0, __fmul_rn(-gcomp(P, a), nrm)), 2.f), dj, dp);
-    return true;
-}
-
-// x_i minus the ghost of x_j across the faces in `mask`; false if a face of
-// the set is h or more from x_j. dp: the ghost's hydrostatic pressure offset.
-template <class F_>
-__device__ __forceinline__ bool ghost_delta(const Params& P, const F_& F, unsigned w, int mask, float4 xi,
-                                            float4 xj, float3& r, float& dp) {
-    r = make_float3(__fsub_rn(xi.x, xj.x), __fsub_rn(xi.y, xj.y), __fsub_rn(xi.z, xj.z));
-    dp = 0.f;
-    if ((mask & 1) && !reflect(P, F, w, 0, xi, xj, r, dp)) return false;
-    if ((mask & 2) && !reflect(P, F, w, 1, xi, xj, r, dp)) return false;
-    if ((mask & 4) && !reflect(P, F, w, 2, xi, xj, r, dp)) return false;
-    return true;
-}
-
-// The ghosts of neighbour x_j (one per non-empty subset of the near faces).
-// Density: adds (1-q)^3 of each ghost within h.
-template <class F_>
-__device__ __forceinline__ void ghost_density_pair(const Params& P, const F_& F, unsigned w, float4 xi, float4 xj,
-                                                   Kahan& acc) {
-    const int nm = 1 << (w & 3u);
-    for (int mask = 1; mask < nm; ++mask) {
-        float3 r;
-        float dp;
-        if (!ghost_delta(P, F, w, mask, xi, xj, r, dp)) continue;
-        const float q = __fmul_rn(dist2(r.x, r.y, r.z), P.inv_h2);
-        if (q >= 1.f) continue;
-        add_poly6(acc, q);
+__device__ __forceinline__ bool near_faces(const Params& P, const F_& F, float4 x, NearFaces& W) {
+    const float lo[3] = {F.x0(), F.y0(), F.z0()}, hi[3] = {F.x1(), F.y1(), F.z1()};
+    bool any = false;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float xa = comp(x, a);
+        const bool lower = xa - lo[a] < P.hf, upper = hi[a] - xa < P.hf;
+        any |= lower | upper;
+        W.nrm[a] = lower || !upper ? 1.f : -1.f;
+        W.plane[a] = lower ? lo[a] : (upper ? hi[a] : -INFINITY);
+        W.di[a] = fmaxf(__fmul_rn(W.nrm[a], __fsub_rn(xa, W.plane[a])), 0.f);
     }
+    return any;
+}
+
+// The ghosts of neighbour x_j, one per non-empty set of the near faces, in
+// the order x, y, xy, z, xz, yz, xyz: add(r, dp) with r = x_i minus the
+// ghost -- a reflected component is nrm (d_i + d_j) -- and dp the ghost's
+// hydrostatic pressure offset (PRESSURE). A face h or more from x_j reflects
+// nothing; one whose reflected component alone reaches h (with a margin over
+// the rounding of the squared distance) cannot bring a ghost into range, so
+// its sets are left out before their distances are formed.
+template <bool PRESSURE, class F>
+__device__ __forceinline__ void for_each_ghost(const Params& P, const NearFaces& W, float4 xi, float4 xj, F&& add) {
+    const float n[3] = {__fsub_rn(xi.x, xj.x), __fsub_rn(xi.y, xj.y), __fsub_rn(xi.z, xj.z)};
+    const float g[3] = {P.gx, P.gy, P.gz};
+    const float reach = P.hf * 1.00001f;
+    float r[3], dj[3], hc[3];
+    bool in[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        dj[a] = fmaxf(__fmul_rn(W.nrm[a], __fsub_rn(comp(xj, a), W.plane[a])), 0.f);
+        const float d = __fadd_rn(W.di[a], dj[a]);
+        in[a] = !(dj[a] >= P.hf) && !(d >= reach);
+        r[a] = __fmul_rn(W.nrm[a], d);
+        hc[a] = PRESSURE ? __fmul_rn(__fmul_rn(P.rho0, __fmul_rn(-g[a], W.nrm[a])), 2.f) : 0.f;
+    }
+    if (!(in[0] || in[1] || in[2])) return;
+#pragma unroll
+    for (int mask = 1; mask < 8; ++mask) {
+        if (((mask & 1) && !in[0]) || ((mask & 2) && !in[1]) || ((mask & 4) && !in[2])) continue;
+        float dp = 0.f;
+        if (PRESSURE) {
+            if (mask & 1) dp = __fmaf_rn(hc[0], dj[0], dp);
+            if (mask & 2) dp = __fmaf_rn(hc[1], dj[1], dp);
+            if (mask & 4) dp = __fmaf_rn(hc[2], dj[2], dp);
+        }
+        add(make_float3(mask & 1 ? r[0] : n[0], mask & 2 ? r[1] : n[1], mask & 4 ? r[2] : n[2]), dp);
+    }
+}
+
+// Density: adds (1-q)^3 of each ghost within h.
+__device__ __forceinline__ void ghost_density_pair(const Params& P, const NearFaces& W, float4 xi, float4 xj,
+                                                   Kahan& acc) {
+    for_each_ghost<false>(P, W, xi, xj, [&](float3 r, float) {
+        const float q = __fmul_rn(dist2(r.x, r.y, r.z), P.inv_h2);
+        if (!(q >= 1.f)) add_poly6(acc, q);
+    });
 }
 
 // Pressure: adds (pV_i + pV_ghost) (1-u)^2 x^ of each ghost within h, the
 // ghost carrying p_j continued hydrostatically across its faces.
-template <class F_>
-__device__ __forceinline__ void ghost_pressure_pair(const Params& P, const F_& F, unsigned w, float4 xi, float4 xj,
-                                                    float pVi, float pj, float3& ap) {
-    const float ir0 = 1.f / __fmul_rn(P.rho0, P.rho0);
-    const int nm = 1 << (w & 3u);
-    for (int mask = 1; mask < nm; ++mask) {
-        float3 r;
-        float dp;
-        if (!ghost_delta(P, F, w, mask, xi, xj, r, dp)) continue;
+__device__ __forceinline__ void ghost_pressure_pair(const Params& P, const NearFaces& W, float4 xi, float4 xj,
+                                                    float pVi, float pj, float ir0, float3& ap) {
+    for_each_ghost<true>(P, W, xi, xj, [&](float3 r, float dp) {
         const float r2 = dist2(r.x, r.y, r.z);
-        if (!(r2 > 0.f) || __fmul_rn(r2, P.inv_h2) >= 1.f) continue;
+        if (!(r2 > 0.f) || __fmul_rn(r2, P.inv_h2) >= 1.f) return;
         const float rinv = rsqrtf(r2);
         const float om = spiky_om(P, r2, rinv);
         const float sc = __fmul_rn(__fmul_rn(__fmul_rn(__fmaf_rn(__fadd_rn(pj, dp), ir0, pVi), om), om), rinv);
         ap.x = __fmaf_rn(sc, r.x, ap.x); ap.y = __fmaf_rn(sc, r.y, ap.y); ap.z = __fmaf_rn(sc, r.z, ap.z);
-    }
+    });
 }
 
 // Ghost terms of particle t, in a second walk of its list that only
@@ -244,22 +249,64 @@ __device__ __forceinline__ void ghost_pressure_pair(const Params& P, const F_& F
 template <bool BATCH = false>
 __device__ __forceinline__ void ghost_density(const Params& P, int t, float4 xi, const float4* pos,
                                               const int* __restrict__ list, int cnt, Kahan& acc) {
-    const auto F = faces_of<BATCH>(P, t);
-    const unsigned wall = near_walls(P, F, xi);
-    if (!(wall & 3u)) return;
-    for_each_nbr(list, P.n, t, cnt, [&](const int j) { ghost_density_pair(P, F, wall, xi, pos[j], acc); });
+    NearFaces W;
+    if (!near_faces(P, faces_of<BATCH>(P, t), xi, W)) return;
+    for_each_nbr(list, P.n, t, cnt, [&](const int j) { ghost_density_pair(P, W, xi, pos[j], acc); });
 }
 
 template <bool BATCH = false>
 __device__ __forceinline__ void ghost_pressure(const Params& P, int t, float4 xi, float pVi,
-                                               const float4* __restrict__ pos, const float* pj_of,
-                                               int pj_stride, const int* __restrict__ list, int cnt, float3& ap) {
-    const auto F = faces_of<BATCH>(P, t);
-    const unsigned wall = near_walls(P, F, xi);
-    if (!(wall & 3u)) return;
+                                               const float4* __restrict__ pos, const float2* rp,
+                                               const int* __restrict__ list, int cnt, float3& ap) {
+    NearFaces W;
+    if (!near_faces(P, faces_of<BATCH>(P, t), xi, W)) return;
+    const float ir0 = 1.f / __fmul_rn(P.rho0, P.rho0);
     for_each_nbr(list, P.n, t, cnt, [&](const int j) {
-        ghost_pressure_pair(P, F, wall, xi, pos[j], pVi, pj_of[(size_t)j * pj_stride], ap);
+        const float4 xj = pos[j];
+        const float pj = rp[j].y;
+        ghost_pressure_pair(P, W, xi, xj, pVi, pj, ir0, ap);
     });
+}
+
+// ---- particles near the walls -----------------------------------------------
+// A particle near a face walks its list twice and sums up to seven ghosts a
+// neighbour. In slot order such particles sit a few to a warp, and the warp
+// waits for them with its other lanes idle. From kWallListMin particles on,
+// the step's reorder therefore lists them (P.wall_list) and flags them by
+// slot, and a sweep with ghost terms launches P.wall_blocks blocks over the
+// list ahead of the blocks over all slots, which skip the listed ones: full
+// warps of wall particles, started first. Each particle is summed by one
+// thread in the same order either way, so the results are the same bits.
+// Density pass / pressure-force pass with the list against without:
+// 78 / 86 against 88 / 96 us at 1,048,576 particles, 36 / 45 against 44 / 58
+// at 290,000; at 97,000, where the pass is one chain of loads and the list
+// adds two, 29 / 30 against 24 / 24 us.
+__device__ __forceinline__ bool in_wall_list(const Params& P, int t) {
+    return P.wall_list && ((P.wall_bits[t >> 5] >> (t & 31)) & 1u);
+}
+
+// The slots of this thread in a launch of BS-thread blocks: f(slot), or f(-1)
+// where it has none. Every lane of a warp makes the same calls.
+template <int BS, bool GHOSTS, class F>
+__device__ __forceinline__ void for_each_slot(const Params& P, F&& f) {
+    if (!GHOSTS) {
+        const int t = blockIdx.x * BS + threadIdx.x;
+        f(t < P.n ? t : -1);
+        return;
+    }
+    const bool wall = (int)blockIdx.x < P.wall_blocks;
+    const int first = ((int)blockIdx.x - (wall ? 0 : P.wall_blocks)) * BS + threadIdx.x;
+    const int end = wall ? *P.wall_count : P.n;
+    int k = first;
+    do {
+        int t = -1;
+        if (k < end) {
+            if (wall) t = P.wall_list[k];
+            else if (!P.wall_blocks || !in_wall_list(P, k)) t = k;
+        }
+        f(t);
+        k += P.wall_blocks * BS;
+    } while (wall && k - (int)(threadIdx.x & 31) < end);
 }
 
 // Boundary particles (config profile; boundary.cu): density psi_b W_ib, as
@@ -436,21 +483,27 @@ struct DensityX {
     }
 };
 
+// Resident threads per SM asked of the sweeps with ghost terms: what the
+// main walk's registers allow (40, 48 or 56 a thread), so that the ghost
+// walk, which few threads take, spills rather than lowering the occupancy of
+// all (density pass at 4M particles: 272 us at 40 registers, 354 at 56).
+constexpr int kDensityThreads = 1536, kForceThreads = 1280, kInitThreads = 1152;
+
 template <bool REF, int NF, bool BATCH, int BS>
-__global__ void __launch_bounds__(BS) k_density_x(Params P, const float4* __restrict__ pos,
-                                                      const float4* __restrict__ vel, const int* __restrict__ counts,
-                                                      const int* __restrict__ list, float2* __restrict__ rp,
-                                                      float* __restrict__ rho_x, int zero_p, float p_scale,
-                                                      float* __restrict__ feats) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= P.n) return;
-    const float4 xi = pos[t];
-    const int count = counts[t];
-    const int cnt = min(count, P.cap);
-    DensityX<REF, NF> D;
-    D.begin(vel, t);
-    for_each_nbr(list, P.n, t, cnt, [&](const int j) { D.pair(P, xi, pos[j], j, vel, rp); });
-    D.template finish<BATCH>(P, t, xi, pos, list, cnt, count, rp, rho_x, zero_p, p_scale, feats);
+__global__ void __launch_bounds__(BS, REF ? 1 : (NF ? kForceThreads : kDensityThreads) / BS)
+    k_density_x(Params P, const float4* __restrict__ pos, const float4* __restrict__ vel,
+                const int* __restrict__ counts, const int* __restrict__ list, float2* __restrict__ rp,
+                float* __restrict__ rho_x, int zero_p, float p_scale, float* __restrict__ feats) {
+    for_each_slot<BS, !REF>(P, [&](const int t) {
+        if (t < 0) return;
+        const float4 xi = pos[t];
+        const int count = counts[t];
+        const int cnt = min(count, P.cap);
+        DensityX<REF, NF> D;
+        D.begin(vel, t);
+        for_each_nbr(list, P.n, t, cnt, [&](const int j) { D.pair(P, xi, pos[j], j, vel, rp); });
+        D.template finish<BATCH>(P, t, xi, pos, list, cnt, count, rp, rho_x, zero_p, p_scale, feats);
+    });
 }
 
 // The neighbour build of one scene (config profile) with the density pass
@@ -502,6 +555,42 @@ struct PairSums {
     float fs;       // sum (1-q)(3-7q) / rho_j           (times -k_surf: surface term)
 };
 
+// Config: p/rho0^2 (the PCISPH linearisation; see k_pci_force_predict).
+template <bool REF>
+__device__ __forceinline__ float pressure_volume(const Params& P, float2 rp) {
+    return REF ? rp.y / (rp.x * rp.x) : rp.y * (1.f / (P.rho0 * P.rho0));
+}
+
+// Adds the pair (i, j) to S; xj, rpj: neighbour j's position, (density, pressure).
+template <bool REF, bool WITH_PRESSURE>
+__device__ __forceinline__ void add_pair(const Params& P, PairSums& S, float4 xi, float4 vi, float pVi, float4 xj,
+                                         float4 vj, float2 rpj) {
+    const float ir0 = 1.f / (P.rho0 * P.rho0);
+    const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
+    const float r2 = dist2(dx, dy, dz);
+    if (!(r2 > 0.f)) return;
+    const float q = r2 * P.inv_h2;
+    if (!REF && q >= 1.f) return;
+    const float rinv = rsqrtf(r2);
+    const float om = 1.f - r2 * rinv * P.inv_h;
+    const float inv_rj = 1.f / rpj.x;
+    const float sv = om * inv_rj;
+    S.fv.x += (vj.x - vi.x) * sv;
+    S.fv.y += (vj.y - vi.y) * sv;
+    S.fv.z += (vj.z - vi.z) * sv;
+    if (WITH_PRESSURE) {
+        const float pVj = REF ? rpj.y * inv_rj * inv_rj : rpj.y * ir0;
+        const float s = (pVi + pVj) * om * om * rinv;
+        S.ap.x += s * dx; S.ap.y += s * dy; S.ap.z += s * dz;
+    }
+    if (REF) {      // surface tension and normals: reference profile only
+        const float t1 = 1.f - q;
+        S.fs += t1 * (3.f - 7.f * q) * inv_rj;
+        const float sn = t1 * t1 * inv_rj;
+        S.nrm.x += dx * sn; S.nrm.y += dy * sn; S.nrm.z += dz * sn;
+    }
+}
+
 template <bool REF, bool WITH_PRESSURE, bool BATCH = false>
 __device__ __forceinline__ PairSums pair_sums(const Params& P, int t, float4 xi, float4 vi, float2 rpi,
                                               const float4* __restrict__ pos, const float4* __restrict__ vel,
@@ -510,40 +599,16 @@ __device__ __forceinline__ PairSums pair_sums(const Params& P, int t, float4 xi,
     PairSums S;
     S.ap = S.fv = S.nrm = make_float3(0.f, 0.f, 0.f);
     S.fs = 0.f;
-    // Config: p/rho0^2 (the PCISPH linearisation; see k_pci_force_predict).
-    const float ir0 = 1.f / (P.rho0 * P.rho0);
-    const float pVi = WITH_PRESSURE ? (REF ? rpi.y / (rpi.x * rpi.x) : rpi.y * ir0) : 0.f;
+    const float pVi = WITH_PRESSURE ? pressure_volume<REF>(P, rpi) : 0.f;
     const int cnt = min(counts[t], P.cap);
     for_each_nbr(list, P.n, t, cnt, [&](const int j) {
         const float4 xj = pos[j];       // the pair's three gathers, ahead of the tests
         const float4 vj = vel[j];
         const float2 rpj = rp[j];
-        const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-        const float r2 = dist2(dx, dy, dz);
-        if (!(r2 > 0.f)) return;
-        const float q = r2 * P.inv_h2;
-        if (!REF && q >= 1.f) return;
-        const float rinv = rsqrtf(r2);
-        const float om = 1.f - r2 * rinv * P.inv_h;
-        const float inv_rj = 1.f / rpj.x;
-        const float sv = om * inv_rj;
-        S.fv.x += (vj.x - vi.x) * sv;
-        S.fv.y += (vj.y - vi.y) * sv;
-        S.fv.z += (vj.z - vi.z) * sv;
-        if (WITH_PRESSURE) {
-            const float pVj = REF ? rpj.y * inv_rj * inv_rj : rpj.y * ir0;
-            const float s = (pVi + pVj) * om * om * rinv;
-            S.ap.x += s * dx; S.ap.y += s * dy; S.ap.z += s * dz;
-        }
-        if (REF) {      // surface tension and normals: reference profile only
-            const float t1 = 1.f - q;
-            S.fs += t1 * (3.f - 7.f * q) * inv_rj;
-            const float sn = t1 * t1 * inv_rj;
-            S.nrm.x += dx * sn; S.nrm.y += dy * sn; S.nrm.z += dz * sn;
-        }
+        add_pair<REF, WITH_PRESSURE>(P, S, xi, vi, pVi, xj, vj, rpj);
     });
     if (WITH_PRESSURE && !REF) {
-        ghost_pressure<BATCH>(P, t, xi, pVi, pos, (const float*)rp + 1, 2, list, cnt, S.ap);
+        ghost_pressure<BATCH>(P, t, xi, pVi, pos, rp, list, cnt, S.ap);
         if (!BATCH) boundary_pressure(P, t, xi, pVi, S.ap);
     }
     return S;
@@ -575,57 +640,78 @@ __global__ void __launch_bounds__(kBlock) k_wcsph_force(Params P, const float4* 
                                                         const int* __restrict__ list, float4* __restrict__ pos_out,
                                                         float4* __restrict__ vel_out, float4* __restrict__ vap_out,
                                                         float4* __restrict__ fnp) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= P.n) return;
-    const float4 xi = pos[t], vi = vel[t], vh = vap[t];
-    const float2 rpi = rp[t];
-    const PairSums S = pair_sums<REF, true>(P, t, xi, vi, rpi, pos, vel, rp, counts, list);
-    const float3 f = nonpressure_force<REF>(P, S, rpi.x);
-    fnp[t] = make_float4(f.x, f.y, f.z, 0.f);
-    const float3 aw = wall_accel<REF>(P, t, xi, vh);
-    const float ir = 1.f / rpi.x;
-    const float3 a = make_float3(f.x * ir + P.k_grad * S.ap.x + aw.x, f.y * ir + P.k_grad * S.ap.y + aw.y,
-                                 f.z * ir + P.k_grad * S.ap.z + aw.z);
-    float3 v = make_float3(vh.x + a.x * P.dt, vh.y + a.y * P.dt, vh.z + a.z * P.dt);
-    float3 x = make_float3(xi.x + v.x * P.dt, xi.y + v.y * P.dt, xi.z + v.z * P.dt);
-    if (REF) box_project(P, t, x, v);   // config WCSPH: penalty walls only
-    pos_out[t] = make_float4(x.x, x.y, x.z, 0.f);
-    vap_out[t] = make_float4(v.x, v.y, v.z, 0.f);
-    vel_out[t] = make_float4((vh.x + v.x) * 0.5f, (vh.y + v.y) * 0.5f, (vh.z + v.z) * 0.5f, 0.f);
+    auto integrate = [&](const int t, const float4 xi, const float2 rpi, const PairSums& S) {
+        const float4 vh = vap[t];
+        const float3 f = nonpressure_force<REF>(P, S, rpi.x);
+        fnp[t] = make_float4(f.x, f.y, f.z, 0.f);
+        const float3 aw = wall_accel<REF>(P, t, xi, vh);
+        const float ir = 1.f / rpi.x;
+        const float3 a = make_float3(f.x * ir + P.k_grad * S.ap.x + aw.x, f.y * ir + P.k_grad * S.ap.y + aw.y,
+                                     f.z * ir + P.k_grad * S.ap.z + aw.z);
+        float3 v = make_float3(vh.x + a.x * P.dt, vh.y + a.y * P.dt, vh.z + a.z * P.dt);
+        float3 x = make_float3(xi.x + v.x * P.dt, xi.y + v.y * P.dt, xi.z + v.z * P.dt);
+        if (REF) box_project(P, t, x, v);   // config WCSPH: penalty walls only
+        pos_out[t] = make_float4(x.x, x.y, x.z, 0.f);
+        vap_out[t] = make_float4(v.x, v.y, v.z, 0.f);
+        vel_out[t] = make_float4((vh.x + v.x) * 0.5f, (vh.y + v.y) * 0.5f, (vh.z + v.z) * 0.5f, 0.f);
+    };
+    for_each_slot<kBlock, !REF>(P, [&](const int t) {
+        if (t < 0) return;
+        const float4 xi = pos[t], vi = vel[t];
+        const float2 rpi = rp[t];
+        integrate(t, xi, rpi, pair_sums<REF, true>(P, t, xi, vi, rpi, pos, vel, rp, counts, list));
+    });
 }
 
 // PCISPH set-up sweep: non-pressure forces at x (and, for a warm start, the
 // pressure acceleration of the carried pressure), then the first prediction.
 template <bool REF, bool WARM, bool BATCH, int BS>
-__global__ void __launch_bounds__(BS) k_pci_init(Params P, const float4* __restrict__ pos,
+__global__ void __launch_bounds__(BS, REF || !WARM ? 1 : kInitThreads / BS) k_pci_init(Params P, const float4* __restrict__ pos,
                                                      const float4* __restrict__ vel, const float4* __restrict__ vap,
                                                      const float2* __restrict__ rp, const int* __restrict__ counts,
                                                      const int* __restrict__ list, float4* __restrict__ fnp,
                                                      float4* __restrict__ xs, float4* __restrict__ vs) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= P.n) return;
-    const float4 xi = pos[t], vi = vel[t], vh = vap[t];
-    const float2 rpi = rp[t];
-    const PairSums S = pair_sums<REF, WARM, BATCH>(P, t, xi, vi, rpi, pos, vel, rp, counts, list);
-    const float3 f = nonpressure_force<REF>(P, S, rpi.x);
-    fnp[t] = make_float4(f.x, f.y, f.z, 0.f);
-    const float3 aw = wall_accel<REF, BATCH>(P, t, xi, vh);
-    const float ir = 1.f / rpi.x;
-    const float ap = WARM ? P.k_grad : 0.f;
-    const float3 a = make_float3(f.x * ir + ap * S.ap.x + aw.x, f.y * ir + ap * S.ap.y + aw.y,
-                                 f.z * ir + ap * S.ap.z + aw.z);
-    const float3 v = make_float3(vh.x + a.x * P.dt, vh.y + a.y * P.dt, vh.z + a.z * P.dt);
-    vs[t] = make_float4(v.x, v.y, v.z, 0.f);
-    xs[t] = make_float4(xi.x + v.x * P.dt, xi.y + v.y * P.dt, xi.z + v.z * P.dt, 0.f);
+    auto predict = [&](const int t, const float4 xi, const float2 rpi, const PairSums& S) {
+        const float4 vh = vap[t];
+        const float3 f = nonpressure_force<REF>(P, S, rpi.x);
+        fnp[t] = make_float4(f.x, f.y, f.z, 0.f);
+        const float3 aw = wall_accel<REF, BATCH>(P, t, xi, vh);
+        const float ir = 1.f / rpi.x;
+        const float ap = WARM ? P.k_grad : 0.f;
+        const float3 a = make_float3(f.x * ir + ap * S.ap.x + aw.x, f.y * ir + ap * S.ap.y + aw.y,
+                                     f.z * ir + ap * S.ap.z + aw.z);
+        const float3 v = make_float3(vh.x + a.x * P.dt, vh.y + a.y * P.dt, vh.z + a.z * P.dt);
+        vs[t] = make_float4(v.x, v.y, v.z, 0.f);
+        xs[t] = make_float4(xi.x + v.x * P.dt, xi.y + v.y * P.dt, xi.z + v.z * P.dt, 0.f);
+    };
+    for_each_slot<BS, !REF && WARM>(P, [&](const int t) {
+        if (t < 0) return;
+        const float4 xi = pos[t], vi = vel[t];
+        const float2 rpi = rp[t];
+        predict(t, xi, rpi, pair_sums<REF, WARM, BATCH>(P, t, xi, vi, rpi, pos, vel, rp, counts, list));
+    });
 }
 
 // PCISPH density pass at x*: rho*, the gradient sums of the pressure
 // increment, the candidate pressure and the FP64 max compression error.
-// Batch: scenes that have converged are left as they are, and the error is
-// the max over each scene (P.err_scene).
-// The density pass for sorted particle t (t < P.n, its scene still
-// iterating): rho* and the candidate pressure into rpc[t]; returns the
-// compression error (rho* - rho0)/rho0 in FP64.
+// The compression error (rho* - rho0)/rho0 in FP64 of sorted particle t, from
+// its compensated sum; rho* and the candidate pressure into rpc[t].
+template <bool REF, class F2, class F2o>
+__device__ __forceinline__ double pci_density_finish(const Params& P, int t, const Kahan& acc, float3 T1, float T2,
+                                                     F2 rp, F2o rpc) {
+    const float drho = density_deviation(P, acc);
+    const float rho = __fadd_rn(P.rho0, drho);
+    float p = rp[t].y;
+    if (REF) {              // per-particle factor, compressed particles only
+        if (drho > 0.f && T2 > 0.f) p += P.k_press * drho / (T1.x * T1.x + T1.y * T1.y + T1.z * T1.z + T2);
+    } else {                // prototype factor, every particle, p >= 0
+        p = fmaxf(0.f, __fmaf_rn(P.k_delta, drho, p));
+    }
+    rpc[t] = make_float2(rho, p);
+    return (double)drho / P.rho0_d;
+}
+
+// The density pass for sorted particle t (t < P.n, its scene still iterating).
 template <bool REF, bool BATCH, class F4, class F2, class F2o>
 __device__ __forceinline__ double pci_density_at(const Params& P, int t, F4 xs, F2 rp, const int* __restrict__ counts,
                                                  const int* __restrict__ list, F2o rpc) {
@@ -654,16 +740,7 @@ __device__ __forceinline__ double pci_density_at(const Params& P, int t, F4 xs, 
         ghost_density<BATCH>(P, t, xi, xs, list, cnt, acc);
         if (!BATCH) boundary_density(P, t, xi, acc, P.bnd_pred ? P.bnd_pred : P.bnd);
     }
-    const float drho = density_deviation(P, acc);
-    const float rho = __fadd_rn(P.rho0, drho);
-    float p = rp[t].y;
-    if (REF) {              // per-particle factor, compressed particles only
-        if (drho > 0.f && T2 > 0.f) p += P.k_press * drho / (T1.x * T1.x + T1.y * T1.y + T1.z * T1.z + T2);
-    } else {                // prototype factor, every particle, p >= 0
-        p = fmaxf(0.f, __fmaf_rn(P.k_delta, drho, p));
-    }
-    rpc[t] = make_float2(rho, p);
-    return (double)drho / P.rho0_d;
+    return pci_density_finish<REF>(P, t, acc, T1, T2, rp, rpc);
 }
 
 // The max of the pass's errors. Batch: per scene (P.err_scene); a warp
@@ -717,28 +794,59 @@ __device__ __forceinline__ void warp_max_error(const Params& P, int sc, double e
 }
 
 template <bool REF, bool BATCH, int BS>
-__global__ void __launch_bounds__(BS) k_pci_density(Params P, const float4* __restrict__ xs,
+__global__ void __launch_bounds__(BS, REF ? 1 : kDensityThreads / BS) k_pci_density(Params P, const float4* __restrict__ xs,
                                                         const float2* __restrict__ rp, const int* __restrict__ counts,
                                                         const int* __restrict__ list, float2* __restrict__ rpc,
                                                         unsigned long long* __restrict__ err_slot) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    double err = -1e300;
-    const int sc = BATCH && t < P.n ? (int)P.slot_scene[t] : -1;
-    if (t < P.n && (!BATCH || P.active[sc])) err = pci_density_at<REF, BATCH>(P, t, xs, rp, counts, list, rpc);
-    warp_max_error<BATCH, BS>(P, sc, err, err_slot);
+    double worst = -1e300;
+    for_each_slot<BS, !REF>(P, [&](const int t) {
+        const int sc = BATCH && t >= 0 ? (int)P.slot_scene[t] : -1;
+        double err = -1e300;
+        if (t >= 0 && (!BATCH || P.active[sc])) err = pci_density_at<REF, BATCH>(P, t, xs, rp, counts, list, rpc);
+        if (BATCH) warp_max_error<true, BS>(P, sc, err, err_slot);
+        else worst = fmax(worst, err);
+    });
+    if (!BATCH) warp_max_error<false, BS>(P, -1, worst, err_slot);
 }
 
-// PCISPH pressure-force pass fused with the next prediction; commits the
-// candidate pressure. Reference profile: at the predicted positions x*, with
-// p/rho*^2 (PciSphSystem_Kernel.cu:88-114 runs on the predicted state).
-// Config profile: at the step's start positions x, with p/rho0^2. That keeps
-// the corrector a linear iteration in p: at x*, x* = x + dt^2 a(x*) is a
-// fixed-point iteration in positions whose gain grows with p dt^2/h^2, and
-// with rho* in p/rho^2 the force feeds back on the density; under a 0.64 m
-// column either one makes the corrector diverge.
+// The pair (i, j) of the pressure force: (pV_i + pV_j) (1-u)^2 x^ into acc.
+template <bool REF>
+__device__ __forceinline__ void add_pressure_pair(const Params& P, float4 xi, float4 xj, float pVi, float2 rj, float ir0,
+                                                  float3& acc) {
+    const float dx = __fsub_rn(xi.x, xj.x), dy = __fsub_rn(xi.y, xj.y), dz = __fsub_rn(xi.z, xj.z);
+    const float r2 = dist2(dx, dy, dz);
+    if (!(r2 > 0.f)) return;
+    if (!REF && __fmul_rn(r2, P.inv_h2) >= 1.f) return;
+    const float rinv = rsqrtf(r2);
+    const float om = spiky_om(P, r2, rinv);
+    // pV_i + pV_j (config: p_j / rho0^2 fused into the sum), then products only
+    const float pv = REF ? pVi + rj.y / (rj.x * rj.x) : __fmaf_rn(rj.y, ir0, pVi);
+    const float s = pv * om * om * rinv;
+    acc.x = __fmaf_rn(s, dx, acc.x); acc.y = __fmaf_rn(s, dy, acc.y); acc.z = __fmaf_rn(s, dz, acc.z);
+}
+
+// From the finished pressure sum of particle t: the next prediction into
+// xs_next[t] and vs[t], and the candidate pressure ri committed to rp[t].
+template <bool REF, bool BATCH>
+__device__ __forceinline__ void pci_force_finish(const Params& P, int t, float2 ri, float3 acc,
+                                                 const float4* __restrict__ pos, const float4* __restrict__ vap,
+                                                 const float4* __restrict__ fnp, float4* xs_next, float4* vs,
+                                                 float2* rp) {
+    const float4 x0 = pos[t], vh = vap[t], f = fnp[t];
+    const float3 aw = wall_accel<REF, BATCH>(P, t, x0, vh);
+    const float ir = 1.f / ri.x;
+    auto accel = [&](float fc, float ac, float wc) {     // f/rho + k_grad sum + wall
+        return __fadd_rn(__fmaf_rn(P.k_grad, ac, __fmul_rn(fc, ir)), wc);
+    };
+    const float3 a = make_float3(accel(f.x, acc.x, aw.x), accel(f.y, acc.y, aw.y), accel(f.z, acc.z, aw.z));
+    const float3 v = make_float3(__fmaf_rn(a.x, P.dt, vh.x), __fmaf_rn(a.y, P.dt, vh.y), __fmaf_rn(a.z, P.dt, vh.z));
+    vs[t] = make_float4(v.x, v.y, v.z, 0.f);
+    xs_next[t] = make_float4(__fmaf_rn(v.x, P.dt, x0.x), __fmaf_rn(v.y, P.dt, x0.y), __fmaf_rn(v.z, P.dt, x0.z), 0.f);
+    rp[t] = ri;
+}
+
 // The pressure-force pass for sorted particle t (t < P.n, its scene still
-// iterating): the next prediction into xs_next[t] and vs[t], and the
-// candidate pressure committed to rp[t].
+// iterating).
 template <bool REF, bool BATCH, class F4, class F2>
 __device__ __forceinline__ void pci_force_at(const Params& P, int t, const float4* __restrict__ pos,
                                              const float4* __restrict__ vap, const float4* __restrict__ fnp, F4 xs,
@@ -755,32 +863,13 @@ __device__ __forceinline__ void pci_force_at(const Params& P, int t, const float
         // costs one dependent load after the list, not two
         const float4 xj = REF ? xs[j] : pos[j];
         const float2 rj = rpc[j];
-        const float dx = __fsub_rn(xi.x, xj.x), dy = __fsub_rn(xi.y, xj.y), dz = __fsub_rn(xi.z, xj.z);
-        const float r2 = dist2(dx, dy, dz);
-        if (!(r2 > 0.f)) return;
-        if (!REF && __fmul_rn(r2, P.inv_h2) >= 1.f) return;
-        const float rinv = rsqrtf(r2);
-        const float om = spiky_om(P, r2, rinv);
-        // pV_i + pV_j (config: p_j / rho0^2 fused into the sum), then products only
-        const float pv = REF ? pVi + rj.y / (rj.x * rj.x) : __fmaf_rn(rj.y, ir0, pVi);
-        const float s = pv * om * om * rinv;
-        acc.x = __fmaf_rn(s, dx, acc.x); acc.y = __fmaf_rn(s, dy, acc.y); acc.z = __fmaf_rn(s, dz, acc.z);
+        add_pressure_pair<REF>(P, xi, xj, pVi, rj, ir0, acc);
     });
     if (!REF) {
-        ghost_pressure<BATCH>(P, t, xi, pVi, pos, (const float*)&rpc[0] + 1, 2, list, cnt, acc);
+        ghost_pressure<BATCH>(P, t, xi, pVi, pos, &rpc[0], list, cnt, acc);
         if (!BATCH) boundary_pressure(P, t, xi, pVi, acc);
     }
-    const float4 x0 = pos[t], vh = vap[t], f = fnp[t];
-    const float3 aw = wall_accel<REF, BATCH>(P, t, x0, vh);
-    const float ir = 1.f / ri.x;
-    auto accel = [&](float fc, float ac, float wc) {     // f/rho + k_grad sum + wall
-        return __fadd_rn(__fmaf_rn(P.k_grad, ac, __fmul_rn(fc, ir)), wc);
-    };
-    const float3 a = make_float3(accel(f.x, acc.x, aw.x), accel(f.y, acc.y, aw.y), accel(f.z, acc.z, aw.z));
-    const float3 v = make_float3(__fmaf_rn(a.x, P.dt, vh.x), __fmaf_rn(a.y, P.dt, vh.y), __fmaf_rn(a.z, P.dt, vh.z));
-    vs[t] = make_float4(v.x, v.y, v.z, 0.f);
-    xs_next[t] = make_float4(__fmaf_rn(v.x, P.dt, x0.x), __fmaf_rn(v.y, P.dt, x0.y), __fmaf_rn(v.z, P.dt, x0.z), 0.f);
-    rp[t] = ri;
+    pci_force_finish<REF, BATCH>(P, t, ri, acc, pos, vap, fnp, xs_next, vs, rp);
 }
 
 // PCISPH pressure-force pass fused with the next prediction; commits the
@@ -792,7 +881,7 @@ __device__ __forceinline__ void pci_force_at(const Params& P, int t, const float
 // with rho* in p/rho^2 the force feeds back on the density; under a 0.64 m
 // column either one makes the corrector diverge.
 template <bool REF, bool BATCH, int BS>
-__global__ void __launch_bounds__(BS) k_pci_force_predict(Params P, const float4* __restrict__ pos,
+__global__ void __launch_bounds__(BS, REF ? 1 : kForceThreads / BS) k_pci_force_predict(Params P, const float4* __restrict__ pos,
                                                               const float4* __restrict__ vap,
                                                               const float4* __restrict__ fnp,
                                                               const float4* __restrict__ xs,
@@ -800,11 +889,11 @@ __global__ void __launch_bounds__(BS) k_pci_force_predict(Params P, const float4
                                                               const int* __restrict__ counts,
                                                               const int* __restrict__ list, float4* __restrict__ xs_next,
                                                               float4* __restrict__ vs, float2* __restrict__ rp) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= P.n) return;
-    if (BATCH && !P.active[P.slot_scene[t]]) return;     // its scene has converged
     if (!BATCH && P.active && !P.active[0]) return;      // single scene, corrector decided on the device: converged
-    pci_force_at<REF, BATCH>(P, t, pos, vap, fnp, xs, rpc, counts, list, xs_next, vs, rp);
+    for_each_slot<BS, !REF>(P, [&](const int t) {
+        if (t < 0 || (BATCH && !P.active[P.slot_scene[t]])) return;     // its scene has converged
+        pci_force_at<REF, BATCH>(P, t, pos, vap, fnp, xs, rpc, counts, list, xs_next, vs, rp);
+    });
 }
 
 // The whole corrector loop of a config-profile scene or batch in one
@@ -925,14 +1014,27 @@ inline int grid_of(int n) { return (n + kBlock - 1) / kBlock; }
 template <int BS>
 inline unsigned blocks_of(int n) { return (unsigned)((n + BS - 1) / BS); }
 
+// P with its wall blocks for launches of BS threads. The list's length is
+// only known on the device: threads for a quarter of the particles (scenes
+// of 100k to 4M list 4 to 25%), 148 x 1024 at most (blocks that find nothing
+// to do cost ~2 ns each); a longer list is strided over.
+template <int BS>
+inline Params with_walls(const Params& P, bool ghosts = true) {
+    Params Q = P;
+    const bool list = ghosts && P.wall_list && P.n >= kWallListMin;
+    Q.wall_blocks = list ? std::min(148 * 1024 / BS, (P.n / 4 + BS - 1) / BS) : 0;
+    return Q;
+}
 
 void launch_density_x(cudaStream_t st, const Params& P, const float4* pos, const float4* vel, const int* counts,
                       const int* list, float2* rp, float* rho_x, int zero_p, float p_scale, float* feats, int nfeat) {
     if (P.n <= 0) return;
     with_block(P.tune.density_block, [&](auto B) {
         constexpr int BS = decltype(B)::value;
+        const Params Q = with_walls<BS>(P);
         auto go = [&](auto kernel) {
-            kernel<<<blocks_of<BS>(P.n), BS, 0, st>>>(P, pos, vel, counts, list, rp, rho_x, zero_p, p_scale, feats);
+            kernel<<<blocks_of<BS>(P.n) + Q.wall_blocks, BS, 0, st>>>(Q, pos, vel, counts, list, rp, rho_x, zero_p,
+                                                                      p_scale, feats);
         };
         const int nf = feats ? (nfeat > 6 ? 7 : 6) : 0;
         if (P.ref) go(k_density_x<true, 0, false, BS>);
@@ -967,12 +1069,10 @@ void launch_wcsph_force(cudaStream_t st, const Params& P, const float4* pos, con
                         const float2* rp, const int* counts, const int* list, float4* pos_out, float4* vel_out,
                         float4* vap_out, float4* fnp) {
     if (P.n <= 0) return;
-    if (P.ref)
-        k_wcsph_force<true><<<grid_of(P.n), kBlock, 0, st>>>(P, pos, vel, vap, rp, counts, list, pos_out, vel_out,
-                                                             vap_out, fnp);
-    else
-        k_wcsph_force<false><<<grid_of(P.n), kBlock, 0, st>>>(P, pos, vel, vap, rp, counts, list, pos_out, vel_out,
-                                                              vap_out, fnp);
+    const Params Q = with_walls<kBlock>(P);
+    auto kernel = P.ref ? k_wcsph_force<true> : k_wcsph_force<false>;
+    kernel<<<grid_of(P.n) + Q.wall_blocks, kBlock, 0, st>>>(Q, pos, vel, vap, rp, counts, list, pos_out, vel_out,
+                                                            vap_out, fnp);
 }
 
 void launch_pci_init(cudaStream_t st, const Params& P, const float4* pos, const float4* vel, const float4* vap,
@@ -981,8 +1081,9 @@ void launch_pci_init(cudaStream_t st, const Params& P, const float4* pos, const 
     if (P.n <= 0) return;
     with_block(P.tune.init_block, [&](auto B) {
         constexpr int BS = decltype(B)::value;
+        const Params Q = with_walls<BS>(P, warm != 0);
         auto go = [&](auto kernel) {
-            kernel<<<blocks_of<BS>(P.n), BS, 0, st>>>(P, pos, vel, vap, rp, counts, list, fnp, xs, vs);
+            kernel<<<blocks_of<BS>(P.n) + Q.wall_blocks, BS, 0, st>>>(Q, pos, vel, vap, rp, counts, list, fnp, xs, vs);
         };
         if (P.ref) { if (warm) go(k_pci_init<true, true, false, BS>); else go(k_pci_init<true, false, false, BS>); }
         else if (P.scenes) { if (warm) go(k_pci_init<false, true, true, BS>); else go(k_pci_init<false, false, true, BS>); }
@@ -996,8 +1097,9 @@ void launch_pci_density(cudaStream_t st, const Params& P, const float4* xs, cons
     if (P.n <= 0) return;
     with_block(P.tune.pci_density_block, [&](auto B) {
         constexpr int BS = decltype(B)::value;
+        const Params Q = with_walls<BS>(P);
         auto go = [&](auto kernel) {
-            kernel<<<blocks_of<BS>(P.n), BS, 0, st>>>(P, xs, rp, counts, list, rpc, err_slot);
+            kernel<<<blocks_of<BS>(P.n) + Q.wall_blocks, BS, 0, st>>>(Q, xs, rp, counts, list, rpc, err_slot);
         };
         if (P.ref) go(k_pci_density<true, false, BS>);
         else if (P.scenes) go(k_pci_density<false, true, BS>);
@@ -1044,8 +1146,10 @@ void launch_pci_force_predict(cudaStream_t st, const Params& P, const float4* po
     if (P.n <= 0) return;
     with_block(P.tune.force_block, [&](auto B) {
         constexpr int BS = decltype(B)::value;
+        const Params Q = with_walls<BS>(P);
         auto go = [&](auto kernel) {
-            kernel<<<blocks_of<BS>(P.n), BS, 0, st>>>(P, pos, vap, fnp, xs, rpc, counts, list, xs_next, vs, rp);
+            kernel<<<blocks_of<BS>(P.n) + Q.wall_blocks, BS, 0, st>>>(Q, pos, vap, fnp, xs, rpc, counts, list, xs_next,
+                                                                      vs, rp);
         };
         if (P.ref) go(k_pci_force_predict<true, false, BS>);
         else if (P.scenes) go(k_pci_force_predict<false, true, BS>);
