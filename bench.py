@@ -50,6 +50,7 @@ UNIT = "particle-steps/s"
 # traffic; neighbour re-reads and list traffic not counted).
 ALG_BYTES = {
     "cell_keys": 24,          # pos 16 -> key + id 8
+    "cell_sort": 16,          # keys and ranks in, sorted keys and slots out
     "radix_sort": 16,         # one read + write of the (key, value) pairs
     "reorder": 77,            # pos, vel, pressure 36 in + 36 out, cell ranges 5
     "reorder_pos": 53,        # after an upload: slot + key 8, pos + id 20 in and out, cell ranges 5
@@ -67,9 +68,10 @@ TUNE_KEYS = ("bucket", "nbr_block", "nbr_schedule", "density_block", "init_block
              "xsph_block")
 
 
-# Kernels per timed group (radix_sort is 3 kernels per 8-bit pass).
+# Kernels per timed group (radix_sort is 3 kernels per 8-bit pass, cell_sort
+# the scan, the placing and the ranking).
 def _kernels_per_group(name: str, sort_passes: int) -> int:
-    return 3 * sort_passes if name == "radix_sort" else 1
+    return 3 * sort_passes if name == "radix_sort" else 3 if name == "cell_sort" else 1
 
 
 CORRECTOR_KERNELS = ("batch_begin", "pci_density", "batch_decide", "pci_force_predict")

@@ -2,8 +2,8 @@
 // uploads/downloads in particle-id order, per-kernel CUDA-event profiling.
 //
 // One psb_step is, on the context's stream:
-//   reset cells of the previous sort -> cell keys -> radix sort (cell, id) ->
-//   reorder + cell ranges -> neighbour lists -> density at x ->
+//   cell keys and counts -> counting sort (cell, id) and cell ranges ->
+//   reorder -> neighbour lists -> density at x ->
 //   WCSPH: forces + leap-frog + walls + interpolation (one sweep)
 //   PCISPH: non-pressure forces + first prediction, then per correction
 //           {density/pressure pass at x*, pressure-force pass + next
@@ -109,6 +109,11 @@ struct psb_ctx {
     uint32_t* cell_start = nullptr;
     uint32_t* cell_end = nullptr;
     size_t ncells = 0;
+    // the counting sort's words (dense_cells; grid.cu): cell_end is then
+    // cell_start + 1, and no cell is ever reset
+    bool dense = false;
+    uint32_t* cell_count = nullptr;
+    uint32_t* tile_sum = nullptr;
     int* nbr_count = nullptr;
     int* nbr_list = nullptr;
     // SPH scratch
@@ -119,8 +124,6 @@ struct psb_ctx {
     float* rho_x = nullptr;
     unsigned long long* err_hist = nullptr;
     int* flags = nullptr;     // [0] overflow [1] max count [2..3] pair total [4] clamped [5] wall list length
-    int* wall_list = nullptr;         // config-profile SPH: slots near the box faces (Params::wall_list)
-    uint32_t* wall_bits = nullptr;
     void* stage = nullptr;    // device staging for uploads/downloads
     // learned warm start
     float* feats = nullptr;   // n_max x 8
@@ -325,10 +328,9 @@ void free_all(psb_ctx* c) {
         cudaFree(c->pos[i]); cudaFree(c->vel[i]); cudaFree(c->vap[i]); cudaFree(c->rp[i]); cudaFree(c->ids[i]);
         cudaFree(c->keys[i]); cudaFree(c->vals[i]); cudaFree(c->xs[i]);
     }
-    cudaFree(c->hist); cudaFree(c->cell_start); cudaFree(c->cell_end); cudaFree(c->nbr_count);
+    cudaFree(c->hist); cudaFree(c->cell_start); cudaFree(c->dense ? c->cell_count : c->cell_end); cudaFree(c->nbr_count);
     cudaFree(c->nbr_list); cudaFree(c->fnp); cudaFree(c->vs); cudaFree(c->rpc); cudaFree(c->rho_x);
     cudaFree(c->err_hist); cudaFree(c->flags); cudaFree(c->stage);
-    cudaFree(c->wall_list); cudaFree(c->wall_bits);
     cudaFree(c->bnd_vel); cudaFree(c->bnd_fext); cudaFree(c->bnd_pred); cudaFree(c->bnd_react);
     cudaFree(c->feats); cudaFree(c->mlp_w); cudaFree(c->mlp_m1); cudaFree(c->mlp_m2); cudaFree(c->mlp_grad); cudaFree(c->mlp_part);
     cudaFree(c->mlp_loss); cudaFree(c->mlp_wbf); cudaFree(c->ds_X); cudaFree(c->ds_T); cudaFree(c->sel);
@@ -552,6 +554,14 @@ int bits_for(size_t ncells) {
     return b;
 }
 
+// Whether a context of n particles sorts by counting over its ncells cells
+// (grid.cu) rather than by radix. Counting touches every cell (~12 B each,
+// little of it past L2: 15 us at 8.3M cells) and every particle about as often
+// as one radix pass of the 2-4 it replaces (28 us each at 1M). It is the
+// faster side up to a few million cells whatever n (the radix passes' launches
+// alone are ~40 us), and beyond that while the cells stay within 24 a particle.
+bool dense_cells(size_t ncells, size_t n) { return ncells <= std::max((size_t)4 << 20, 24 * n); }
+
 // Whether the density pass at x is folded into the neighbour build
 // (schedule 2): one config-profile PCISPH scene; batches, the reference
 // profile, WCSPH and DEM run schedule 2 as schedule 0.
@@ -567,14 +577,29 @@ int build(psb_ctx* c, bool keep_p = false, bool features = false) {
     const int n = c->n;
     const int rs = c->sorted >= 0 ? c->sorted : c->stale;       // cells occupied by the previous sort
     const int rn = c->sorted >= 0 ? c->sorted_n : c->stale_n;
-    if (rs >= 0) timed(c, "reset_cells", [&] { psb::launch_reset_cells(st, rn, c->keys[rs], c->cell_start); });
+    if (rs >= 0 && !c->dense)
+        timed(c, "reset_cells", [&] { psb::launch_reset_cells(st, rn, c->keys[rs], c->cell_start); });
     c->stale = -1;
     cudaMemsetAsync(c->flags, 0, 8 * sizeof(int), st);
-    timed(c, "cell_keys", [&] {
-        psb::launch_cell_keys(st, P, c->pos[c->cs], c->ids[c->cr], c->keys[0], c->vals[0], &c->flags[4]);
-    });
     int res = 0;
-    timed(c, "radix_sort", [&] { res = psb::radix_sort(st, n, c->key_bits, c->keys, c->vals, c->hist, c->hist_blocks); });
+    uint32_t* range_start = c->cell_start;      // the reorder records the cell ranges
+    if (c->dense) {
+        timed(c, "cell_keys", [&] {
+            psb::launch_cell_count(st, P, c->pos[c->cs], c->keys[0], c->vals[0], c->cell_count, c->tile_sum, &c->flags[4]);
+        });
+        // the predictor's x* buffer is free until the set-up sweep
+        timed(c, "cell_sort", [&] {
+            psb::launch_cell_sort(st, n, c->ncells, c->ids[c->cr], c->keys[0], c->vals[0], c->cell_count, c->tile_sum,
+                                  c->cell_start, reinterpret_cast<uint2*>(c->xs[0]), c->keys[1], c->vals[1]);
+        });
+        res = 1;
+        range_start = nullptr;
+    } else {
+        timed(c, "cell_keys", [&] {
+            psb::launch_cell_keys(st, P, c->pos[c->cs], c->ids[c->cr], c->keys[0], c->vals[0], &c->flags[4]);
+        });
+        timed(c, "radix_sort", [&] { res = psb::radix_sort(st, n, c->key_bits, c->keys, c->vals, c->hist, c->hist_blocks); });
+    }
     const int os = c->cs, orr = c->cr, ns = os ^ 1, nr = orr ^ 1;
     // The first step after an upload gathers the positions first and the
     // rest of the state after its neighbour build, once the upload's copies
@@ -584,12 +609,12 @@ int build(psb_ctx* c, bool keep_p = false, bool features = false) {
     if (split) {
         timed(c, "reorder_pos", [&] {
             psb::launch_reorder_pos(st, P, c->keys[res], c->vals[res], c->pos[os], c->ids[orr], c->pos[ns], c->ids[nr],
-                                    c->cell_start, c->cell_end);
+                                    range_start, c->cell_end);
         });
     } else {
         timed(c, "reorder", [&] {
             psb::launch_reorder(st, P, c->keys[res], c->vals[res], c->pos[os], c->vel[os], c->vap[os], c->rp[orr],
-                                c->ids[orr], c->pos[ns], c->vel[ns], c->vap[ns], c->rp[nr], c->ids[nr], c->cell_start,
+                                c->ids[orr], c->pos[ns], c->vel[ns], c->vap[ns], c->rp[nr], c->ids[nr], range_start,
                                 c->cell_end);
         });
     }
@@ -1033,10 +1058,27 @@ int create_impl(const psb_scene* scene, size_t ncells, psb_ctx** out) {
         rc = dalloc(c, &c->vals[i], n); if (rc) break;
         rc = dalloc(c, &c->xs[i], n); if (rc) break;
     }
-    if (!rc) rc = dalloc(c, &c->hist, (size_t)256 * c->hist_blocks + 256);
-    if (!rc) rc = dalloc(c, &c->cell_start, c->ncells);
-    if (!rc) rc = dalloc(c, &c->cell_end, c->ncells);
-    if (!rc) rc = dalloc(c, &c->nbr_count, n);
+    c->dense = dense_cells(c->ncells, n);
+    if (c->dense) {
+        const size_t words = psb::cell_sort_cells(c->ncells), tiles = psb::cell_sort_tiles(c->ncells);
+        if (!rc) rc = dalloc(c, &c->cell_start, words);
+        if (!rc) rc = dalloc(c, &c->cell_count, words + tiles);
+        c->cell_end = c->cell_start + 1;
+        c->tile_sum = c->cell_count + words;
+        if (!rc && cudaMemset(c->cell_count, 0, sizeof(uint32_t) * (words + tiles)) != cudaSuccess) rc = PSB_ECUDA;
+    } else {
+        if (!rc) rc = dalloc(c, &c->hist, (size_t)256 * c->hist_blocks + 256);
+        if (!rc) rc = dalloc(c, &c->cell_start, c->ncells);
+        if (!rc) rc = dalloc(c, &c->cell_end, c->ncells);
+        if (!rc && cudaMemset(c->cell_start, 0xFF, sizeof(uint32_t) * c->ncells) != cudaSuccess) rc = PSB_ECUDA;
+    }
+    // the neighbour counts, and (config-profile SPH) the wall list and its flags
+    const bool ghosts = !c->P.ref && !c->P.dem;
+    if (!rc) rc = dalloc(c, &c->nbr_count, ghosts ? 2 * n + (n + 31) / 32 : n);
+    if (ghosts) {
+        c->P.wall_list = c->nbr_count + n;
+        c->P.wall_bits = (uint32_t*)c->nbr_count + 2 * n;
+    }
     if (!rc) rc = dalloc(c, &c->nbr_list, psb::nbr_list_ints(n, c->cap));
     if (!rc) rc = dalloc(c, &c->fnp, n);
     if (!rc) rc = dalloc(c, &c->vs, n);
@@ -1044,13 +1086,7 @@ int create_impl(const psb_scene* scene, size_t ncells, psb_ctx** out) {
     if (!rc) rc = dalloc(c, &c->rho_x, n);
     if (!rc) rc = dalloc(c, &c->err_hist, PSB_MAX_ITERS + 1);
     if (!rc) rc = dalloc(c, &c->flags, 8);
-    if (!c->P.ref && !c->P.dem) {       // the profile with wall ghosts
-        if (!rc) rc = dalloc(c, &c->wall_list, n);
-        if (!rc) rc = dalloc(c, &c->wall_bits, (n + 31) / 32);
-        c->P.wall_list = c->wall_list;
-        c->P.wall_bits = c->wall_bits;
-        c->P.wall_count = c->flags + 5;
-    }
+    if (ghosts) c->P.wall_count = c->flags + 5;
     // uploads and downloads stage every array at once: 3 x 12 + 2 x 4 bytes
     if (!rc) rc = dalloc(c, (char**)&c->stage, n * 48);
     if (!rc) rc = dalloc(c, &c->feats, n * 8);
@@ -1065,7 +1101,6 @@ int create_impl(const psb_scene* scene, size_t ncells, psb_ctx** out) {
     if (!rc && cudaMemset(c->mlp_wbf, 0, 2 * psb::kMlpParams) != cudaSuccess) rc = PSB_ECUDA;
     if (!rc && cudaMallocHost((void**)&c->h_err, sizeof(unsigned long long) * (PSB_MAX_ITERS + 1)) != cudaSuccess) rc = PSB_ENOMEM;
     if (!rc && cudaMallocHost((void**)&c->h_flags, 8 * sizeof(int)) != cudaSuccess) rc = PSB_ENOMEM;
-    if (!rc && cudaMemset(c->cell_start, 0xFF, sizeof(uint32_t) * c->ncells) != cudaSuccess) rc = PSB_ECUDA;
     if (!rc && cudaMemset(c->err_hist, 0, sizeof(unsigned long long) * (PSB_MAX_ITERS + 1)) != cudaSuccess) rc = PSB_ECUDA;
     if (!rc && cudaDeviceSynchronize() != cudaSuccess) rc = PSB_ECUDA;
     if (rc) {

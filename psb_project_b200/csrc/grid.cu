@@ -15,6 +15,8 @@
 // neighbour order is deterministic; particles outside the grid are clamped
 // into the border cells (the reference writes out of bounds there); lists
 // are bounded (overflow raises a flag, never a trap).
+#include <algorithm>
+
 #include "psb_internal.cuh"
 
 namespace psb {
@@ -36,6 +38,22 @@ __global__ void k_reset_cells(int n, const uint32_t* __restrict__ sorted_keys, u
     if (s == 0 || sorted_keys[s - 1] != k) cell_start[k] = kEmpty;
 }
 
+// Cell of the particle in slot s; c is set where it was clamped.
+template <bool BATCH>
+__device__ __forceinline__ uint32_t cell_key(const Params& P, int s, float4 p, int& c) {
+    const Grid g = BATCH ? P.scenes[P.slot_scene[s]].g : P.g;
+    const uint32_t base = BATCH ? P.scenes[P.slot_scene[s]].cell_base : 0u;
+    const int i = cell_coord(p.x, g.gx, g.cell, g.nx, c);
+    const int j = cell_coord(p.y, g.gy, g.cell, g.ny, c);
+    const int k = cell_coord(p.z, g.gz, g.cell, g.nz, c);
+    return base + (uint32_t)i + (uint32_t)j * (uint32_t)g.nx + (uint32_t)k * (uint32_t)g.nx * (uint32_t)g.ny;
+}
+
+__device__ __forceinline__ void count_clamped(int c, int* __restrict__ clamped) {
+    const unsigned ballot = __ballot_sync(__activemask(), c);
+    if (ballot && (threadIdx.x & 31) == __ffs(ballot) - 1) atomicAdd(clamped, __popc(ballot));
+}
+
 // Cell key of every particle, written at its id so that a stable sort of
 // the id-ordered keys yields (cell, id) order. A batch gives each scene its
 // own grid and a block of keys after the previous scene's, so the sort keeps
@@ -46,18 +64,12 @@ __global__ void k_cell_keys(Params P, const float4* __restrict__ pos, const int*
                             int* __restrict__ clamped) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= P.n) return;
-    const float4 p = pos[s];
-    const Grid g = BATCH ? P.scenes[P.slot_scene[s]].g : P.g;
-    const uint32_t base = BATCH ? P.scenes[P.slot_scene[s]].cell_base : 0u;
     int c = 0;
-    const int i = cell_coord(p.x, g.gx, g.cell, g.nx, c);
-    const int j = cell_coord(p.y, g.gy, g.cell, g.ny, c);
-    const int k = cell_coord(p.z, g.gz, g.cell, g.nz, c);
+    const uint32_t key = cell_key<BATCH>(P, s, pos[s], c);
     const int id = ids[s];
-    keys_by_id[id] = base + (uint32_t)i + (uint32_t)j * (uint32_t)g.nx + (uint32_t)k * (uint32_t)g.nx * (uint32_t)g.ny;
+    keys_by_id[id] = key;
     slot_by_id[id] = (uint32_t)s;
-    const unsigned ballot = __ballot_sync(__activemask(), c);
-    if (ballot && (threadIdx.x & 31) == __ffs(ballot) - 1) atomicAdd(clamped, __popc(ballot));
+    count_clamped(c, clamped);
 }
 
 // ---- LSD radix sort, 8-bit digits, three kernels per pass ----------------
@@ -171,8 +183,10 @@ __global__ void __launch_bounds__(kBlock) k_radix_scatter(int n, int shift, int 
 }
 
 // Lists slot t (position x) in P.wall_list when it lies near a box face, and
-// writes the warp's flag word; every lane of the warp calls it. One atomic
-// add per warp that has such a particle; the list's order is left open.
+// writes the warp's flag word; every thread of the block calls it. One atomic
+// add per block that has such a particle (one per warp queued at the count's
+// address: 40 us of the positions' reorder at 1M, 14 without); the list's
+// order is left open.
 template <bool BATCH>
 __device__ __forceinline__ void list_near_walls(const Params& P, int t, float4 x) {
     if (!P.wall_list || P.n < kWallListMin) return;
@@ -188,19 +202,219 @@ __device__ __forceinline__ void list_near_walls(const Params& P, int t, float4 x
                x.z - lo_z < reach || hi_z - x.z < reach;
     }
     const unsigned word = __ballot_sync(0xffffffffu, near);
-    const int lane = threadIdx.x & 31;
-    int base = 0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ int s_count[kBlock / 32], s_base;
     if (lane == 0) {
         if (t < P.n) P.wall_bits[t >> 5] = word;
-        if (word) base = atomicAdd(P.wall_count, __popc(word));
+        s_count[warp] = __popc(word);
     }
-    if (!word) return;
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (near) P.wall_list[base + __popc(word & ((1u << lane) - 1u))] = t;
+    __syncthreads();
+    int before = 0, total = 0;
+#pragma unroll
+    for (int w = 0; w < kBlock / 32; ++w) {
+        if (w < warp) before += s_count[w];
+        total += s_count[w];
+    }
+    if (total == 0) return;
+    if (threadIdx.x == 0) s_base = atomicAdd(P.wall_count, total);
+    __syncthreads();
+    if (near) P.wall_list[s_base + before + __popc(word & ((1u << lane) - 1u))] = t;
+}
+
+// ---- sort of up to kSmallSort pairs in one block -----------------------------
+// Below this size the passes above are launches: 8 kernels of 2-5 us each for
+// 5,000 pairs, 45 us with the gaps. One block keeps the pairs in registers
+// and shared memory through every pass (same 8-bit digits, same stable order)
+// and touches global memory once each way. Warp w owns items 256 w .. 256 w +
+// 255, a row of 32 per turn: a row's equal digits are found with
+// __match_any_sync and ranked by lane behind the warp's count so far; the
+// (digit, warp) counts are then scanned and each pair moves to its place.
+constexpr int kSmallSort = 8192, kSmallThreads = 1024, kSmallItems = kSmallSort / kSmallThreads;
+struct SmallSortSmem {
+    uint32_t key[kSmallSort], val[kSmallSort];
+    uint16_t count[256][kSmallThreads / 32];      // per digit and warp, then exclusive offsets
+    uint32_t warp_sum[kSmallThreads / 32];
+};
+
+__global__ void __launch_bounds__(kSmallThreads) k_small_sort(int n, int bits, const uint32_t* keys_in,
+                                                              const uint32_t* vals_in, uint32_t* keys_out,
+                                                              uint32_t* vals_out) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    SmallSortSmem& S = *reinterpret_cast<SmallSortSmem*>(smem_raw);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    uint32_t key[kSmallItems], val[kSmallItems], rank[kSmallItems];
+    const int first = warp * 32 * kSmallItems + lane;
+#pragma unroll
+    for (int r = 0; r < kSmallItems; ++r) {
+        const int i = first + r * 32;
+        key[r] = i < n ? keys_in[i] : 0u;
+        val[r] = i < n ? vals_in[i] : 0u;
+    }
+    for (int shift = 0; shift < bits; shift += 8) {
+        for (int i = tid; i < 256 * (kSmallThreads / 32) / 2; i += kSmallThreads) ((uint32_t*)S.count)[i] = 0u;
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kSmallItems; ++r) {
+            if (first - lane + r * 32 >= n) break;               // warp-uniform
+            const bool valid = first + r * 32 < n;
+            const uint32_t d = (key[r] >> shift) & 255u;
+            const unsigned peers = __match_any_sync(0xffffffffu, valid ? d : 256u);
+            uint32_t before = 0u;
+            if (valid) before = S.count[d][warp];
+            __syncwarp();
+            rank[r] = before + __popc(peers & ((1u << lane) - 1u));
+            if (valid && lane == __ffs(peers) - 1) S.count[d][warp] = (uint16_t)(before + __popc(peers));
+            __syncwarp();
+        }
+        __syncthreads();
+        // exclusive scan over (digit, warp), eight entries a thread
+        uint16_t* c = &S.count[0][0] + tid * 8;
+        uint32_t v[8], tot = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) { v[k] = tot; tot += c[k]; }
+        uint32_t x = tot;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) S.warp_sum[warp] = x;
+        __syncthreads();
+        if (warp == 0) {
+            const uint32_t w = S.warp_sum[lane];
+            uint32_t y = w;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t z = __shfl_up_sync(0xffffffffu, y, o);
+                if (lane >= o) y += z;
+            }
+            S.warp_sum[lane] = y - w;
+        }
+        __syncthreads();
+        const uint32_t base = S.warp_sum[warp] + x - tot;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) c[k] = (uint16_t)(base + v[k]);
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kSmallItems; ++r) {
+            if (first + r * 32 < n) {
+                const uint32_t dst = S.count[(key[r] >> shift) & 255u][warp] + rank[r];
+                S.key[dst] = key[r];
+                S.val[dst] = val[r];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kSmallItems; ++r) {
+            const int i = first + r * 32;
+            if (i < n) { key[r] = S.key[i]; val[r] = S.val[i]; }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < kSmallItems; ++r) {
+        const int i = first + r * 32;
+        if (i < n) { keys_out[i] = key[r]; vals_out[i] = val[r]; }
+    }
+}
+
+// ---- counting sort by cell ------------------------------------------------------
+// A step's particles are sorted over cells whose number is known, so one
+// counting pass replaces the radix passes: count the cells' particles, scan
+// the counts over the grid, place each particle in its cell's range, then
+// order every cell's few particles by id (the arrival order is the atomics').
+// The result is the radix sort's, (cell, id) order, and the scanned counts
+// are the cell ranges of every cell, empty ones included: cell c holds slots
+// [cell_start[c], cell_start[c + 1]).
+constexpr int kScanCells = 8192;      // cells per block of the scan, 32 per thread
+
+// Keys by slot, and each particle's arrival rank in its cell; one atomic per
+// distinct cell and per distinct scan tile of a warp (slots are nearly in
+// cell order from the previous step, so a warp holds a few of each).
+template <bool BATCH>
+__global__ void __launch_bounds__(kBlock) k_cell_count(Params P, const float4* __restrict__ pos,
+                                                       uint32_t* __restrict__ keys, uint32_t* __restrict__ ranks,
+                                                       uint32_t* __restrict__ cell_count,
+                                                       uint32_t* __restrict__ tile_sum, int* __restrict__ clamped) {
+    const int s = blockIdx.x * kBlock + threadIdx.x, lane = threadIdx.x & 31;
+    const bool valid = s < P.n;
+    int c = 0;
+    const uint32_t key = valid ? cell_key<BATCH>(P, s, pos[s], c) : kEmpty;
+    const unsigned peers = __match_any_sync(0xffffffffu, key);
+    const int leader = __ffs(peers) - 1;
+    uint32_t before = 0u;
+    if (valid && lane == leader) before = atomicAdd(&cell_count[key], (uint32_t)__popc(peers));
+    before = __shfl_sync(0xffffffffu, before, leader);
+    const unsigned tile = valid ? key / kScanCells : kEmpty;
+    const unsigned mates = __match_any_sync(0xffffffffu, tile);
+    if (!valid) return;
+    if (lane == __ffs(mates) - 1) atomicAdd(&tile_sum[tile], (uint32_t)__popc(mates));
+    keys[s] = key;
+    ranks[s] = before + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+    count_clamped(c, clamped);
+}
+
+// Exclusive scan of the counts of one tile of cells, behind the particles of
+// the tiles before it; leaves the counts at zero for the next step. A tile
+// without particles (most of a dam break's box) only writes.
+__global__ void __launch_bounds__(kBlock) k_cell_scan(uint32_t* __restrict__ cell_count,
+                                                      const uint32_t* __restrict__ tile_sum,
+                                                      uint32_t* __restrict__ cell_start) {
+    __shared__ uint32_t s_warp[kBlock / 32];
+    const int tile = blockIdx.x, tid = threadIdx.x;
+    uint32_t mine = 0, run;
+    for (int i = tid; i < tile; i += kBlock) mine += tile_sum[i];
+    block_exclusive_scan(mine, s_warp, run);
+    const uint32_t here = tile_sum[tile];
+    const size_t first = (size_t)tile * kScanCells + tid * 4;
+    for (int r = 0; r < kScanCells; r += kBlock * 4) {
+        uint4 start = make_uint4(run, run, run, run);
+        if (here) {
+            uint4* at = reinterpret_cast<uint4*>(cell_count + first + r);
+            const uint4 v = *at;
+            uint32_t tot;
+            start.x += block_exclusive_scan(v.x + v.y + v.z + v.w, s_warp, tot);
+            start.y = start.x + v.x;
+            start.z = start.y + v.y;
+            start.w = start.z + v.z;
+            run += tot;
+            *at = make_uint4(0u, 0u, 0u, 0u);
+        }
+        *reinterpret_cast<uint4*>(cell_start + first + r) = start;
+    }
+    if (tid == 0 && tile == (int)gridDim.x - 1) cell_start[(size_t)(tile + 1) * kScanCells] = run;
+}
+
+// Each particle's (id, slot) into its cell's range, in arrival order; clears
+// the tile sums for the next step.
+__global__ void __launch_bounds__(kBlock) k_cell_place(int n, int ntiles, const uint32_t* __restrict__ keys,
+                                                       const uint32_t* __restrict__ ranks, const int* __restrict__ ids,
+                                                       const uint32_t* __restrict__ cell_start,
+                                                       uint2* __restrict__ placed, uint32_t* __restrict__ tile_sum) {
+    const int s = blockIdx.x * kBlock + threadIdx.x;
+    if (s < ntiles) tile_sum[s] = 0u;
+    if (s >= n) return;
+    placed[cell_start[keys[s]] + ranks[s]] = make_uint2((uint32_t)ids[s], (uint32_t)s);
+}
+
+// Orders every cell's particles by id: a particle's place is the number of
+// smaller ids in its cell.
+__global__ void __launch_bounds__(kBlock) k_cell_rank(int n, const uint32_t* __restrict__ keys,
+                                                      const uint2* __restrict__ placed,
+                                                      const uint32_t* __restrict__ cell_start,
+                                                      uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out) {
+    const int p = blockIdx.x * kBlock + threadIdx.x;
+    if (p >= n) return;
+    const uint2 me = placed[p];
+    const uint32_t key = keys[me.y];
+    const uint32_t lo = cell_start[key], hi = cell_start[key + 1];
+    uint32_t t = lo;
+    for (uint32_t q = lo; q < hi; ++q) t += placed[q].x < me.x ? 1u : 0u;
+    keys_out[t] = key;
+    vals_out[t] = me.y;
 }
 
 // Gathers the particle state into sorted order and records each occupied
-// cell's [start, end) slot range.
+// cell's [start, end) slot range (cell_start null: the counting sort has).
 template <bool BATCH>
 __global__ void k_reorder(Params P, const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals,
                           const float4* __restrict__ pos, const float4* __restrict__ vel,
@@ -219,6 +433,7 @@ __global__ void k_reorder(Params P, const uint32_t* __restrict__ keys, const uin
     vap2[t] = vap[s];
     rp2[t] = rp[s];
     ids2[t] = ids[s];
+    if (!cell_start) return;
     const uint32_t k = keys[t];
     if (t == 0 || keys[t - 1] != k) cell_start[k] = (uint32_t)t;
     if (t == n - 1 || keys[t + 1] != k) cell_end[k] = (uint32_t)t + 1u;
@@ -240,6 +455,7 @@ __global__ void k_reorder_pos(Params P, const uint32_t* __restrict__ keys, const
     if (t >= n) return;
     pos2[t] = x;
     ids2[t] = ids[s];
+    if (!cell_start) return;
     const uint32_t k = keys[t];
     if (t == 0 || keys[t - 1] != k) cell_start[k] = (uint32_t)t;
     if (t == n - 1 || keys[t + 1] != k) cell_end[k] = (uint32_t)t + 1u;
@@ -406,9 +622,38 @@ void launch_cell_keys(cudaStream_t st, const Params& P, const float4* pos, const
 
 int radix_blocks(int n) { return (n + kTile - 1) / kTile; }
 
+bool small_sort(cudaStream_t st, int n, int bits, const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,
+                uint32_t* vals_out) {
+    if (n > kSmallSort) return false;
+    cudaFuncSetAttribute(k_small_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmallSortSmem));
+    k_small_sort<<<1, kSmallThreads, sizeof(SmallSortSmem), st>>>(n, bits, keys_in, vals_in, keys_out, vals_out);
+    return true;
+}
+
+size_t cell_sort_tiles(size_t ncells) { return (ncells + kScanCells - 1) / kScanCells; }
+size_t cell_sort_cells(size_t ncells) { return cell_sort_tiles(ncells) * kScanCells + 4; }
+
+void launch_cell_count(cudaStream_t st, const Params& P, const float4* pos, uint32_t* keys, uint32_t* ranks,
+                       uint32_t* cell_count, uint32_t* tile_sum, int* clamped) {
+    if (P.n <= 0) return;
+    auto kernel = P.scenes ? k_cell_count<true> : k_cell_count<false>;
+    kernel<<<grid_of(P.n), kBlock, 0, st>>>(P, pos, keys, ranks, cell_count, tile_sum, clamped);
+}
+
+void launch_cell_sort(cudaStream_t st, int n, size_t ncells, const int* ids, const uint32_t* keys, const uint32_t* ranks,
+                      uint32_t* cell_count, uint32_t* tile_sum, uint32_t* cell_start, uint2* placed, uint32_t* keys_out,
+                      uint32_t* vals_out) {
+    if (n <= 0) return;
+    const int tiles = (int)cell_sort_tiles(ncells);
+    k_cell_scan<<<tiles, kBlock, 0, st>>>(cell_count, tile_sum, cell_start);
+    k_cell_place<<<grid_of(std::max(n, tiles)), kBlock, 0, st>>>(n, tiles, keys, ranks, ids, cell_start, placed, tile_sum);
+    k_cell_rank<<<grid_of(n), kBlock, 0, st>>>(n, keys, placed, cell_start, keys_out, vals_out);
+}
+
 int radix_sort(cudaStream_t st, int n, int bits, uint32_t* keys[2], uint32_t* vals[2], uint32_t* hist, int nblocks_cap) {
     const int nb = radix_blocks(n);
     if (nb > nblocks_cap || n <= 0) return 0;
+    if (small_sort(st, n, bits, keys[0], vals[0], keys[0], vals[0])) return 0;
     int cur = 0;
     for (int shift = 0; shift < bits; shift += 8) {
         k_radix_hist<<<nb, kBlock, 0, st>>>(n, shift, nb, keys[cur], hist);

@@ -100,6 +100,12 @@ extern "C" int psb_sort_cells_noalloc(const uint32_t* keys_in, const uint32_t* v
                      cudaGetErrorString(pending));
         return PSB_ECUDA;
     }
+    if (psb::small_sort((cudaStream_t)stream, n, key_bits, keys_in, vals_in, keys_out, vals_out)) {
+        const cudaError_t e = cudaGetLastError();
+        if (e == cudaSuccess) return PSB_OK;
+        std::fprintf(stderr, "psb_sort_cells_noalloc: %s\n", cudaGetErrorString(e));
+        return PSB_ECUDA;
+    }
     uint32_t* scratch = nullptr;
     int rc = scratch_for_current_device(&scratch);
     if (rc != PSB_OK) return rc;

@@ -263,9 +263,27 @@ void launch_cell_keys(cudaStream_t st, const Params& P, const float4* pos, const
 // hist holds 256 * radix_blocks(n) + 256 words.
 int radix_sort(cudaStream_t st, int n, int bits, uint32_t* keys[2], uint32_t* vals[2], uint32_t* hist, int nblocks_cap);
 int radix_blocks(int n);
+// The same for n that one block holds (false: too many, nothing launched);
+// the outputs may be the inputs.
+bool small_sort(cudaStream_t st, int n, int bits, const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,
+                uint32_t* vals_out);
+// Counting sort of the particles by (cell, id) over a grid of ncells cells:
+// launch_cell_count writes each slot's key and arrival rank and raises the
+// counts; launch_cell_sort turns the counts into cell_start (every cell; slots
+// [cell_start[c], cell_start[c + 1])), writes the sorted keys and the old slot
+// of each sorted one, and leaves counts and tile sums at zero, as both must
+// be before the first count. cell_count and cell_start hold
+// cell_sort_cells(ncells) words, tile_sum cell_sort_tiles(ncells); placed: n.
+size_t cell_sort_tiles(size_t ncells);
+size_t cell_sort_cells(size_t ncells);
+void launch_cell_count(cudaStream_t st, const Params& P, const float4* pos, uint32_t* keys, uint32_t* ranks,
+                       uint32_t* cell_count, uint32_t* tile_sum, int* clamped);
+void launch_cell_sort(cudaStream_t st, int n, size_t ncells, const int* ids, const uint32_t* keys, const uint32_t* ranks,
+                      uint32_t* cell_count, uint32_t* tile_sum, uint32_t* cell_start, uint2* placed, uint32_t* keys_out,
+                      uint32_t* vals_out);
 // The whole state into sorted order, with the cell ranges; or in two
 // launches: positions, ids and cell ranges (what the neighbour build reads),
-// then the rest.
+// then the rest. cell_start null: the ranges are there already.
 // Both also list the particles near the box faces (P.wall_list).
 void launch_reorder(cudaStream_t st, const Params& P, const uint32_t* keys, const uint32_t* vals, const float4* pos,
                     const float4* vel, const float4* vap, const float2* rp, const int* ids, float4* pos2, float4* vel2,
