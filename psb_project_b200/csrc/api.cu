@@ -89,6 +89,8 @@ struct psb_ctx {
     int device = 0;
     int n = 0, n_max = 0, cap = 0;
     cudaStream_t stream = nullptr;
+    void* slab = nullptr;       // the device buffers below that psb_create makes, in one allocation
+    void* h_slab = nullptr;     // the pinned ones
     // particle state, double-buffered for the reorder: cs indexes pos/vel/vap,
     // cr indexes rp/ids
     float4* pos[2] = {};
@@ -324,21 +326,12 @@ int dalloc(psb_ctx* c, T** p, size_t count) {
 }
 
 void free_all(psb_ctx* c) {
-    for (int i = 0; i < 2; ++i) {
-        cudaFree(c->pos[i]); cudaFree(c->vel[i]); cudaFree(c->vap[i]); cudaFree(c->rp[i]); cudaFree(c->ids[i]);
-        cudaFree(c->keys[i]); cudaFree(c->vals[i]); cudaFree(c->xs[i]);
-    }
-    cudaFree(c->hist); cudaFree(c->cell_start); cudaFree(c->dense ? c->cell_count : c->cell_end); cudaFree(c->nbr_count);
-    cudaFree(c->nbr_list); cudaFree(c->fnp); cudaFree(c->vs); cudaFree(c->rpc); cudaFree(c->rho_x);
-    cudaFree(c->err_hist); cudaFree(c->flags); cudaFree(c->stage);
+    cudaFree(c->slab);
+    cudaFreeHost(c->h_slab);
     cudaFree(c->bnd_vel); cudaFree(c->bnd_fext); cudaFree(c->bnd_pred); cudaFree(c->bnd_react);
-    cudaFree(c->feats); cudaFree(c->mlp_w); cudaFree(c->mlp_m1); cudaFree(c->mlp_m2); cudaFree(c->mlp_grad); cudaFree(c->mlp_part);
-    cudaFree(c->mlp_loss); cudaFree(c->mlp_wbf); cudaFree(c->ds_X); cudaFree(c->ds_T); cudaFree(c->sel);
+    cudaFree(c->ds_X); cudaFree(c->ds_T); cudaFree(c->sel);
     cudaFree(c->iso); cudaFree(c->mc_cube); cudaFree(c->mc_edge); cudaFree(c->mc_scratch); cudaFree(c->mc_vert);
     cudaFree(c->mc_tri);
-    cudaFreeHost(c->h_err); cudaFreeHost(c->h_flags);
-    cudaFree(c->d_scenes); cudaFree(c->d_slot_scene); cudaFree(c->d_active); cudaFree(c->d_err_scene);
-    cudaFree(c->d_err_sh); cudaFree(c->d_loop);
     cudaFree(c->diag_rows); cudaFree(c->diag_out);
     cudaFree(c->bnd_raw); cudaFree(c->bnd_sorted); cudaFree(c->bnd_ids); cudaFree(c->bnd_iota); cudaFree(c->bnd_w);
     for (int i = 0; i < 2; ++i) { cudaFree(c->bnd_keys[i]); cudaFree(c->bnd_vals[i]); }
@@ -347,7 +340,6 @@ void free_all(psb_ctx* c) {
     cudaFree(c->d_coll);
     for (float* d : c->coll_data) cudaFree(d);
     for (auto& e : c->emitters) { cudaFree(e.d_list); cudaFree(e.d_faces); }
-    cudaFreeHost(c->h_loop); cudaFreeHost(c->h_err_sh);
     for (auto& g : c->gexec) if (g) { cudaGraphExecDestroy(g); g = nullptr; }
     if (c->cap_stream) cudaStreamDestroy(c->cap_stream);
     if (c->cap_main) cudaStreamDestroy(c->cap_main);
@@ -1028,8 +1020,9 @@ const char* psb_last_error(const psb_ctx* c) { return c ? c->err.c_str() : ""; }
 
 namespace {
 
-// Context and device buffers for `scene` (validated) over `ncells` grid cells.
-int create_impl(const psb_scene* scene, size_t ncells, psb_ctx** out) {
+// Context and device buffers for `scene` (validated) over `ncells` grid
+// cells; a batch's S scenes share them.
+int create_impl(const psb_scene* scene, size_t ncells, int S, bool batch, psb_ctx** out) {
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
         cudaGetLastError();
@@ -1046,62 +1039,93 @@ int create_impl(const psb_scene* scene, size_t ncells, psb_ctx** out) {
     c->key_bits = bits_for(c->ncells);
     c->hist_blocks = psb::radix_blocks(c->n_max);
     cudaGetDevice(&c->device);
-    const size_t n = (size_t)c->n_max;
-    int rc = PSB_OK;
-    for (int i = 0; i < 2 && rc == PSB_OK; ++i) {
-        rc = dalloc(c, &c->pos[i], n); if (rc) break;
-        rc = dalloc(c, &c->vel[i], n); if (rc) break;
-        rc = dalloc(c, &c->vap[i], n); if (rc) break;
-        rc = dalloc(c, &c->rp[i], n); if (rc) break;
-        rc = dalloc(c, &c->ids[i], n); if (rc) break;
-        rc = dalloc(c, &c->keys[i], n); if (rc) break;
-        rc = dalloc(c, &c->vals[i], n); if (rc) break;
-        rc = dalloc(c, &c->xs[i], n); if (rc) break;
-    }
+    const size_t n = (size_t)c->n_max, s_ = (size_t)S;
     c->dense = dense_cells(c->ncells, n);
-    if (c->dense) {
-        const size_t words = psb::cell_sort_cells(c->ncells), tiles = psb::cell_sort_tiles(c->ncells);
-        if (!rc) rc = dalloc(c, &c->cell_start, words);
-        if (!rc) rc = dalloc(c, &c->cell_count, words + tiles);
-        c->cell_end = c->cell_start + 1;
-        c->tile_sum = c->cell_count + words;
-        if (!rc && cudaMemset(c->cell_count, 0, sizeof(uint32_t) * (words + tiles)) != cudaSuccess) rc = PSB_ECUDA;
-    } else {
-        if (!rc) rc = dalloc(c, &c->hist, (size_t)256 * c->hist_blocks + 256);
-        if (!rc) rc = dalloc(c, &c->cell_start, c->ncells);
-        if (!rc) rc = dalloc(c, &c->cell_end, c->ncells);
-        if (!rc && cudaMemset(c->cell_start, 0xFF, sizeof(uint32_t) * c->ncells) != cudaSuccess) rc = PSB_ECUDA;
-    }
-    // the neighbour counts, and (config-profile SPH) the wall list and its flags
     const bool ghosts = !c->P.ref && !c->P.dem;
-    if (!rc) rc = dalloc(c, &c->nbr_count, ghosts ? 2 * n + (n + 31) / 32 : n);
-    if (ghosts) {
-        c->P.wall_list = c->nbr_count + n;
-        c->P.wall_bits = (uint32_t*)c->nbr_count + 2 * n;
+    const size_t words = psb::cell_sort_cells(c->ncells), tiles = psb::cell_sort_tiles(c->ncells);
+    // The buffers a context always has, in one device and one pinned block:
+    // the first turn adds up their sizes, the second places them.
+    size_t dev_bytes = 0, host_bytes = 0;
+    auto layout = [&] {
+        size_t at = 0;
+        auto take = [&](auto& p, size_t count) {
+            p = c->slab ? reinterpret_cast<std::decay_t<decltype(p)>>((char*)c->slab + at) : nullptr;
+            at += (std::max<size_t>(count, 1) * sizeof(*p) + 511) & ~(size_t)511;
+        };
+        for (int i = 0; i < 2; ++i) {
+            take(c->pos[i], n); take(c->vel[i], n); take(c->vap[i], n); take(c->rp[i], n); take(c->ids[i], n);
+            take(c->keys[i], n); take(c->vals[i], n); take(c->xs[i], n);
+        }
+        if (c->dense) {
+            take(c->cell_start, words);
+            take(c->cell_count, words + tiles);
+            c->cell_end = c->cell_start + 1;
+            c->tile_sum = c->cell_count + words;
+        } else {
+            take(c->hist, (size_t)256 * c->hist_blocks + 256);
+            take(c->cell_start, c->ncells);
+            take(c->cell_end, c->ncells);
+        }
+        take(c->nbr_count, n); take(c->nbr_list, psb::nbr_list_ints(n, c->cap));
+        take(c->fnp, n); take(c->vs, n); take(c->rpc, n); take(c->rho_x, n);
+        take(c->err_hist, PSB_MAX_ITERS + 1); take(c->flags, 8);
+        if (ghosts) {       // config-profile SPH: the wall list and its flags
+            take(c->P.wall_list, n);
+            take(c->P.wall_bits, (n + 31) / 32);
+            c->P.wall_count = c->flags + 5;
+        }
+        char* stage = nullptr;      // uploads and downloads stage every array at once: 3 x 12 + 2 x 4 bytes
+        take(stage, n * 48);
+        c->stage = stage;
+        take(c->feats, n * 8);
+        take(c->mlp_w, psb::kMlpParams); take(c->mlp_m1, psb::kMlpParams); take(c->mlp_m2, psb::kMlpParams);
+        take(c->mlp_grad, psb::kMlpParams); take(c->mlp_part, psb::kMlpGradPartials); take(c->mlp_loss, 1);
+        uint16_t* wbf = nullptr;
+        take(wbf, psb::kMlpParams);
+        c->mlp_wbf = wbf;
+        // the device-side corrector's words for S scenes (batch.cu)
+        take(c->d_active, s_); take(c->d_err_scene, s_); take(c->d_err_sh, (PSB_MAX_ITERS + 1) * s_);
+        take(c->d_loop, 2 + 4 * s_);
+        if (batch) { take(c->d_scenes, s_); take(c->d_slot_scene, n); }
+        dev_bytes = at;
+        at = 0;
+        auto pin = [&](auto& p, size_t count) {
+            p = c->h_slab ? reinterpret_cast<std::decay_t<decltype(p)>>((char*)c->h_slab + at) : nullptr;
+            at += (count * sizeof(*p) + 63) & ~(size_t)63;
+        };
+        pin(c->h_err, PSB_MAX_ITERS + 1); pin(c->h_flags, 8); pin(c->h_loop, 2 + 4 * s_);
+        pin(c->h_err_sh, (PSB_MAX_ITERS + 1) * s_);
+        host_bytes = at;
+    };
+    layout();
+    char *dev = nullptr, *host = nullptr;
+    int rc = dalloc(c, &dev, dev_bytes);
+    if (!rc && cudaMallocHost((void**)&host, host_bytes) != cudaSuccess) rc = PSB_ENOMEM;
+    c->slab = dev;
+    c->h_slab = host;
+    if (!rc) {
+        layout();
+        std::memset(host, 0, host_bytes);
+        auto fill = [&](void* p, int v, size_t bytes) {
+            if (!rc && cudaMemsetAsync(p, v, bytes, nullptr) != cudaSuccess) rc = PSB_ECUDA;
+        };
+        if (c->dense) fill(c->cell_count, 0, sizeof(uint32_t) * (words + tiles));
+        else fill(c->cell_start, 0xFF, sizeof(uint32_t) * c->ncells);
+        fill(c->mlp_w, 0, sizeof(float) * psb::kMlpParams);
+        fill(c->mlp_wbf, 0, 2 * psb::kMlpParams);
+        fill(c->err_hist, 0, sizeof(unsigned long long) * (PSB_MAX_ITERS + 1));
+        fill(c->d_loop, 0, sizeof(int) * (2 + 4 * s_));
+        fill(c->d_active, 1, s_);
+        fill(c->d_err_scene, 0, sizeof(unsigned long long) * s_);
+        fill(c->d_err_sh, 0, sizeof(unsigned long long) * (PSB_MAX_ITERS + 1) * s_);
     }
-    if (!rc) rc = dalloc(c, &c->nbr_list, psb::nbr_list_ints(n, c->cap));
-    if (!rc) rc = dalloc(c, &c->fnp, n);
-    if (!rc) rc = dalloc(c, &c->vs, n);
-    if (!rc) rc = dalloc(c, &c->rpc, n);
-    if (!rc) rc = dalloc(c, &c->rho_x, n);
-    if (!rc) rc = dalloc(c, &c->err_hist, PSB_MAX_ITERS + 1);
-    if (!rc) rc = dalloc(c, &c->flags, 8);
-    if (ghosts) c->P.wall_count = c->flags + 5;
-    // uploads and downloads stage every array at once: 3 x 12 + 2 x 4 bytes
-    if (!rc) rc = dalloc(c, (char**)&c->stage, n * 48);
-    if (!rc) rc = dalloc(c, &c->feats, n * 8);
-    if (!rc) rc = dalloc(c, &c->mlp_w, psb::kMlpParams);
-    if (!rc) rc = dalloc(c, &c->mlp_m1, psb::kMlpParams);
-    if (!rc) rc = dalloc(c, &c->mlp_m2, psb::kMlpParams);
-    if (!rc) rc = dalloc(c, &c->mlp_grad, psb::kMlpParams);
-    if (!rc) rc = dalloc(c, &c->mlp_part, psb::kMlpGradPartials);
-    if (!rc) rc = dalloc(c, &c->mlp_loss, 1);
-    if (!rc) rc = dalloc(c, (uint16_t**)&c->mlp_wbf, psb::kMlpParams);
-    if (!rc && cudaMemset(c->mlp_w, 0, sizeof(float) * psb::kMlpParams) != cudaSuccess) rc = PSB_ECUDA;
-    if (!rc && cudaMemset(c->mlp_wbf, 0, 2 * psb::kMlpParams) != cudaSuccess) rc = PSB_ECUDA;
-    if (!rc && cudaMallocHost((void**)&c->h_err, sizeof(unsigned long long) * (PSB_MAX_ITERS + 1)) != cudaSuccess) rc = PSB_ENOMEM;
-    if (!rc && cudaMallocHost((void**)&c->h_flags, 8 * sizeof(int)) != cudaSuccess) rc = PSB_ENOMEM;
-    if (!rc && cudaMemset(c->err_hist, 0, sizeof(unsigned long long) * (PSB_MAX_ITERS + 1)) != cudaSuccess) rc = PSB_ECUDA;
+    if (!rc) rc = cuda_check(c, cudaStreamCreateWithFlags(&c->cap_stream, cudaStreamNonBlocking), "stream");
+    if (!rc) rc = cuda_check(c, cudaStreamCreateWithFlags(&c->cap_main, cudaStreamNonBlocking), "stream");
+    if (!rc) rc = cuda_check(c, cudaStreamCreateWithFlags(&c->copy_st, cudaStreamNonBlocking), "stream");
+    if (!rc) rc = cuda_check(c, cudaEventCreateWithFlags(&c->ev_in, cudaEventDisableTiming), "event");
+    if (!rc) rc = cuda_check(c, cudaEventCreateWithFlags(&c->ev_tail, cudaEventDisableTiming), "event");
+    // a step's graph waits on ev_in: give it a first, completed record
+    if (!rc) rc = cuda_check(c, cudaEventRecord(c->ev_in, c->copy_st), "event");
     if (!rc && cudaDeviceSynchronize() != cudaSuccess) rc = PSB_ECUDA;
     if (rc) {
         std::fprintf(stderr, "psb_create: %s\n", c->err.empty() ? "allocation failed" : c->err.c_str());
@@ -1110,7 +1134,7 @@ int create_impl(const psb_scene* scene, size_t ncells, psb_ctx** out) {
         delete c;
         return rc;
     }
-    std::memset(c->h_err, 0, sizeof(unsigned long long) * (PSB_MAX_ITERS + 1));
+    c->nscenes = S;
     {   // pressure scale of the learned warm start: rho0 |g| 0.1 m
         const double g = std::sqrt((double)scene->gravity[0] * scene->gravity[0] +
                                    (double)scene->gravity[1] * scene->gravity[1] +
@@ -1145,35 +1169,6 @@ const char* batch_mismatch(const psb_scene& a, const psb_scene& b) {
     return nullptr;
 }
 
-// The device-side corrector's words for S scenes (batch.cu), their pinned
-// mirrors, and the streams a CUDA-graph capture runs on.
-int alloc_loop(psb_ctx* c, int S) {
-    int rc = PSB_OK;
-    if (!rc) rc = dalloc(c, &c->d_active, S);
-    if (!rc) rc = dalloc(c, &c->d_err_scene, S);
-    if (!rc) rc = dalloc(c, &c->d_err_sh, (size_t)(PSB_MAX_ITERS + 1) * S);
-    if (!rc) rc = dalloc(c, &c->d_loop, 2 + 4 * (size_t)S);
-    if (!rc && cudaMallocHost((void**)&c->h_loop, sizeof(int) * (2 + 4 * (size_t)S)) != cudaSuccess) rc = PSB_ENOMEM;
-    if (!rc && cudaMallocHost((void**)&c->h_err_sh, sizeof(unsigned long long) * (PSB_MAX_ITERS + 1) * S) != cudaSuccess)
-        rc = PSB_ENOMEM;
-    if (!rc) rc = cuda_check(c, cudaMemset(c->d_loop, 0, sizeof(int) * (2 + 4 * (size_t)S)), "loop");
-    if (!rc) rc = cuda_check(c, cudaMemset(c->d_active, 1, S), "active");
-    if (!rc) rc = cuda_check(c, cudaMemset(c->d_err_scene, 0, sizeof(unsigned long long) * S), "err");
-    if (!rc) rc = cuda_check(c, cudaMemset(c->d_err_sh, 0, sizeof(unsigned long long) * (PSB_MAX_ITERS + 1) * S), "err");
-    if (!rc) rc = cuda_check(c, cudaStreamCreateWithFlags(&c->cap_stream, cudaStreamNonBlocking), "stream");
-    if (!rc) rc = cuda_check(c, cudaStreamCreateWithFlags(&c->cap_main, cudaStreamNonBlocking), "stream");
-    if (!rc) rc = cuda_check(c, cudaStreamCreateWithFlags(&c->copy_st, cudaStreamNonBlocking), "stream");
-    if (!rc) rc = cuda_check(c, cudaEventCreateWithFlags(&c->ev_in, cudaEventDisableTiming), "event");
-    if (!rc) rc = cuda_check(c, cudaEventCreateWithFlags(&c->ev_tail, cudaEventDisableTiming), "event");
-    // a step's graph waits on ev_in: give it a first, completed record
-    if (!rc) rc = cuda_check(c, cudaEventRecord(c->ev_in, c->copy_st), "event");
-    if (!rc) {
-        std::memset(c->h_loop, 0, sizeof(int) * (2 + 4 * (size_t)S));
-        std::memset(c->h_err_sh, 0, sizeof(unsigned long long) * (PSB_MAX_ITERS + 1) * S);
-    }
-    return rc;
-}
-
 }  // namespace
 
 extern "C" {
@@ -1186,16 +1181,7 @@ int psb_create(const psb_scene* scene, psb_ctx** out) {
         std::fprintf(stderr, "psb_create: %s\n", why.c_str());
         return PSB_EINVAL;
     }
-    PSB_TRY(create_impl(scene, (size_t)scene->dims[0] * scene->dims[1] * scene->dims[2], out));
-    psb_ctx* c = *out;
-    if (const int rc = alloc_loop(c, 1)) {
-        std::fprintf(stderr, "psb_create: %s\n", c->err.c_str());
-        free_all(c);
-        delete c;
-        *out = nullptr;
-        return rc;
-    }
-    return PSB_OK;
+    return create_impl(scene, (size_t)scene->dims[0] * scene->dims[1] * scene->dims[2], 1, false, out);
 }
 
 int psb_create_batch(const psb_scene* scenes, int32_t n_scenes, psb_ctx** out) {
@@ -1223,10 +1209,9 @@ int psb_create_batch(const psb_scene* scenes, int32_t n_scenes, psb_ctx** out) {
     psb_scene u = scenes[0];
     u.n_max = (int32_t)total;
     psb_ctx* c = nullptr;
-    PSB_TRY(create_impl(&u, cells, &c));
     const int S = n_scenes;
+    PSB_TRY(create_impl(&u, cells, S, true, &c));
     c->batch = true;
-    c->nscenes = S;
     c->first.assign(S + 1, 0);
     c->geom.resize(S);
     std::vector<uint16_t> slot_scene((size_t)total);
@@ -1252,11 +1237,8 @@ int psb_create_batch(const psb_scene* scenes, int32_t n_scenes, psb_ctx** out) {
         std::fill(slot_scene.begin() + c->first[s], slot_scene.begin() + c->first[s + 1], (uint16_t)s);
     }
     int rc = PSB_OK;
-    if (!rc) rc = dalloc(c, &c->d_scenes, S);
-    if (!rc) rc = dalloc(c, &c->d_slot_scene, (size_t)total);
     if (!rc) rc = cuda_check(c, cudaMemcpy(c->d_scenes, c->geom.data(), sizeof(psb::SceneGeom) * S, cudaMemcpyHostToDevice), "geom");
     if (!rc) rc = cuda_check(c, cudaMemcpy(c->d_slot_scene, slot_scene.data(), 2 * (size_t)total, cudaMemcpyHostToDevice), "slots");
-    if (!rc) rc = alloc_loop(c, S);
     if (rc) {
         std::fprintf(stderr, "psb_create_batch: %s\n", c->err.c_str());
         free_all(c);
