@@ -1041,6 +1041,7 @@ int create_impl(const psb_scene* scene, size_t ncells, int S, bool batch, psb_ct
     cudaGetDevice(&c->device);
     const size_t n = (size_t)c->n_max, s_ = (size_t)S;
     c->dense = dense_cells(c->ncells, n);
+    c->P.dense_cells = c->dense;
     const bool ghosts = !c->P.ref && !c->P.dem;
     const size_t words = psb::cell_sort_cells(c->ncells), tiles = psb::cell_sort_tiles(c->ncells);
     // The buffers a context always has, in one device and one pinned block:
@@ -1053,7 +1054,8 @@ int create_impl(const psb_scene* scene, size_t ncells, int S, bool batch, psb_ct
             at += (std::max<size_t>(count, 1) * sizeof(*p) + 511) & ~(size_t)511;
         };
         for (int i = 0; i < 2; ++i) {
-            take(c->pos[i], n); take(c->vel[i], n); take(c->vap[i], n); take(c->rp[i], n); take(c->ids[i], n);
+            take(c->pos[i], n + 3);     // the neighbour build reads a row in fours, up to three past its end
+            take(c->vel[i], n); take(c->vap[i], n); take(c->rp[i], n); take(c->ids[i], n);
             take(c->keys[i], n); take(c->vals[i], n); take(c->xs[i], n);
         }
         if (c->dense) {

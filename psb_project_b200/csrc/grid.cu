@@ -476,29 +476,145 @@ __global__ void k_reorder_state(int n, const uint32_t* __restrict__ vals, const 
 
 // Per-thread schedule: one thread per sorted particle. The three cells of a
 // grid row are adjacent in sorted order, so each of the nine rows is one
-// contiguous slot range; candidates are visited in increasing slot order and
+// contiguous slot range; candidates are taken in increasing slot order and
 // the list is sorted. In a batch the walk stays inside the particle's
 // scene's grid.
+//
+// ~216 candidates are tested for ~33 kept, so the test is kept to the load,
+// six FP32 operations and one shift: with e = |d|^2 - h^2 in one FMA chain, a
+// funnel shift collects e's sign into the row's mask, and a running minimum
+// of |e| says whether any candidate of the row came within rounding of the
+// cut-off -- only then is the row gone over again with the reference's FP64
+// test. The masks of the nine rows wait in shared memory; the list is then
+// written quad by quad, every lane's k-th quad in the same store (512
+// contiguous bytes a warp), where one 4-byte store per entry was a sector
+// write for each of 34M entries at 1M particles.
+// A candidate used to cost ~30 issued instructions (its own accept branch,
+// taken by some lane nearly every time) and costs ~10 now.
+constexpr int kRows = 9;
+
+// The candidates of one row, slots [lo, lo + m) with 1 <= m <= 32: bit 31 - c
+// of the result is set when slot lo + c is a neighbour of the particle at pi.
+// Reads up to three slots past the range (pos is padded by as many).
+__device__ __forceinline__ uint32_t row_mask(const Params& P, float4 pi, const float4* __restrict__ pos, uint32_t lo,
+                                             uint32_t m) {
+    const float4* __restrict__ x = pos + lo;
+    uint32_t mask = 0u;
+    float near = INFINITY;
+    auto excess = [&](float4 pj) {
+        const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+        return __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmaf_rn(dx, dx, -P.h2)));
+    };
+    for (uint32_t c = 0; c < m; c += 4) {
+        const float4 a0 = x[c], a1 = x[c + 1], a2 = x[c + 2], a3 = x[c + 3];
+        const float e0 = excess(a0), e1 = excess(a1), e2 = excess(a2), e3 = excess(a3);
+        mask = __funnelshift_l(__float_as_uint(e0), mask, 1);
+        mask = __funnelshift_l(__float_as_uint(e1), mask, 1);
+        mask = __funnelshift_l(__float_as_uint(e2), mask, 1);
+        mask = __funnelshift_l(__float_as_uint(e3), mask, 1);
+        near = fminf(fminf(near, fminf(fabsf(e0), fabsf(e1))), fminf(fabsf(e2), fabsf(e3)));
+    }
+    mask = (mask << (32u - ((m + 3u) & ~3u))) & (kEmpty << (32u - m));
+    // h2_hi - h2 is 1e-5 h^2, some thirty times the rounding of e near h
+    const float band = P.h2_hi - P.h2;
+    if (near <= band) {
+        for (uint32_t c = 0; c < m; ++c) {
+            const float4 pj = x[c];
+            if (!(fabsf(excess(pj)) <= band)) continue;
+            const uint32_t bit = 0x80000000u >> c;
+            if (exact_neighbor(pi, pj, P.h2_exact)) mask |= bit;
+            else mask &= ~bit;
+        }
+    }
+    return mask;
+}
+
 template <bool BATCH, int BS>
 __global__ void __launch_bounds__(BS) k_build_nbr(Params P, const float4* __restrict__ pos,
                                                   const uint32_t* __restrict__ keys,
                                                   const uint32_t* __restrict__ cell_start,
                                                   const uint32_t* __restrict__ cell_end, int* __restrict__ counts,
                                                   int* __restrict__ list, int* __restrict__ flags) {
-    const int t = blockIdx.x * BS + threadIdx.x;
+    __shared__ uint32_t s_first[kRows][BS], s_mask[kRows][BS];     // each thread uses its own column
+    const int tid = threadIdx.x;
+    const int t = blockIdx.x * BS + tid;
     const bool valid = t < P.n;       // every lane stays for the warp reductions below
     const int n = P.n;
     int cnt = 0;
     if (valid) {
-        int* wq = list + nbr_index(0, n, t);
-        const size_t qstride = (size_t)4 * (size_t)n;
-        walk_neighbours<BATCH>(P, t, pos[t], pos, keys, cell_start, cell_end, [&](uint32_t q, float4) {
-            // one 4-byte store per entry (buffering four in registers measured
-            // slower); wq is entry cnt's quad, nbr_index(cnt, n, t) - (cnt & 3)
-            if (cnt < P.cap) wq[cnt & 3] = (int)q;
-            ++cnt;
-            if ((cnt & 3) == 0 && cnt < P.cap) wq += qstride;
-        });
+        const Grid g = BATCH ? P.scenes[P.slot_scene[t]].g : P.g;
+        const uint32_t base = BATCH ? P.scenes[P.slot_scene[t]].cell_base : 0u;
+        const uint32_t nx = (uint32_t)g.nx, ny = (uint32_t)g.ny;
+        const uint32_t key = keys[t] - base;
+        const int ci = (int)(key % nx), cj = (int)((key / nx) % ny), ck = (int)(key / (nx * ny));
+        const int a0 = max(ci - 1, 0), a1 = min(ci + 1, g.nx - 1);
+        // the nine rows' slot ranges: independent loads, in flight together
+        uint32_t longest = 0u;
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+            const int j = cj + r % 3 - 1, k = ck + r / 3 - 1;
+            uint32_t lo = 0u, hi = 0u;
+            if (j >= 0 && j < g.ny && k >= 0 && k < g.nz) {
+                const uint32_t row = base + (uint32_t)j * nx + (uint32_t)k * nx * ny;
+                if (P.dense_cells) {
+                    lo = cell_start[row + a0];
+                    hi = cell_end[row + a1];
+                } else {
+                    row_range(cell_start, cell_end, row, a0, a1, lo, hi);
+                }
+            }
+            s_first[r][tid] = lo;
+            s_mask[r][tid] = hi;
+            longest = max(longest, hi - lo);
+        }
+        const float4 pi = pos[t];
+        if (longest <= 32u) {
+            for (int r = 0; r < kRows; ++r) {
+                const uint32_t lo = s_first[r][tid], m = s_mask[r][tid] - lo;
+                const uint32_t mask = m ? row_mask(P, pi, pos, lo, m) : 0u;
+                s_mask[r][tid] = mask;
+                cnt += __popc(mask);
+            }
+            // the set bits of the nine masks in order, four to a store
+            const int kept = min(cnt, P.cap);
+            int4* __restrict__ out = reinterpret_cast<int4*>(list) + t;
+            int r = -1;
+            uint32_t mask = 0u, q = 0u;
+            auto next = [&] {
+                while (mask == 0u) {
+                    ++r;
+                    mask = s_mask[r][tid];
+                    q = s_first[r][tid];
+                }
+                const int z = __clz((int)mask);
+                mask = (mask << z) << 1;
+                q += (uint32_t)z;
+                return (int)q++;
+            };
+            for (int c = 0; c < kept; c += 4, out += n) {
+                int4 e = make_int4(0, 0, 0, 0);
+                e.x = next();
+                if (c + 1 < kept) e.y = next();
+                if (c + 2 < kept) e.z = next();
+                if (c + 3 < kept) e.w = next();
+                *out = e;
+            }
+        } else {        // a row of more than 32 candidates: 32 at a time, an entry a store
+            for (int r = 0; r < kRows; ++r) {
+                const uint32_t hi = s_mask[r][tid];
+                for (uint32_t lo = s_first[r][tid]; lo < hi; lo += 32u) {
+                    uint32_t mask = row_mask(P, pi, pos, lo, min(hi - lo, 32u)), q = lo;
+                    while (mask) {
+                        const int z = __clz((int)mask);
+                        mask = (mask << z) << 1;
+                        q += (uint32_t)z;
+                        if (cnt < P.cap) list[nbr_index(cnt, n, t)] = (int)q;
+                        ++q;
+                        ++cnt;
+                    }
+                }
+            }
+        }
         counts[t] = cnt;
         if (cnt > P.cap) atomicOr(&flags[0], 1);
     }

@@ -126,6 +126,7 @@ struct Params {
     int* wall_count;
     uint32_t* wall_bits;
     int wall_blocks;
+    int dense_cells;    // the cell ranges cover every cell (the counting sort's), empty ones included
 };
 
 // Distance to a face, in h, up to which the reorder lists a particle: past
@@ -208,6 +209,22 @@ __device__ __forceinline__ void nbr_flags(int cnt, int* __restrict__ flags) {
         atomicMax(&flags[1], m);
         atomicAdd((unsigned long long*)&flags[2], tot);
     }
+}
+
+// Slots of cells a0..a1 of a row where empty cells hold kEmpty (the radix
+// sort's ranges): lo = hi = 0 when all are empty.
+__device__ __forceinline__ void row_range(const uint32_t* __restrict__ cell_start,
+                                          const uint32_t* __restrict__ cell_end, uint32_t row, int a0, int a1,
+                                          uint32_t& lo, uint32_t& hi) {
+    lo = kEmpty;
+    hi = 0u;
+    for (int a = a0; a <= a1; ++a) {
+        const uint32_t s = cell_start[row + a];
+        if (s == kEmpty) continue;
+        if (lo == kEmpty) lo = s;
+        hi = cell_end[row + a];
+    }
+    if (lo == kEmpty) lo = 0u;
 }
 
 // The 27-cell walk of sorted particle t (one thread per particle): the three
