@@ -120,8 +120,8 @@ struct psb_ctx {
     int* nbr_list = nullptr;
     // SPH scratch
     float4* fnp = nullptr;
-    float4* xs[2] = {};
-    float4* vs = nullptr;
+    psb::Soa3 xs[2] = {};
+    psb::Soa3 vs{};
     float2* rpc = nullptr;
     float* rho_x = nullptr;
     unsigned long long* err_hist = nullptr;
@@ -582,7 +582,7 @@ int build(psb_ctx* c, bool keep_p = false, bool features = false) {
         // the predictor's x* buffer is free until the set-up sweep
         timed(c, "cell_sort", [&] {
             psb::launch_cell_sort(st, n, c->ncells, c->ids[c->cr], c->keys[0], c->vals[0], c->cell_count, c->tile_sum,
-                                  c->cell_start, reinterpret_cast<uint2*>(c->xs[0]), c->keys[1], c->vals[1]);
+                                  c->cell_start, reinterpret_cast<uint2*>(c->xs[0].xy), c->keys[1], c->vals[1]);
         });
         res = 1;
         range_start = nullptr;
@@ -614,7 +614,7 @@ int build(psb_ctx* c, bool keep_p = false, bool features = false) {
         if (!split) return;
         wait_inputs(c, st);
         timed(c, "reorder_state", [&] {
-            psb::launch_reorder_state(st, n, c->vals[res], c->vel[os], c->vap[os], c->rp[orr], c->vel[ns], c->vap[ns],
+            psb::launch_reorder_state(st, P, c->vals[res], c->vel[os], c->vap[os], c->rp[orr], c->vel[ns], c->vap[ns],
                                       c->rp[nr]);
         });
     };
@@ -635,7 +635,7 @@ int build(psb_ctx* c, bool keep_p = false, bool features = false) {
     if (fused_density(c, P)) {
         reorder_state();
         timed(c, "build_nbr", [&] {
-            psb::launch_build_density(st, P, c->pos[c->cs], c->vel[c->cs], c->keys[res], c->cell_start, c->cell_end,
+            psb::launch_build_density(st, P, c->pos[c->cs], c->keys[res], c->cell_start, c->cell_end,
                                       c->nbr_count, c->nbr_list, c->flags, c->rp[c->cr], c->rho_x, zero_p, c->p_scale,
                                       feats, nfeat);
         });
@@ -647,7 +647,7 @@ int build(psb_ctx* c, bool keep_p = false, bool features = false) {
         reorder_state();
         if (!P.dem)
             timed(c, "density_x", [&] {
-                psb::launch_density_x(st, P, c->pos[c->cs], c->vel[c->cs], c->nbr_count, c->nbr_list, c->rp[c->cr],
+                psb::launch_density_x(st, P, c->nbr_count, c->nbr_list, c->rp[c->cr],
                                       c->rho_x, zero_p, c->p_scale, feats, nfeat);
             });
     }
@@ -697,7 +697,7 @@ int batch_corrector(psb_ctx* c, const Params& P, int s, int r, bool capture) {
     if (c->corrector == PSB_CORRECTOR_PERSISTENT && max_it > 0 && !moving) {     // begins the loop itself
         cudaError_t e = cudaSuccess;
         timed(c, "corrector_persistent", [&] {
-            e = psb::launch_corrector_persistent(st, P, c->pos[s], c->vap[s], c->fnp, c->xs[0], c->rp[r], c->rpc,
+            e = psb::launch_corrector_persistent(st, P, c->vap[s], c->fnp, c->xs[0], c->rp[r], c->rpc,
                                                  c->nbr_count, c->nbr_list, c->vs, S, c->sc.min_iters, max_it,
                                                  c->sc.eta, c->d_active, c->d_err_scene, c->d_err_sh, c->d_loop);
         });
@@ -718,7 +718,7 @@ int batch_corrector(psb_ctx* c, const Params& P, int s, int r, bool capture) {
                                      c->d_err_sh, c->d_loop, h, set_handle);
         });
         timed(c, "pci_force_predict", [&] {
-            psb::launch_pci_force_predict(bs, P, c->pos[s], c->vap[s], c->fnp, c->xs[1], c->rpc, c->nbr_count,
+            psb::launch_pci_force_predict(bs, P, c->vap[s], c->fnp, c->xs[1], c->rpc, c->nbr_count,
                                           c->nbr_list, c->xs[0], c->vs, c->rp[r]);
         });
         // the boundary predicted with the pressures the fluid's prediction
@@ -776,18 +776,18 @@ int enqueue_loop_step(psb_ctx* c, bool capture) {
     if (moving) P.bnd_pred = c->bnd_pred;
     if (mode == PSB_WARM_LEARNED) {
         timed(c, "mlp_infer", [&] {
-            psb::launch_mlp_infer(st, c->mlp_arch, c->n, c->feats, c->mlp_wbf, c->p_scale, c->rp[r]);
+            psb::launch_mlp_infer(st, c->mlp_arch, c->n, c->feats, c->mlp_wbf, c->p_scale, c->rp[r], P.zp);
         });
     } else if (mode == PSB_WARM_ZERO && collect) {
         psb::launch_zero_pressure(st, c->n, c->rp[r]);
     }
     timed(c, "pci_init", [&] {
-        psb::launch_pci_init(st, P, c->pos[s], c->vel[s], c->vap[s], c->rp[r], c->nbr_count, c->nbr_list,
+        psb::launch_pci_init(st, P, c->vap[s], c->rp[r], c->nbr_count, c->nbr_list,
                              mode == PSB_WARM_ZERO ? 0 : 1, c->fnp, c->xs[0], c->vs);
     });
     if (moving) move_boundary(c, st, P, s, r);     // the boundary's first prediction, with the initial pressure
     PSB_TRY(batch_corrector(c, P, s, r, capture));
-    const float4* v_commit = c->vs;
+    psb::Soa3 v_commit = c->vs;
     if (P.xsph_k != 0.f) {
         timed(c, "xsph", [&] { psb::launch_xsph(st, P, c->xs[0], c->vs, c->nbr_count, c->nbr_list, c->xs[1]); });
         v_commit = c->xs[1];
@@ -953,7 +953,7 @@ int step_once(psb_ctx* c, bool last) {
     } else if (!P.pci) {
         const int o = s ^ 1;
         timed(c, "wcsph_force", [&] {
-            psb::launch_wcsph_force(st, P, c->pos[s], c->vel[s], c->vap[s], c->rp[r], c->nbr_count, c->nbr_list,
+            psb::launch_wcsph_force(st, P, c->vap[s], c->rp[r], c->nbr_count, c->nbr_list,
                                     c->pos[o], c->vel[o], c->vap[o], c->fnp);
         });
         if (P.n_coll > 0)
@@ -967,7 +967,7 @@ int step_once(psb_ctx* c, bool last) {
         // reference-profile PCISPH: exactly three corrections from p = 0
         // (PciSphSystem.cu:30-61), no host round trip
         timed(c, "pci_init", [&] {
-            psb::launch_pci_init(st, P, c->pos[s], c->vel[s], c->vap[s], c->rp[r], c->nbr_count, c->nbr_list, 0,
+            psb::launch_pci_init(st, P, c->vap[s], c->rp[r], c->nbr_count, c->nbr_list, 0,
                                  c->fnp, c->xs[0], c->vs);
         });
         constexpr int kRefIters = 3;
@@ -977,7 +977,7 @@ int step_once(psb_ctx* c, bool last) {
                 psb::launch_pci_density(st, P, c->xs[xi], c->rp[r], c->nbr_count, c->nbr_list, c->rpc, &c->err_hist[k]);
             });
             timed(c, "pci_force_predict", [&] {
-                psb::launch_pci_force_predict(st, P, c->pos[s], c->vap[s], c->fnp, c->xs[xi], c->rpc, c->nbr_count,
+                psb::launch_pci_force_predict(st, P, c->vap[s], c->fnp, c->xs[xi], c->rpc, c->nbr_count,
                                               c->nbr_list, c->xs[xi ^ 1], c->vs, c->rp[r]);
             });
             xi ^= 1;
@@ -1056,7 +1056,8 @@ int create_impl(const psb_scene* scene, size_t ncells, int S, bool batch, psb_ct
         for (int i = 0; i < 2; ++i) {
             take(c->pos[i], n + 3);     // the neighbour build reads a row in fours, up to three past its end
             take(c->vel[i], n); take(c->vap[i], n); take(c->rp[i], n); take(c->ids[i], n);
-            take(c->keys[i], n); take(c->vals[i], n); take(c->xs[i], n);
+            take(c->keys[i], n); take(c->vals[i], n);
+            take(c->xs[i].xy, n); take(c->xs[i].z, n);
         }
         if (c->dense) {
             take(c->cell_start, words);
@@ -1069,8 +1070,12 @@ int create_impl(const psb_scene* scene, size_t ncells, int S, bool batch, psb_ct
             take(c->cell_end, c->ncells);
         }
         take(c->nbr_count, n); take(c->nbr_list, psb::nbr_list_ints(n, c->cap));
-        take(c->fnp, n); take(c->vs, n); take(c->rpc, n); take(c->rho_x, n);
+        take(c->fnp, n); take(c->vs.xy, n); take(c->vs.z, n); take(c->rpc, n); take(c->rho_x, n);
         take(c->err_hist, PSB_MAX_ITERS + 1); take(c->flags, 8);
+        if (!c->P.dem) {
+            take(c->P.x0.xy, n); take(c->P.x0.z, n); take(c->P.v0.xy, n); take(c->P.v0.z, n);
+            take(c->P.zp, n); take(c->P.vr, n);
+        }
         if (ghosts) {       // config-profile SPH: the wall list and its flags
             take(c->P.wall_list, n);
             take(c->P.wall_bits, (n + 31) / 32);
@@ -1615,7 +1620,7 @@ int psb_presolve(psb_ctx* c, int32_t iters) {
     cudaMemsetAsync(c->err_hist, 0, sizeof(unsigned long long) * (PSB_MAX_ITERS + 1), st);
     if (c->batch) cudaMemsetAsync(c->d_active, 1, c->nscenes, st);     // every scene takes every pass
     timed(c, "pci_init", [&] {
-        psb::launch_pci_init(st, P, c->pos[s], c->vel[s], c->vap[s], c->rp[r], c->nbr_count, c->nbr_list, 1, c->fnp,
+        psb::launch_pci_init(st, P, c->vap[s], c->rp[r], c->nbr_count, c->nbr_list, 1, c->fnp,
                              c->xs[0], c->vs);
     });
     int xi = 0;
@@ -1625,7 +1630,7 @@ int psb_presolve(psb_ctx* c, int32_t iters) {
                                     &c->err_hist[k < PSB_MAX_ITERS ? k : PSB_MAX_ITERS]);
         });
         timed(c, "pci_force_predict", [&] {
-            psb::launch_pci_force_predict(st, P, c->pos[s], c->vap[s], c->fnp, c->xs[xi], c->rpc, c->nbr_count,
+            psb::launch_pci_force_predict(st, P, c->vap[s], c->fnp, c->xs[xi], c->rpc, c->nbr_count,
                                           c->nbr_list, c->xs[xi ^ 1], c->vs, c->rp[r]);
         });
         xi ^= 1;
@@ -1673,7 +1678,7 @@ int psb_warm_start(psb_ctx* c, float* features, float* pressure) {
             // pressure, an input of the next step, stays in place
             const float2* src = c->rp[c->cr];
             if (mode == PSB_WARM_LEARNED) {
-                psb::launch_mlp_infer(st, c->mlp_arch, n, c->feats, c->mlp_wbf, c->p_scale, c->rpc);
+                psb::launch_mlp_infer(st, c->mlp_arch, n, c->feats, c->mlp_wbf, c->p_scale, c->rpc, nullptr);
                 src = c->rpc;
             }
             k_scatter_rp<<<blocks(n), psb::kBlock, 0, st>>>(n, ids, src, 1, stage);
@@ -2501,7 +2506,7 @@ int psb_autotune(psb_ctx* c, int32_t trials, psb_tune* out) {
     // so that all three do the same work.
     tune_one(0, [&](const Params& Q) {
         if (fused_density(c, Q)) {
-            psb::launch_build_density(st, Q, c->pos[s], c->vel[s], c->keys[c->sorted], c->cell_start, c->cell_end,
+            psb::launch_build_density(st, Q, c->pos[s], c->keys[c->sorted], c->cell_start, c->cell_end,
                                       c->nbr_count, c->nbr_list, c->flags, c->rp[r], c->rho_x, 0, c->p_scale,
                                       feats ? c->feats : nullptr, psb::mlp_inputs(c->mlp_arch));
             return;
@@ -2511,25 +2516,25 @@ int psb_autotune(psb_ctx* c, int32_t trials, psb_tune* out) {
         if (can_fuse_density(c, Q)) {
             Params D = Q;
             D.tune = psb::Tune{};
-            psb::launch_density_x(st, D, c->pos[s], c->vel[s], c->nbr_count, c->nbr_list, c->rp[r], c->rho_x, 0,
+            psb::launch_density_x(st, D, c->nbr_count, c->nbr_list, c->rp[r], c->rho_x, 0,
                                   c->p_scale, feats ? c->feats : nullptr, psb::mlp_inputs(c->mlp_arch));
         }
     });
     if (sph)
         tune_one(1, [&](const Params& Q) {
-            psb::launch_density_x(st, Q, c->pos[s], c->vel[s], c->nbr_count, c->nbr_list, c->rp[r], c->rho_x, 0,
+            psb::launch_density_x(st, Q, c->nbr_count, c->nbr_list, c->rp[r], c->rho_x, 0,
                                   c->p_scale, feats ? c->feats : nullptr, psb::mlp_inputs(c->mlp_arch));
         });
     if (pci) {
         tune_one(2, [&](const Params& Q) {
-            psb::launch_pci_init(st, Q, c->pos[s], c->vel[s], c->vap[s], c->rp[r], c->nbr_count, c->nbr_list, warm,
+            psb::launch_pci_init(st, Q, c->vap[s], c->rp[r], c->nbr_count, c->nbr_list, warm,
                                  c->fnp, c->xs[0], c->vs);
         });
         tune_one(3, [&](const Params& Q) {
             psb::launch_pci_density(st, Q, c->xs[0], c->rp[r], c->nbr_count, c->nbr_list, c->rpc, &c->err_hist[0]);
         });
         tune_one(4, [&](const Params& Q) {
-            psb::launch_pci_force_predict(st, Q, c->pos[s], c->vap[s], c->fnp, c->xs[0], c->rpc, c->nbr_count,
+            psb::launch_pci_force_predict(st, Q, c->vap[s], c->fnp, c->xs[0], c->rpc, c->nbr_count,
                                           c->nbr_list, c->xs[1], c->vs, c->rp[r]);
         });
         tune_one(5, [&](const Params& Q) {

@@ -428,8 +428,15 @@ __global__ void k_reorder(Params P, const uint32_t* __restrict__ keys, const uin
     const float4 x = t < n ? pos[s] : make_float4(0.f, 0.f, 0.f, 0.f);
     list_near_walls<BATCH>(P, t, x);
     if (t >= n) return;
+    const float4 v = vel[s];
     pos2[t] = x;
-    vel2[t] = vel[s];
+    vel2[t] = v;
+    if (P.x0.xy) {
+        P.x0.xy[t] = make_float2(x.x, x.y);
+        P.x0.z[t] = x.z;
+        P.v0.xy[t] = make_float2(v.x, v.y);
+        P.v0.z[t] = v.z;
+    }
     vap2[t] = vap[s];
     rp2[t] = rp[s];
     ids2[t] = ids[s];
@@ -454,6 +461,10 @@ __global__ void k_reorder_pos(Params P, const uint32_t* __restrict__ keys, const
     list_near_walls<BATCH>(P, t, x);
     if (t >= n) return;
     pos2[t] = x;
+    if (P.x0.xy) {
+        P.x0.xy[t] = make_float2(x.x, x.y);
+        P.x0.z[t] = x.z;
+    }
     ids2[t] = ids[s];
     if (!cell_start) return;
     const uint32_t k = keys[t];
@@ -463,13 +474,18 @@ __global__ void k_reorder_pos(Params P, const uint32_t* __restrict__ keys, const
 
 // Gathers velocities, half-step velocities and (density, pressure) into
 // sorted order.
-__global__ void k_reorder_state(int n, const uint32_t* __restrict__ vals, const float4* __restrict__ vel,
+__global__ void k_reorder_state(Params P, const uint32_t* __restrict__ vals, const float4* __restrict__ vel,
                                 const float4* __restrict__ vap, const float2* __restrict__ rp,
                                 float4* __restrict__ vel2, float4* __restrict__ vap2, float2* __restrict__ rp2) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
+    if (t >= P.n) return;
     const uint32_t s = vals[t];
-    vel2[t] = vel[s];
+    const float4 v = vel[s];
+    vel2[t] = v;
+    if (P.v0.xy) {
+        P.v0.xy[t] = make_float2(v.x, v.y);
+        P.v0.z[t] = v.z;
+    }
     vap2[t] = vap[s];
     rp2[t] = rp[s];
 }
@@ -797,9 +813,9 @@ void launch_reorder_pos(cudaStream_t st, const Params& P, const uint32_t* keys, 
     kernel<<<grid_of(P.n), kBlock, 0, st>>>(P, keys, vals, pos, ids, pos2, ids2, cell_start, cell_end);
 }
 
-void launch_reorder_state(cudaStream_t st, int n, const uint32_t* vals, const float4* vel, const float4* vap,
+void launch_reorder_state(cudaStream_t st, const Params& P, const uint32_t* vals, const float4* vel, const float4* vap,
                           const float2* rp, float4* vel2, float4* vap2, float2* rp2) {
-    if (n > 0) k_reorder_state<<<grid_of(n), kBlock, 0, st>>>(n, vals, vel, vap, rp, vel2, vap2, rp2);
+    if (P.n > 0) k_reorder_state<<<grid_of(P.n), kBlock, 0, st>>>(P, vals, vel, vap, rp, vel2, vap2, rp2);
 }
 
 void launch_build_nbr(cudaStream_t st, const Params& P, const float4* pos, const uint32_t* keys,

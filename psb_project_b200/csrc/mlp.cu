@@ -185,7 +185,8 @@ __device__ __forceinline__ void layer64(float (&z)[8][4], const uint32_t (&a)[4]
 template <int NIN, int ACT>
 __global__ void __launch_bounds__(256) k_mlp_infer_mma(int n, const float* __restrict__ feats,
                                                        const __nv_bfloat16* __restrict__ w, float p_scale,
-                                                       float2* __restrict__ rp, float* __restrict__ y_raw) {
+                                                       float2* __restrict__ rp, float2* __restrict__ zp,
+                                                       float* __restrict__ y_raw) {
     __shared__ uint32_t sW1[kH * kW1Stride];
     __shared__ uint32_t sW2[kH * kRow];
     __shared__ float sB1[kH], sB2[kH], sW3[kH];
@@ -233,8 +234,11 @@ __global__ void __launch_bounds__(256) k_mlp_infer_mma(int n, const float* __res
                 if (r0 < n) y_raw[r0] = y0 + sB3;
                 if (r1 < n) y_raw[r1] = y1 + sB3;
             } else {
-                if (r0 < n) rp[r0].y = fmaxf(0.f, y0 + sB3) * p_scale;
-                if (r1 < n) rp[r1].y = fmaxf(0.f, y1 + sB3) * p_scale;
+                const float p0 = fmaxf(0.f, y0 + sB3) * p_scale, p1 = fmaxf(0.f, y1 + sB3) * p_scale;
+                if (r0 < n) rp[r0].y = p0;
+                if (r1 < n) rp[r1].y = p1;
+                if (zp && r0 < n) zp[r0].y = p0;
+                if (zp && r1 < n) zp[r1].y = p1;
             }
         }
     }
@@ -535,13 +539,14 @@ void with_arch(int arch, F&& f) {
     else f(std::integral_constant<int, 6>{}, std::integral_constant<int, kSilu>{});
 }
 
-void infer(cudaStream_t st, int arch, int n, const float* feats, const void* wbf, float p_scale, float2* rp, float* y) {
+void infer(cudaStream_t st, int arch, int n, const float* feats, const void* wbf, float p_scale, float2* rp, float2* zp,
+           float* y) {
     if (n <= 0) return;
     const int tiles = (n + 15) / 16;
     const int blocks = std::min((tiles + 7) / 8, 148 * 8);      // 8 warps per block, grid-stride over tiles
     with_arch(arch, [&](auto nin, auto a) {
         k_mlp_infer_mma<decltype(nin)::value, decltype(a)::value>
-            <<<blocks, 256, 0, st>>>(n, feats, (const __nv_bfloat16*)wbf, p_scale, rp, y);
+            <<<blocks, 256, 0, st>>>(n, feats, (const __nv_bfloat16*)wbf, p_scale, rp, zp, y);
     });
 }
 
@@ -555,14 +560,14 @@ void launch_zero_pressure(cudaStream_t st, int n, float2* rp) {
 }
 
 void launch_mlp_infer(cudaStream_t st, int arch, int n, const float* feats, const void* wbf, float p_scale,
-                      float2* rp) {
-    infer(st, arch, n, feats, wbf, p_scale, rp, nullptr);
+                      float2* rp, float2* zp) {
+    infer(st, arch, n, feats, wbf, p_scale, rp, zp, nullptr);
 }
 
 // Host-facing forward through the tensor-core kernel the warm start uses
 // (rows of stride 8).
 void launch_mlp_forward(cudaStream_t st, int arch, int n, const float* X, const void* wbf, float* y) {
-    infer(st, arch, n, X, wbf, 1.f, nullptr, y);
+    infer(st, arch, n, X, wbf, 1.f, nullptr, nullptr, y);
 }
 
 void launch_mlp_grad(cudaStream_t st, int arch, int batch, const float* X, const float* T, const uint32_t* sel,

@@ -10,7 +10,7 @@
 // Per-step scratch: sort keys/values (2 x 2 x 4 B), cell_start/cell_end
 // (dense over the grid, only occupied cells are ever written or reset),
 // neighbour lists (slot-major quads, see nbr_index; c < count[s]), and the
-// PCISPH predictor buffers xs[2] (float4), vs (float4), rpc (float2),
+// PCISPH predictor buffers xs[2] and vs (Soa3), rpc (float2),
 // fnp (float4 non-pressure force density), rho_x (float).
 #pragma once
 #include <cuda_runtime.h>
@@ -51,6 +51,16 @@ struct Tune {
 // Uniform per-scene constants, FP32 in normalised form (q = r^2/h^2, u = r/h)
 // so that no intermediate leaves FP32 range; derived on the host in FP64.
 struct Collider;     // colliders.cuh
+
+// A vector field split for gathers: a neighbour's vector is an 8-byte and a
+// 4-byte load. The sweeps' gathers are bound by L1 wavefronts -- a warp's 32
+// neighbours lie in ~10 lines of a float4 array, ~5 of the 8-byte one, ~3 of
+// the 4-byte one -- so the split costs fewer of them than one 16-byte load
+// (density pass at 1M particles alone: 55 against 66 us).
+struct Soa3 {
+    float2* xy;
+    float* z;
+};
 
 struct Params {
     int n;
@@ -126,6 +136,13 @@ struct Params {
     int* wall_count;
     uint32_t* wall_bits;
     int wall_blocks;
+    // SPH: the step's start positions and velocities in sorted order, as its
+    // sweeps gather them, written by the reorder; and the two z components
+    // once more beside the scalar that the pressure and set-up sums want with
+    // them: (z, pressure) and (v_z, density). The density passes write those.
+    Soa3 x0, v0;
+    float2* zp;
+    float2* vr;
     int dense_cells;    // the cell ranges cover every cell (the counting sort's), empty ones included
 };
 
@@ -151,26 +168,23 @@ inline void with_block(int bs, F&& f) {
 __host__ __device__ inline size_t nbr_index(int c, int n, int t) { return ((size_t)(c >> 2) * n + t) * 4 + (c & 3); }
 inline size_t nbr_list_ints(size_t n, int cap) { return n * (size_t)((cap + 3) & ~3); }
 
-// f(j) for the first cnt entries of slot t's list, in order; quads in
-// flight per thread: PSB_NBR_UNROLL (a build setting). 1 measured fastest
-// on B200 at 1M particles (density pass 119 us against 140 us at 2 and
-// 170 us at 4): the four gathers of one quad already overlap, and fewer
-// registers keep more warps resident.
-#ifndef PSB_NBR_UNROLL
-#define PSB_NBR_UNROLL 1
-#endif
-constexpr int kNbrUnroll = PSB_NBR_UNROLL;
+// f(j) for the first cnt entries of slot t's list, in order. The next quad's
+// load is issued behind the current quad's gathers, so a quad costs one
+// latency, not two (density pass at 1M particles alone: 61 against 66 us).
 template <class F>
 __device__ __forceinline__ void for_each_nbr(const int* __restrict__ list, int n, int t, int cnt, F&& f) {
     const int4* __restrict__ L = reinterpret_cast<const int4*>(list) + t;
+    int4 q = make_int4(0, 0, 0, 0);
+    if (cnt > 0) q = __ldg(L);
     int c = 0;
-#pragma unroll kNbrUnroll
     for (; c + 4 <= cnt; c += 4) {
-        const int4 q = __ldg(L + (size_t)(c >> 2) * n);
+        int4 next = q;
+        L += n;
+        if (c + 4 < cnt) next = __ldg(L);
         f(q.x); f(q.y); f(q.z); f(q.w);
+        q = next;
     }
     if (c < cnt) {
-        const int4 q = __ldg(L + (size_t)(c >> 2) * n);
         f(q.x);
         if (c + 1 < cnt) f(q.y);
         if (c + 2 < cnt) f(q.z);
@@ -307,37 +321,32 @@ void launch_reorder(cudaStream_t st, const Params& P, const uint32_t* keys, cons
                     float4* vap2, float2* rp2, int* ids2, uint32_t* cell_start, uint32_t* cell_end);
 void launch_reorder_pos(cudaStream_t st, const Params& P, const uint32_t* keys, const uint32_t* vals, const float4* pos,
                         const int* ids, float4* pos2, int* ids2, uint32_t* cell_start, uint32_t* cell_end);
-void launch_reorder_state(cudaStream_t st, int n, const uint32_t* vals, const float4* vel, const float4* vap,
+void launch_reorder_state(cudaStream_t st, const Params& P, const uint32_t* vals, const float4* vel, const float4* vap,
                           const float2* rp, float4* vel2, float4* vap2, float2* rp2);
 void launch_build_nbr(cudaStream_t st, const Params& P, const float4* pos, const uint32_t* keys,
                       const uint32_t* cell_start, const uint32_t* cell_end, int* counts, int* list, int* flags);
 // (sph.cu) The per-thread neighbour build of one config-profile scene with the
 // density pass at x folded in: lists, counts and flags as launch_build_nbr,
 // then density, pressure and features as launch_density_x.
-void launch_build_density(cudaStream_t st, const Params& P, const float4* pos, const float4* vel, const uint32_t* keys,
+void launch_build_density(cudaStream_t st, const Params& P, const float4* pos, const uint32_t* keys,
                           const uint32_t* cell_start, const uint32_t* cell_end, int* counts, int* list, int* flags,
                           float2* rp, float* rho_x, int zero_p, float p_scale, float* feats, int nfeat);
 
 // ---- launchers (sph.cu) ---------------------------------------------------
 // feats != nullptr: also the warm start's inputs f0 .. f(nfeat - 1), nfeat 6 or 7.
-void launch_density_x(cudaStream_t st, const Params& P, const float4* pos, const float4* vel, const int* counts,
-                      const int* list, float2* rp, float* rho_x, int zero_p, float p_scale = 1.f,
+void launch_density_x(cudaStream_t st, const Params& P, const int* counts, const int* list, float2* rp, float* rho_x, int zero_p, float p_scale = 1.f,
                       float* feats = nullptr, int nfeat = 7);
-void launch_wcsph_force(cudaStream_t st, const Params& P, const float4* pos, const float4* vel, const float4* vap,
-                        const float2* rp, const int* counts, const int* list, float4* pos_out, float4* vel_out,
+void launch_wcsph_force(cudaStream_t st, const Params& P, const float4* vap, const float2* rp, const int* counts, const int* list, float4* pos_out, float4* vel_out,
                         float4* vap_out, float4* fnp);
-void launch_pci_init(cudaStream_t st, const Params& P, const float4* pos, const float4* vel, const float4* vap,
-                     const float2* rp, const int* counts, const int* list, int warm, float4* fnp, float4* xs,
-                     float4* vs);
-void launch_pci_density(cudaStream_t st, const Params& P, const float4* xs, const float2* rp, const int* counts,
+void launch_pci_init(cudaStream_t st, const Params& P, const float4* vap, const float2* rp, const int* counts,
+                     const int* list, int warm, float4* fnp, Soa3 xs, Soa3 vs);
+void launch_pci_density(cudaStream_t st, const Params& P, Soa3 xs, const float2* rp, const int* counts,
                         const int* list, float2* rpc, unsigned long long* err_slot);
-void launch_pci_force_predict(cudaStream_t st, const Params& P, const float4* pos, const float4* vap,
-                              const float4* fnp, const float4* xs, const float2* rpc, const int* counts,
-                              const int* list, float4* xs_next, float4* vs, float2* rp);
-void launch_pci_commit(cudaStream_t st, const Params& P, const float4* xs, const float4* vs, const float2* rpc,
+void launch_pci_force_predict(cudaStream_t st, const Params& P, const float4* vap, const float4* fnp, Soa3 xs,
+                              const float2* rpc, const int* counts, const int* list, Soa3 xs_next, Soa3 vs, float2* rp);
+void launch_pci_commit(cudaStream_t st, const Params& P, Soa3 xs, Soa3 vs, const float2* rpc,
                        int have_density_pass, float4* pos, float4* vel, float4* vap, float2* rp);
-void launch_xsph(cudaStream_t st, const Params& P, const float4* xs, const float4* vs, const int* counts,
-                 const int* list, float4* vs_out);
+void launch_xsph(cudaStream_t st, const Params& P, Soa3 xs, Soa3 vs, const int* counts, const int* list, Soa3 vs_out);
 void launch_dem_step(cudaStream_t st, const Params& P, const float4* pos, const float4* vel, const int* counts,
                      const int* list, float4* pos_out, float4* vel_out, float4* vap_out, float4* force);
 // The force on each sphere (slot order) that the next step would apply
@@ -356,9 +365,8 @@ void launch_batch_decide(cudaStream_t st, int S, int min_it, int max_it, double 
 // The whole corrector loop of a config-profile scene or batch as one
 // cooperative launch (begin, then {density pass, decision, pressure-force
 // pass} until the decision ends it). Returns the launch's error.
-cudaError_t launch_corrector_persistent(cudaStream_t st, const Params& P, const float4* pos, const float4* vap,
-                                        const float4* fnp, float4* xs, float2* rp, float2* rpc, const int* counts,
-                                        const int* list, float4* vs, int S, int min_it, int max_it, double eta,
+cudaError_t launch_corrector_persistent(cudaStream_t st, const Params& P, const float4* vap, const float4* fnp, Soa3 xs,
+                                        float2* rp, float2* rpc, const int* counts, const int* list, Soa3 vs, int S, int min_it, int max_it, double eta,
                                         uint8_t* active, unsigned long long* err_scene, unsigned long long* err_hist,
                                         int* loop);
 
@@ -444,7 +452,9 @@ void launch_mc_polygonize_slots(cudaStream_t st, const double* node4, int nx, in
 constexpr int kMlpParams = 4737;   // the larger network's parameters: 7x64 + 64 + 64x64 + 64 + 64 + 1
 int mlp_inputs(int arch);
 int mlp_params(int arch);
-void launch_mlp_infer(cudaStream_t st, int arch, int n, const float* feats, const void* wbf, float p_scale, float2* rp);
+// The initial pressures into rp[].y and, where given, zp[].y.
+void launch_mlp_infer(cudaStream_t st, int arch, int n, const float* feats, const void* wbf, float p_scale, float2* rp,
+                      float2* zp);
 void launch_mlp_forward(cudaStream_t st, int arch, int n, const float* X, const void* wbf, float* y);
 // Training blocks per minibatch (at most) and the gradient partials they
 // write: kMlpGradBlocks rows of kMlpParams + 1 floats (the caller's buffer).

@@ -83,6 +83,17 @@ __device__ __forceinline__ float density_deviation(const Params& P, const Kahan&
 
 __device__ __forceinline__ float3 f3(float4 a) { return make_float3(a.x, a.y, a.z); }
 
+// Element j of a split vector field (plain loads: the persistent corrector
+// rewrites some of them between its passes).
+__device__ __forceinline__ float4 at(const Soa3& a, int j) {
+    const float2 xy = a.xy[j];
+    return make_float4(xy.x, xy.y, a.z[j], 0.f);
+}
+__device__ __forceinline__ void put(const Soa3& a, int t, float x, float y, float z) {
+    a.xy[t] = make_float2(x, y);
+    a.z[t] = z;
+}
+
 // The box faces that bound particle t (slot t): the scene's own (kernel
 // parameters, read where used) or, in a batch, its scene's table entry.
 template <bool BATCH> struct Faces;
@@ -242,29 +253,24 @@ __device__ __forceinline__ void ghost_pressure_pair(const Params& P, const NearF
 // particles within h of a face take (the walls are evaluated at xi). Kept
 // out of the main walk: a per-neighbour wall test there slows every
 // particle more than the separate walk costs the few near the faces.
-// The positions (ghost_density) and pressures (ghost_pressure) may be ones
-// that the persistent corrector rewrites between its passes, so they are
-// not declared __restrict__ here: a kernel whose own arguments are
-// restrict-qualified read-only arrays still gets read-only-cache loads.
 template <bool BATCH = false>
-__device__ __forceinline__ void ghost_density(const Params& P, int t, float4 xi, const float4* pos,
+__device__ __forceinline__ void ghost_density(const Params& P, int t, float4 xi, const Soa3& x,
                                               const int* __restrict__ list, int cnt, Kahan& acc) {
     NearFaces W;
     if (!near_faces(P, faces_of<BATCH>(P, t), xi, W)) return;
-    for_each_nbr(list, P.n, t, cnt, [&](const int j) { ghost_density_pair(P, W, xi, pos[j], acc); });
+    for_each_nbr(list, P.n, t, cnt, [&](const int j) { ghost_density_pair(P, W, xi, at(x, j), acc); });
 }
 
+// The neighbours at the step's start positions with the pressures of P.zp.
 template <bool BATCH = false>
 __device__ __forceinline__ void ghost_pressure(const Params& P, int t, float4 xi, float pVi,
-                                               const float4* __restrict__ pos, const float2* rp,
                                                const int* __restrict__ list, int cnt, float3& ap) {
     NearFaces W;
     if (!near_faces(P, faces_of<BATCH>(P, t), xi, W)) return;
     const float ir0 = 1.f / __fmul_rn(P.rho0, P.rho0);
     for_each_nbr(list, P.n, t, cnt, [&](const int j) {
-        const float4 xj = pos[j];
-        const float pj = rp[j].y;
-        ghost_pressure_pair(P, W, xi, xj, pVi, pj, ir0, ap);
+        const float2 xy = P.x0.xy[j], zp = P.zp[j];
+        ghost_pressure_pair(P, W, xi, make_float4(xy.x, xy.y, zp.x, 0.f), pVi, zp.y, ir0, ap);
     });
 }
 
@@ -405,15 +411,14 @@ struct DensityX {
     float3 gr = make_float3(0.f, 0.f, 0.f);
     float4 vi = make_float4(0.f, 0.f, 0.f, 0.f);
 
-    __device__ __forceinline__ void begin(const float4* __restrict__ vel, int t) {
-        if (FEAT) vi = vel[t];
+    __device__ __forceinline__ void begin(const Params& P, int t) {
+        if (FEAT) vi = at(P.v0, t);
     }
     // neighbour j at xj (r2 = dist2 of xi - xj); rp[j].y is the carried
     // pressure, which the pass writes back unchanged
-    __device__ __forceinline__ void pair(const Params& P, float4 xi, float4 xj, int j, const float4* __restrict__ vel,
-                                         const float2* __restrict__ rp) {
+    __device__ __forceinline__ void pair(const Params& P, float4 xi, float4 xj, int j, const float2* __restrict__ rp) {
         // the pair's other gathers issue with its position, ahead of the tests
-        const float4 vj = FEAT ? vel[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 vj = FEAT ? at(P.v0, j) : make_float4(0.f, 0.f, 0.f, 0.f);
         const float pj = SMOOTH_P ? rp[j].y : 0.f;
         const float dx = __fsub_rn(xi.x, xj.x), dy = __fsub_rn(xi.y, xj.y), dz = __fsub_rn(xi.z, xj.z);
         const float r2 = dist2(dx, dy, dz);
@@ -441,12 +446,11 @@ struct DensityX {
     // wall ghosts and boundary particles (config), then density, pressure
     // (EOS, or the carried / zeroed PCISPH pressure) and the features
     template <bool BATCH>
-    __device__ __forceinline__ void finish(const Params& P, int t, float4 xi, const float4* __restrict__ pos,
-                                           const int* __restrict__ list, int cnt, int count, float2* __restrict__ rp,
+    __device__ __forceinline__ void finish(const Params& P, int t, float4 xi, const int* __restrict__ list, int cnt, int count, float2* __restrict__ rp,
                                            float* __restrict__ rho_x, int zero_p, float p_scale,
                                            float* __restrict__ feats) {
         if (!REF) {
-            ghost_density<BATCH>(P, t, xi, pos, list, cnt, acc);
+            ghost_density<BATCH>(P, t, xi, P.x0, list, cnt, acc);
             if (!BATCH) boundary_density(P, t, xi, acc, P.bnd);
         }
         const float drho = density_deviation(P, acc);
@@ -480,6 +484,9 @@ struct DensityX {
         }
         rp[t] = make_float2(rho, p);
         rho_x[t] = rho;
+        // what the set-up or force sweep gathers beside the xy components
+        P.zp[t] = make_float2(xi.z, p);
+        P.vr[t] = make_float2(FEAT ? vi.z : P.v0.z[t], rho);
     }
 };
 
@@ -491,18 +498,17 @@ constexpr int kDensityThreads = 1536, kForceThreads = 1280, kInitThreads = 1152;
 
 template <bool REF, int NF, bool BATCH, int BS>
 __global__ void __launch_bounds__(BS, REF ? 1 : (NF ? kForceThreads : kDensityThreads) / BS)
-    k_density_x(Params P, const float4* __restrict__ pos, const float4* __restrict__ vel,
-                const int* __restrict__ counts, const int* __restrict__ list, float2* __restrict__ rp,
+    k_density_x(Params P, const int* __restrict__ counts, const int* __restrict__ list, float2* __restrict__ rp,
                 float* __restrict__ rho_x, int zero_p, float p_scale, float* __restrict__ feats) {
     for_each_slot<BS, !REF>(P, [&](const int t) {
         if (t < 0) return;
-        const float4 xi = pos[t];
+        const float4 xi = at(P.x0, t);
         const int count = counts[t];
         const int cnt = min(count, P.cap);
         DensityX<REF, NF> D;
-        D.begin(vel, t);
-        for_each_nbr(list, P.n, t, cnt, [&](const int j) { D.pair(P, xi, pos[j], j, vel, rp); });
-        D.template finish<BATCH>(P, t, xi, pos, list, cnt, count, rp, rho_x, zero_p, p_scale, feats);
+        D.begin(P, t);
+        for_each_nbr(list, P.n, t, cnt, [&](const int j) { D.pair(P, xi, at(P.x0, j), j, rp); });
+        D.template finish<BATCH>(P, t, xi, list, cnt, count, rp, rho_x, zero_p, p_scale, feats);
     });
 }
 
@@ -514,7 +520,6 @@ __global__ void __launch_bounds__(BS, REF ? 1 : (NF ? kForceThreads : kDensityTh
 // and boundary terms then walk the list this thread has just written.
 template <int NF, int BS>
 __global__ void __launch_bounds__(BS) k_build_density(Params P, const float4* __restrict__ pos,
-                                                          const float4* __restrict__ vel,
                                                           const uint32_t* __restrict__ keys,
                                                           const uint32_t* __restrict__ cell_start,
                                                           const uint32_t* __restrict__ cell_end,
@@ -528,20 +533,20 @@ __global__ void __launch_bounds__(BS) k_build_density(Params P, const float4* __
     if (valid) {
         const float4 pi = pos[t];
         DensityX<false, NF> D;
-        D.begin(vel, t);
+        D.begin(P, t);
         int* wq = list + nbr_index(0, P.n, t);
         const size_t qstride = (size_t)4 * (size_t)P.n;
         walk_neighbours<false>(P, t, pi, pos, keys, cell_start, cell_end, [&](uint32_t q, float4 pj) {
             if (cnt < P.cap) {
                 wq[cnt & 3] = (int)q;
-                D.pair(P, pi, pj, (int)q, vel, rp);
+                D.pair(P, pi, pj, (int)q, rp);
             }
             ++cnt;
             if ((cnt & 3) == 0 && cnt < P.cap) wq += qstride;
         });
         counts[t] = cnt;
         if (cnt > P.cap) atomicOr(&flags[0], 1);
-        D.template finish<false>(P, t, pi, pos, list, min(cnt, P.cap), cnt, rp, rho_x, zero_p, p_scale, feats);
+        D.template finish<false>(P, t, pi, list, min(cnt, P.cap), cnt, rp, rho_x, zero_p, p_scale, feats);
     }
     nbr_flags(cnt, flags);
 }
@@ -593,22 +598,20 @@ __device__ __forceinline__ void add_pair(const Params& P, PairSums& S, float4 xi
 
 template <bool REF, bool WITH_PRESSURE, bool BATCH = false>
 __device__ __forceinline__ PairSums pair_sums(const Params& P, int t, float4 xi, float4 vi, float2 rpi,
-                                              const float4* __restrict__ pos, const float4* __restrict__ vel,
-                                              const float2* __restrict__ rp, const int* __restrict__ counts,
-                                              const int* __restrict__ list) {
+                                              const int* __restrict__ counts, const int* __restrict__ list) {
     PairSums S;
     S.ap = S.fv = S.nrm = make_float3(0.f, 0.f, 0.f);
     S.fs = 0.f;
     const float pVi = WITH_PRESSURE ? pressure_volume<REF>(P, rpi) : 0.f;
     const int cnt = min(counts[t], P.cap);
     for_each_nbr(list, P.n, t, cnt, [&](const int j) {
-        const float4 xj = pos[j];       // the pair's three gathers, ahead of the tests
-        const float4 vj = vel[j];
-        const float2 rpj = rp[j];
-        add_pair<REF, WITH_PRESSURE>(P, S, xi, vi, pVi, xj, vj, rpj);
+        // the pair's four 8-byte gathers, ahead of the tests
+        const float2 xy = P.x0.xy[j], zp = P.zp[j], vxy = P.v0.xy[j], vr = P.vr[j];
+        add_pair<REF, WITH_PRESSURE>(P, S, xi, vi, pVi, make_float4(xy.x, xy.y, zp.x, 0.f),
+                                     make_float4(vxy.x, vxy.y, vr.x, 0.f), make_float2(vr.y, zp.y));
     });
     if (WITH_PRESSURE && !REF) {
-        ghost_pressure<BATCH>(P, t, xi, pVi, pos, rp, list, cnt, S.ap);
+        ghost_pressure<BATCH>(P, t, xi, pVi, list, cnt, S.ap);
         if (!BATCH) boundary_pressure(P, t, xi, pVi, S.ap);
     }
     return S;
@@ -634,9 +637,7 @@ __device__ __forceinline__ float3 nonpressure_force(const Params& P, const PairS
 
 // WCSPH: forces, leap-frog, walls and velocity interpolation in one sweep.
 template <bool REF>
-__global__ void __launch_bounds__(kBlock) k_wcsph_force(Params P, const float4* __restrict__ pos,
-                                                        const float4* __restrict__ vel, const float4* __restrict__ vap,
-                                                        const float2* __restrict__ rp, const int* __restrict__ counts,
+__global__ void __launch_bounds__(kBlock) k_wcsph_force(Params P, const float4* __restrict__ vap, const float2* __restrict__ rp, const int* __restrict__ counts,
                                                         const int* __restrict__ list, float4* __restrict__ pos_out,
                                                         float4* __restrict__ vel_out, float4* __restrict__ vap_out,
                                                         float4* __restrict__ fnp) {
@@ -657,20 +658,18 @@ __global__ void __launch_bounds__(kBlock) k_wcsph_force(Params P, const float4* 
     };
     for_each_slot<kBlock, !REF>(P, [&](const int t) {
         if (t < 0) return;
-        const float4 xi = pos[t], vi = vel[t];
+        const float4 xi = at(P.x0, t), vi = at(P.v0, t);
         const float2 rpi = rp[t];
-        integrate(t, xi, rpi, pair_sums<REF, true>(P, t, xi, vi, rpi, pos, vel, rp, counts, list));
+        integrate(t, xi, rpi, pair_sums<REF, true>(P, t, xi, vi, rpi, counts, list));
     });
 }
 
 // PCISPH set-up sweep: non-pressure forces at x (and, for a warm start, the
 // pressure acceleration of the carried pressure), then the first prediction.
 template <bool REF, bool WARM, bool BATCH, int BS>
-__global__ void __launch_bounds__(BS, REF || !WARM ? 1 : kInitThreads / BS) k_pci_init(Params P, const float4* __restrict__ pos,
-                                                     const float4* __restrict__ vel, const float4* __restrict__ vap,
-                                                     const float2* __restrict__ rp, const int* __restrict__ counts,
-                                                     const int* __restrict__ list, float4* __restrict__ fnp,
-                                                     float4* __restrict__ xs, float4* __restrict__ vs) {
+__global__ void __launch_bounds__(BS, REF || !WARM ? 1 : kInitThreads / BS) k_pci_init(
+    Params P, const float4* __restrict__ vap, const float2* __restrict__ rp, const int* __restrict__ counts,
+    const int* __restrict__ list, float4* __restrict__ fnp, Soa3 xs, Soa3 vs) {
     auto predict = [&](const int t, const float4 xi, const float2 rpi, const PairSums& S) {
         const float4 vh = vap[t];
         const float3 f = nonpressure_force<REF>(P, S, rpi.x);
@@ -681,14 +680,14 @@ __global__ void __launch_bounds__(BS, REF || !WARM ? 1 : kInitThreads / BS) k_pc
         const float3 a = make_float3(f.x * ir + ap * S.ap.x + aw.x, f.y * ir + ap * S.ap.y + aw.y,
                                      f.z * ir + ap * S.ap.z + aw.z);
         const float3 v = make_float3(vh.x + a.x * P.dt, vh.y + a.y * P.dt, vh.z + a.z * P.dt);
-        vs[t] = make_float4(v.x, v.y, v.z, 0.f);
-        xs[t] = make_float4(xi.x + v.x * P.dt, xi.y + v.y * P.dt, xi.z + v.z * P.dt, 0.f);
+        put(vs, t, v.x, v.y, v.z);
+        put(xs, t, xi.x + v.x * P.dt, xi.y + v.y * P.dt, xi.z + v.z * P.dt);
     };
     for_each_slot<BS, !REF && WARM>(P, [&](const int t) {
         if (t < 0) return;
-        const float4 xi = pos[t], vi = vel[t];
+        const float4 xi = at(P.x0, t), vi = at(P.v0, t);
         const float2 rpi = rp[t];
-        predict(t, xi, rpi, pair_sums<REF, WARM, BATCH>(P, t, xi, vi, rpi, pos, vel, rp, counts, list));
+        predict(t, xi, rpi, pair_sums<REF, WARM, BATCH>(P, t, xi, vi, rpi, counts, list));
     });
 }
 
@@ -708,20 +707,21 @@ __device__ __forceinline__ double pci_density_finish(const Params& P, int t, con
         p = fmaxf(0.f, __fmaf_rn(P.k_delta, drho, p));
     }
     rpc[t] = make_float2(rho, p);
+    if (!REF) P.zp[t] = make_float2(P.x0.z[t], p);     // as the pressure-force pass gathers it
     return (double)drho / P.rho0_d;
 }
 
 // The density pass for sorted particle t (t < P.n, its scene still iterating).
-template <bool REF, bool BATCH, class F4, class F2, class F2o>
-__device__ __forceinline__ double pci_density_at(const Params& P, int t, F4 xs, F2 rp, const int* __restrict__ counts,
+template <bool REF, bool BATCH, class F2, class F2o>
+__device__ __forceinline__ double pci_density_at(const Params& P, int t, const Soa3& xs, F2 rp, const int* __restrict__ counts,
                                                  const int* __restrict__ list, F2o rpc) {
-    const float4 xi = xs[t];
+    const float4 xi = at(xs, t);
     const int cnt = min(counts[t], P.cap);
     Kahan acc;
     float3 T1 = make_float3(0.f, 0.f, 0.f);
     float T2 = 0.f;
     for_each_nbr(list, P.n, t, cnt, [&](const int j) {
-        const float4 xj = xs[j];
+        const float4 xj = at(xs, j);
         const float dx = __fsub_rn(xi.x, xj.x), dy = __fsub_rn(xi.y, xj.y), dz = __fsub_rn(xi.z, xj.z);
         const float r2 = dist2(dx, dy, dz);
         const float q = __fmul_rn(r2, P.inv_h2);
@@ -743,6 +743,17 @@ __device__ __forceinline__ double pci_density_at(const Params& P, int t, F4 xs, 
     return pci_density_finish<REF>(P, t, acc, T1, T2, rp, rpc);
 }
 
+// Raises *slot to err (ordered encoding; -1e300: no error). The slot only
+// grows during a pass, so a value at or below what it already holds needs no
+// atomic. Atomics on one sector retire one after another in L2, and a batch's
+// scene words share a few sectors: its density pass took 218 us with an
+// atomic from every warp (64 scenes, 2.3M particles), 171 us with the test.
+__device__ __forceinline__ void raise_error(unsigned long long* slot, double err) {
+    if (!(err > -1e300)) return;
+    const unsigned long long e = order_double(err);
+    if (e > *(volatile unsigned long long*)slot) atomicMax(slot, e);
+}
+
 // The max of the pass's errors. Batch: per scene (P.err_scene); a warp
 // inside one scene reduces first, one straddling two or more reduces per
 // lane; sc = the slot's scene, -1 for none. Single scene (the persistent
@@ -756,9 +767,9 @@ __device__ __forceinline__ void reduce_error(const Params& P, int sc, double err
         if (__all_sync(0xffffffffu, sc == sc0 || sc < 0)) {
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) err = fmax(err, __shfl_xor_sync(0xffffffffu, err, o));
-            if ((threadIdx.x & 31) == 0 && sc0 >= 0 && err > -1e300) atomicMax(&P.err_scene[sc0], order_double(err));
-        } else if (sc >= 0 && err > -1e300) {
-            atomicMax(&P.err_scene[sc], order_double(err));
+            if ((threadIdx.x & 31) == 0 && sc0 >= 0) raise_error(&P.err_scene[sc0], err);
+        } else if (sc >= 0) {
+            raise_error(&P.err_scene[sc], err);
         }
     } else {
 #pragma unroll
@@ -768,7 +779,7 @@ __device__ __forceinline__ void reduce_error(const Params& P, int sc, double err
         if (threadIdx.x == 0) {
             double m = s_err[0];
             for (int w = 1; w < BS / 32; ++w) m = fmax(m, s_err[w]);
-            if (m > -1e300) atomicMax(err_slot, order_double(m));
+            raise_error(err_slot, m);
         }
         __syncthreads();
     }
@@ -789,12 +800,12 @@ __device__ __forceinline__ void warp_max_error(const Params& P, int sc, double e
     } else {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) err = fmax(err, __shfl_xor_sync(0xffffffffu, err, o));
-        if ((threadIdx.x & 31) == 0 && err > -1e300) atomicMax(err_slot, order_double(err));
+        if ((threadIdx.x & 31) == 0) raise_error(err_slot, err);
     }
 }
 
 template <bool REF, bool BATCH, int BS>
-__global__ void __launch_bounds__(BS, REF ? 1 : kDensityThreads / BS) k_pci_density(Params P, const float4* __restrict__ xs,
+__global__ void __launch_bounds__(BS, REF ? 1 : kDensityThreads / BS) k_pci_density(Params P, Soa3 xs,
                                                         const float2* __restrict__ rp, const int* __restrict__ counts,
                                                         const int* __restrict__ list, float2* __restrict__ rpc,
                                                         unsigned long long* __restrict__ err_slot) {
@@ -829,10 +840,9 @@ __device__ __forceinline__ void add_pressure_pair(const Params& P, float4 xi, fl
 // xs_next[t] and vs[t], and the candidate pressure ri committed to rp[t].
 template <bool REF, bool BATCH>
 __device__ __forceinline__ void pci_force_finish(const Params& P, int t, float2 ri, float3 acc,
-                                                 const float4* __restrict__ pos, const float4* __restrict__ vap,
-                                                 const float4* __restrict__ fnp, float4* xs_next, float4* vs,
-                                                 float2* rp) {
-    const float4 x0 = pos[t], vh = vap[t], f = fnp[t];
+                                                 const float4* __restrict__ vap, const float4* __restrict__ fnp,
+                                                 const Soa3& xs_next, const Soa3& vs, float2* rp) {
+    const float4 x0 = at(P.x0, t), vh = vap[t], f = fnp[t];
     const float3 aw = wall_accel<REF, BATCH>(P, t, x0, vh);
     const float ir = 1.f / ri.x;
     auto accel = [&](float fc, float ac, float wc) {     // f/rho + k_grad sum + wall
@@ -840,36 +850,41 @@ __device__ __forceinline__ void pci_force_finish(const Params& P, int t, float2 
     };
     const float3 a = make_float3(accel(f.x, acc.x, aw.x), accel(f.y, acc.y, aw.y), accel(f.z, acc.z, aw.z));
     const float3 v = make_float3(__fmaf_rn(a.x, P.dt, vh.x), __fmaf_rn(a.y, P.dt, vh.y), __fmaf_rn(a.z, P.dt, vh.z));
-    vs[t] = make_float4(v.x, v.y, v.z, 0.f);
-    xs_next[t] = make_float4(__fmaf_rn(v.x, P.dt, x0.x), __fmaf_rn(v.y, P.dt, x0.y), __fmaf_rn(v.z, P.dt, x0.z), 0.f);
+    put(vs, t, v.x, v.y, v.z);
+    put(xs_next, t, __fmaf_rn(v.x, P.dt, x0.x), __fmaf_rn(v.y, P.dt, x0.y), __fmaf_rn(v.z, P.dt, x0.z));
     rp[t] = ri;
 }
 
 // The pressure-force pass for sorted particle t (t < P.n, its scene still
 // iterating).
-template <bool REF, bool BATCH, class F4, class F2>
-__device__ __forceinline__ void pci_force_at(const Params& P, int t, const float4* __restrict__ pos,
-                                             const float4* __restrict__ vap, const float4* __restrict__ fnp, F4 xs,
-                                             F2 rpc, const int* __restrict__ counts, const int* __restrict__ list,
-                                             float4* xs_next, float4* vs, float2* rp) {
-    const float4 xi = REF ? xs[t] : pos[t];
+template <bool REF, bool BATCH, class F2>
+__device__ __forceinline__ void pci_force_at(const Params& P, int t, const float4* __restrict__ vap,
+                                             const float4* __restrict__ fnp, const Soa3& xs, F2 rpc,
+                                             const int* __restrict__ counts, const int* __restrict__ list,
+                                             const Soa3& xs_next, const Soa3& vs, float2* rp) {
+    const float4 xi = REF ? at(xs, t) : at(P.x0, t);
     const float2 ri = rpc[t];
     const float ir0 = 1.f / __fmul_rn(P.rho0, P.rho0);
     const float pVi = REF ? ri.y / __fmul_rn(ri.x, ri.x) : __fmul_rn(ri.y, ir0);
     const int cnt = min(counts[t], P.cap);
     float3 acc = make_float3(0.f, 0.f, 0.f);
     for_each_nbr(list, P.n, t, cnt, [&](const int j) {
-        // both gathers of the pair issue before its distance test, so a pair
-        // costs one dependent load after the list, not two
-        const float4 xj = REF ? xs[j] : pos[j];
-        const float2 rj = rpc[j];
-        add_pressure_pair<REF>(P, xi, xj, pVi, rj, ir0, acc);
+        // the pair's gathers issue before its distance test, so a pair costs
+        // one dependent load after the list, not two
+        if (REF) {
+            const float4 xj = at(xs, j);
+            const float2 rj = rpc[j];
+            add_pressure_pair<REF>(P, xi, xj, pVi, rj, ir0, acc);
+        } else {
+            const float2 xy = P.x0.xy[j], zp = P.zp[j];
+            add_pressure_pair<REF>(P, xi, make_float4(xy.x, xy.y, zp.x, 0.f), pVi, zp, ir0, acc);
+        }
     });
     if (!REF) {
-        ghost_pressure<BATCH>(P, t, xi, pVi, pos, &rpc[0], list, cnt, acc);
+        ghost_pressure<BATCH>(P, t, xi, pVi, list, cnt, acc);
         if (!BATCH) boundary_pressure(P, t, xi, pVi, acc);
     }
-    pci_force_finish<REF, BATCH>(P, t, ri, acc, pos, vap, fnp, xs_next, vs, rp);
+    pci_force_finish<REF, BATCH>(P, t, ri, acc, vap, fnp, xs_next, vs, rp);
 }
 
 // PCISPH pressure-force pass fused with the next prediction; commits the
@@ -881,18 +896,13 @@ __device__ __forceinline__ void pci_force_at(const Params& P, int t, const float
 // with rho* in p/rho^2 the force feeds back on the density; under a 0.64 m
 // column either one makes the corrector diverge.
 template <bool REF, bool BATCH, int BS>
-__global__ void __launch_bounds__(BS, REF ? 1 : kForceThreads / BS) k_pci_force_predict(Params P, const float4* __restrict__ pos,
-                                                              const float4* __restrict__ vap,
-                                                              const float4* __restrict__ fnp,
-                                                              const float4* __restrict__ xs,
-                                                              const float2* __restrict__ rpc,
-                                                              const int* __restrict__ counts,
-                                                              const int* __restrict__ list, float4* __restrict__ xs_next,
-                                                              float4* __restrict__ vs, float2* __restrict__ rp) {
+__global__ void __launch_bounds__(BS, REF ? 1 : kForceThreads / BS) k_pci_force_predict(
+    Params P, const float4* __restrict__ vap, const float4* __restrict__ fnp, Soa3 xs, const float2* __restrict__ rpc,
+    const int* __restrict__ counts, const int* __restrict__ list, Soa3 xs_next, Soa3 vs, float2* __restrict__ rp) {
     if (!BATCH && P.active && !P.active[0]) return;      // single scene, corrector decided on the device: converged
     for_each_slot<BS, !REF>(P, [&](const int t) {
         if (t < 0 || (BATCH && !P.active[P.slot_scene[t]])) return;     // its scene has converged
-        pci_force_at<REF, BATCH>(P, t, pos, vap, fnp, xs, rpc, counts, list, xs_next, vs, rp);
+        pci_force_at<REF, BATCH>(P, t, vap, fnp, xs, rpc, counts, list, xs_next, vs, rp);
     });
 }
 
@@ -908,15 +918,10 @@ __global__ void __launch_bounds__(BS, REF ? 1 : kForceThreads / BS) k_pci_force_
 // Five resident blocks of 256 per SM (at most 48 registers, no spills),
 // the occupancy of the separate pressure-force pass.
 template <bool BATCH, int BS>
-__global__ void __launch_bounds__(BS, 5) k_corrector_persistent(Params P, const float4* __restrict__ pos,
-                                                                 const float4* __restrict__ vap,
-                                                                 const float4* __restrict__ fnp, float4* xs, float2* rp,
-                                                                 float2* rpc, const int* __restrict__ counts,
-                                                                 const int* __restrict__ list, float4* vs,
-                                                                 unsigned long long* err_slot, int S, int min_it,
-                                                                 int max_it, double eta, uint8_t* active,
-                                                                 unsigned long long* err_scene,
-                                                                 unsigned long long* err_hist, int* loop) {
+__global__ void __launch_bounds__(BS, 5) k_corrector_persistent(
+    Params P, const float4* __restrict__ vap, const float4* __restrict__ fnp, Soa3 xs, float2* rp, float2* rpc,
+    const int* __restrict__ counts, const int* __restrict__ list, Soa3 vs, unsigned long long* err_slot, int S, int min_it,
+    int max_it, double eta, uint8_t* active, unsigned long long* err_scene, unsigned long long* err_hist, int* loop) {
     cg::grid_group grid = cg::this_grid();
     __shared__ double s_err[BS / 32];
     __shared__ int s_any;
@@ -931,7 +936,7 @@ __global__ void __launch_bounds__(BS, 5) k_corrector_persistent(Params P, const 
             double err = -1e300;
             const int sc = BATCH && t < P.n ? (int)P.slot_scene[t] : -1;
             const volatile uint8_t* act = active;
-            if (t < P.n && (!BATCH || act[sc])) err = pci_density_at<false, BATCH>(P, t, (const float4*)xs, (const float2*)rp, counts, list, rpc);
+            if (t < P.n && (!BATCH || act[sc])) err = pci_density_at<false, BATCH>(P, t, xs, (const float2*)rp, counts, list, rpc);
             if (BATCH) reduce_error<true, BS>(P, sc, err, err_slot, s_err);
             else emax = fmax(emax, err);
         }
@@ -946,8 +951,7 @@ __global__ void __launch_bounds__(BS, 5) k_corrector_persistent(Params P, const 
             if (t >= P.n) continue;
             const volatile uint8_t* act = active;
             if (!act[BATCH ? (int)P.slot_scene[t] : 0]) continue;
-            pci_force_at<false, BATCH>(P, t, pos, vap, fnp, (const float4*)xs, (const float2*)rpc, counts, list, xs,
-                                       vs, rp);
+            pci_force_at<false, BATCH>(P, t, vap, fnp, xs, (const float2*)rpc, counts, list, xs, vs, rp);
         }
         if (!cont) break;
         grid.sync();
@@ -957,14 +961,13 @@ __global__ void __launch_bounds__(BS, 5) k_corrector_persistent(Params P, const 
 // Commit of the last prediction, walls, collision objects (COLL: the start
 // position pos[t] is read before it is overwritten), velocity interpolation.
 template <bool BATCH, bool COLL>
-__global__ void __launch_bounds__(kBlock) k_pci_commit(Params P, const float4* __restrict__ xs,
-                                                       const float4* __restrict__ vs, const float2* __restrict__ rpc,
+__global__ void __launch_bounds__(kBlock) k_pci_commit(Params P, Soa3 xs, Soa3 vs, const float2* __restrict__ rpc,
                                                        int have_density_pass, float4* __restrict__ pos,
                                                        float4* __restrict__ vel, float4* __restrict__ vap,
                                                        float2* __restrict__ rp) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= P.n) return;
-    float3 x = f3(xs[t]), v = f3(vs[t]);
+    float3 x = f3(at(xs, t)), v = f3(at(vs, t));
     const float4 vh = vap[t];
     box_project<BATCH>(P, t, x, v);
     if constexpr (COLL) {
@@ -984,24 +987,22 @@ __global__ void __launch_bounds__(kBlock) k_pci_commit(Params P, const float4* _
 // config PCISPH: v_i + xsph sum_j (m/rho0) W_ij (v_j - v_i) over the list at
 // x*, W the poly6 kernel (m W = k_rho (1-q)^3). Positions are not moved.
 template <int BS>
-__global__ void __launch_bounds__(BS) k_xsph(Params P, const float4* __restrict__ xs,
-                                                 const float4* __restrict__ vs, const int* __restrict__ counts,
-                                                 const int* __restrict__ list, float4* __restrict__ vs_out) {
+__global__ void __launch_bounds__(BS) k_xsph(Params P, Soa3 xs, Soa3 vs, const int* __restrict__ counts,
+                                                 const int* __restrict__ list, Soa3 vs_out) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= P.n) return;
-    const float4 xi = xs[t], vi = vs[t];
+    const float4 xi = at(xs, t), vi = at(vs, t);
     const int cnt = min(counts[t], P.cap);
     float3 dv = make_float3(0.f, 0.f, 0.f);
     for_each_nbr(list, P.n, t, cnt, [&](const int j) {
-        const float4 xj = xs[j];
+        const float4 xj = at(xs, j), vj = at(vs, j);
         const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
         const float q = dist2(dx, dy, dz) * P.inv_h2;
         if (q >= 1.f) return;
-        const float4 vj = vs[j];
         const float w = (1.f - q) * (1.f - q) * (1.f - q);
         dv.x += w * (vj.x - vi.x); dv.y += w * (vj.y - vi.y); dv.z += w * (vj.z - vi.z);
     });
-    vs_out[t] = make_float4(vi.x + P.xsph_k * dv.x, vi.y + P.xsph_k * dv.y, vi.z + P.xsph_k * dv.z, 0.f);
+    put(vs_out, t, vi.x + P.xsph_k * dv.x, vi.y + P.xsph_k * dv.y, vi.z + P.xsph_k * dv.z);
 }
 
 inline int grid_of(int n) { return (n + kBlock - 1) / kBlock; }
@@ -1026,15 +1027,14 @@ inline Params with_walls(const Params& P, bool ghosts = true) {
     return Q;
 }
 
-void launch_density_x(cudaStream_t st, const Params& P, const float4* pos, const float4* vel, const int* counts,
-                      const int* list, float2* rp, float* rho_x, int zero_p, float p_scale, float* feats, int nfeat) {
+void launch_density_x(cudaStream_t st, const Params& P, const int* counts, const int* list, float2* rp, float* rho_x,
+                      int zero_p, float p_scale, float* feats, int nfeat) {
     if (P.n <= 0) return;
     with_block(P.tune.density_block, [&](auto B) {
         constexpr int BS = decltype(B)::value;
         const Params Q = with_walls<BS>(P);
         auto go = [&](auto kernel) {
-            kernel<<<blocks_of<BS>(P.n) + Q.wall_blocks, BS, 0, st>>>(Q, pos, vel, counts, list, rp, rho_x, zero_p,
-                                                                      p_scale, feats);
+            kernel<<<blocks_of<BS>(P.n) + Q.wall_blocks, BS, 0, st>>>(Q, counts, list, rp, rho_x, zero_p, p_scale, feats);
         };
         const int nf = feats ? (nfeat > 6 ? 7 : 6) : 0;
         if (P.ref) go(k_density_x<true, 0, false, BS>);
@@ -1048,15 +1048,15 @@ void launch_density_x(cudaStream_t st, const Params& P, const float4* pos, const
     });
 }
 
-void launch_build_density(cudaStream_t st, const Params& P, const float4* pos, const float4* vel, const uint32_t* keys,
+void launch_build_density(cudaStream_t st, const Params& P, const float4* pos, const uint32_t* keys,
                           const uint32_t* cell_start, const uint32_t* cell_end, int* counts, int* list, int* flags,
                           float2* rp, float* rho_x, int zero_p, float p_scale, float* feats, int nfeat) {
     if (P.n <= 0) return;
     with_block(P.tune.nbr_block, [&](auto B) {
         constexpr int BS = decltype(B)::value;
         auto go = [&](auto kernel) {
-            kernel<<<blocks_of<BS>(P.n), BS, 0, st>>>(P, pos, vel, keys, cell_start, cell_end, counts, list, flags, rp,
-                                                      rho_x, zero_p, p_scale, feats);
+            kernel<<<blocks_of<BS>(P.n), BS, 0, st>>>(P, pos, keys, cell_start, cell_end, counts, list, flags, rp, rho_x,
+                                                      zero_p, p_scale, feats);
         };
         const int nf = feats ? (nfeat > 6 ? 7 : 6) : 0;
         if (nf == 7) go(k_build_density<7, BS>);
@@ -1065,25 +1065,23 @@ void launch_build_density(cudaStream_t st, const Params& P, const float4* pos, c
     });
 }
 
-void launch_wcsph_force(cudaStream_t st, const Params& P, const float4* pos, const float4* vel, const float4* vap,
-                        const float2* rp, const int* counts, const int* list, float4* pos_out, float4* vel_out,
+void launch_wcsph_force(cudaStream_t st, const Params& P, const float4* vap, const float2* rp, const int* counts,
+                        const int* list, float4* pos_out, float4* vel_out,
                         float4* vap_out, float4* fnp) {
     if (P.n <= 0) return;
     const Params Q = with_walls<kBlock>(P);
     auto kernel = P.ref ? k_wcsph_force<true> : k_wcsph_force<false>;
-    kernel<<<grid_of(P.n) + Q.wall_blocks, kBlock, 0, st>>>(Q, pos, vel, vap, rp, counts, list, pos_out, vel_out,
-                                                            vap_out, fnp);
+    kernel<<<grid_of(P.n) + Q.wall_blocks, kBlock, 0, st>>>(Q, vap, rp, counts, list, pos_out, vel_out, vap_out, fnp);
 }
 
-void launch_pci_init(cudaStream_t st, const Params& P, const float4* pos, const float4* vel, const float4* vap,
-                     const float2* rp, const int* counts, const int* list, int warm, float4* fnp, float4* xs,
-                     float4* vs) {
+void launch_pci_init(cudaStream_t st, const Params& P, const float4* vap, const float2* rp, const int* counts,
+                     const int* list, int warm, float4* fnp, Soa3 xs, Soa3 vs) {
     if (P.n <= 0) return;
     with_block(P.tune.init_block, [&](auto B) {
         constexpr int BS = decltype(B)::value;
         const Params Q = with_walls<BS>(P, warm != 0);
         auto go = [&](auto kernel) {
-            kernel<<<blocks_of<BS>(P.n) + Q.wall_blocks, BS, 0, st>>>(Q, pos, vel, vap, rp, counts, list, fnp, xs, vs);
+            kernel<<<blocks_of<BS>(P.n) + Q.wall_blocks, BS, 0, st>>>(Q, vap, rp, counts, list, fnp, xs, vs);
         };
         if (P.ref) { if (warm) go(k_pci_init<true, true, false, BS>); else go(k_pci_init<true, false, false, BS>); }
         else if (P.scenes) { if (warm) go(k_pci_init<false, true, true, BS>); else go(k_pci_init<false, false, true, BS>); }
@@ -1092,8 +1090,8 @@ void launch_pci_init(cudaStream_t st, const Params& P, const float4* pos, const 
     });
 }
 
-void launch_pci_density(cudaStream_t st, const Params& P, const float4* xs, const float2* rp, const int* counts,
-                        const int* list, float2* rpc, unsigned long long* err_slot) {
+void launch_pci_density(cudaStream_t st, const Params& P, Soa3 xs, const float2* rp, const int* counts, const int* list,
+                        float2* rpc, unsigned long long* err_slot) {
     if (P.n <= 0) return;
     with_block(P.tune.pci_density_block, [&](auto B) {
         constexpr int BS = decltype(B)::value;
@@ -1107,9 +1105,8 @@ void launch_pci_density(cudaStream_t st, const Params& P, const float4* xs, cons
     });
 }
 
-cudaError_t launch_corrector_persistent(cudaStream_t st, const Params& P, const float4* pos, const float4* vap,
-                                        const float4* fnp, float4* xs, float2* rp, float2* rpc, const int* counts,
-                                        const int* list, float4* vs, int S, int min_it, int max_it, double eta,
+cudaError_t launch_corrector_persistent(cudaStream_t st, const Params& P, const float4* vap, const float4* fnp, Soa3 xs,
+                                        float2* rp, float2* rpc, const int* counts, const int* list, Soa3 vs, int S, int min_it, int max_it, double eta,
                                         uint8_t* active, unsigned long long* err_scene, unsigned long long* err_hist,
                                         int* loop) {
     constexpr int BS = 256;
@@ -1134,22 +1131,21 @@ cudaError_t launch_corrector_persistent(cudaStream_t st, const Params& P, const 
         attr[0].val.cooperative = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, kernel, P, pos, vap, fnp, xs, rp, rpc, counts, list, vs, err_slot, S, min_it,
+        return cudaLaunchKernelEx(&cfg, kernel, P, vap, fnp, xs, rp, rpc, counts, list, vs, err_slot, S, min_it,
                                   max_it, eta, active, err_scene, err_hist, loop);
     };
     if (P.ref) return cudaErrorInvalidValue;
     return P.scenes ? go(k_corrector_persistent<true, BS>) : go(k_corrector_persistent<false, BS>);
 }
-void launch_pci_force_predict(cudaStream_t st, const Params& P, const float4* pos, const float4* vap,
-                              const float4* fnp, const float4* xs, const float2* rpc, const int* counts,
-                              const int* list, float4* xs_next, float4* vs, float2* rp) {
+
+void launch_pci_force_predict(cudaStream_t st, const Params& P, const float4* vap, const float4* fnp, Soa3 xs,
+                              const float2* rpc, const int* counts, const int* list, Soa3 xs_next, Soa3 vs, float2* rp) {
     if (P.n <= 0) return;
     with_block(P.tune.force_block, [&](auto B) {
         constexpr int BS = decltype(B)::value;
         const Params Q = with_walls<BS>(P);
         auto go = [&](auto kernel) {
-            kernel<<<blocks_of<BS>(P.n) + Q.wall_blocks, BS, 0, st>>>(Q, pos, vap, fnp, xs, rpc, counts, list, xs_next,
-                                                                      vs, rp);
+            kernel<<<blocks_of<BS>(P.n) + Q.wall_blocks, BS, 0, st>>>(Q, vap, fnp, xs, rpc, counts, list, xs_next, vs, rp);
         };
         if (P.ref) go(k_pci_force_predict<true, false, BS>);
         else if (P.scenes) go(k_pci_force_predict<false, true, BS>);
@@ -1157,8 +1153,7 @@ void launch_pci_force_predict(cudaStream_t st, const Params& P, const float4* po
     });
 }
 
-void launch_xsph(cudaStream_t st, const Params& P, const float4* xs, const float4* vs, const int* counts,
-                 const int* list, float4* vs_out) {
+void launch_xsph(cudaStream_t st, const Params& P, Soa3 xs, Soa3 vs, const int* counts, const int* list, Soa3 vs_out) {
     if (P.n <= 0) return;
     with_block(P.tune.xsph_block, [&](auto B) {
         constexpr int BS = decltype(B)::value;
@@ -1166,7 +1161,7 @@ void launch_xsph(cudaStream_t st, const Params& P, const float4* xs, const float
     });
 }
 
-void launch_pci_commit(cudaStream_t st, const Params& P, const float4* xs, const float4* vs, const float2* rpc,
+void launch_pci_commit(cudaStream_t st, const Params& P, Soa3 xs, Soa3 vs, const float2* rpc,
                        int have_density_pass, float4* pos, float4* vel, float4* vap, float2* rp) {
     if (P.n <= 0) return;
     if (P.scenes)
