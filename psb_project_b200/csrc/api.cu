@@ -149,12 +149,12 @@ struct psb_ctx {
     int sel_cap = 0;
     // iso field and marching cubes (grown on demand)
     double* iso = nullptr;
-    uint32_t* mc_cube = nullptr;   // per-node triangle counts -> offsets
-    uint32_t* mc_edge = nullptr;   // per-edge flags -> vertex offsets
-    uint32_t* mc_scratch = nullptr;
+    uint16_t* mc_case = nullptr;   // per node: edge flags and cube case
+    uint32_t* mc_first = nullptr;  // per node: its first vertex
+    uint32_t* mc_block = nullptr;  // per block of nodes: vertices, then triangles -> offsets; then the scan's scratch
     float* mc_vert = nullptr;
     int32_t* mc_tri = nullptr;
-    long long iso_cap = 0, mc_cube_cap = 0, mc_edge_cap = 0, mc_scratch_cap = 0, mc_vert_cap = 0, mc_tri_cap = 0;
+    long long iso_cap = 0, mc_case_cap = 0, mc_first_cap = 0, mc_block_cap = 0, mc_vert_cap = 0, mc_tri_cap = 0;
     bool mc_table = false;
     // batched scenes (psb_create_batch); a single scene has nscenes == 1 and batch == false
     bool batch = false;
@@ -330,7 +330,7 @@ void free_all(psb_ctx* c) {
     cudaFreeHost(c->h_slab);
     cudaFree(c->bnd_vel); cudaFree(c->bnd_fext); cudaFree(c->bnd_pred); cudaFree(c->bnd_react);
     cudaFree(c->ds_X); cudaFree(c->ds_T); cudaFree(c->sel);
-    cudaFree(c->iso); cudaFree(c->mc_cube); cudaFree(c->mc_edge); cudaFree(c->mc_scratch); cudaFree(c->mc_vert);
+    cudaFree(c->iso); cudaFree(c->mc_case); cudaFree(c->mc_first); cudaFree(c->mc_block); cudaFree(c->mc_vert);
     cudaFree(c->mc_tri);
     cudaFree(c->diag_rows); cudaFree(c->diag_out);
     cudaFree(c->bnd_raw); cudaFree(c->bnd_sorted); cudaFree(c->bnd_ids); cudaFree(c->bnd_iota); cudaFree(c->bnd_w);
@@ -1768,6 +1768,7 @@ int iso_on_device(psb_ctx* c, const psb_iso_grid* g, double level, psb::IsoParam
         Q.ring = (int)std::floor(1.0 / g->scale);
     } else {
         Q.ring = 1;      // cell >= h
+        Q.r = h;
         Q.inv_r2 = 1.0 / (h * h);
         Q.k_colour = 315.0 * c->sc.mass / (64.0 * 3.14159265358979323846 * h * h * h);
     }
@@ -1777,7 +1778,8 @@ int iso_on_device(psb_ctx* c, const psb_iso_grid* g, double level, psb::IsoParam
     Params P = c->P;
     P.n = c->n;
     timed(c, "iso_field", [&] {
-        psb::launch_iso_field(c->stream, Q, P, c->pos[c->cs], c->rp[c->cr], c->cell_start, c->cell_end, c->iso);
+        psb::launch_iso_field(c->stream, Q, P, c->pos[c->cs], c->rp[c->cr], c->cell_start, c->cell_end,
+                              reinterpret_cast<double*>(c->xs[0].xy), c->iso);     // x* is free between steps
     });
     return cuda_check(c, cudaGetLastError(), "iso field");
 }
@@ -2247,22 +2249,20 @@ int psb_extract_surface(psb_ctx* c, const psb_iso_grid* g, double level, float* 
         psb::mc_upload_table(st);
         c->mc_table = true;
     }
-    // counts per cube (indexed by its lowest node) and per node edge, one
-    // trailing zero each: their in-place exclusive scans end in the totals
-    const long long cube_n = nn + 1, edge_n = 3 * nn + 1;
-    PSB_TRY(grow(c, &c->mc_cube, &c->mc_cube_cap, cube_n));
-    PSB_TRY(grow(c, &c->mc_edge, &c->mc_edge_cap, edge_n));
-    PSB_TRY(grow(c, &c->mc_scratch, &c->mc_scratch_cap, psb::scan_scratch_words(edge_n)));
-    timed(c, "mc_classify", [&] { psb::launch_mc_classify(st, Q, c->iso, c->mc_cube, c->mc_edge); });
+    const long long nb = psb::mc_blocks(Q), words = psb::scan_scratch_words(2 * (nb + 1));
+    PSB_TRY(grow(c, &c->mc_case, &c->mc_case_cap, nn));
+    PSB_TRY(grow(c, &c->mc_first, &c->mc_first_cap, nn));
+    PSB_TRY(grow(c, &c->mc_block, &c->mc_block_cap, 2 * (nb + 1) + words));
+    uint32_t *verts = c->mc_block, *tris = verts + nb + 1, *scratch = tris + nb + 1;
+    timed(c, "mc_classify", [&] { psb::launch_mc_classify(st, Q, c->iso, c->mc_case, verts, tris); });
     timed(c, "mc_scan", [&] {
-        psb::scan_exclusive_u32(st, edge_n, c->mc_edge, c->mc_scratch);
-        psb::scan_exclusive_u32(st, cube_n, c->mc_cube, c->mc_scratch);
+        psb::scan_exclusive_u32(st, 2 * (nb + 1), verts, scratch);      // both in one: the triangles' behind the vertices'
     });
     uint32_t tot[2] = {0, 0};
-    PSB_TRY(cuda_check(c, cudaMemcpyAsync(&tot[0], c->mc_edge + 3 * nn, 4, cudaMemcpyDeviceToHost, st), "mc"));
-    PSB_TRY(cuda_check(c, cudaMemcpyAsync(&tot[1], c->mc_cube + nn, 4, cudaMemcpyDeviceToHost, st), "mc"));
+    PSB_TRY(cuda_check(c, cudaMemcpyAsync(&tot[0], verts + nb, 4, cudaMemcpyDeviceToHost, st), "mc"));
+    PSB_TRY(cuda_check(c, cudaMemcpyAsync(&tot[1], tris + nb, 4, cudaMemcpyDeviceToHost, st), "mc"));
     PSB_TRY(cuda_check(c, cudaStreamSynchronize(st), "mc"));
-    const int64_t nv = tot[0], nt = tot[1];
+    const int64_t nv = tot[0], nt = tot[1] - tot[0];
     const bool fits = (!vertices || nv <= *n_vertices) && (!triangles || nt <= *n_triangles);
     *n_vertices = nv;
     *n_triangles = nt;
@@ -2270,7 +2270,7 @@ int psb_extract_surface(psb_ctx* c, const psb_iso_grid* g, double level, float* 
     if (!fits) return fail(c, PSB_EINVAL, "psb_extract_surface: output buffers too small (counts returned)");
     PSB_TRY(grow(c, &c->mc_vert, &c->mc_vert_cap, 3 * (nv > 0 ? nv : 1)));
     PSB_TRY(grow(c, &c->mc_tri, &c->mc_tri_cap, 3 * (nt > 0 ? nt : 1)));
-    timed(c, "mc_emit", [&] { psb::launch_mc_emit(st, Q, c->iso, c->mc_edge, c->mc_cube, c->mc_vert, c->mc_tri); });
+    timed(c, "mc_emit", [&] { psb::launch_mc_emit(st, Q, c->iso, c->mc_case, verts, tris, c->mc_first, c->mc_vert, c->mc_tri); });
     if (vertices && nv)
         PSB_TRY(cuda_check(c, cudaMemcpyAsync(vertices, c->mc_vert, sizeof(float) * 3 * nv, cudaMemcpyDeviceToHost, st), "mc"));
     if (triangles && nt)

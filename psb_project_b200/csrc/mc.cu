@@ -16,7 +16,7 @@
 // and welds vertices on the host in O(V^2) (SurfaceSPH.cpp:120-186); here
 // every active grid edge owns one vertex (its index is the edge's rank in an
 // exclusive scan), so the mesh is welded by construction, and triangles are
-// written compacted through a second scan.
+// written compacted through a second one.
 //
 // The triangle table is generated here, not copied: for each of the 256
 // cases the active edges of every cube face are joined into segments (a face
@@ -27,6 +27,8 @@
 // corners, so neighbouring cubes agree on every shared face and the surface
 // is closed wherever the field is.
 #include <cuda_runtime.h>
+#include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstdint>
@@ -48,7 +50,25 @@ constexpr int kFace[6][4] = {{0, 1, 2, 3}, {4, 5, 6, 7}, {0, 3, 7, 4}, {1, 2, 6,
 __constant__ int c_corner[8][3] = PSB_MC_CORNERS;
 __constant__ int c_edge[12][2] = PSB_MC_EDGES;
 
+// For each edge, 5 bits: the corner offset of its lower node (x, y, z) and its axis.
+constexpr uint64_t edge_pack() {
+    uint64_t p = 0;
+    for (int e = 0; e < 12; ++e) {
+        const int* a = kCorner[kEdge[e][0]];
+        const int* b = kCorner[kEdge[e][1]];
+        const int* lo = a[0] + a[1] + a[2] <= b[0] + b[1] + b[2] ? a : b;
+        const int* hi = lo == a ? b : a;
+        const int axis = hi[0] != lo[0] ? 0 : (hi[1] != lo[1] ? 1 : 2);
+        p |= (uint64_t)(lo[0] | lo[1] << 1 | lo[2] << 2 | axis << 3) << (5 * e);
+    }
+    return p;
+}
+constexpr uint64_t kEdgePack = edge_pack();
+
 __constant__ int8_t c_tri[256][kMcMaxTri * 3];
+// The same table in global memory: the lanes of a warp read different cases,
+// which constant memory serves one at a time.
+__device__ int8_t g_tri[256][kMcMaxTri * 3];
 __constant__ uint8_t c_ntri[256];
 
 int edge_of(int a, int b) {
@@ -132,106 +152,246 @@ void mc_build_table(uint8_t ntri[256], int8_t tri[256][kMcMaxTri * 3]) {
 namespace {
 
 // ---- iso field ----------------------------------------------------------------
-template <bool REF>
-__global__ void k_iso_field(IsoParams Q, Params P, const float4* __restrict__ pos, const float2* __restrict__ rp,
-                            const uint32_t* __restrict__ cell_start, const uint32_t* __restrict__ cell_end,
-                            double* __restrict__ iso) {
-    const long long node = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long nn = (long long)Q.dims[0] * Q.dims[1] * Q.dims[2];
-    if (node >= nn) return;
-    const int ix = (int)(node % Q.dims[0]);
-    const int iy = (int)((node / Q.dims[0]) % Q.dims[1]);
-    const int iz = (int)(node / ((long long)Q.dims[0] * Q.dims[1]));
-    const double px = Q.origin[0] + ix * Q.spacing[0];
-    const double py = Q.origin[1] + iy * Q.spacing[1];
-    const double pz = Q.origin[2] + iz * Q.spacing[2];
-    // particle-grid cell of the node, as the reference computes it
-    const int I = (int)floor((px - (double)P.g.gx) / (double)P.g.cell);
-    const int J = (int)floor((py - (double)P.g.gy) / (double)P.g.cell);
-    const int K = (int)floor((pz - (double)P.g.gz) / (double)P.g.cell);
+// k_colour / rho_j of every particle (config profile): the division once a
+// particle rather than once a (node, particle) pair.
+__global__ void k_iso_weight(int n, double k_colour, const float2* __restrict__ rp, double* __restrict__ w) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < n) w[t] = k_colour / (double)rp[t].x;
+}
+
+// A thread takes a brick of E^3 nodes, a warp 4 x 2 x 4 threads, a block 1 x 2
+// x 2 warps. The cells of a grid row are adjacent in slot order, so the rings
+// of a thread's nodes are a few contiguous slot ranges. The sums are FP64, but
+// 85% of a ring's particles lie outside the radius: those are dropped by an
+// FP32 test against the nearest of the thread's nodes, with a margin over its
+// own rounding (32 candidates to a mask), and only the rest, in order, see the
+// FP64 distances. Config profile: a particle within the radius lies in the
+// node's ring, so going over the union of several rings adds nothing to any
+// of them, and a candidate is loaded once for eight nodes. The field was bound
+// by L1 wavefronts (93% of the data pipe with a node a thread, FP64 17%):
+// 128^3 nodes over 262,144 particles took 518 us in node order with every
+// candidate in FP64, 475 with the FP32 test, 412 with a warp's nodes in a
+// brick, 273 with 2 x 2 x 1 nodes a thread, 247 with 2 x 2 x 2. Nodes further
+// apart than half a cell share too little and take a thread each, and so do
+// the nodes of grids too small to fill the chip with eighths (64^3: 77 us
+// with a node a thread, 112 with eight; 80^3: 85 with eight, 117 for the kernel
+// before) and the reference profile's, whose ring may cut the radius off.
+constexpr long long kIsoBrickNodes = 393216;
+
+template <bool REF, int E>
+__global__ void __launch_bounds__(128) k_iso_field(IsoParams Q, Params P, const float4* __restrict__ pos,
+                                                   const double* __restrict__ weight,
+                                                   const uint32_t* __restrict__ cell_start,
+                                                   const uint32_t* __restrict__ cell_end, double* __restrict__ iso) {
+    const int l = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const unsigned bx = (Q.dims[0] + 4 * E - 1) / (4 * E), by = (Q.dims[1] + 4 * E - 1) / (4 * E);
+    const int ix = ((int)(blockIdx.x % bx) * 4 + (l & 3)) * E;
+    const int iy = ((int)(blockIdx.x / bx % by) * 4 + (wp & 1) * 2 + (l >> 2 & 1)) * E;
+    const int iz = ((int)(blockIdx.x / (bx * by)) * 8 + (wp >> 1) * 4 + (l >> 3)) * E;
+    if (ix >= Q.dims[0] || iy >= Q.dims[1] || iz >= Q.dims[2]) return;
+    double px[E], py[E], pz[E];
+    float fx[E], fy[E], fz[E];
+    int lo_x = INT_MAX, hi_x = INT_MIN, lo_y = INT_MAX, hi_y = INT_MIN, lo_z = INT_MAX, hi_z = INT_MIN;
+    // particle-grid cells of the nodes, as the reference computes them
+    float far = 0.f;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        px[e] = Q.origin[0] + (ix + e) * Q.spacing[0];
+        py[e] = Q.origin[1] + (iy + e) * Q.spacing[1];
+        const int I = (int)floor((px[e] - (double)P.g.gx) / (double)P.g.cell);
+        const int J = (int)floor((py[e] - (double)P.g.gy) / (double)P.g.cell);
+        pz[e] = Q.origin[2] + (iz + e) * Q.spacing[2];
+        const int K = (int)floor((pz[e] - (double)P.g.gz) / (double)P.g.cell);
+        lo_x = min(lo_x, I); hi_x = max(hi_x, I);
+        lo_y = min(lo_y, J); hi_y = max(hi_y, J);
+        lo_z = min(lo_z, K); hi_z = max(hi_z, K);
+        fx[e] = (float)px[e];
+        fy[e] = (float)py[e];
+        fz[e] = (float)pz[e];
+        far = fmaxf(far, fmaxf(fmaxf(fabsf(fx[e]), fabsf(fy[e])), fabsf(fz[e])));
+    }
     const int ring = Q.ring;
-    double acc = 0.0;
-    for (int i = I - ring; i <= I + ring; ++i) {
-        if (i < 0 || i >= P.g.nx) continue;
-        for (int j = J - ring; j <= J + ring; ++j) {
-            if (j < 0 || j >= P.g.ny) continue;
-            for (int k = K - ring; k <= K + ring; ++k) {
-                if (k < 0 || k >= P.g.nz) continue;
-                const uint32_t c = (uint32_t)i + (uint32_t)j * P.g.nx + (uint32_t)k * P.g.nx * P.g.ny;
-                const uint32_t s = cell_start[c];
-                if (s == kEmpty) continue;
-                const uint32_t e = cell_end[c];
-                for (uint32_t t = s; t < e; ++t) {
+    const int a0 = max(lo_x - ring, 0), a1 = min(hi_x + ring, P.g.nx - 1);
+    double acc[E][E][E] = {};
+    // radius of the FP32 test: a node and a particle within the ring are each
+    // rounded by at most 2^-24 of their largest coordinate
+    far += (float)(ring + 1) * P.g.cell;
+    const float reach = (float)Q.r * 1.0001f + far * 5e-7f;
+    const float r2 = -(reach * reach);
+    const int k1 = min(hi_z + ring, P.g.nz - 1), j1 = min(hi_y + ring, P.g.ny - 1);
+    for (int k = max(lo_z - ring, 0); k <= k1 && a0 <= a1; ++k) {
+        for (int j = max(lo_y - ring, 0); j <= j1; ++j) {
+            const uint32_t row = (uint32_t)j * P.g.nx + (uint32_t)k * P.g.nx * P.g.ny;
+            uint32_t lo, hi;
+            if (P.dense_cells) {
+                lo = cell_start[row + a0];
+                hi = cell_end[row + a1];
+            } else {
+                row_range(cell_start, cell_end, row, a0, a1, lo, hi);
+            }
+            for (; lo < hi; lo += 32u) {
+                const uint32_t m = min(hi - lo, 32u);
+                uint32_t mask = 0u;
+                for (uint32_t c = 0; c < m; c += 2) {
+#pragma unroll
+                    for (uint32_t u = 0; u < 2; ++u) {
+                        const float4 x = pos[lo + c + u];       // padded past the last particle
+                        float best = INFINITY;
+#pragma unroll
+                        for (int g = 0; g < E; ++g) {
+                            const float dz = fz[g] - x.z;
+                            const float bz = __fmaf_rn(dz, dz, r2);
+#pragma unroll
+                            for (int f = 0; f < E; ++f) {
+                                const float dy = fy[f] - x.y;
+                                const float b = __fmaf_rn(dy, dy, bz);
+#pragma unroll
+                                for (int e = 0; e < E; ++e) {
+                                    const float dx = fx[e] - x.x;
+                                    const float d = __fmaf_rn(dx, dx, b);
+                                    best = E == 1 ? d : fminf(best, d);
+                                }
+                            }
+                        }
+                        // a NaN position stays in, as in the FP64 test (fminf passes over it)
+                        const bool in = !(best >= 0.f && best < INFINITY);
+                        mask = mask << 1 | (in ? 1u : 0u);
+                    }
+                }
+                mask = (mask << (32u - ((m + 1u) & ~1u))) & (kEmpty << (32u - m));
+                uint32_t t = lo;
+                while (mask) {
+                    const int z = __clz((int)mask);
+                    mask = (mask << z) << 1;
+                    t += (uint32_t)z;
                     const float4 x = pos[t];
-                    const double dx = px - x.x, dy = py - x.y, dz = pz - x.z;
-                    const double d2 = dx * dx + dy * dy + dz * dz;
                     if (REF) {
+                        const double dx = px[0] - x.x, dy = py[0] - x.y, dz = pz[0] - x.z;
+                        const double d2 = dx * dx + dy * dy + dz * dz;
                         // d = length(pos1 - pos2); (1/powf(r,6)) * powf(r*r - d*d, 3) in float
                         const double d = sqrt(d2);
-                        if (!(d <= Q.r)) continue;
-                        const float term = (1.f / powf((float)Q.r, 6.f)) * powf((float)(Q.r * Q.r - d * d), 3.f);
-                        acc += (double)term;
+                        if (d <= Q.r) {
+                            const float term = (1.f / powf((float)Q.r, 6.f)) * powf((float)(Q.r * Q.r - d * d), 3.f);
+                            acc[0][0][0] += (double)term;
+                        }
                     } else {
-                        const double q = d2 * Q.inv_r2;
-                        if (q >= 1.0) continue;
-                        const double w = 1.0 - q;
-                        acc += Q.k_colour * (w * w * w) / (double)rp[t].x;
+                        const double wt = weight[t];
+#pragma unroll
+                        for (int g = 0; g < E; ++g) {
+                            const double dz = pz[g] - x.z, dz2 = dz * dz;
+#pragma unroll
+                            for (int f = 0; f < E; ++f) {
+                                const double dy = py[f] - x.y, dy2 = dy * dy + dz2;
+#pragma unroll
+                                for (int e = 0; e < E; ++e) {
+                                    const double dx = px[e] - x.x;
+                                    const double q = (dx * dx + dy2) * Q.inv_r2;
+                                    if (!(q >= 1.0)) {
+                                        const double w = 1.0 - q;
+                                        acc[g][f][e] += w * w * w * wt;
+                                    }
+                                }
+                            }
+                        }
                     }
+                    ++t;
                 }
             }
         }
     }
-    iso[node] = acc;
+#pragma unroll
+    for (int g = 0; g < E; ++g)
+#pragma unroll
+        for (int f = 0; f < E; ++f)
+#pragma unroll
+            for (int e = 0; e < E; ++e)
+                if (ix + e < Q.dims[0] && iy + f < Q.dims[1] && iz + g < Q.dims[2])
+                    iso[ix + e + (size_t)Q.dims[0] * (iy + f + (size_t)Q.dims[1] * (iz + g))] = acc[g][f][e];
 }
 
 // ---- marching cubes -----------------------------------------------------------
-__device__ __forceinline__ int cube_case(const IsoParams& Q, const double* __restrict__ iso, int x, int y, int z) {
-    const long long sx = 1, sy = Q.dims[0], sz = (long long)Q.dims[0] * Q.dims[1];
-    const long long b = x + y * sy + z * sz;
-    int cs = 0;
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        const long long o = b + c_corner[c][0] * sx + c_corner[c][1] * sy + c_corner[c][2] * sz;
-        if (iso[o] <= Q.level) cs |= 1 << c;
+// Nodes and their coordinates fit 30 bits (psb_extract_surface's limit).
+struct NodeAt {
+    int x, y, z;
+};
+__device__ __forceinline__ NodeAt node_at(const IsoParams& Q, unsigned node) {
+    const unsigned plane = node / (unsigned)Q.dims[0];
+    return {(int)(node - plane * Q.dims[0]), (int)(plane % (unsigned)Q.dims[1]), (int)(plane / (unsigned)Q.dims[1])};
+}
+
+// The active edges (+x, +y, +z, bits 0-2) and the cube case (bits 8-15) of a
+// node, from the corners of the cube it is the lowest node of. A node on a
+// far face has no cube: case 0.
+__device__ __forceinline__ unsigned node_case(const IsoParams& Q, const double* __restrict__ iso, unsigned node,
+                                              const NodeAt& p) {
+    const unsigned sy = Q.dims[0], sz = sy * Q.dims[1];
+    const bool ix = p.x + 1 < Q.dims[0], iy = p.y + 1 < Q.dims[1], iz = p.z + 1 < Q.dims[2];
+    auto in = [&](unsigned o) { return iso[o] <= Q.level; };
+    const bool c0 = in(node);
+    const bool cx = ix ? in(node + 1) : c0, cy = iy ? in(node + sy) : c0, cz = iz ? in(node + sz) : c0;
+    unsigned r = (c0 != cx ? 1u : 0u) | (c0 != cy ? 2u : 0u) | (c0 != cz ? 4u : 0u);
+    if (ix && iy && iz) {       // corners 0..7: 000 100 101 001 010 110 111 011
+        unsigned cs = (c0 ? 1u : 0u) | (cx ? 2u : 0u) | (in(node + 1 + sz) ? 4u : 0u) | (cz ? 8u : 0u) |
+                      (cy ? 16u : 0u) | (in(node + 1 + sy) ? 32u : 0u) | (in(node + 1 + sy + sz) ? 64u : 0u) |
+                      (in(node + sy + sz) ? 128u : 0u);
+        r |= cs << 8;
     }
-    return cs;
+    return r;
 }
 
-__device__ __forceinline__ bool edge_active(const IsoParams& Q, const double* __restrict__ iso, long long node,
-                                            int axis, int x, int y, int z) {
-    const int c = axis == 0 ? x : (axis == 1 ? y : z);
-    if (c + 1 >= Q.dims[axis]) return false;
-    const long long step = axis == 0 ? 1 : (axis == 1 ? Q.dims[0] : (long long)Q.dims[0] * Q.dims[1]);
-    return (iso[node] <= Q.level) != (iso[node + step] <= Q.level);
-}
+constexpr int kMcBlock = 256;
 
-// Per cube (indexed by its lowest node): triangle count. Per node: 0/1 for
-// each of its +x, +y, +z edges crossing the level. Both arrays carry one
-// trailing zero so that their in-place exclusive scans end in the totals.
-__global__ void k_mc_classify(IsoParams Q, const double* __restrict__ iso, uint32_t* __restrict__ cube_tris,
-                              uint32_t* __restrict__ edge_flag) {
-    const long long node = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long nn = (long long)Q.dims[0] * Q.dims[1] * Q.dims[2];
-    if (node == nn) { cube_tris[nn] = 0; edge_flag[3 * nn] = 0; }
-    if (node >= nn) return;
-    const int x = (int)(node % Q.dims[0]);
-    const int y = (int)((node / Q.dims[0]) % Q.dims[1]);
-    const int z = (int)(node / ((long long)Q.dims[0] * Q.dims[1]));
+// Exclusive rank of (a, b) over the block in thread order, and the block's
+// totals; both below 2^16 (at most 3 and 10 a thread).
+__device__ __forceinline__ uint2 block_rank(unsigned a, unsigned b, uint2& total) {
+    __shared__ unsigned s_warp[kMcBlock / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned v = a | b << 16;
+    unsigned x = v;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) edge_flag[3 * node + a] = edge_active(Q, iso, node, a, x, y, z) ? 1u : 0u;
-    uint32_t nt = 0;
-    if (x + 1 < Q.dims[0] && y + 1 < Q.dims[1] && z + 1 < Q.dims[2]) nt = c_ntri[cube_case(Q, iso, x, y, z)];
-    cube_tris[node] = nt;
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) s_warp[warp] = x;
+    __syncthreads();
+    unsigned before = 0, all = 0;
+#pragma unroll
+    for (int w = 0; w < kMcBlock / 32; ++w) {
+        if (w < warp) before += s_warp[w];
+        all += s_warp[w];
+    }
+    total = make_uint2(all & 0xffffu, all >> 16);
+    const unsigned e = before + x - v;
+    return make_uint2(e & 0xffffu, e >> 16);
 }
 
-// Global edge id (node * 3 + axis) of cube edge e of the cube at (x, y, z).
-__device__ __forceinline__ long long global_edge(const IsoParams& Q, int x, int y, int z, int e) {
-    const int a = c_edge[e][0], b = c_edge[e][1];
-    const int lo = (c_corner[a][0] + c_corner[a][1] + c_corner[a][2]) <= (c_corner[b][0] + c_corner[b][1] + c_corner[b][2]) ? a : b;
-    const int hi = lo == a ? b : a;
-    const int axis = c_corner[hi][0] != c_corner[lo][0] ? 0 : (c_corner[hi][1] != c_corner[lo][1] ? 1 : 2);
-    const long long nx = x + c_corner[lo][0], ny = y + c_corner[lo][1], nz = z + c_corner[lo][2];
-    return 3 * (nx + ny * Q.dims[0] + nz * (long long)Q.dims[0] * Q.dims[1]) + axis;
+// Pass 1: every node's edge flags and cube case, and the vertices and
+// triangles of each block of nodes. The offsets are scanned over the blocks
+// alone (a word each for 256 nodes); pass 2 ranks inside a block again. A
+// count per edge and per cube, scanned in full, was 33 MB of counters on
+// 128^3 nodes: 31 us to write, 75 to scan and 85 for an emission pass with a
+// thread per edge.
+__global__ void __launch_bounds__(kMcBlock) k_mc_classify(IsoParams Q, const double* __restrict__ iso,
+                                                          uint16_t* __restrict__ cases,
+                                                          uint32_t* __restrict__ block_vert,
+                                                          uint32_t* __restrict__ block_tri) {
+    const unsigned nn = (unsigned)Q.dims[0] * Q.dims[1] * Q.dims[2];
+    const unsigned node = blockIdx.x * kMcBlock + threadIdx.x;
+    unsigned nv = 0, nt = 0;
+    if (node < nn) {
+        const unsigned r = node_case(Q, iso, node, node_at(Q, node));
+        cases[node] = (uint16_t)r;
+        nv = __popc(r & 7u);
+        nt = c_ntri[r >> 8];
+    }
+    uint2 total;
+    block_rank(nv, nt, total);
+    if (threadIdx.x == 0) {
+        block_vert[blockIdx.x] = total.x;
+        block_tri[blockIdx.x] = total.y;
+        if (blockIdx.x == gridDim.x - 1) block_vert[gridDim.x] = block_tri[gridDim.x] = 0u;     // their scans' totals
+    }
 }
 
 // vertexInterpolate_MarchingCube (MarchingCube_Kernel.cu:143-155)
@@ -243,42 +403,59 @@ __device__ __forceinline__ double interp(double level, double v1, double v2, dou
     return p1 + mu * (p2 - p1);
 }
 
-__global__ void k_mc_vertices(IsoParams Q, const double* __restrict__ iso, const uint32_t* __restrict__ edge_off,
-                              float* __restrict__ vert) {
-    const long long ge = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long nn = (long long)Q.dims[0] * Q.dims[1] * Q.dims[2];
-    if (ge >= 3 * nn) return;
-    const long long node = ge / 3;
-    const int axis = (int)(ge % 3);
-    const int x = (int)(node % Q.dims[0]);
-    const int y = (int)((node / Q.dims[0]) % Q.dims[1]);
-    const int z = (int)(node / ((long long)Q.dims[0] * Q.dims[1]));
-    if (!edge_active(Q, iso, node, axis, x, y, z)) return;
-    const long long step = axis == 0 ? 1 : (axis == 1 ? Q.dims[0] : (long long)Q.dims[0] * Q.dims[1]);
-    const double v1 = iso[node], v2 = iso[node + step];
-    const double p[3] = {Q.origin[0] + x * Q.spacing[0], Q.origin[1] + y * Q.spacing[1], Q.origin[2] + z * Q.spacing[2]};
-    const uint32_t o = edge_off[ge];
-    for (int d = 0; d < 3; ++d) {
-        const double q = d == axis ? p[d] + Q.spacing[d] : p[d];
-        vert[3 * (size_t)o + d] = (float)interp(Q.level, v1, v2, p[d], q);
+// Pass 2: the vertices of a node's active edges, and the index of its first.
+__global__ void __launch_bounds__(kMcBlock) k_mc_vertices(IsoParams Q, const double* __restrict__ iso,
+                                                          const uint16_t* __restrict__ cases,
+                                                          const uint32_t* __restrict__ block_vert,
+                                                          uint32_t* __restrict__ first, float* __restrict__ vert) {
+    const unsigned nn = (unsigned)Q.dims[0] * Q.dims[1] * Q.dims[2];
+    const unsigned node = blockIdx.x * kMcBlock + threadIdx.x;
+    if (block_vert[blockIdx.x + 1] == block_vert[blockIdx.x]) return;       // no active edge in the block
+    const unsigned edges = node < nn ? cases[node] & 7u : 0u;
+    uint2 total;
+    uint32_t o = block_vert[blockIdx.x] + block_rank(__popc(edges), 0u, total).x;
+    if (!edges) return;
+    first[node] = o;
+    const NodeAt n = node_at(Q, node);
+    const double p[3] = {Q.origin[0] + n.x * Q.spacing[0], Q.origin[1] + n.y * Q.spacing[1],
+                         Q.origin[2] + n.z * Q.spacing[2]};
+    const unsigned step[3] = {1u, (unsigned)Q.dims[0], (unsigned)Q.dims[0] * Q.dims[1]};
+    const double v1 = iso[node];
+#pragma unroll
+    for (int axis = 0; axis < 3; ++axis) {
+        if (!(edges >> axis & 1u)) continue;
+        const double v2 = iso[node + step[axis]];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const double q = d == axis ? p[d] + Q.spacing[d] : p[d];
+            vert[3 * (size_t)o + d] = (float)interp(Q.level, v1, v2, p[d], q);
+        }
+        ++o;
     }
 }
 
-__global__ void k_mc_triangles(IsoParams Q, const double* __restrict__ iso, const uint32_t* __restrict__ tri_off,
-                               const uint32_t* __restrict__ edge_off, int32_t* __restrict__ tris) {
-    const long long node = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long nn = (long long)Q.dims[0] * Q.dims[1] * Q.dims[2];
-    if (node >= nn) return;
-    const int x = (int)(node % Q.dims[0]);
-    const int y = (int)((node / Q.dims[0]) % Q.dims[1]);
-    const int z = (int)(node / ((long long)Q.dims[0] * Q.dims[1]));
-    if (x + 1 >= Q.dims[0] || y + 1 >= Q.dims[1] || z + 1 >= Q.dims[2]) return;
-    const int cs = cube_case(Q, iso, x, y, z);
-    const uint32_t base = tri_off[node];
+// Vertex index of cube edge e of the cube whose lowest node is `node`: the
+// edge's own lower node's first vertex plus its active edges of lower axes.
+__device__ __forceinline__ uint32_t edge_vertex(const IsoParams& Q, const uint16_t* __restrict__ cases,
+                                                const uint32_t* __restrict__ first, unsigned node, int e) {
+    const unsigned p = (unsigned)(kEdgePack >> (5 * e));
+    const unsigned m = node + (p & 1u) + (p >> 1 & 1u) * Q.dims[0] + (p >> 2 & 1u) * (unsigned)Q.dims[0] * Q.dims[1];
+    return first[m] + __popc(cases[m] & ((1u << (p >> 3 & 3u)) - 1u));
+}
+
+__global__ void __launch_bounds__(kMcBlock) k_mc_triangles(IsoParams Q, const uint16_t* __restrict__ cases,
+                                                           const uint32_t* __restrict__ block_tri,
+                                                           const uint32_t* __restrict__ first,
+                                                           int32_t* __restrict__ tris) {
+    const unsigned nn = (unsigned)Q.dims[0] * Q.dims[1] * Q.dims[2];
+    const unsigned node = blockIdx.x * kMcBlock + threadIdx.x;
+    if (block_tri[blockIdx.x + 1] == block_tri[blockIdx.x]) return;
+    const int cs = node < nn ? cases[node] >> 8 : 0;
     const int nt = c_ntri[cs];
-    for (int t = 0; t < nt; ++t)
-        for (int k = 0; k < 3; ++k)
-            tris[3 * ((size_t)base + t) + k] = (int32_t)edge_off[global_edge(Q, x, y, z, c_tri[cs][3 * t + k])];
+    uint2 total;
+    // the triangles' counts are scanned behind the vertices': less their total
+    int32_t* __restrict__ out = tris + 3 * (size_t)(block_tri[blockIdx.x] - block_tri[0] + block_rank(0u, nt, total).y);
+    for (int k = 0; k < 3 * nt; ++k) out[k] = (int32_t)edge_vertex(Q, cases, first, node, g_tri[cs][k]);
 }
 
 // polygonize_MarchingCube_Kernel (MarchingCube_Kernel.cu:36-139) on the
@@ -389,6 +566,7 @@ void mc_upload_table(cudaStream_t st) {
     }
     cudaMemcpyToSymbolAsync(c_ntri, ntri, sizeof(ntri), 0, cudaMemcpyHostToDevice, st);
     cudaMemcpyToSymbolAsync(c_tri, tri, sizeof(tri), 0, cudaMemcpyHostToDevice, st);
+    cudaMemcpyToSymbolAsync(g_tri, tri, sizeof(tri), 0, cudaMemcpyHostToDevice, st);
 }
 
 long long scan_scratch_words(long long n) {
@@ -415,24 +593,32 @@ void scan_exclusive_u32(cudaStream_t st, long long n, uint32_t* data, uint32_t* 
 }
 
 void launch_iso_field(cudaStream_t st, const IsoParams& Q, const Params& P, const float4* pos, const float2* rp,
-                      const uint32_t* cell_start, const uint32_t* cell_end, double* iso) {
+                      const uint32_t* cell_start, const uint32_t* cell_end, double* weight, double* iso) {
     const long long nn = (long long)Q.dims[0] * Q.dims[1] * Q.dims[2];
     if (nn <= 0) return;
-    if (P.ref) k_iso_field<true><<<blocks_for(nn, 256), 256, 0, st>>>(Q, P, pos, rp, cell_start, cell_end, iso);
-    else k_iso_field<false><<<blocks_for(nn, 256), 256, 0, st>>>(Q, P, pos, rp, cell_start, cell_end, iso);
+    if (!P.ref) k_iso_weight<<<blocks_for(P.n, 256), 256, 0, st>>>(P.n, Q.k_colour, rp, weight);
+    const double widest = std::max(Q.spacing[0], std::max(Q.spacing[1], Q.spacing[2]));
+    const int edge = !P.ref && nn >= kIsoBrickNodes && 2.0 * widest <= (double)P.g.cell ? 2 : 1;
+    auto kernel = P.ref ? k_iso_field<true, 1> : edge == 2 ? k_iso_field<false, 2> : k_iso_field<false, 1>;
+    const long long xy = 4 * edge, z = 8 * edge;
+    const long long blocks = ((Q.dims[0] + xy - 1) / xy) * ((Q.dims[1] + xy - 1) / xy) * ((Q.dims[2] + z - 1) / z);
+    kernel<<<(unsigned)blocks, 128, 0, st>>>(Q, P, pos, weight, cell_start, cell_end, iso);
 }
 
-void launch_mc_classify(cudaStream_t st, const IsoParams& Q, const double* iso, uint32_t* cube_tris,
-                        uint32_t* edge_flag) {
-    const long long nn = (long long)Q.dims[0] * Q.dims[1] * Q.dims[2];
-    k_mc_classify<<<blocks_for(nn + 1, 256), 256, 0, st>>>(Q, iso, cube_tris, edge_flag);
+long long mc_blocks(const IsoParams& Q) {
+    return ((long long)Q.dims[0] * Q.dims[1] * Q.dims[2] + kMcBlock - 1) / kMcBlock;
 }
 
-void launch_mc_emit(cudaStream_t st, const IsoParams& Q, const double* iso, const uint32_t* edge_off,
-                    const uint32_t* tri_off, float* vert, int32_t* tris) {
-    const long long nn = (long long)Q.dims[0] * Q.dims[1] * Q.dims[2];
-    k_mc_vertices<<<blocks_for(3 * nn, 256), 256, 0, st>>>(Q, iso, edge_off, vert);
-    k_mc_triangles<<<blocks_for(nn, 256), 256, 0, st>>>(Q, iso, tri_off, edge_off, tris);
+void launch_mc_classify(cudaStream_t st, const IsoParams& Q, const double* iso, uint16_t* cases, uint32_t* block_vert,
+                        uint32_t* block_tri) {
+    k_mc_classify<<<(unsigned)mc_blocks(Q), kMcBlock, 0, st>>>(Q, iso, cases, block_vert, block_tri);
+}
+
+void launch_mc_emit(cudaStream_t st, const IsoParams& Q, const double* iso, const uint16_t* cases,
+                    const uint32_t* block_vert, const uint32_t* block_tri, uint32_t* first, float* vert, int32_t* tris) {
+    const unsigned blocks = (unsigned)mc_blocks(Q);
+    k_mc_vertices<<<blocks, kMcBlock, 0, st>>>(Q, iso, cases, block_vert, first, vert);
+    k_mc_triangles<<<blocks, kMcBlock, 0, st>>>(Q, cases, block_tri, first, tris);
 }
 
 }  // namespace psb

@@ -427,7 +427,7 @@ struct IsoParams {
     double spacing[3];  // node spacing per axis
     int dims[3];        // nodes per axis
     double level;       // iso level of the surface
-    double r;           // REF: influence radius h / scale
+    double r;           // influence radius (REF: h / scale; CONFIG: h)
     int ring;           // cells of the particle grid walked on each side of the node's cell
     double inv_r2;      // CONFIG: 1 / h^2
     double k_colour;    // CONFIG: m 315 / (64 pi h^3): c(x) = k_colour sum (1 - q)^3 / rho_j
@@ -437,11 +437,15 @@ void mc_upload_table(cudaStream_t st);
 long long scan_scratch_words(long long n);
 void scan_exclusive_u32(cudaStream_t st, long long n, uint32_t* data, uint32_t* scratch);
 void launch_iso_field(cudaStream_t st, const IsoParams& Q, const Params& P, const float4* pos, const float2* rp,
-                      const uint32_t* cell_start, const uint32_t* cell_end, double* iso);
-void launch_mc_classify(cudaStream_t st, const IsoParams& Q, const double* iso, uint32_t* cube_tris,
-                        uint32_t* edge_flag);
-void launch_mc_emit(cudaStream_t st, const IsoParams& Q, const double* iso, const uint32_t* edge_off,
-                    const uint32_t* tri_off, float* vert, int32_t* tris);
+                      const uint32_t* cell_start, const uint32_t* cell_end, double* weight, double* iso);
+// Marching cubes: edge flags and cube case per node, vertices and triangles
+// per block of nodes (mc_blocks of them, one trailing word for the scan's
+// total); then, from the scanned block counts, the mesh. first: a word per node.
+long long mc_blocks(const IsoParams& Q);
+void launch_mc_classify(cudaStream_t st, const IsoParams& Q, const double* iso, uint16_t* cases, uint32_t* block_vert,
+                        uint32_t* block_tri);
+void launch_mc_emit(cudaStream_t st, const IsoParams& Q, const double* iso, const uint16_t* cases,
+                    const uint32_t* block_vert, const uint32_t* block_tri, uint32_t* first, float* vert, int32_t* tris);
 // The reference's polygonizer layout (compat): double4 nodes, per-cube vertex
 // slots and counts; synchronous, reports a slot overflow on stderr.
 void launch_mc_polygonize_slots(cudaStream_t st, const double* node4, int nx, int ny, int nz, double level, int* count,
