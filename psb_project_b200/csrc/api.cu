@@ -145,8 +145,6 @@ struct psb_ctx {
     uint64_t ds_cap = 0, ds_rows = 0;
     int collect_stride = 0;
     int64_t collect_steps = 0;
-    uint32_t* sel = nullptr;
-    int sel_cap = 0;
     // iso field and marching cubes (grown on demand)
     double* iso = nullptr;
     uint16_t* mc_case = nullptr;   // per node: edge flags and cube case
@@ -329,7 +327,7 @@ void free_all(psb_ctx* c) {
     cudaFree(c->slab);
     cudaFreeHost(c->h_slab);
     cudaFree(c->bnd_vel); cudaFree(c->bnd_fext); cudaFree(c->bnd_pred); cudaFree(c->bnd_react);
-    cudaFree(c->ds_X); cudaFree(c->ds_T); cudaFree(c->sel);
+    cudaFree(c->ds_X); cudaFree(c->ds_T);
     cudaFree(c->iso); cudaFree(c->mc_case); cudaFree(c->mc_first); cudaFree(c->mc_block); cudaFree(c->mc_vert);
     cudaFree(c->mc_tri);
     cudaFree(c->diag_rows); cudaFree(c->diag_out);
@@ -1544,23 +1542,13 @@ int psb_mlp_train(psb_ctx* c, int32_t iters, int32_t batch, float lr, uint64_t s
     if (!c->mlp_set) return fail(c, PSB_ESTATE, "psb_mlp_train: set initial weights first");
     enter(c);
     cudaStream_t st = c->stream;
-    if (batch > c->sel_cap) {
-        cudaStreamSynchronize(st);
-        cudaFree(c->sel);
-        c->sel = nullptr;
-        c->sel_cap = 0;
-        PSB_TRY(dalloc(c, &c->sel, (size_t)batch));
-        c->sel_cap = batch;
-    }
     for (int it = 0; it < iters; ++it) {
-        psb::launch_mlp_sample(st, batch, rows, seed + 0x100000001ull * (uint64_t)(c->mlp_step + 1), c->sel);
-        timed(c, "mlp_train", [&] {
-            psb::launch_mlp_grad(st, c->mlp_arch, batch, c->ds_X, c->ds_T, c->sel, c->mlp_wbf, c->mlp_part, c->mlp_grad,
-                                 c->mlp_loss);
-        });
+        const uint64_t draw = seed + 0x100000001ull * (uint64_t)(c->mlp_step + 1);
         ++c->mlp_step;
-        psb::launch_adam(st, psb::mlp_params(c->mlp_arch), c->mlp_w, c->mlp_grad, c->mlp_m1, c->mlp_m2, c->mlp_wbf, lr,
-                         c->mlp_step);
+        timed(c, "mlp_train", [&] {
+            psb::launch_mlp_step(st, c->mlp_arch, batch, c->ds_X, c->ds_T, rows, draw, c->mlp_part, c->mlp_grad,
+                                 c->mlp_loss, c->mlp_w, c->mlp_m1, c->mlp_m2, c->mlp_wbf, lr, c->mlp_step);
+        });
     }
     if (loss) {
         PSB_TRY(cuda_check(c, cudaMemcpyAsync(loss, c->mlp_loss, sizeof(float), cudaMemcpyDeviceToHost, st), "loss"));
@@ -1584,7 +1572,7 @@ static int mlp_host_call(psb_ctx* c, const float* X, const float* T, int32_t n, 
         rc = cuda_check(c, cudaMemcpyAsync(y, dy, sizeof(float) * n, cudaMemcpyDeviceToHost, st), "mlp");
     }
     if (!rc && grad) {
-        psb::launch_mlp_grad(st, c->mlp_arch, n, dX, dT, nullptr, c->mlp_wbf, c->mlp_part, c->mlp_grad, c->mlp_loss);
+        psb::launch_mlp_grad(st, c->mlp_arch, n, dX, dT, c->mlp_wbf, c->mlp_part, c->mlp_grad, c->mlp_loss);
         rc = cuda_check(c, cudaMemcpyAsync(grad, c->mlp_grad, sizeof(float) * psb::mlp_params(c->mlp_arch),
                                            cudaMemcpyDeviceToHost, st), "mlp");
         if (!rc && loss) rc = cuda_check(c, cudaMemcpyAsync(loss, c->mlp_loss, sizeof(float), cudaMemcpyDeviceToHost, st), "mlp");

@@ -55,6 +55,7 @@ struct Layout {
 };
 static_assert(Layout<7>::N == kMlpParams, "the largest network's parameter count");
 static_assert(Layout<6>::N == 4673, "the configured network's parameter count");
+static_assert(Layout<6>::W2 % 2 == 0 && Layout<7>::W2 % 2 == 0, "W2 is read as 32-bit pairs");
 
 enum { kSilu = 0, kRelu = 1 };
 
@@ -73,12 +74,22 @@ __device__ __forceinline__ float act(float z) {
     return fmaf(hz, tanh_approx(hz), hz);         // z sigma(z) = z/2 (1 + tanh(z/2))
 }
 
+// The activation and its derivative from one tanh: z becomes act'(z).
 template <int ACT>
-__device__ __forceinline__ float act_grad(float z) {
-    if (ACT == kRelu) return z > 0.f ? 1.f : 0.f;
-    const float s = fmaf(0.5f, tanh_approx(0.5f * z), 0.5f);    // sigma(z)
-    return s * fmaf(z, 1.f - s, 1.f);                            // sigma (1 + z (1 - sigma))
+__device__ __forceinline__ float act_and_grad(float& z) {
+    if (ACT == kRelu) {
+        const float a = fmaxf(z, 0.f);
+        z = z > 0.f ? 1.f : 0.f;
+        return a;
+    }
+    const float hz = 0.5f * z, t = tanh_approx(hz);
+    const float s = fmaf(0.5f, t, 0.5f);                // sigma(z)
+    z = s * fmaf(z, 1.f - s, 1.f);                      // sigma (1 + z (1 - sigma))
+    return fmaf(hz, t, hz);
 }
+
+__device__ __forceinline__ float bf_lo(uint32_t v) { return __uint_as_float(v << 16); }
+__device__ __forceinline__ float bf_hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
@@ -114,12 +125,17 @@ __device__ __forceinline__ void stage_weights(const __nv_bfloat16* __restrict__ 
         const float hi = k + 1 < NIN ? __bfloat162float(w[L::W1 + r * NIN + k + 1]) : 0.f;
         sW1[i] = pack_bf16(lo, hi);
     }
-    for (int i = threadIdx.x; i < kH * 32; i += blockDim.x) {
-        const int r = i / 32, k = 2 * (i % 32);
-        sW2[r * kRow + i % 32] = pack_bf16(__bfloat162float(w[L::W2 + r * kH + k]), __bfloat162float(w[L::W2 + r * kH + k + 1]));
-        if (sW2T)       // [k][j]: pairs along j (rows of W2)
-            sW2T[r * kRow + i % 32] =
-                pack_bf16(__bfloat162float(w[L::W2 + k * kH + r]), __bfloat162float(w[L::W2 + (k + 1) * kH + r]));
+    // W2's rows are pairs already (its offset is even); its transpose pairs
+    // up the halves of two rows
+    const uint32_t* w2 = reinterpret_cast<const uint32_t*>(w + L::W2);
+    for (int i = threadIdx.x; i < kH * 32; i += blockDim.x) sW2[(i / 32) * kRow + i % 32] = w2[i];
+    if (sW2T) {
+        for (int i = threadIdx.x; i < kH / 2 * 32; i += blockDim.x) {
+            const int k = i / 32, r = i % 32;         // rows 2k, 2k + 1; columns 2r, 2r + 1
+            const uint32_t lo = w2[2 * k * 32 + r], hi = w2[(2 * k + 1) * 32 + r];
+            sW2T[2 * r * kRow + k] = __byte_perm(lo, hi, 0x5410);
+            sW2T[(2 * r + 1) * kRow + k] = __byte_perm(lo, hi, 0x7632);
+        }
     }
     for (int i = threadIdx.x; i < kH; i += blockDim.x) {
         sB1[i] = __bfloat162float(w[L::B1 + i]);
@@ -196,20 +212,23 @@ __global__ void __launch_bounds__(256) k_mlp_infer_mma(int n, const float* __res
 
     const int lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
     const int warps_total = gridDim.x * (blockDim.x >> 5);
-    for (int tile = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); tile * 16 < n; tile += warps_total) {
+    const int first = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    // inputs 2 tig, 2 tig + 1 of the tile's rows gid and gid + 8 (the rows of
+    // feats hold 8, zero past NIN); the next tile's load while this one runs
+    float2 f0 = make_float2(0.f, 0.f), f1 = f0;
+    auto fetch = [&](int tile) {
         const int r0 = tile * 16 + gid, r1 = r0 + 8;
-        uint32_t a0 = 0u, a1 = 0u;
-        {
-            const int k = 2 * tig;
-            if (k < NIN) {
-                const float f00 = r0 < n ? feats[(size_t)r0 * 8 + k] : 0.f;
-                const float f01 = r0 < n && k + 1 < NIN ? feats[(size_t)r0 * 8 + k + 1] : 0.f;
-                const float f10 = r1 < n ? feats[(size_t)r1 * 8 + k] : 0.f;
-                const float f11 = r1 < n && k + 1 < NIN ? feats[(size_t)r1 * 8 + k + 1] : 0.f;
-                a0 = pack_bf16(f00, f01);
-                a1 = pack_bf16(f10, f11);
-            }
-        }
+        const float2* __restrict__ F = reinterpret_cast<const float2*>(feats) + tig;
+        f0 = r0 < n ? F[(size_t)r0 * 4] : make_float2(0.f, 0.f);
+        f1 = r1 < n ? F[(size_t)r1 * 4] : make_float2(0.f, 0.f);
+    };
+    if (first * 16 < n) fetch(first);
+    for (int tile = first; tile * 16 < n; tile += warps_total) {
+        const int r0 = tile * 16 + gid, r1 = r0 + 8;
+        const int k = 2 * tig;
+        const uint32_t a0 = k < NIN ? pack_bf16(f0.x, k + 1 < NIN ? f0.y : 0.f) : 0u;
+        const uint32_t a1 = k < NIN ? pack_bf16(f1.x, k + 1 < NIN ? f1.y : 0.f) : 0u;
+        if ((long long)(tile + warps_total) * 16 < n) fetch(tile + warps_total);
         float z[8][4];
         layer1(z, a0, a1, sW1, sB1, gid, tig);
         uint32_t h1[4][4];
@@ -220,10 +239,12 @@ __global__ void __launch_bounds__(256) k_mlp_infer_mma(int n, const float* __res
         for (int nt = 0; nt < 8; ++nt) {     // output layer on the BF16-rounded activations
             const int col = nt * 8 + 2 * tig;
             const float w30 = sW3[col], w31 = sW3[col + 1];
-            y0 = fmaf(w30, bf(act<ACT>(z[nt][0])), y0);
-            y0 = fmaf(w31, bf(act<ACT>(z[nt][1])), y0);
-            y1 = fmaf(w30, bf(act<ACT>(z[nt][2])), y1);
-            y1 = fmaf(w31, bf(act<ACT>(z[nt][3])), y1);
+            const uint32_t p0 = pack_bf16(act<ACT>(z[nt][0]), act<ACT>(z[nt][1]));
+            const uint32_t p1 = pack_bf16(act<ACT>(z[nt][2]), act<ACT>(z[nt][3]));
+            y0 = fmaf(w30, bf_lo(p0), y0);
+            y0 = fmaf(w31, bf_hi(p0), y0);
+            y1 = fmaf(w30, bf_lo(p1), y1);
+            y1 = fmaf(w31, bf_hi(p1), y1);
         }
         y0 += __shfl_xor_sync(0xffffffffu, y0, 1);
         y0 += __shfl_xor_sync(0xffffffffu, y0, 2);
@@ -278,26 +299,54 @@ __device__ __forceinline__ float row_sum(float v) {
     return v;
 }
 
+// Sample b of the minibatch `seed`: uniform over [0, rows), SplitMix64.
+__device__ __forceinline__ uint32_t sample_row(uint64_t rows, uint64_t seed, uint32_t b) {
+    uint64_t z = seed + 0x9E3779B97F4A7C15ull * (uint64_t)(b + 1u);
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+    z ^= z >> 31;
+    return (uint32_t)(z % rows);
+}
+
 // Mean-squared-error loss and its gradient over `batch` samples (sample b:
-// row sel[b] of X (stride 8) and T, or row b without sel). Each block
+// row sample_row(rows, seed, b) of X (stride 8) and T, or row b with rows 0). Each block
 // writes its partial sums -- every parameter's gradient at its layout
 // index, the loss at kMlpParams -- to its own row of `partial` (kPartStride
 // floats); k_grad_reduce adds the rows in block order. No atomics: the
 // gradient, and so the trained network, is the same bits on every run.
 template <int NIN, int ACT>
-__global__ void __launch_bounds__(kTrainWarps * 32) k_mlp_train_mma(int batch, const float* __restrict__ X,
+__global__ void __launch_bounds__(kTrainWarps * 32, ACT == kRelu ? 3 : 1) k_mlp_train_mma(int batch, const float* __restrict__ X,
                                                                   const float* __restrict__ T,
-                                                                  const uint32_t* __restrict__ sel,
+                                                                  uint64_t rows, uint64_t seed,
                                                                   const __nv_bfloat16* __restrict__ w,
                                                                   float* __restrict__ partial) {
     using L = Layout<NIN>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TrainSmem& S = *reinterpret_cast<TrainSmem*>(smem_raw);
+    const int lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3, wp = threadIdx.x >> 5;
+    const int m0 = wp * 16 + gid, m1 = m0 + 8;                 // rows of this warp in a block tile
+    const int k = 2 * tig;
+    // a tile's samples: two inputs of two rows and the rows' targets; the
+    // first tile's are on their way while the weights are staged, the next
+    // one's while a tile is worked on
+    float x00, x01, x10, x11, t0, t1;
+    auto fetch = [&](int tile) {
+        const int r0 = tile * kTrainRows + m0, r1 = r0 + 8;
+        const bool v0 = r0 < batch, v1 = r1 < batch;
+        const uint32_t row0 = v0 ? (rows ? sample_row(rows, seed, r0) : (uint32_t)r0) : 0u;
+        const uint32_t row1 = v1 ? (rows ? sample_row(rows, seed, r1) : (uint32_t)r1) : 0u;
+        x00 = v0 && k < NIN ? X[(size_t)row0 * 8 + k] : 0.f;
+        x01 = v0 && k + 1 < NIN ? X[(size_t)row0 * 8 + k + 1] : 0.f;
+        x10 = v1 && k < NIN ? X[(size_t)row1 * 8 + k] : 0.f;
+        x11 = v1 && k + 1 < NIN ? X[(size_t)row1 * 8 + k + 1] : 0.f;
+        t0 = v0 ? T[row0] : 0.f;
+        t1 = v1 ? T[row1] : 0.f;
+    };
+    fetch(blockIdx.x);
     stage_weights<NIN>(w, S.W1, S.W2, S.W2T, S.B1, S.B2, S.W3, &S.B3);
     for (int i = threadIdx.x; i < kTrainWarps * (3 * kH + 2); i += blockDim.x) (&S.G[0][0])[i] = 0.f;
     __syncthreads();
 
-    const int lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3, wp = threadIdx.x >> 5;
     const float inv_b = 1.f / (float)batch;
     float gW2[8][4], gW1[4];
 #pragma unroll
@@ -306,38 +355,56 @@ __global__ void __launch_bounds__(kTrainWarps * 32) k_mlp_train_mma(int batch, c
     float g_b3 = 0.f, g_loss = 0.f;
 
     for (int tile = blockIdx.x; tile * kTrainRows < batch; tile += gridDim.x) {
-        const int m0 = wp * 16 + gid, m1 = m0 + 8;                 // rows of this warp in the block tile
         const int r0 = tile * kTrainRows + m0, r1 = r0 + 8;
         const bool v0 = r0 < batch, v1 = r1 < batch;
-        const uint32_t row0 = v0 ? (sel ? sel[r0] : (uint32_t)r0) : 0u;
-        const uint32_t row1 = v1 ? (sel ? sel[r1] : (uint32_t)r1) : 0u;
-        const int k = 2 * tig;
-        const float x00 = v0 && k < NIN ? bf(X[(size_t)row0 * 8 + k]) : 0.f;
-        const float x01 = v0 && k + 1 < NIN ? bf(X[(size_t)row0 * 8 + k + 1]) : 0.f;
-        const float x10 = v1 && k < NIN ? bf(X[(size_t)row1 * 8 + k]) : 0.f;
-        const float x11 = v1 && k + 1 < NIN ? bf(X[(size_t)row1 * 8 + k + 1]) : 0.f;
+        const float f00 = bf(x00), f01 = bf(x01), f10 = bf(x10), f11 = bf(x11), y0t = t0, y1t = t1;
+        if (tile + (int)gridDim.x < (batch + kTrainRows - 1) / kTrainRows) fetch(tile + gridDim.x);
         // ---- forward
         float z1[8][4];
-        layer1(z1, pack_bf16(x00, x01), pack_bf16(x10, x11), S.W1, S.B1, gid, tig);
-        uint32_t a[4][4];
-        to_a_frags(a, z1, [](float v) { return act<ACT>(v); });
+        layer1(z1, pack_bf16(f00, f01), pack_bf16(f10, f11), S.W1, S.B1, gid, tig);
+        // Each unit's tanh is taken once (three times before: forward, weight
+        // gradients and derivative were each their own): the activations stay
+        // as the BF16 pairs they are rounded to, z1 and z2 turn into act'(z).
+        uint32_t a[4][4];       // h1, as layer 2's A fragments (to_a_frags)
+#pragma unroll
+        for (int nt = 0; nt < 8; ++nt) {
+            float h[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) h[q] = act_and_grad<ACT>(z1[nt][q]);
+            const uint32_t p0 = pack_bf16(h[0], h[1]), p1 = pack_bf16(h[2], h[3]);
+            a[nt / 2][2 * (nt & 1)] = p0;
+            a[nt / 2][2 * (nt & 1) + 1] = p1;
+            // and transposed, an operand of the weight-gradient products
+            const int col = nt * 8 + 2 * tig;
+            unsigned short* H = reinterpret_cast<unsigned short*>(S.H1T);
+            H[col * kTRow + m0] = (unsigned short)p0;
+            H[(col + 1) * kTRow + m0] = (unsigned short)(p0 >> 16);
+            H[col * kTRow + m1] = (unsigned short)p1;
+            H[(col + 1) * kTRow + m1] = (unsigned short)(p1 >> 16);
+        }
         float z2[8][4];
         layer64(z2, a, S.W2, S.B2, gid, tig);
         float y0 = 0.f, y1 = 0.f;
+        uint32_t h2[8][2];      // BF16 pairs of the two columns, rows m0 and m1
 #pragma unroll
         for (int nt = 0; nt < 8; ++nt) {
             const int col = nt * 8 + 2 * tig;
-            y0 = fmaf(S.W3[col], bf(act<ACT>(z2[nt][0])), y0);
-            y0 = fmaf(S.W3[col + 1], bf(act<ACT>(z2[nt][1])), y0);
-            y1 = fmaf(S.W3[col], bf(act<ACT>(z2[nt][2])), y1);
-            y1 = fmaf(S.W3[col + 1], bf(act<ACT>(z2[nt][3])), y1);
+            float h[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) h[q] = act_and_grad<ACT>(z2[nt][q]);
+            h2[nt][0] = pack_bf16(h[0], h[1]);
+            h2[nt][1] = pack_bf16(h[2], h[3]);
+            y0 = fmaf(S.W3[col], bf_lo(h2[nt][0]), y0);
+            y0 = fmaf(S.W3[col + 1], bf_hi(h2[nt][0]), y0);
+            y1 = fmaf(S.W3[col], bf_lo(h2[nt][1]), y1);
+            y1 = fmaf(S.W3[col + 1], bf_hi(h2[nt][1]), y1);
         }
         y0 += __shfl_xor_sync(0xffffffffu, y0, 1);
         y0 += __shfl_xor_sync(0xffffffffu, y0, 2);
         y1 += __shfl_xor_sync(0xffffffffu, y1, 1);
         y1 += __shfl_xor_sync(0xffffffffu, y1, 2);
-        const float e0 = v0 ? y0 + S.B3 - T[row0] : 0.f;
-        const float e1 = v1 ? y1 + S.B3 - T[row1] : 0.f;
+        const float e0 = v0 ? y0 + S.B3 - y0t : 0.f;
+        const float e1 = v1 ? y1 + S.B3 - y1t : 0.f;
         const float dy0 = 2.f * e0 * inv_b, dy1 = 2.f * e1 * inv_b;   // d(mean e^2)/dy
         if (tig == 0) {
             g_b3 += dy0 + dy1;
@@ -349,9 +416,10 @@ __global__ void __launch_bounds__(kTrainWarps * 32) k_mlp_train_mma(int batch, c
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
                 const int col = nt * 8 + 2 * tig + c;
-                const float gw3 = row_sum(dy0 * bf(act<ACT>(z2[nt][c])) + dy1 * bf(act<ACT>(z2[nt][2 + c])));
-                const float d0 = dy0 * S.W3[col] * act_grad<ACT>(z2[nt][c]);
-                const float d1 = dy1 * S.W3[col] * act_grad<ACT>(z2[nt][2 + c]);
+                const float a0 = c ? bf_hi(h2[nt][0]) : bf_lo(h2[nt][0]), a1 = c ? bf_hi(h2[nt][1]) : bf_lo(h2[nt][1]);
+                const float gw3 = row_sum(dy0 * a0 + dy1 * a1);
+                const float d0 = dy0 * S.W3[col] * z2[nt][c];
+                const float d1 = dy1 * S.W3[col] * z2[nt][2 + c];
                 const float gb2 = row_sum(d0 + d1);
                 if (gid == 0) {         // one lane per column in the warp
                     S.G[wp][2 * kH + col] += gw3;
@@ -370,23 +438,21 @@ __global__ void __launch_bounds__(kTrainWarps * 32) k_mlp_train_mma(int batch, c
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
                 const int col = nt * 8 + 2 * tig + c;
-                const float d0 = dh[nt][c] * act_grad<ACT>(z1[nt][c]);
-                const float d1 = dh[nt][2 + c] * act_grad<ACT>(z1[nt][2 + c]);
+                const float d0 = dh[nt][c] * z1[nt][c];
+                const float d1 = dh[nt][2 + c] * z1[nt][2 + c];
                 const float gb1 = row_sum(d0 + d1);
                 if (gid == 0) S.G[wp][col] += gb1;
                 // the tile's operands of the weight-gradient products, transposed
-                S.H1T[col * kTRow + m0] = __float2bfloat16_rn(act<ACT>(z1[nt][c]));
-                S.H1T[col * kTRow + m1] = __float2bfloat16_rn(act<ACT>(z1[nt][2 + c]));
                 S.D2T[col * kTRow + m0] = __float2bfloat16_rn(z2[nt][c]);
                 S.D2T[col * kTRow + m1] = __float2bfloat16_rn(z2[nt][2 + c]);
                 S.D1T[col * kTRow + m0] = __float2bfloat16_rn(d0);
                 S.D1T[col * kTRow + m1] = __float2bfloat16_rn(d1);
             }
         }
-        S.XT[k * kTRow + m0] = __float2bfloat16_rn(x00);
-        S.XT[(k + 1) * kTRow + m0] = __float2bfloat16_rn(x01);
-        S.XT[k * kTRow + m1] = __float2bfloat16_rn(x10);
-        S.XT[(k + 1) * kTRow + m1] = __float2bfloat16_rn(x11);
+        S.XT[k * kTRow + m0] = __float2bfloat16_rn(f00);
+        S.XT[(k + 1) * kTRow + m0] = __float2bfloat16_rn(f01);
+        S.XT[k * kTRow + m1] = __float2bfloat16_rn(f10);
+        S.XT[(k + 1) * kTRow + m1] = __float2bfloat16_rn(f11);
         __syncthreads();
         // ---- weight gradients over the tile's 64 samples: warp wp takes
         // rows [16 wp, 16 wp + 16) of dW2 (= dz2^T h1) and dW1 (= dz1^T x)
@@ -455,18 +521,29 @@ __global__ void __launch_bounds__(kTrainWarps * 32) k_mlp_train_mma(int batch, c
     }
 }
 
+// Adam's state and constants; wmaster null: the gradient only.
+struct AdamStep {
+    float* wmaster;
+    float* m1;
+    float* m2;
+    __nv_bfloat16* wbf;
+    float lr, b1, b2, eps, c1, c2;
+};
+
 // grad[p] (p < np) and the loss: the blocks' partial rows added in a fixed
 // order. Warp w of a block adds rows w, w + 8, ... for 32 consecutive
-// entries; the eight warp sums are then added in warp order.
+// entries, sixteen loads in flight (11 MB come from L2 on 147 blocks: with
+// four it was latency, 10 us); the eight warp sums are then added in warp
+// order. The thread that ends with a parameter's gradient takes its Adam step.
 __global__ void __launch_bounds__(256) k_grad_reduce(int nblocks, int np, const float* __restrict__ partial,
-                                                     float* __restrict__ grad, float* __restrict__ loss) {
+                                                     float* __restrict__ grad, float* __restrict__ loss, AdamStep A) {
     __shared__ float s[8][33];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int q = blockIdx.x * 32 + lane;                 // q == np: the loss
     const int src = q < np ? q : kMlpParams;
     float v = 0.f;
     if (q <= np) {
-#pragma unroll 4
+#pragma unroll 16
         for (int b = w; b < nblocks; b += 8) v += partial[(size_t)b * kPartStride + src];
     }
     s[w][lane] = v;
@@ -475,40 +552,26 @@ __global__ void __launch_bounds__(256) k_grad_reduce(int nblocks, int np, const 
         float t = s[0][lane];
 #pragma unroll
         for (int k = 1; k < 8; ++k) t += s[k][lane];
-        if (q < np) grad[q] = t;
-        else *loss = t;
+        if (q == np) {
+            *loss = t;
+            return;
+        }
+        grad[q] = t;
+        if (A.wmaster) {
+            const float m = A.b1 * A.m1[q] + (1.f - A.b1) * t;
+            const float u = A.b2 * A.m2[q] + (1.f - A.b2) * t * t;
+            A.m1[q] = m;
+            A.m2[q] = u;
+            const float wm = A.wmaster[q] - A.lr * (m / A.c1) / (sqrtf(u / A.c2) + A.eps);
+            A.wmaster[q] = wm;
+            A.wbf[q] = __float2bfloat16_rn(wm);
+        }
     }
-}
-
-__global__ void k_adam(int np, float* __restrict__ wmaster, const float* __restrict__ grad, float* __restrict__ m1,
-                       float* __restrict__ m2, __nv_bfloat16* __restrict__ wbf, float lr, float b1, float b2,
-                       float eps, float c1, float c2) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= np) return;
-    const float g = grad[i];
-    const float m = b1 * m1[i] + (1.f - b1) * g;
-    const float v = b2 * m2[i] + (1.f - b2) * g * g;
-    m1[i] = m;
-    m2[i] = v;
-    const float w = wmaster[i] - lr * (m / c1) / (sqrtf(v / c2) + eps);
-    wmaster[i] = w;
-    wbf[i] = __float2bfloat16_rn(w);
 }
 
 __global__ void k_to_bf16(int np, const float* __restrict__ w, __nv_bfloat16* __restrict__ wbf) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < np) wbf[i] = __float2bfloat16_rn(w[i]);
-}
-
-// Samples: uniform over [0, size) from SplitMix64 of (seed, iteration, b).
-__global__ void k_sample(int batch, uint64_t size, uint64_t seed, uint32_t* __restrict__ sel) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= batch) return;
-    uint64_t z = seed + 0x9E3779B97F4A7C15ull * (uint64_t)(b + 1);
-    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-    z ^= z >> 31;
-    sel[b] = (uint32_t)(z % size);
 }
 
 // Appends (features, converged pressure) of every stride-th slot, from
@@ -570,34 +633,39 @@ void launch_mlp_forward(cudaStream_t st, int arch, int n, const float* X, const 
     infer(st, arch, n, X, wbf, 1.f, nullptr, nullptr, y);
 }
 
-void launch_mlp_grad(cudaStream_t st, int arch, int batch, const float* X, const float* T, const uint32_t* sel,
-                     const void* wbf, float* partial, float* grad, float* loss) {
-    if (batch <= 0) {
-        cudaMemsetAsync(grad, 0, sizeof(float) * kMlpParams, st);
-        cudaMemsetAsync(loss, 0, sizeof(float), st);
-        return;
-    }
+namespace {
+void grad_launch(cudaStream_t st, int arch, int batch, const float* X, const float* T, uint64_t rows, uint64_t seed,
+                 const void* wbf, float* partial, float* grad, float* loss, const AdamStep& adam) {
     const int tiles = (batch + kTrainRows - 1) / kTrainRows;
     const int blocks = std::min(tiles, kMlpGradBlocks);
     with_arch(arch, [&](auto nin, auto a) {
         auto kernel = k_mlp_train_mma<decltype(nin)::value, decltype(a)::value>;
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TrainSmem));
-        kernel<<<blocks, kTrainWarps * 32, sizeof(TrainSmem), st>>>(batch, X, T, sel, (const __nv_bfloat16*)wbf,
+        kernel<<<blocks, kTrainWarps * 32, sizeof(TrainSmem), st>>>(batch, X, T, rows, seed, (const __nv_bfloat16*)wbf,
                                                                     partial);
     });
     const int np = mlp_params(arch);
-    k_grad_reduce<<<(np + 1 + 31) / 32, 256, 0, st>>>(blocks, np, partial, grad, loss);
+    k_grad_reduce<<<(np + 1 + 31) / 32, 256, 0, st>>>(blocks, np, partial, grad, loss, adam);
+}
+}  // namespace
+
+void launch_mlp_grad(cudaStream_t st, int arch, int batch, const float* X, const float* T, const void* wbf,
+                     float* partial, float* grad, float* loss) {
+    if (batch <= 0) {
+        cudaMemsetAsync(grad, 0, sizeof(float) * kMlpParams, st);
+        cudaMemsetAsync(loss, 0, sizeof(float), st);
+        return;
+    }
+    grad_launch(st, arch, batch, X, T, 0, 0, wbf, partial, grad, loss, AdamStep{});
 }
 
-void launch_mlp_sample(cudaStream_t st, int batch, uint64_t size, uint64_t seed, uint32_t* sel) {
-    if (batch > 0) k_sample<<<grid_of(batch), kBlock, 0, st>>>(batch, size, seed, sel);
-}
-
-void launch_adam(cudaStream_t st, int np, float* w, const float* grad, float* m1, float* m2, void* wbf, float lr,
-                 int step) {
+void launch_mlp_step(cudaStream_t st, int arch, int batch, const float* X, const float* T, uint64_t rows, uint64_t seed,
+                     float* partial, float* grad, float* loss, float* w, float* m1, float* m2, void* wbf, float lr,
+                     int step) {
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - powf(b1, (float)step), c2 = 1.f - powf(b2, (float)step);
-    k_adam<<<grid_of(np), kBlock, 0, st>>>(np, w, grad, m1, m2, (__nv_bfloat16*)wbf, lr, b1, b2, 1e-8f, c1, c2);
+    grad_launch(st, arch, batch, X, T, rows, seed, wbf, partial, grad, loss,
+                AdamStep{w, m1, m2, (__nv_bfloat16*)wbf, lr, b1, b2, 1e-8f, c1, c2});
 }
 
 void launch_to_bf16(cudaStream_t st, int np, const float* w, void* wbf) {

@@ -464,11 +464,12 @@ void launch_mlp_forward(cudaStream_t st, int arch, int n, const float* X, const 
 // write: kMlpGradBlocks rows of kMlpParams + 1 floats (the caller's buffer).
 constexpr int kMlpGradBlocks = 148 * 4;
 constexpr size_t kMlpGradPartials = (size_t)kMlpGradBlocks * (kMlpParams + 1);
-void launch_mlp_grad(cudaStream_t st, int arch, int batch, const float* X, const float* T, const uint32_t* sel,
-                     const void* wbf, float* partial, float* grad, float* loss);
-void launch_mlp_sample(cudaStream_t st, int batch, uint64_t size, uint64_t seed, uint32_t* sel);
-void launch_adam(cudaStream_t st, int np, float* w, const float* grad, float* m1, float* m2, void* wbf, float lr,
-                 int step);
+void launch_mlp_grad(cudaStream_t st, int arch, int batch, const float* X, const float* T, const void* wbf,
+                     float* partial, float* grad, float* loss);
+// One Adam step on a minibatch drawn from `rows` recorded rows (rows > 0).
+void launch_mlp_step(cudaStream_t st, int arch, int batch, const float* X, const float* T, uint64_t rows, uint64_t seed,
+                     float* partial, float* grad, float* loss, float* w, float* m1, float* m2, void* wbf, float lr,
+                     int step);
 void launch_to_bf16(cudaStream_t st, int np, const float* w, void* wbf);
 void launch_collect(cudaStream_t st, int n, int stride, int offset, uint64_t base, uint64_t cap, const float* feats,
                     const float2* rp, float p_scale, float* X, float* T);
