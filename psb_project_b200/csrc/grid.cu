@@ -355,33 +355,73 @@ __global__ void __launch_bounds__(kBlock) k_cell_count(Params P, const float4* _
 
 // Exclusive scan of the counts of one tile of cells, behind the particles of
 // the tiles before it; leaves the counts at zero for the next step. A tile
-// without particles (most of a dam break's box) only writes.
+// without particles (most of a dam break's box) only writes. Cells are scanned
+// in rows of 1,024, four to a thread: all rows' counts are loaded at once, each
+// warp scans its part of every row, and the 64 (row, warp) totals are scanned
+// by one warp -- two barriers; a block scan per row, one after another, took
+// 12 us for the five tiles of a 38,000-cell grid.
 __global__ void __launch_bounds__(kBlock) k_cell_scan(uint32_t* __restrict__ cell_count,
                                                       const uint32_t* __restrict__ tile_sum,
                                                       uint32_t* __restrict__ cell_start) {
-    __shared__ uint32_t s_warp[kBlock / 32];
-    const int tile = blockIdx.x, tid = threadIdx.x;
-    uint32_t mine = 0, run;
-    for (int i = tid; i < tile; i += kBlock) mine += tile_sum[i];
-    block_exclusive_scan(mine, s_warp, run);
-    const uint32_t here = tile_sum[tile];
+    constexpr int kRowsPerTile = kScanCells / (kBlock * 4), kWarps = kBlock / 32;
+    static_assert(kRowsPerTile * kWarps == 64, "one warp scans the (row, warp) totals, two each");
+    __shared__ uint32_t s_warp[kWarps], s_total[kRowsPerTile * kWarps];
+    const int tile = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const size_t first = (size_t)tile * kScanCells + tid * 4;
-    for (int r = 0; r < kScanCells; r += kBlock * 4) {
-        uint4 start = make_uint4(run, run, run, run);
-        if (here) {
-            uint4* at = reinterpret_cast<uint4*>(cell_count + first + r);
-            const uint4 v = *at;
-            uint32_t tot;
-            start.x += block_exclusive_scan(v.x + v.y + v.z + v.w, s_warp, tot);
-            start.y = start.x + v.x;
-            start.z = start.y + v.y;
-            start.w = start.z + v.z;
-            run += tot;
-            *at = make_uint4(0u, 0u, 0u, 0u);
-        }
-        *reinterpret_cast<uint4*>(cell_start + first + r) = start;
+    const uint32_t here = tile_sum[tile];
+    uint4 v[kRowsPerTile];
+    if (here) {
+#pragma unroll
+        for (int r = 0; r < kRowsPerTile; ++r) v[r] = *reinterpret_cast<const uint4*>(cell_count + first + r * kBlock * 4);
     }
-    if (tid == 0 && tile == (int)gridDim.x - 1) cell_start[(size_t)(tile + 1) * kScanCells] = run;
+    uint32_t mine = 0, before;
+    for (int i = tid; i < tile; i += kBlock) mine += tile_sum[i];
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if (lane == 0) s_warp[warp] = mine;
+    uint32_t e[kRowsPerTile];       // exclusive within the warp's part of the row
+    if (here) {
+#pragma unroll
+        for (int r = 0; r < kRowsPerTile; ++r) {
+            const uint32_t t = v[r].x + v[r].y + v[r].z + v[r].w;
+            uint32_t x = t;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            e[r] = x - t;
+            if (lane == 31) s_total[r * kWarps + warp] = x;
+        }
+    }
+    __syncthreads();
+    before = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) before += s_warp[w];
+    if (here && warp == 0) {
+        const uint32_t a = s_total[2 * lane], b = s_total[2 * lane + 1];
+        uint32_t x = a + b;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        s_total[2 * lane] = x - a - b;
+        s_total[2 * lane + 1] = x - b;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kRowsPerTile; ++r) {
+        uint4 start = make_uint4(before, before, before, before);
+        if (here) {
+            start.x += s_total[r * kWarps + warp] + e[r];
+            start.y = start.x + v[r].x;
+            start.z = start.y + v[r].y;
+            start.w = start.z + v[r].z;
+            *reinterpret_cast<uint4*>(cell_count + first + r * kBlock * 4) = make_uint4(0u, 0u, 0u, 0u);
+        }
+        *reinterpret_cast<uint4*>(cell_start + first + r * kBlock * 4) = start;
+    }
+    if (tid == 0 && tile == (int)gridDim.x - 1) cell_start[(size_t)(tile + 1) * kScanCells] = before + here;
 }
 
 // Each particle's (id, slot) into its cell's range, in arrival order; clears
