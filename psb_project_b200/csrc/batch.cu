@@ -28,6 +28,7 @@ __global__ void __launch_bounds__(kLoopThreads) k_batch_begin(int S, int max_it,
                                                              unsigned long long* __restrict__ err_scene,
                                                              unsigned long long* __restrict__ err_hist, int hist_len,
                                                              int* __restrict__ loop) {
+    after_previous();
     corrector_begin(S, max_it, active, err_scene, err_hist, hist_len, loop);
 }
 
@@ -37,6 +38,7 @@ __global__ void __launch_bounds__(kLoopThreads) k_batch_decide(int S, int min_it
                                                               unsigned long long* __restrict__ err_hist,
                                                               int* __restrict__ loop,
                                                               cudaGraphConditionalHandle handle, int set_handle) {
+    after_previous();
     __shared__ int any;
     const int cont = corrector_decide(S, min_it, max_it, eta, active, err_scene, err_hist, loop, &any);
     if (threadIdx.x == 0 && set_handle) cudaGraphSetConditional(handle, cont ? 1u : 0u);
@@ -46,14 +48,14 @@ __global__ void __launch_bounds__(kLoopThreads) k_batch_decide(int S, int min_it
 
 void launch_batch_begin(cudaStream_t st, int S, int max_it, uint8_t* active, unsigned long long* err_scene,
                         unsigned long long* err_hist, int hist_len, int* loop) {
-    k_batch_begin<<<1, kLoopThreads, 0, st>>>(S, max_it, active, err_scene, err_hist, hist_len, loop);
+    launch_chained(k_batch_begin, 1, kLoopThreads, 0, st, S, max_it, active, err_scene, err_hist, hist_len, loop);
 }
 
 void launch_batch_decide(cudaStream_t st, int S, int min_it, int max_it, double eta, uint8_t* active,
                          unsigned long long* err_scene, unsigned long long* err_hist, int* loop,
                          cudaGraphConditionalHandle handle, int set_handle) {
-    k_batch_decide<<<1, kLoopThreads, 0, st>>>(S, min_it, max_it, eta, active, err_scene, err_hist, loop, handle,
-                                               set_handle);
+    launch_chained(k_batch_decide, 1, kLoopThreads, 0, st, S, min_it, max_it, eta, active, err_scene, err_hist, loop,
+                   handle, set_handle);
 }
 
 }  // namespace psb

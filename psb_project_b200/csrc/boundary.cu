@@ -87,6 +87,7 @@ __global__ void __launch_bounds__(kBlock) k_build_bnd_nbr(Params P, const float4
                                                           const uint32_t* __restrict__ bnd_start,
                                                           const uint32_t* __restrict__ bnd_end, int* __restrict__ counts,
                                                           int* __restrict__ list, int* __restrict__ flags) {
+    after_previous();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= P.n) return;
     const float4 pi = pos[t];
@@ -189,6 +190,7 @@ __global__ void __launch_bounds__(kBlock) k_bnd_move(Params P, int nb, const flo
                                                      const float4* __restrict__ vel, const float4* __restrict__ fext,
                                                      float inv_mass, float4* __restrict__ pred,
                                                      float4* __restrict__ force) {
+    after_previous();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nb) return;
     const float4 xb = P.bnd[b];
@@ -213,8 +215,8 @@ void launch_bnd_move(cudaStream_t st, const Params& P, int nb, const float4* flu
                      const uint32_t* cell_start, const uint32_t* cell_end, const float4* vel, const float4* fext,
                      float inv_mass, float4* pred, float4* force) {
     if (nb > 0)
-        k_bnd_move<<<blocks_for(nb), kBlock, 0, st>>>(P, nb, fluid_pos, fluid_rp, cell_start, cell_end, vel, fext,
-                                                      inv_mass, pred, force);
+        launch_chained(k_bnd_move, blocks_for(nb), kBlock, 0, st, P, nb, fluid_pos, fluid_rp, cell_start, cell_end,
+                       vel, fext, inv_mass, pred, force);
 }
 
 void launch_bnd_gather4(cudaStream_t st, int nb, const int* ids, const float4* src, float4* dst) {
@@ -246,7 +248,8 @@ int launch_bnd_prepare(cudaStream_t st, const Params& P, int nb, const float4* r
 void launch_build_bnd_nbr(cudaStream_t st, const Params& P, const float4* pos, const uint32_t* keys,
                           const uint32_t* bnd_start, const uint32_t* bnd_end, int* counts, int* list, int* flags) {
     if (P.n > 0)
-        k_build_bnd_nbr<<<blocks_for(P.n), kBlock, 0, st>>>(P, pos, keys, bnd_start, bnd_end, counts, list, flags);
+        launch_chained(k_build_bnd_nbr, blocks_for(P.n), kBlock, 0, st, P, pos, keys, bnd_start, bnd_end, counts,
+                       list, flags);
 }
 
 }  // namespace psb

@@ -49,6 +49,7 @@ __global__ void __launch_bounds__(kBlock) k_dem_step(Params P, const float4* __r
                                                      const int* __restrict__ list, float4* __restrict__ pos_out,
                                                      float4* __restrict__ vel_out, float4* __restrict__ vap_out,
                                                      float4* __restrict__ force) {
+    after_previous();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= P.n) return;
     const float4 xa = pos[t], va = vel[t];
@@ -103,20 +104,22 @@ void launch_dem_step(cudaStream_t st, const Params& P, const float4* pos, const 
                      const int* list, float4* pos_out, float4* vel_out, float4* vap_out, float4* force) {
     if (P.n <= 0) return;
     if (P.ref)
-        k_dem_step<true><<<grid_of(P.n), kBlock, 0, st>>>(P, pos, vel, counts, list, pos_out, vel_out, vap_out, force);
+        launch_chained(k_dem_step<true>, grid_of(P.n), kBlock, 0, st, P, pos, vel, counts, list, pos_out, vel_out,
+                       vap_out, force);
     else
-        k_dem_step<false><<<grid_of(P.n), kBlock, 0, st>>>(P, pos, vel, counts, list, pos_out, vel_out, vap_out, force);
+        launch_chained(k_dem_step<false>, grid_of(P.n), kBlock, 0, st, P, pos, vel, counts, list, pos_out, vel_out,
+                       vap_out, force);
 }
 
 void launch_dem_forces(cudaStream_t st, const Params& P, const float4* pos, const float4* vel, const int* counts,
                        const int* list, float4* force) {
     if (P.n <= 0) return;
     if (P.ref)
-        k_dem_step<true, false><<<grid_of(P.n), kBlock, 0, st>>>(P, pos, vel, counts, list, nullptr, nullptr, nullptr,
-                                                                 force);
+        launch_chained(k_dem_step<true, false>, grid_of(P.n), kBlock, 0, st, P, pos, vel, counts, list, nullptr,
+                       nullptr, nullptr, force);
     else
-        k_dem_step<false, false><<<grid_of(P.n), kBlock, 0, st>>>(P, pos, vel, counts, list, nullptr, nullptr, nullptr,
-                                                                  force);
+        launch_chained(k_dem_step<false, false>, grid_of(P.n), kBlock, 0, st, P, pos, vel, counts, list, nullptr,
+                       nullptr, nullptr, force);
 }
 
 }  // namespace psb

@@ -62,6 +62,7 @@ template <bool BATCH>
 __global__ void k_cell_keys(Params P, const float4* __restrict__ pos, const int* __restrict__ ids,
                             uint32_t* __restrict__ keys_by_id, uint32_t* __restrict__ slot_by_id,
                             int* __restrict__ clamped) {
+    after_previous();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= P.n) return;
     int c = 0;
@@ -78,6 +79,7 @@ constexpr int kTile = kBlock * kItems;         // 2048 keys per block
 
 __global__ void k_radix_hist(int n, int shift, int nblocks, const uint32_t* __restrict__ keys,
                              uint32_t* __restrict__ hist) {
+    after_previous();
     __shared__ uint32_t h[256];
     h[threadIdx.x] = 0;
     __syncthreads();
@@ -122,6 +124,7 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* s
 // in place and writes the digit's total.
 __global__ void __launch_bounds__(kBlock) k_radix_scan(int nb, uint32_t* __restrict__ hist,
                                                        uint32_t* __restrict__ totals) {
+    after_previous();
     __shared__ uint32_t s_warp[kBlock / 32];
     uint32_t* h = hist + (size_t)blockIdx.x * nb;
     uint32_t carry = 0;
@@ -146,6 +149,7 @@ __global__ void __launch_bounds__(kBlock) k_radix_scatter(int n, int shift, int 
                                                           uint32_t* __restrict__ vals_out,
                                                           const uint32_t* __restrict__ offsets,
                                                           const uint32_t* __restrict__ totals) {
+    after_previous();
     __shared__ uint32_t s_off[256];
     __shared__ uint32_t s_wc[kBlock / 32][256];
     __shared__ uint32_t s_warp[kBlock / 32];
@@ -335,6 +339,7 @@ __global__ void __launch_bounds__(kBlock) k_cell_count(Params P, const float4* _
                                                        uint32_t* __restrict__ keys, uint32_t* __restrict__ ranks,
                                                        uint32_t* __restrict__ cell_count,
                                                        uint32_t* __restrict__ tile_sum, int* __restrict__ clamped) {
+    after_previous();
     const int s = blockIdx.x * kBlock + threadIdx.x, lane = threadIdx.x & 31;
     const bool valid = s < P.n;
     int c = 0;
@@ -363,6 +368,7 @@ __global__ void __launch_bounds__(kBlock) k_cell_count(Params P, const float4* _
 __global__ void __launch_bounds__(kBlock) k_cell_scan(uint32_t* __restrict__ cell_count,
                                                       const uint32_t* __restrict__ tile_sum,
                                                       uint32_t* __restrict__ cell_start) {
+    after_previous();
     constexpr int kRowsPerTile = kScanCells / (kBlock * 4), kWarps = kBlock / 32;
     static_assert(kRowsPerTile * kWarps == 64, "one warp scans the (row, warp) totals, two each");
     __shared__ uint32_t s_warp[kWarps], s_total[kRowsPerTile * kWarps];
@@ -430,6 +436,7 @@ __global__ void __launch_bounds__(kBlock) k_cell_place(int n, int ntiles, const 
                                                        const uint32_t* __restrict__ ranks, const int* __restrict__ ids,
                                                        const uint32_t* __restrict__ cell_start,
                                                        uint2* __restrict__ placed, uint32_t* __restrict__ tile_sum) {
+    after_previous();
     const int s = blockIdx.x * kBlock + threadIdx.x;
     if (s < ntiles) tile_sum[s] = 0u;
     if (s >= n) return;
@@ -442,6 +449,7 @@ __global__ void __launch_bounds__(kBlock) k_cell_rank(int n, const uint32_t* __r
                                                       const uint2* __restrict__ placed,
                                                       const uint32_t* __restrict__ cell_start,
                                                       uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out) {
+    after_previous();
     const int p = blockIdx.x * kBlock + threadIdx.x;
     if (p >= n) return;
     const uint2 me = placed[p];
@@ -462,6 +470,7 @@ __global__ void k_reorder(Params P, const uint32_t* __restrict__ keys, const uin
                           float4* __restrict__ pos2, float4* __restrict__ vel2, float4* __restrict__ vap2,
                           float2* __restrict__ rp2, int* __restrict__ ids2, uint32_t* __restrict__ cell_start,
                           uint32_t* __restrict__ cell_end) {
+    after_previous();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = P.n;
     const uint32_t s = t < n ? vals[t] : 0u;
@@ -494,6 +503,7 @@ __global__ void k_reorder_pos(Params P, const uint32_t* __restrict__ keys, const
                               const float4* __restrict__ pos, const int* __restrict__ ids, float4* __restrict__ pos2,
                               int* __restrict__ ids2, uint32_t* __restrict__ cell_start,
                               uint32_t* __restrict__ cell_end) {
+    after_previous();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = P.n;
     const uint32_t s = t < n ? vals[t] : 0u;
@@ -517,6 +527,7 @@ __global__ void k_reorder_pos(Params P, const uint32_t* __restrict__ keys, const
 __global__ void k_reorder_state(Params P, const uint32_t* __restrict__ vals, const float4* __restrict__ vel,
                                 const float4* __restrict__ vap, const float2* __restrict__ rp,
                                 float4* __restrict__ vel2, float4* __restrict__ vap2, float2* __restrict__ rp2) {
+    after_previous();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= P.n) return;
     const uint32_t s = vals[t];
@@ -597,6 +608,7 @@ __global__ void __launch_bounds__(BS) k_build_nbr(Params P, const float4* __rest
                                                   const uint32_t* __restrict__ cell_start,
                                                   const uint32_t* __restrict__ cell_end, int* __restrict__ counts,
                                                   int* __restrict__ list, int* __restrict__ flags) {
+    after_previous();
     __shared__ uint32_t s_first[kRows][BS], s_mask[kRows][BS];     // each thread uses its own column
     const int tid = threadIdx.x;
     const int t = blockIdx.x * BS + tid;
@@ -700,6 +712,7 @@ __global__ void __launch_bounds__(BS) k_build_nbr_tile(Params P, const float4* _
                                                        const uint32_t* __restrict__ cell_end,
                                                        int* __restrict__ counts, int* __restrict__ list,
                                                        int* __restrict__ flags) {
+    after_previous();
     __shared__ float4 s_tile[BS];
     float4* tile = s_tile + (threadIdx.x & ~31u);
     const int lane = threadIdx.x & 31;
@@ -823,9 +836,10 @@ void launch_cell_sort(cudaStream_t st, int n, size_t ncells, const int* ids, con
                       uint32_t* vals_out) {
     if (n <= 0) return;
     const int tiles = (int)cell_sort_tiles(ncells);
-    k_cell_scan<<<tiles, kBlock, 0, st>>>(cell_count, tile_sum, cell_start);
-    k_cell_place<<<grid_of(std::max(n, tiles)), kBlock, 0, st>>>(n, tiles, keys, ranks, ids, cell_start, placed, tile_sum);
-    k_cell_rank<<<grid_of(n), kBlock, 0, st>>>(n, keys, placed, cell_start, keys_out, vals_out);
+    launch_chained(k_cell_scan, tiles, kBlock, 0, st, cell_count, tile_sum, cell_start);
+    launch_chained(k_cell_place, grid_of(std::max(n, tiles)), kBlock, 0, st, n, tiles, keys, ranks, ids, cell_start,
+                   placed, tile_sum);
+    launch_chained(k_cell_rank, grid_of(n), kBlock, 0, st, n, keys, placed, cell_start, keys_out, vals_out);
 }
 
 int radix_sort(cudaStream_t st, int n, int bits, uint32_t* keys[2], uint32_t* vals[2], uint32_t* hist, int nblocks_cap) {
@@ -834,10 +848,10 @@ int radix_sort(cudaStream_t st, int n, int bits, uint32_t* keys[2], uint32_t* va
     if (small_sort(st, n, bits, keys[0], vals[0], keys[0], vals[0])) return 0;
     int cur = 0;
     for (int shift = 0; shift < bits; shift += 8) {
-        k_radix_hist<<<nb, kBlock, 0, st>>>(n, shift, nb, keys[cur], hist);
-        k_radix_scan<<<256, kBlock, 0, st>>>(nb, hist, hist + (size_t)256 * nb);
-        k_radix_scatter<<<nb, kBlock, 0, st>>>(n, shift, nb, keys[cur], vals[cur], keys[cur ^ 1], vals[cur ^ 1], hist,
-                                               hist + (size_t)256 * nb);
+        launch_chained(k_radix_hist, nb, kBlock, 0, st, n, shift, nb, keys[cur], hist);
+        launch_chained(k_radix_scan, 256, kBlock, 0, st, nb, hist, hist + (size_t)256 * nb);
+        launch_chained(k_radix_scatter, nb, kBlock, 0, st, n, shift, nb, keys[cur], vals[cur], keys[cur ^ 1],
+                       vals[cur ^ 1], hist, hist + (size_t)256 * nb);
         cur ^= 1;
     }
     return cur;
@@ -848,15 +862,15 @@ void launch_reorder(cudaStream_t st, const Params& P, const uint32_t* keys, cons
                     float4* vap2, float2* rp2, int* ids2, uint32_t* cell_start, uint32_t* cell_end) {
     if (P.n <= 0) return;
     auto kernel = P.scenes ? k_reorder<true> : k_reorder<false>;
-    kernel<<<grid_of(P.n), kBlock, 0, st>>>(P, keys, vals, pos, vel, vap, rp, ids, pos2, vel2, vap2, rp2, ids2,
-                                            cell_start, cell_end);
+    launch_chained(kernel, grid_of(P.n), kBlock, 0, st, P, keys, vals, pos, vel, vap, rp, ids, pos2, vel2, vap2, rp2,
+                   ids2, cell_start, cell_end);
 }
 
 void launch_reorder_pos(cudaStream_t st, const Params& P, const uint32_t* keys, const uint32_t* vals, const float4* pos,
                         const int* ids, float4* pos2, int* ids2, uint32_t* cell_start, uint32_t* cell_end) {
     if (P.n <= 0) return;
     auto kernel = P.scenes ? k_reorder_pos<true> : k_reorder_pos<false>;
-    kernel<<<grid_of(P.n), kBlock, 0, st>>>(P, keys, vals, pos, ids, pos2, ids2, cell_start, cell_end);
+    launch_chained(kernel, grid_of(P.n), kBlock, 0, st, P, keys, vals, pos, ids, pos2, ids2, cell_start, cell_end);
 }
 
 void launch_reorder_state(cudaStream_t st, const Params& P, const uint32_t* vals, const float4* vel, const float4* vap,
@@ -870,7 +884,9 @@ void launch_build_nbr(cudaStream_t st, const Params& P, const float4* pos, const
     with_block(P.tune.nbr_block, [&](auto B) {
         constexpr int BS = decltype(B)::value;
         const unsigned g = (unsigned)((P.n + BS - 1) / BS);
-        auto go = [&](auto kernel) { kernel<<<g, BS, 0, st>>>(P, pos, keys, cell_start, cell_end, counts, list, flags); };
+        auto go = [&](auto kernel) {
+            launch_chained(kernel, g, BS, 0, st, P, pos, keys, cell_start, cell_end, counts, list, flags);
+        };
         if (P.tune.nbr_schedule == 1) {
             if (P.scenes) go(k_build_nbr_tile<true, BS>); else go(k_build_nbr_tile<false, BS>);
         } else {

@@ -155,6 +155,7 @@ namespace {
 // k_colour / rho_j of every particle (config profile): the division once a
 // particle rather than once a (node, particle) pair.
 __global__ void k_iso_weight(int n, double k_colour, const float2* __restrict__ rp, double* __restrict__ w) {
+    after_previous();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < n) w[t] = k_colour / (double)rp[t].x;
 }
@@ -183,6 +184,7 @@ __global__ void __launch_bounds__(128) k_iso_field(IsoParams Q, Params P, const 
                                                    const double* __restrict__ weight,
                                                    const uint32_t* __restrict__ cell_start,
                                                    const uint32_t* __restrict__ cell_end, double* __restrict__ iso) {
+    after_previous();
     const int l = threadIdx.x & 31, wp = threadIdx.x >> 5;
     const unsigned bx = (Q.dims[0] + 4 * E - 1) / (4 * E), by = (Q.dims[1] + 4 * E - 1) / (4 * E);
     const int ix = ((int)(blockIdx.x % bx) * 4 + (l & 3)) * E;
@@ -376,6 +378,7 @@ __global__ void __launch_bounds__(kMcBlock) k_mc_classify(IsoParams Q, const dou
                                                           uint16_t* __restrict__ cases,
                                                           uint32_t* __restrict__ block_vert,
                                                           uint32_t* __restrict__ block_tri) {
+    after_previous();
     const unsigned nn = (unsigned)Q.dims[0] * Q.dims[1] * Q.dims[2];
     const unsigned node = blockIdx.x * kMcBlock + threadIdx.x;
     unsigned nv = 0, nt = 0;
@@ -408,6 +411,7 @@ __global__ void __launch_bounds__(kMcBlock) k_mc_vertices(IsoParams Q, const dou
                                                           const uint16_t* __restrict__ cases,
                                                           const uint32_t* __restrict__ block_vert,
                                                           uint32_t* __restrict__ first, float* __restrict__ vert) {
+    after_previous();
     const unsigned nn = (unsigned)Q.dims[0] * Q.dims[1] * Q.dims[2];
     const unsigned node = blockIdx.x * kMcBlock + threadIdx.x;
     if (block_vert[blockIdx.x + 1] == block_vert[blockIdx.x]) return;       // no active edge in the block
@@ -447,6 +451,7 @@ __global__ void __launch_bounds__(kMcBlock) k_mc_triangles(IsoParams Q, const ui
                                                            const uint32_t* __restrict__ block_tri,
                                                            const uint32_t* __restrict__ first,
                                                            int32_t* __restrict__ tris) {
+    after_previous();
     const unsigned nn = (unsigned)Q.dims[0] * Q.dims[1] * Q.dims[2];
     const unsigned node = blockIdx.x * kMcBlock + threadIdx.x;
     if (block_tri[blockIdx.x + 1] == block_tri[blockIdx.x]) return;
@@ -602,7 +607,7 @@ void launch_iso_field(cudaStream_t st, const IsoParams& Q, const Params& P, cons
     auto kernel = P.ref ? k_iso_field<true, 1> : edge == 2 ? k_iso_field<false, 2> : k_iso_field<false, 1>;
     const long long xy = 4 * edge, z = 8 * edge;
     const long long blocks = ((Q.dims[0] + xy - 1) / xy) * ((Q.dims[1] + xy - 1) / xy) * ((Q.dims[2] + z - 1) / z);
-    kernel<<<(unsigned)blocks, 128, 0, st>>>(Q, P, pos, weight, cell_start, cell_end, iso);
+    launch_chained(kernel, (unsigned)blocks, 128, 0, st, Q, P, pos, weight, cell_start, cell_end, iso);
 }
 
 long long mc_blocks(const IsoParams& Q) {
@@ -611,14 +616,14 @@ long long mc_blocks(const IsoParams& Q) {
 
 void launch_mc_classify(cudaStream_t st, const IsoParams& Q, const double* iso, uint16_t* cases, uint32_t* block_vert,
                         uint32_t* block_tri) {
-    k_mc_classify<<<(unsigned)mc_blocks(Q), kMcBlock, 0, st>>>(Q, iso, cases, block_vert, block_tri);
+    launch_chained(k_mc_classify, (unsigned)mc_blocks(Q), kMcBlock, 0, st, Q, iso, cases, block_vert, block_tri);
 }
 
 void launch_mc_emit(cudaStream_t st, const IsoParams& Q, const double* iso, const uint16_t* cases,
                     const uint32_t* block_vert, const uint32_t* block_tri, uint32_t* first, float* vert, int32_t* tris) {
     const unsigned blocks = (unsigned)mc_blocks(Q);
-    k_mc_vertices<<<blocks, kMcBlock, 0, st>>>(Q, iso, cases, block_vert, first, vert);
-    k_mc_triangles<<<blocks, kMcBlock, 0, st>>>(Q, cases, block_tri, first, tris);
+    launch_chained(k_mc_vertices, blocks, kMcBlock, 0, st, Q, iso, cases, block_vert, first, vert);
+    launch_chained(k_mc_triangles, blocks, kMcBlock, 0, st, Q, cases, block_tri, first, tris);
 }
 
 }  // namespace psb

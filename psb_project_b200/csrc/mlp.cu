@@ -203,6 +203,7 @@ __global__ void __launch_bounds__(256) k_mlp_infer_mma(int n, const float* __res
                                                        const __nv_bfloat16* __restrict__ w, float p_scale,
                                                        float2* __restrict__ rp, float2* __restrict__ zp,
                                                        float* __restrict__ y_raw) {
+    after_previous();
     __shared__ uint32_t sW1[kH * kW1Stride];
     __shared__ uint32_t sW2[kH * kRow];
     __shared__ float sB1[kH], sB2[kH], sW3[kH];
@@ -321,6 +322,7 @@ __global__ void __launch_bounds__(kTrainWarps * 32, ACT == kRelu ? 3 : 1) k_mlp_
                                                                   const __nv_bfloat16* __restrict__ w,
                                                                   float* __restrict__ partial) {
     using L = Layout<NIN>;
+    after_previous();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TrainSmem& S = *reinterpret_cast<TrainSmem*>(smem_raw);
     const int lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3, wp = threadIdx.x >> 5;
@@ -537,6 +539,7 @@ struct AdamStep {
 // order. The thread that ends with a parameter's gradient takes its Adam step.
 __global__ void __launch_bounds__(256) k_grad_reduce(int nblocks, int np, const float* __restrict__ partial,
                                                      float* __restrict__ grad, float* __restrict__ loss, AdamStep A) {
+    after_previous();
     __shared__ float s[8][33];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int q = blockIdx.x * 32 + lane;                 // q == np: the loss
@@ -608,8 +611,8 @@ void infer(cudaStream_t st, int arch, int n, const float* feats, const void* wbf
     const int tiles = (n + 15) / 16;
     const int blocks = std::min((tiles + 7) / 8, 148 * 8);      // 8 warps per block, grid-stride over tiles
     with_arch(arch, [&](auto nin, auto a) {
-        k_mlp_infer_mma<decltype(nin)::value, decltype(a)::value>
-            <<<blocks, 256, 0, st>>>(n, feats, (const __nv_bfloat16*)wbf, p_scale, rp, zp, y);
+        launch_chained(k_mlp_infer_mma<decltype(nin)::value, decltype(a)::value>, blocks, 256, 0, st, n, feats,
+                       (const __nv_bfloat16*)wbf, p_scale, rp, zp, y);
     });
 }
 
@@ -641,11 +644,11 @@ void grad_launch(cudaStream_t st, int arch, int batch, const float* X, const flo
     with_arch(arch, [&](auto nin, auto a) {
         auto kernel = k_mlp_train_mma<decltype(nin)::value, decltype(a)::value>;
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TrainSmem));
-        kernel<<<blocks, kTrainWarps * 32, sizeof(TrainSmem), st>>>(batch, X, T, rows, seed, (const __nv_bfloat16*)wbf,
-                                                                    partial);
+        launch_chained(kernel, blocks, kTrainWarps * 32, sizeof(TrainSmem), st, batch, X, T, rows, seed,
+                       (const __nv_bfloat16*)wbf, partial);
     });
     const int np = mlp_params(arch);
-    k_grad_reduce<<<(np + 1 + 31) / 32, 256, 0, st>>>(blocks, np, partial, grad, loss, adam);
+    launch_chained(k_grad_reduce, (np + 1 + 31) / 32, 256, 0, st, blocks, np, partial, grad, loss, adam);
 }
 }  // namespace
 

@@ -500,6 +500,7 @@ template <bool REF, int NF, bool BATCH, int BS>
 __global__ void __launch_bounds__(BS, REF ? 1 : (NF ? kForceThreads : kDensityThreads) / BS)
     k_density_x(Params P, const int* __restrict__ counts, const int* __restrict__ list, float2* __restrict__ rp,
                 float* __restrict__ rho_x, int zero_p, float p_scale, float* __restrict__ feats) {
+    after_previous();
     for_each_slot<BS, !REF>(P, [&](const int t) {
         if (t < 0) return;
         const float4 xi = at(P.x0, t);
@@ -527,6 +528,7 @@ __global__ void __launch_bounds__(BS) k_build_density(Params P, const float4* __
                                                           int* __restrict__ flags, float2* __restrict__ rp,
                                                           float* __restrict__ rho_x, int zero_p, float p_scale,
                                                           float* __restrict__ feats) {
+    after_previous();
     const int t = blockIdx.x * BS + threadIdx.x;
     const bool valid = t < P.n;     // every lane stays for the warp reductions below
     int cnt = 0;
@@ -641,6 +643,7 @@ __global__ void __launch_bounds__(kBlock) k_wcsph_force(Params P, const float4* 
                                                         const int* __restrict__ list, float4* __restrict__ pos_out,
                                                         float4* __restrict__ vel_out, float4* __restrict__ vap_out,
                                                         float4* __restrict__ fnp) {
+    after_previous();
     auto integrate = [&](const int t, const float4 xi, const float2 rpi, const PairSums& S) {
         const float4 vh = vap[t];
         const float3 f = nonpressure_force<REF>(P, S, rpi.x);
@@ -670,6 +673,7 @@ template <bool REF, bool WARM, bool BATCH, int BS>
 __global__ void __launch_bounds__(BS, REF || !WARM ? 1 : kInitThreads / BS) k_pci_init(
     Params P, const float4* __restrict__ vap, const float2* __restrict__ rp, const int* __restrict__ counts,
     const int* __restrict__ list, float4* __restrict__ fnp, Soa3 xs, Soa3 vs) {
+    after_previous();
     auto predict = [&](const int t, const float4 xi, const float2 rpi, const PairSums& S) {
         const float4 vh = vap[t];
         const float3 f = nonpressure_force<REF>(P, S, rpi.x);
@@ -809,6 +813,7 @@ __global__ void __launch_bounds__(BS, REF ? 1 : kDensityThreads / BS) k_pci_dens
                                                         const float2* __restrict__ rp, const int* __restrict__ counts,
                                                         const int* __restrict__ list, float2* __restrict__ rpc,
                                                         unsigned long long* __restrict__ err_slot) {
+    after_previous();
     double worst = -1e300;
     for_each_slot<BS, !REF>(P, [&](const int t) {
         const int sc = BATCH && t >= 0 ? (int)P.slot_scene[t] : -1;
@@ -899,6 +904,7 @@ template <bool REF, bool BATCH, int BS>
 __global__ void __launch_bounds__(BS, REF ? 1 : kForceThreads / BS) k_pci_force_predict(
     Params P, const float4* __restrict__ vap, const float4* __restrict__ fnp, Soa3 xs, const float2* __restrict__ rpc,
     const int* __restrict__ counts, const int* __restrict__ list, Soa3 xs_next, Soa3 vs, float2* __restrict__ rp) {
+    after_previous();
     if (!BATCH && P.active && !P.active[0]) return;      // single scene, corrector decided on the device: converged
     for_each_slot<BS, !REF>(P, [&](const int t) {
         if (t < 0 || (BATCH && !P.active[P.slot_scene[t]])) return;     // its scene has converged
@@ -965,6 +971,7 @@ __global__ void __launch_bounds__(kBlock) k_pci_commit(Params P, Soa3 xs, Soa3 v
                                                        int have_density_pass, float4* __restrict__ pos,
                                                        float4* __restrict__ vel, float4* __restrict__ vap,
                                                        float2* __restrict__ rp) {
+    after_previous();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= P.n) return;
     float3 x = f3(at(xs, t)), v = f3(at(vs, t));
@@ -989,6 +996,7 @@ __global__ void __launch_bounds__(kBlock) k_pci_commit(Params P, Soa3 xs, Soa3 v
 template <int BS>
 __global__ void __launch_bounds__(BS) k_xsph(Params P, Soa3 xs, Soa3 vs, const int* __restrict__ counts,
                                                  const int* __restrict__ list, Soa3 vs_out) {
+    after_previous();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= P.n) return;
     const float4 xi = at(xs, t), vi = at(vs, t);
@@ -1034,7 +1042,8 @@ void launch_density_x(cudaStream_t st, const Params& P, const int* counts, const
         constexpr int BS = decltype(B)::value;
         const Params Q = with_walls<BS>(P);
         auto go = [&](auto kernel) {
-            kernel<<<blocks_of<BS>(P.n) + Q.wall_blocks, BS, 0, st>>>(Q, counts, list, rp, rho_x, zero_p, p_scale, feats);
+            launch_chained(kernel, blocks_of<BS>(P.n) + Q.wall_blocks, BS, 0, st, Q, counts, list, rp, rho_x, zero_p,
+                           p_scale, feats);
         };
         const int nf = feats ? (nfeat > 6 ? 7 : 6) : 0;
         if (P.ref) go(k_density_x<true, 0, false, BS>);
@@ -1055,8 +1064,8 @@ void launch_build_density(cudaStream_t st, const Params& P, const float4* pos, c
     with_block(P.tune.nbr_block, [&](auto B) {
         constexpr int BS = decltype(B)::value;
         auto go = [&](auto kernel) {
-            kernel<<<blocks_of<BS>(P.n), BS, 0, st>>>(P, pos, keys, cell_start, cell_end, counts, list, flags, rp, rho_x,
-                                                      zero_p, p_scale, feats);
+            launch_chained(kernel, blocks_of<BS>(P.n), BS, 0, st, P, pos, keys, cell_start, cell_end, counts, list,
+                           flags, rp, rho_x, zero_p, p_scale, feats);
         };
         const int nf = feats ? (nfeat > 6 ? 7 : 6) : 0;
         if (nf == 7) go(k_build_density<7, BS>);
@@ -1071,7 +1080,8 @@ void launch_wcsph_force(cudaStream_t st, const Params& P, const float4* vap, con
     if (P.n <= 0) return;
     const Params Q = with_walls<kBlock>(P);
     auto kernel = P.ref ? k_wcsph_force<true> : k_wcsph_force<false>;
-    kernel<<<grid_of(P.n) + Q.wall_blocks, kBlock, 0, st>>>(Q, vap, rp, counts, list, pos_out, vel_out, vap_out, fnp);
+    launch_chained(kernel, grid_of(P.n) + Q.wall_blocks, kBlock, 0, st, Q, vap, rp, counts, list, pos_out, vel_out,
+                   vap_out, fnp);
 }
 
 void launch_pci_init(cudaStream_t st, const Params& P, const float4* vap, const float2* rp, const int* counts,
@@ -1081,7 +1091,8 @@ void launch_pci_init(cudaStream_t st, const Params& P, const float4* vap, const 
         constexpr int BS = decltype(B)::value;
         const Params Q = with_walls<BS>(P, warm != 0);
         auto go = [&](auto kernel) {
-            kernel<<<blocks_of<BS>(P.n) + Q.wall_blocks, BS, 0, st>>>(Q, vap, rp, counts, list, fnp, xs, vs);
+            launch_chained(kernel, blocks_of<BS>(P.n) + Q.wall_blocks, BS, 0, st, Q, vap, rp, counts, list, fnp, xs,
+                           vs);
         };
         if (P.ref) { if (warm) go(k_pci_init<true, true, false, BS>); else go(k_pci_init<true, false, false, BS>); }
         else if (P.scenes) { if (warm) go(k_pci_init<false, true, true, BS>); else go(k_pci_init<false, false, true, BS>); }
@@ -1097,7 +1108,8 @@ void launch_pci_density(cudaStream_t st, const Params& P, Soa3 xs, const float2*
         constexpr int BS = decltype(B)::value;
         const Params Q = with_walls<BS>(P);
         auto go = [&](auto kernel) {
-            kernel<<<blocks_of<BS>(P.n) + Q.wall_blocks, BS, 0, st>>>(Q, xs, rp, counts, list, rpc, err_slot);
+            launch_chained(kernel, blocks_of<BS>(P.n) + Q.wall_blocks, BS, 0, st, Q, xs, rp, counts, list, rpc,
+                           err_slot);
         };
         if (P.ref) go(k_pci_density<true, false, BS>);
         else if (P.scenes) go(k_pci_density<false, true, BS>);
@@ -1145,7 +1157,8 @@ void launch_pci_force_predict(cudaStream_t st, const Params& P, const float4* va
         constexpr int BS = decltype(B)::value;
         const Params Q = with_walls<BS>(P);
         auto go = [&](auto kernel) {
-            kernel<<<blocks_of<BS>(P.n) + Q.wall_blocks, BS, 0, st>>>(Q, vap, fnp, xs, rpc, counts, list, xs_next, vs, rp);
+            launch_chained(kernel, blocks_of<BS>(P.n) + Q.wall_blocks, BS, 0, st, Q, vap, fnp, xs, rpc, counts, list,
+                           xs_next, vs, rp);
         };
         if (P.ref) go(k_pci_force_predict<true, false, BS>);
         else if (P.scenes) go(k_pci_force_predict<false, true, BS>);
