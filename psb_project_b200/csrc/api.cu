@@ -126,6 +126,7 @@ struct psb_ctx {
     float* rho_x = nullptr;
     unsigned long long* err_hist = nullptr;
     int* flags = nullptr;     // [0] overflow [1] max count [2..3] pair total [4] clamped [5] wall list length
+                              // [6] clamped, as counted before the others are cleared
     void* stage = nullptr;    // device staging for uploads/downloads
     // learned warm start
     float* feats = nullptr;   // n_max x 8
@@ -570,17 +571,18 @@ int build(psb_ctx* c, bool keep_p = false, bool features = false) {
     if (rs >= 0 && !c->dense)
         timed(c, "reset_cells", [&] { psb::launch_reset_cells(st, rn, c->keys[rs], c->cell_start); });
     c->stale = -1;
-    cudaMemsetAsync(c->flags, 0, 8 * sizeof(int), st);
+    // the counting sort clears the words itself
+    if (!c->dense || n <= 0) cudaMemsetAsync(c->flags, 0, 8 * sizeof(int), st);
     int res = 0;
     uint32_t* range_start = c->cell_start;      // the reorder records the cell ranges
     if (c->dense) {
         timed(c, "cell_keys", [&] {
-            psb::launch_cell_count(st, P, c->pos[c->cs], c->keys[0], c->vals[0], c->cell_count, c->tile_sum, &c->flags[4]);
+            psb::launch_cell_count(st, P, c->pos[c->cs], c->keys[0], c->vals[0], c->cell_count, c->tile_sum, &c->flags[6]);
         });
         // the predictor's x* buffer is free until the set-up sweep
         timed(c, "cell_sort", [&] {
             psb::launch_cell_sort(st, n, c->ncells, c->ids[c->cr], c->keys[0], c->vals[0], c->cell_count, c->tile_sum,
-                                  c->cell_start, reinterpret_cast<uint2*>(c->xs[0].xy), c->keys[1], c->vals[1]);
+                                  c->cell_start, c->flags, reinterpret_cast<uint2*>(c->xs[0].xy), c->keys[1], c->vals[1]);
         });
         res = 1;
         range_start = nullptr;
@@ -933,7 +935,6 @@ int step_once(psb_ctx* c, bool last) {
     P.n = c->n;
     const int s = c->cs, r = c->cr;
     int iters = 0, converged = 1;
-    cudaMemsetAsync(c->err_hist, 0, sizeof(unsigned long long) * (PSB_MAX_ITERS + 1), st);
     if (P.dem) {
         const int o = s ^ 1;
         P.slot_ids = c->ids[r];
@@ -964,6 +965,7 @@ int step_once(psb_ctx* c, bool last) {
     } else {
         // reference-profile PCISPH: exactly three corrections from p = 0
         // (PciSphSystem.cu:30-61), no host round trip
+        cudaMemsetAsync(c->err_hist, 0, sizeof(unsigned long long) * (PSB_MAX_ITERS + 1), st);
         timed(c, "pci_init", [&] {
             psb::launch_pci_init(st, P, c->vap[s], c->rp[r], c->nbr_count, c->nbr_list, 0,
                                  c->fnp, c->xs[0], c->vs);
@@ -1119,6 +1121,7 @@ int create_impl(const psb_scene* scene, size_t ncells, int S, bool batch, psb_ct
         fill(c->mlp_w, 0, sizeof(float) * psb::kMlpParams);
         fill(c->mlp_wbf, 0, 2 * psb::kMlpParams);
         fill(c->err_hist, 0, sizeof(unsigned long long) * (PSB_MAX_ITERS + 1));
+        fill(c->flags, 0, 8 * sizeof(int));
         fill(c->d_loop, 0, sizeof(int) * (2 + 4 * s_));
         fill(c->d_active, 1, s_);
         fill(c->d_err_scene, 0, sizeof(unsigned long long) * s_);

@@ -367,8 +367,16 @@ __global__ void __launch_bounds__(kBlock) k_cell_count(Params P, const float4* _
 // 12 us for the five tiles of a 38,000-cell grid.
 __global__ void __launch_bounds__(kBlock) k_cell_scan(uint32_t* __restrict__ cell_count,
                                                       const uint32_t* __restrict__ tile_sum,
-                                                      uint32_t* __restrict__ cell_start) {
+                                                      uint32_t* __restrict__ cell_start, int* __restrict__ flags) {
     after_previous();
+    // the build's words: cleared here, not by a memset before the count pass,
+    // which cannot be placed early (16 DEM steps 597 -> 493 us without it and
+    // the error history's); the count pass has left its clamped count in flags[6]
+    if (blockIdx.x == 0 && threadIdx.x < 8) {
+        const int clamped = flags[6];
+        __syncwarp(0xffu);
+        flags[threadIdx.x] = threadIdx.x == 4 ? clamped : 0;
+    }
     constexpr int kRowsPerTile = kScanCells / (kBlock * 4), kWarps = kBlock / 32;
     static_assert(kRowsPerTile * kWarps == 64, "one warp scans the (row, warp) totals, two each");
     __shared__ uint32_t s_warp[kWarps], s_total[kRowsPerTile * kWarps];
@@ -828,15 +836,15 @@ void launch_cell_count(cudaStream_t st, const Params& P, const float4* pos, uint
                        uint32_t* cell_count, uint32_t* tile_sum, int* clamped) {
     if (P.n <= 0) return;
     auto kernel = P.scenes ? k_cell_count<true> : k_cell_count<false>;
-    kernel<<<grid_of(P.n), kBlock, 0, st>>>(P, pos, keys, ranks, cell_count, tile_sum, clamped);
+    launch_chained(kernel, grid_of(P.n), kBlock, 0, st, P, pos, keys, ranks, cell_count, tile_sum, clamped);
 }
 
 void launch_cell_sort(cudaStream_t st, int n, size_t ncells, const int* ids, const uint32_t* keys, const uint32_t* ranks,
-                      uint32_t* cell_count, uint32_t* tile_sum, uint32_t* cell_start, uint2* placed, uint32_t* keys_out,
-                      uint32_t* vals_out) {
+                      uint32_t* cell_count, uint32_t* tile_sum, uint32_t* cell_start, int* flags, uint2* placed,
+                      uint32_t* keys_out, uint32_t* vals_out) {
     if (n <= 0) return;
     const int tiles = (int)cell_sort_tiles(ncells);
-    launch_chained(k_cell_scan, tiles, kBlock, 0, st, cell_count, tile_sum, cell_start);
+    launch_chained(k_cell_scan, tiles, kBlock, 0, st, cell_count, tile_sum, cell_start, flags);
     launch_chained(k_cell_place, grid_of(std::max(n, tiles)), kBlock, 0, st, n, tiles, keys, ranks, ids, cell_start,
                    placed, tile_sum);
     launch_chained(k_cell_rank, grid_of(n), kBlock, 0, st, n, keys, placed, cell_start, keys_out, vals_out);

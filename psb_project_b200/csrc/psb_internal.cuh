@@ -344,15 +344,17 @@ bool small_sort(cudaStream_t st, int n, int bits, const uint32_t* keys_in, const
 // counts; launch_cell_sort turns the counts into cell_start (every cell; slots
 // [cell_start[c], cell_start[c + 1])), writes the sorted keys and the old slot
 // of each sorted one, and leaves counts and tile sums at zero, as both must
-// be before the first count. cell_count and cell_start hold
-// cell_sort_cells(ncells) words, tile_sum cell_sort_tiles(ncells); placed: n.
+// be before the first count; it clears the eight words at flags, keeping the
+// count of clamped particles that the count pass left at flags[6] in flags[4].
+// cell_count and cell_start hold cell_sort_cells(ncells) words, tile_sum
+// cell_sort_tiles(ncells); placed: n.
 size_t cell_sort_tiles(size_t ncells);
 size_t cell_sort_cells(size_t ncells);
 void launch_cell_count(cudaStream_t st, const Params& P, const float4* pos, uint32_t* keys, uint32_t* ranks,
                        uint32_t* cell_count, uint32_t* tile_sum, int* clamped);
 void launch_cell_sort(cudaStream_t st, int n, size_t ncells, const int* ids, const uint32_t* keys, const uint32_t* ranks,
-                      uint32_t* cell_count, uint32_t* tile_sum, uint32_t* cell_start, uint2* placed, uint32_t* keys_out,
-                      uint32_t* vals_out);
+                      uint32_t* cell_count, uint32_t* tile_sum, uint32_t* cell_start, int* flags, uint2* placed,
+                      uint32_t* keys_out, uint32_t* vals_out);
 // The whole state into sorted order, with the cell ranges; or in two
 // launches: positions, ids and cell ranges (what the neighbour build reads),
 // then the rest. cell_start null: the ranges are there already.
