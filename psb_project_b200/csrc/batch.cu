@@ -7,9 +7,9 @@
 // least min_iters corrections) and decides whether another pass is needed.
 // The pressure-force pass that follows skips retired scenes, so each scene
 // ends in the state it has when stepped alone: the same passes, in the same
-// order, on the same data. The decision reaches the host as one word, or,
-// inside a CUDA graph, the conditional handle of the while node that
-// repeats {density pass, decision, pressure-force pass}.
+// order, on the same data. The decision reaches the host as one word, written
+// into its memory, or, inside a CUDA graph, the conditional handle of the
+// while node that repeats {density pass, decision, pressure-force pass}.
 //
 // Loop words (device int array): [0] the pass index k, [1] continue,
 // [2, 2 + S) corrections per scene, [2 + S, 2 + 2S) converged per scene,
@@ -37,11 +37,13 @@ __global__ void __launch_bounds__(kLoopThreads) k_batch_decide(int S, int min_it
                                                               unsigned long long* __restrict__ err_scene,
                                                               unsigned long long* __restrict__ err_hist,
                                                               int* __restrict__ loop,
-                                                              cudaGraphConditionalHandle handle, int set_handle) {
+                                                              cudaGraphConditionalHandle handle, int set_handle,
+                                                              int* host_word) {
     after_previous();
     __shared__ int any;
     const int cont = corrector_decide(S, min_it, max_it, eta, active, err_scene, err_hist, loop, &any);
     if (threadIdx.x == 0 && set_handle) cudaGraphSetConditional(handle, cont ? 1u : 0u);
+    if (threadIdx.x == 0 && host_word) *(volatile int*)host_word = 1 + cont;
 }
 
 }  // namespace
@@ -53,9 +55,9 @@ void launch_batch_begin(cudaStream_t st, int S, int max_it, uint8_t* active, uns
 
 void launch_batch_decide(cudaStream_t st, int S, int min_it, int max_it, double eta, uint8_t* active,
                          unsigned long long* err_scene, unsigned long long* err_hist, int* loop,
-                         cudaGraphConditionalHandle handle, int set_handle) {
+                         cudaGraphConditionalHandle handle, int set_handle, int* host_word) {
     launch_chained(k_batch_decide, 1, kLoopThreads, 0, st, S, min_it, max_it, eta, active, err_scene, err_hist, loop,
-                   handle, set_handle);
+                   handle, set_handle, host_word);
 }
 
 }  // namespace psb

@@ -399,12 +399,13 @@ void launch_dem_forces(cudaStream_t st, const Params& P, const float4* pos, cons
 
 // ---- batched scenes: the corrector loop on the device (batch.cu) ---------------
 // loop: [0] pass index, [1] continue, [2, 2 + S) corrections, [2 + S, 2 + 2S) converged,
-// [2 + 2S, 2 + 3S) corrections summed over steps, [2 + 3S, 2 + 4S) unconverged steps
+// [2 + 2S, 2 + 3S) corrections summed over steps, [2 + 3S, 2 + 4S) unconverged steps;
+// host_word (if not null): set to 1 (stop) or 2 (another pass) by the decision
 void launch_batch_begin(cudaStream_t st, int S, int max_it, uint8_t* active, unsigned long long* err_scene,
                         unsigned long long* err_hist, int hist_len, int* loop);
 void launch_batch_decide(cudaStream_t st, int S, int min_it, int max_it, double eta, uint8_t* active,
                          unsigned long long* err_scene, unsigned long long* err_hist, int* loop,
-                         cudaGraphConditionalHandle handle, int set_handle);
+                         cudaGraphConditionalHandle handle, int set_handle, int* host_word);
 // The whole corrector loop of a config-profile scene or batch as one
 // cooperative launch (begin, then {density pass, decision, pressure-force
 // pass} until the decision ends it). Returns the launch's error.
