@@ -127,54 +127,173 @@ __global__ void __launch_bounds__(kBlock) k_build_bnd_nbr(Params P, const float4
 // F_b = - sum_j m a_j^b over the fluid particles j within h of the
 // boundary particle at xb, a_j^b = k_grad (psi_b / m) pV_j (1-u)^2 x^_jb
 // the mirrored-pressure acceleration the boundary particle gives j (sph.cu,
-// boundary_pressure); the fluid's cells are walked around xb.
+// boundary_pressure); the fluid's cells are walked around xb, row by row in
+// slot order. Two forms of the same sum, term by term in the same order:
+//   * one thread a boundary particle: ~216 candidates, one after another, a
+//     chain of ~20 us whatever the number of particles up to ~30k;
+//   * one warp a boundary particle: the lanes take 32 candidates of a row at
+//     a time, all nine rows' loads in flight together, and queue the accepted
+//     ones in slot order in shared memory; three lanes then add the queue, a
+//     component each. A shorter chain, but several times the instructions.
+// k_bnd_move, solids immersed in 262k fluid particles, threads against warps:
+// 500 boundary particles 27 and 8.8 us, 2,000 24 and 9.3, 8,000 19.5 and
+// 16.4, 16,000 19.5 and 23: warps up to kBndWarps.
+constexpr int kBndWarps = 8192;
+
+// The first cell of the walk in each direction, and the one behind the last.
+struct BndCells {
+    int lo[3], hi[3];
+};
+__device__ __forceinline__ BndCells bnd_cells(const Params& P, float4 xb) {
+    BndCells c;
+    const float lo[3] = {P.g.gx, P.g.gy, P.g.gz};
+    const float x[3] = {xb.x, xb.y, xb.z};
+    const int dims[3] = {P.g.nx, P.g.ny, P.g.nz};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const double q = floor(((double)x[a] - (double)lo[a]) / (double)P.g.cell);
+        const int i = q < 0.0 ? 0 : (q >= (double)dims[a] ? dims[a] - 1 : (int)q);
+        c.lo[a] = max(i - 1, 0);
+        c.hi[a] = min(i + 2, dims[a]);
+    }
+    return c;
+}
+
+// The slots of the walk's cells of row (j, k).
+__device__ __forceinline__ void bnd_row(const Params& P, const BndCells& c, int j, int k,
+                                        const uint32_t* __restrict__ cell_start, const uint32_t* __restrict__ cell_end,
+                                        uint32_t& lo, uint32_t& hi) {
+    const uint32_t row = (uint32_t)j * (uint32_t)P.g.nx + (uint32_t)k * (uint32_t)P.g.nx * (uint32_t)P.g.ny;
+    if (P.dense_cells) {
+        lo = cell_start[row + c.lo[0]];
+        hi = cell_end[row + c.hi[0] - 1];
+    } else {
+        row_range(cell_start, cell_end, row, c.lo[0], c.hi[0] - 1, lo, hi);
+    }
+}
+
+// d = x_j - x_b and its weight in the sum; false if the pair has none.
+__device__ __forceinline__ bool bnd_pair(const Params& P, float4 xb, float4 xj, const float& pj, float4& t) {
+    const float ir0 = 1.f / (P.rho0 * P.rho0);
+    const float dx = xj.x - xb.x, dy = xj.y - xb.y, dz = xj.z - xb.z;
+    const float r2 = dist2(dx, dy, dz);
+    if (!(r2 > 0.f) || r2 * P.inv_h2 >= 1.f) return false;
+    const float rinv = rsqrtf(r2);
+    const float om = __fmaf_rn(-(r2 * rinv), P.inv_h, 1.f);      // rounded alike in both forms
+    t = make_float4(dx, dy, dz, pj * ir0 * om * om * rinv);
+    return true;
+}
+
 __device__ float3 bnd_reaction_at(const Params& P, float4 xb, const float4* __restrict__ fluid_pos,
                                   const float2* __restrict__ fluid_rp, const uint32_t* __restrict__ cell_start,
                                   const uint32_t* __restrict__ cell_end) {
-    const int nx = P.g.nx, ny = P.g.ny, nz = P.g.nz;
-    int c[3];
-    const float lo[3] = {P.g.gx, P.g.gy, P.g.gz};
-    const float x[3] = {xb.x, xb.y, xb.z};
-    const int dims[3] = {nx, ny, nz};
-    for (int a = 0; a < 3; ++a) {
-        const double q = floor(((double)x[a] - (double)lo[a]) / (double)P.g.cell);
-        c[a] = q < 0.0 ? 0 : (q >= (double)dims[a] ? dims[a] - 1 : (int)q);
-    }
-    const float ir0 = 1.f / (P.rho0 * P.rho0);
+    const BndCells c = bnd_cells(P, xb);
     float3 s = make_float3(0.f, 0.f, 0.f);
-    for (int k = max(c[2] - 1, 0); k <= min(c[2] + 1, nz - 1); ++k)
-        for (int j = max(c[1] - 1, 0); j <= min(c[1] + 1, ny - 1); ++j) {
-            const uint32_t row = (uint32_t)j * (uint32_t)nx + (uint32_t)k * (uint32_t)nx * (uint32_t)ny;
-            for (int a = max(c[0] - 1, 0); a <= min(c[0] + 1, nx - 1); ++a) {
-                const uint32_t q0 = cell_start[row + a];
-                if (q0 == kEmpty) continue;
-                const uint32_t q1 = cell_end[row + a];
-                for (uint32_t q = q0; q < q1; ++q) {
-                    const float4 xj = fluid_pos[q];
-                    const float dx = xj.x - xb.x, dy = xj.y - xb.y, dz = xj.z - xb.z;
-                    const float r2 = dx * dx + dy * dy + dz * dz;
-                    if (!(r2 > 0.f) || r2 * P.inv_h2 >= 1.f) continue;
-                    const float rinv = rsqrtf(r2);
-                    const float om = 1.f - r2 * rinv * P.inv_h;
-                    const float w = fluid_rp[q].y * ir0 * om * om * rinv;
-                    s.x += w * dx; s.y += w * dy; s.z += w * dz;
-                }
+    for (int k = c.lo[2]; k < c.hi[2]; ++k)
+        for (int j = c.lo[1]; j < c.hi[1]; ++j) {
+            uint32_t lo, hi;
+            bnd_row(P, c, j, k, cell_start, cell_end, lo, hi);
+            for (uint32_t q = lo; q < hi; ++q) {
+                float4 t;
+                if (!bnd_pair(P, xb, fluid_pos[q], fluid_rp[q].y, t)) continue;
+                s.x = __fmaf_rn(t.w, t.x, s.x); s.y = __fmaf_rn(t.w, t.y, s.y); s.z = __fmaf_rn(t.w, t.z, s.z);
             }
         }
     const float k = -P.mass * P.k_grad * xb.w;
     return make_float3(k * s.x, k * s.y, k * s.z);
 }
 
-// Boundary slot b's reaction at the fluid's state.
+// The same by a whole warp (every lane calls it, every lane gets the sum);
+// queue: kBndQueue entries of the warp's own.
+constexpr int kBndQueue = 9 * 32;
+__device__ float3 bnd_reaction_warp(const Params& P, float4 xb, const float4* __restrict__ fluid_pos,
+                                    const float2* __restrict__ fluid_rp, const uint32_t* __restrict__ cell_start,
+                                    const uint32_t* __restrict__ cell_end, float4* queue) {
+    const int lane = threadIdx.x & 31;
+    const BndCells c = bnd_cells(P, xb);
+    // lane r < 9 finds row r's slots; a row outside the grid has none
+    uint32_t lo = 0u, hi = 0u;
+    {
+        const int j = c.lo[1] + lane % 3, k = c.lo[2] + lane / 3;
+        if (lane < 9 && j < c.hi[1] && k < c.hi[2]) bnd_row(P, c, j, k, cell_start, cell_end, lo, hi);
+    }
+    float4 x[9];
+    float p[9];
+#pragma unroll
+    for (int r = 0; r < 9; ++r) {
+        const uint32_t q = __shfl_sync(0xffffffffu, lo, r) + lane;
+        const bool in = q < __shfl_sync(0xffffffffu, hi, r);
+        x[r] = in ? fluid_pos[q] : make_float4(0.f, 0.f, 0.f, 0.f);
+        p[r] = in ? fluid_rp[q].y : 0.f;
+    }
+    float s = 0.f;          // lanes 0, 1, 2: the sum's x, y, z
+    int queued = 0;
+    auto add_queue = [&] {
+        __syncwarp();
+        if (lane < 3) {
+            const float* e = reinterpret_cast<const float*>(queue);
+#pragma unroll 4
+            for (int i = 0; i < queued; ++i) s = __fmaf_rn(e[4 * i + 3], e[4 * i + lane], s);
+        }
+        __syncwarp();
+        queued = 0;
+    };
+#pragma unroll
+    for (int r = 0; r < 9; ++r) {
+        const uint32_t q0 = __shfl_sync(0xffffffffu, lo, r), q1 = __shfl_sync(0xffffffffu, hi, r);
+        float4 xj = x[r];
+        float pj = p[r];
+        for (uint32_t q = q0 + lane; q - lane < q1; q += 32u) {
+            if (q - lane != q0 && q < q1) {         // past the row's first 32: loaded here
+                xj = fluid_pos[q];
+                pj = fluid_rp[q].y;
+            }
+            float4 t;
+            const bool take = q < q1 && bnd_pair(P, xb, xj, pj, t);
+            const unsigned taken = __ballot_sync(0xffffffffu, take);
+            if (take) queue[queued + __popc(taken & ((1u << lane) - 1u))] = t;
+            queued += __popc(taken);
+            if (queued > kBndQueue - 32) add_queue();
+        }
+    }
+    add_queue();
+    const float k = -P.mass * P.k_grad * xb.w;
+    return make_float3(k * __shfl_sync(0xffffffffu, s, 0), k * __shfl_sync(0xffffffffu, s, 1),
+                       k * __shfl_sync(0xffffffffu, s, 2));
+}
+
+// f(b, x_b, F) for the block's boundary slots b < nb, F the reaction on b.
+template <bool WARP, class Fn>
+__device__ __forceinline__ void for_each_reaction(const Params& P, int nb, const float4* __restrict__ fluid_pos,
+                                                  const float2* __restrict__ fluid_rp,
+                                                  const uint32_t* __restrict__ cell_start,
+                                                  const uint32_t* __restrict__ cell_end, Fn&& f) {
+    const int i = blockIdx.x * kBlock + threadIdx.x;
+    if constexpr (WARP) {
+        __shared__ float4 s_queue[kBlock / 32][kBndQueue];
+        const int b = i >> 5;
+        if (b >= nb) return;
+        const float4 xb = P.bnd[b];
+        const float3 F = bnd_reaction_warp(P, xb, fluid_pos, fluid_rp, cell_start, cell_end,
+                                           s_queue[threadIdx.x >> 5]);
+        if ((threadIdx.x & 31) == 0) f(b, xb, F);
+    } else {
+        if (i >= nb) return;
+        const float4 xb = P.bnd[i];
+        f(i, xb, bnd_reaction_at(P, xb, fluid_pos, fluid_rp, cell_start, cell_end));
+    }
+}
+
+// Boundary slots' reaction at the fluid's state.
+template <bool WARP>
 __global__ void __launch_bounds__(kBlock) k_bnd_reaction(Params P, int nb, const float4* __restrict__ fluid_pos,
                                                          const float2* __restrict__ fluid_rp,
                                                          const uint32_t* __restrict__ cell_start,
                                                          const uint32_t* __restrict__ cell_end,
                                                          float4* __restrict__ force) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nb) return;
-    const float3 F = bnd_reaction_at(P, P.bnd[b], fluid_pos, fluid_rp, cell_start, cell_end);
-    force[b] = make_float4(F.x, F.y, F.z, 0.f);
+    for_each_reaction<WARP>(P, nb, fluid_pos, fluid_rp, cell_start, cell_end, [&](int b, float4, float3 F) {
+        force[b] = make_float4(F.x, F.y, F.z, 0.f);
+    });
 }
 
 // Moving boundary: the reaction at the committed pressures of the current
@@ -183,6 +302,7 @@ __global__ void __launch_bounds__(kBlock) k_bnd_reaction(Params P, int nb, const
 // position updates are the DEM step's (v += (f + F) / m dt, x += v dt), so
 // the spheres' next positions are the last prediction's wherever no wall
 // projects them.
+template <bool WARP>
 __global__ void __launch_bounds__(kBlock) k_bnd_move(Params P, int nb, const float4* __restrict__ fluid_pos,
                                                      const float2* __restrict__ fluid_rp,
                                                      const uint32_t* __restrict__ cell_start,
@@ -191,17 +311,18 @@ __global__ void __launch_bounds__(kBlock) k_bnd_move(Params P, int nb, const flo
                                                      float inv_mass, float4* __restrict__ pred,
                                                      float4* __restrict__ force) {
     after_previous();
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nb) return;
-    const float4 xb = P.bnd[b];
-    const float3 F = bnd_reaction_at(P, xb, fluid_pos, fluid_rp, cell_start, cell_end);
-    const float4 v0 = vel[b], f = fext[b];
-    const float vx = v0.x + (f.x + F.x) * inv_mass * P.dt;
-    const float vy = v0.y + (f.y + F.y) * inv_mass * P.dt;
-    const float vz = v0.z + (f.z + F.z) * inv_mass * P.dt;
-    pred[b] = make_float4(xb.x + vx * P.dt, xb.y + vy * P.dt, xb.z + vz * P.dt, xb.w);
-    force[b] = make_float4(F.x, F.y, F.z, 0.f);
+    for_each_reaction<WARP>(P, nb, fluid_pos, fluid_rp, cell_start, cell_end, [&](int b, float4 xb, float3 F) {
+        const float4 v0 = vel[b], f = fext[b];
+        const float vx = v0.x + (f.x + F.x) * inv_mass * P.dt;
+        const float vy = v0.y + (f.y + F.y) * inv_mass * P.dt;
+        const float vz = v0.z + (f.z + F.z) * inv_mass * P.dt;
+        pred[b] = make_float4(xb.x + vx * P.dt, xb.y + vy * P.dt, xb.z + vz * P.dt, xb.w);
+        force[b] = make_float4(F.x, F.y, F.z, 0.f);
+    });
 }
+
+// Threads for nb boundary particles' reactions.
+inline int reaction_threads(int nb) { return nb <= kBndWarps ? nb * 32 : nb; }
 
 __global__ void k_gather4(int nb, const int* __restrict__ ids, const float4* __restrict__ src,
                           float4* __restrict__ dst) {
@@ -214,9 +335,10 @@ __global__ void k_gather4(int nb, const int* __restrict__ ids, const float4* __r
 void launch_bnd_move(cudaStream_t st, const Params& P, int nb, const float4* fluid_pos, const float2* fluid_rp,
                      const uint32_t* cell_start, const uint32_t* cell_end, const float4* vel, const float4* fext,
                      float inv_mass, float4* pred, float4* force) {
-    if (nb > 0)
-        launch_chained(k_bnd_move, blocks_for(nb), kBlock, 0, st, P, nb, fluid_pos, fluid_rp, cell_start, cell_end,
-                       vel, fext, inv_mass, pred, force);
+    if (nb <= 0) return;
+    auto kernel = nb <= kBndWarps ? k_bnd_move<true> : k_bnd_move<false>;
+    launch_chained(kernel, blocks_for(reaction_threads(nb)), kBlock, 0, st, P, nb, fluid_pos, fluid_rp, cell_start,
+                   cell_end, vel, fext, inv_mass, pred, force);
 }
 
 void launch_bnd_gather4(cudaStream_t st, int nb, const int* ids, const float4* src, float4* dst) {
@@ -225,8 +347,9 @@ void launch_bnd_gather4(cudaStream_t st, int nb, const int* ids, const float4* s
 
 void launch_bnd_reaction(cudaStream_t st, const Params& P, int nb, const float4* fluid_pos, const float2* fluid_rp,
                          const uint32_t* cell_start, const uint32_t* cell_end, float4* force) {
-    if (nb > 0)
-        k_bnd_reaction<<<blocks_for(nb), kBlock, 0, st>>>(P, nb, fluid_pos, fluid_rp, cell_start, cell_end, force);
+    if (nb <= 0) return;
+    auto kernel = nb <= kBndWarps ? k_bnd_reaction<true> : k_bnd_reaction<false>;
+    kernel<<<blocks_for(reaction_threads(nb)), kBlock, 0, st>>>(P, nb, fluid_pos, fluid_rp, cell_start, cell_end, force);
 }
 
 int launch_bnd_prepare(cudaStream_t st, const Params& P, int nb, const float4* raw, int* iota, uint32_t* keys[2],
