@@ -140,7 +140,8 @@ struct Params {
     // SPH: the step's start positions and velocities in sorted order, as its
     // sweeps gather them, written by the reorder; and the two z components
     // once more beside the scalar that the pressure and set-up sums want with
-    // them: (z, pressure) and (v_z, density). The density passes write those.
+    // them: (z, pressure) and (v_z, 1 / density) -- the division once a particle,
+    // not once a pair. The density passes write those.
     Soa3 x0, v0;
     float2* zp;
     float2* vr;

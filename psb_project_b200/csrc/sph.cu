@@ -486,15 +486,15 @@ struct DensityX {
         rho_x[t] = rho;
         // what the set-up or force sweep gathers beside the xy components
         P.zp[t] = make_float2(xi.z, p);
-        P.vr[t] = make_float2(FEAT ? vi.z : P.v0.z[t], rho);
+        P.vr[t] = make_float2(FEAT ? vi.z : P.v0.z[t], 1.f / rho);
     }
 };
 
 // Resident threads per SM asked of the sweeps with ghost terms: what the
-// main walk's registers allow (40, 48 or 56 a thread), so that the ghost
+// main walk's registers allow (40 or 48 a thread), so that the ghost
 // walk, which few threads take, spills rather than lowering the occupancy of
 // all (density pass at 4M particles: 272 us at 40 registers, 354 at 56).
-constexpr int kDensityThreads = 1536, kForceThreads = 1280, kInitThreads = 1152;
+constexpr int kDensityThreads = 1536, kForceThreads = 1280;
 
 template <bool REF, int NF, bool BATCH, int BS>
 __global__ void __launch_bounds__(BS, REF ? 1 : (NF ? kForceThreads : kDensityThreads) / BS)
@@ -568,10 +568,10 @@ __device__ __forceinline__ float pressure_volume(const Params& P, float2 rp) {
     return REF ? rp.y / (rp.x * rp.x) : rp.y * (1.f / (P.rho0 * P.rho0));
 }
 
-// Adds the pair (i, j) to S; xj, rpj: neighbour j's position, (density, pressure).
+// Adds the pair (i, j) to S; xj, inv_rj, pj: neighbour j's position, 1 / density, pressure.
 template <bool REF, bool WITH_PRESSURE>
 __device__ __forceinline__ void add_pair(const Params& P, PairSums& S, float4 xi, float4 vi, float pVi, float4 xj,
-                                         float4 vj, float2 rpj) {
+                                         float4 vj, float inv_rj, float pj) {
     const float ir0 = 1.f / (P.rho0 * P.rho0);
     const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
     const float r2 = dist2(dx, dy, dz);
@@ -580,13 +580,12 @@ __device__ __forceinline__ void add_pair(const Params& P, PairSums& S, float4 xi
     if (!REF && q >= 1.f) return;
     const float rinv = rsqrtf(r2);
     const float om = 1.f - r2 * rinv * P.inv_h;
-    const float inv_rj = 1.f / rpj.x;
     const float sv = om * inv_rj;
     S.fv.x += (vj.x - vi.x) * sv;
     S.fv.y += (vj.y - vi.y) * sv;
     S.fv.z += (vj.z - vi.z) * sv;
     if (WITH_PRESSURE) {
-        const float pVj = REF ? rpj.y * inv_rj * inv_rj : rpj.y * ir0;
+        const float pVj = REF ? pj * inv_rj * inv_rj : pj * ir0;
         const float s = (pVi + pVj) * om * om * rinv;
         S.ap.x += s * dx; S.ap.y += s * dy; S.ap.z += s * dz;
     }
@@ -610,7 +609,7 @@ __device__ __forceinline__ PairSums pair_sums(const Params& P, int t, float4 xi,
         // the pair's four 8-byte gathers, ahead of the tests
         const float2 xy = P.x0.xy[j], zp = P.zp[j], vxy = P.v0.xy[j], vr = P.vr[j];
         add_pair<REF, WITH_PRESSURE>(P, S, xi, vi, pVi, make_float4(xy.x, xy.y, zp.x, 0.f),
-                                     make_float4(vxy.x, vxy.y, vr.x, 0.f), make_float2(vr.y, zp.y));
+                                     make_float4(vxy.x, vxy.y, vr.x, 0.f), vr.y, zp.y);
     });
     if (WITH_PRESSURE && !REF) {
         ghost_pressure<BATCH>(P, t, xi, pVi, list, cnt, S.ap);
@@ -669,8 +668,11 @@ __global__ void __launch_bounds__(kBlock) k_wcsph_force(Params P, const float4* 
 
 // PCISPH set-up sweep: non-pressure forces at x (and, for a warm start, the
 // pressure acceleration of the carried pressure), then the first prediction.
+// Four 8-byte gathers a pair: bound by L1 wavefronts. With 1 / rho_j gathered
+// instead of rho_j (the division was ~10 of 79 instructions a pair) it takes
+// 147 us at 1M particles against 166, 538 at 4M against 613.
 template <bool REF, bool WARM, bool BATCH, int BS>
-__global__ void __launch_bounds__(BS, REF || !WARM ? 1 : kInitThreads / BS) k_pci_init(
+__global__ void __launch_bounds__(BS, REF || !WARM ? 1 : kForceThreads / BS) k_pci_init(
     Params P, const float4* __restrict__ vap, const float2* __restrict__ rp, const int* __restrict__ counts,
     const int* __restrict__ list, float4* __restrict__ fnp, Soa3 xs, Soa3 vs) {
     after_previous();
