@@ -1076,7 +1076,7 @@ int create_impl(const psb_scene* scene, size_t ncells, int S, bool batch, psb_ct
             at += (std::max<size_t>(count, 1) * sizeof(*p) + 511) & ~(size_t)511;
         };
         for (int i = 0; i < 2; ++i) {
-            take(c->pos[i], n + 3);     // the neighbour build reads a row in fours, up to three past its end
+            take(c->pos[i], n + 3);     // the iso field reads a row in fours, up to three past its end
             take(c->vel[i], n); take(c->vap[i], n); take(c->rp[i], n); take(c->ids[i], n);
             take(c->keys[i], n); take(c->vals[i], n);
             take(c->xs[i].xy, n); take(c->xs[i].z, n);
@@ -1094,8 +1094,10 @@ int create_impl(const psb_scene* scene, size_t ncells, int S, bool batch, psb_ct
         take(c->nbr_count, n); take(c->nbr_list, psb::nbr_list_ints(n, c->cap));
         take(c->fnp, n); take(c->vs.xy, n); take(c->vs.z, n); take(c->rpc, n); take(c->rho_x, n);
         take(c->err_hist, PSB_MAX_ITERS + 1); take(c->flags, 8);
+        // (the neighbour build reads these in aligned fours, within take's rounding)
+        take(c->P.cx, n); take(c->P.cy, n); take(c->P.x0.z, n);
         if (!c->P.dem) {
-            take(c->P.x0.xy, n); take(c->P.x0.z, n); take(c->P.v0.xy, n); take(c->P.v0.z, n);
+            take(c->P.x0.xy, n); take(c->P.v0.xy, n); take(c->P.v0.z, n);
             take(c->P.zp, n); take(c->P.vr, n);
         }
         if (ghosts) {       // config-profile SPH: the wall list and its flags

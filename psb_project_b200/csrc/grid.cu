@@ -488,9 +488,11 @@ __global__ void k_reorder(Params P, const uint32_t* __restrict__ keys, const uin
     const float4 v = vel[s];
     pos2[t] = x;
     vel2[t] = v;
+    P.cx[t] = x.x;
+    P.cy[t] = x.y;
+    P.x0.z[t] = x.z;
     if (P.x0.xy) {
         P.x0.xy[t] = make_float2(x.x, x.y);
-        P.x0.z[t] = x.z;
         P.v0.xy[t] = make_float2(v.x, v.y);
         P.v0.z[t] = v.z;
     }
@@ -519,9 +521,11 @@ __global__ void k_reorder_pos(Params P, const uint32_t* __restrict__ keys, const
     list_near_walls<BATCH>(P, t, x);
     if (t >= n) return;
     pos2[t] = x;
+    P.cx[t] = x.x;
+    P.cy[t] = x.y;
+    P.x0.z[t] = x.z;
     if (P.x0.xy) {
         P.x0.xy[t] = make_float2(x.x, x.y);
-        P.x0.z[t] = x.z;
     }
     ids2[t] = ids[s];
     if (!cell_start) return;
@@ -555,53 +559,79 @@ __global__ void k_reorder_state(Params P, const uint32_t* __restrict__ vals, con
 // the list is sorted. In a batch the walk stays inside the particle's
 // scene's grid.
 //
-// ~216 candidates are tested for ~33 kept, so the test is kept to the load,
-// six FP32 operations and one shift: with e = |d|^2 - h^2 in one FMA chain, a
-// funnel shift collects e's sign into the row's mask, and a second mask says
-// which fours of candidates hold one within rounding of the cut-off: only
-// those are gone over again with the reference's FP64 test. (A block of fluid
-// started on a lattice of spacing h/2 has candidates at exactly h in five of
-// its nine rows; going over the whole row took 198 us at 1M such particles
-// and 26.9 at 16k, the fours 184 and 23.0.) The masks of the nine rows wait in shared memory; the list is then
-// written quad by quad, every lane's k-th quad in the same store (512
-// contiguous bytes a warp), where one 4-byte store per entry was a sector
-// write for each of 34M entries at 1M particles.
-// A candidate used to cost ~30 issued instructions (its own accept branch,
-// taken by some lane nearly every time) and costs ~10 now.
+// ~216 candidates are tested for ~33 kept, so the kernel is bound by the
+// instructions and the L1 wavefronts of the test. It is kept to seven
+// instructions a candidate: x, y and z lie in arrays of their own (the reorder
+// writes them beside the position), a row is read in aligned fours -- three
+// 16-byte loads for four candidates instead of four -- and two candidates
+// share an instruction of the FMA chain e = |d|^2 - h^2 (f32x2). A funnel
+// shift collects e's sign into the row's mask, and a second mask says which
+// fours hold a candidate within rounding of the cut-off: only those are gone
+// over again with the reference's FP64 test. (A block of fluid started on a
+// lattice of spacing h/2 has candidates at exactly h in five of its nine rows;
+// going over the whole row took 198 us at 1M such particles and 26.9 at 16k,
+// the fours 184 and 23.0.) The masks of the nine rows wait in shared memory;
+// the list is then written quad by quad, every lane's k-th quad in the same
+// store (512 contiguous bytes a warp), where one 4-byte store per entry was a
+// sector write for each of 34M entries at 1M particles.
+// One candidate after another from the float4 positions, eleven instructions
+// each: 184 us at 1M particles, 654 at 4M, 36 at 97k; now 151, 555 and 27.
+// Loading a four ahead of the one in use: 12 registers more, 163 us at 1M.
 constexpr int kRows = 9;
 
-// The candidates of one row, slots [lo, lo + m) with 1 <= m <= 32: bit 31 - c
-// of the result is set when slot lo + c is a neighbour of the particle at pi.
-// Reads up to three slots past the range (pos is padded by as many).
-__device__ __forceinline__ uint32_t row_mask(const Params& P, float4 pi, const float4* __restrict__ pos, uint32_t lo,
-                                             uint32_t m) {
-    const float4* __restrict__ x = pos + lo;
+// Two FP32 operations of one instruction.
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 d;
+    asm("add.rn.f32x2 %0, %1, %2;"
+        : "=l"(reinterpret_cast<unsigned long long&>(d))
+        : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
+    return d;
+}
+__device__ __forceinline__ float2 square_plus2(float2 a, float2 c) {
+    float2 d;
+    asm("fma.rn.f32x2 %0, %1, %1, %2;"
+        : "=l"(reinterpret_cast<unsigned long long&>(d))
+        : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(c)));
+    return d;
+}
+
+// The candidates of the row [lo, hi) among the 32 slots from w on (a multiple
+// of four below hi): bit 31 - c of the result is set when slot w + c is one
+// and a neighbour of the particle at pi. Reads whole fours.
+__device__ __forceinline__ uint32_t row_mask(const Params& P, float4 pi, uint32_t w, uint32_t lo, uint32_t hi) {
+    const float4* __restrict__ X = reinterpret_cast<const float4*>(P.cx + w);
+    const float4* __restrict__ Y = reinterpret_cast<const float4*>(P.cy + w);
+    const float4* __restrict__ Z = reinterpret_cast<const float4*>(P.x0.z + w);
     // h2_hi - h2 is 1e-5 h^2, some thirty times the rounding of e near h
     const float band = P.h2_hi - P.h2;
+    const uint32_t first = lo > w ? lo - w : 0u, end = min(hi - w, 32u), groups = (end + 3u) >> 2;
     uint32_t mask = 0u, close = 0u;      // close: one bit per four candidates, the last four lowest
-    auto excess = [&](float4 pj) {
-        const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-        return __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmaf_rn(dx, dx, -P.h2)));
+    const float2 px = make_float2(-pi.x, -pi.x), py = make_float2(-pi.y, -pi.y), pz = make_float2(-pi.z, -pi.z);
+    const float2 cut = make_float2(-P.h2, -P.h2);
+    auto excess = [&](float2 x, float2 y, float2 z) {
+        return square_plus2(add2(z, pz), square_plus2(add2(y, py), square_plus2(add2(x, px), cut)));
     };
-    for (uint32_t c = 0; c < m; c += 4) {
-        const float4 a0 = x[c], a1 = x[c + 1], a2 = x[c + 2], a3 = x[c + 3];
-        const float e0 = excess(a0), e1 = excess(a1), e2 = excess(a2), e3 = excess(a3);
-        mask = __funnelshift_l(__float_as_uint(e0), mask, 1);
-        mask = __funnelshift_l(__float_as_uint(e1), mask, 1);
-        mask = __funnelshift_l(__float_as_uint(e2), mask, 1);
-        mask = __funnelshift_l(__float_as_uint(e3), mask, 1);
-        const float near = fminf(fminf(fabsf(e0), fabsf(e1)), fminf(fabsf(e2), fabsf(e3)));
+    for (uint32_t g = 0; g < groups; ++g) {
+        const float4 x = X[g], y = Y[g], z = Z[g];
+        const float2 a = excess(make_float2(x.x, x.y), make_float2(y.x, y.y), make_float2(z.x, z.y));
+        const float2 b = excess(make_float2(x.z, x.w), make_float2(y.z, y.w), make_float2(z.z, z.w));
+        mask = __funnelshift_l(__float_as_uint(a.x), mask, 1);
+        mask = __funnelshift_l(__float_as_uint(a.y), mask, 1);
+        mask = __funnelshift_l(__float_as_uint(b.x), mask, 1);
+        mask = __funnelshift_l(__float_as_uint(b.y), mask, 1);
+        const float near = fminf(fminf(fabsf(a.x), fabsf(a.y)), fminf(fabsf(b.x), fabsf(b.y)));
         close = __funnelshift_l(__float_as_uint(near - band), close, 1);
     }
-    const uint32_t groups = (m + 3u) >> 2;
-    mask = (mask << (32u - 4u * groups)) & (kEmpty << (32u - m));
+    mask = (mask << (32u - 4u * groups)) & (kEmpty << (32u - end)) & (kEmpty >> first);
     while (close) {
         const uint32_t low = (uint32_t)__ffs((int)close) - 1u;
         close &= close - 1u;
         const uint32_t c0 = 4u * (groups - 1u - low);
-        for (uint32_t c = c0; c < min(c0 + 4u, m); ++c) {
-            const float4 pj = x[c];
-            if (!(fabsf(excess(pj)) <= band)) continue;
+        for (uint32_t c = max(c0, first); c < min(c0 + 4u, end); ++c) {
+            const float4 pj = make_float4(P.cx[w + c], P.cy[w + c], P.x0.z[w + c], 0.f);
+            const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+            const float e = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmaf_rn(dx, dx, -P.h2)));
+            if (!(fabsf(e) <= band)) continue;
             const uint32_t bit = 0x80000000u >> c;
             if (exact_neighbor(pi, pj, P.h2_exact)) mask |= bit;
             else mask &= ~bit;
@@ -611,8 +641,7 @@ __device__ __forceinline__ uint32_t row_mask(const Params& P, float4 pi, const f
 }
 
 template <bool BATCH, int BS>
-__global__ void __launch_bounds__(BS) k_build_nbr(Params P, const float4* __restrict__ pos,
-                                                  const uint32_t* __restrict__ keys,
+__global__ void __launch_bounds__(BS) k_build_nbr(Params P, const uint32_t* __restrict__ keys,
                                                   const uint32_t* __restrict__ cell_start,
                                                   const uint32_t* __restrict__ cell_end, int* __restrict__ counts,
                                                   int* __restrict__ list, int* __restrict__ flags) {
@@ -647,13 +676,14 @@ __global__ void __launch_bounds__(BS) k_build_nbr(Params P, const float4* __rest
             }
             s_first[r][tid] = lo;
             s_mask[r][tid] = hi;
-            longest = max(longest, hi - lo);
+            longest = max(longest, hi - (lo & ~3u));
         }
-        const float4 pi = pos[t];
+        const float4 pi = make_float4(P.cx[t], P.cy[t], P.x0.z[t], 0.f);
         if (longest <= 32u) {
             for (int r = 0; r < kRows; ++r) {
-                const uint32_t lo = s_first[r][tid], m = s_mask[r][tid] - lo;
-                const uint32_t mask = m ? row_mask(P, pi, pos, lo, m) : 0u;
+                const uint32_t lo = s_first[r][tid], hi = s_mask[r][tid], w = lo & ~3u;
+                const uint32_t mask = lo < hi ? row_mask(P, pi, w, lo, hi) : 0u;
+                s_first[r][tid] = w;
                 s_mask[r][tid] = mask;
                 cnt += __popc(mask);
             }
@@ -683,9 +713,10 @@ __global__ void __launch_bounds__(BS) k_build_nbr(Params P, const float4* __rest
             }
         } else {        // a row of more than 32 candidates: 32 at a time, an entry a store
             for (int r = 0; r < kRows; ++r) {
-                const uint32_t hi = s_mask[r][tid];
-                for (uint32_t lo = s_first[r][tid]; lo < hi; lo += 32u) {
-                    uint32_t mask = row_mask(P, pi, pos, lo, min(hi - lo, 32u)), q = lo;
+                const uint32_t lo = s_first[r][tid], hi = s_mask[r][tid];
+                if (lo >= hi) continue;
+                for (uint32_t w = lo & ~3u; w < hi; w += 32u) {
+                    uint32_t mask = row_mask(P, pi, w, lo, hi), q = w;
                     while (mask) {
                         const int z = __clz((int)mask);
                         mask = (mask << z) << 1;
@@ -893,10 +924,13 @@ void launch_build_nbr(cudaStream_t st, const Params& P, const float4* pos, const
         constexpr int BS = decltype(B)::value;
         const unsigned g = (unsigned)((P.n + BS - 1) / BS);
         auto go = [&](auto kernel) {
+            launch_chained(kernel, g, BS, 0, st, P, keys, cell_start, cell_end, counts, list, flags);
+        };
+        auto go_tile = [&](auto kernel) {
             launch_chained(kernel, g, BS, 0, st, P, pos, keys, cell_start, cell_end, counts, list, flags);
         };
         if (P.tune.nbr_schedule == 1) {
-            if (P.scenes) go(k_build_nbr_tile<true, BS>); else go(k_build_nbr_tile<false, BS>);
+            if (P.scenes) go_tile(k_build_nbr_tile<true, BS>); else go_tile(k_build_nbr_tile<false, BS>);
         } else {
             if (P.scenes) go(k_build_nbr<true, BS>); else go(k_build_nbr<false, BS>);
         }

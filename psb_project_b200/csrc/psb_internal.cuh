@@ -143,6 +143,7 @@ struct Params {
     // them: (z, pressure) and (v_z, 1 / density) -- the division once a particle,
     // not once a pair. The density passes write those.
     Soa3 x0, v0;
+    float *cx, *cy;     // x0's x and y once more, each alone, for the neighbour build (DEM: with x0.z, all it has of x0)
     float2* zp;
     float2* vr;
     int dense_cells;    // the cell ranges cover every cell (the counting sort's), empty ones included
