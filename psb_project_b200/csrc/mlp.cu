@@ -322,7 +322,6 @@ __global__ void __launch_bounds__(kTrainWarps * 32, ACT == kRelu ? 3 : 1) k_mlp_
                                                                   const __nv_bfloat16* __restrict__ w,
                                                                   float* __restrict__ partial) {
     using L = Layout<NIN>;
-    after_previous();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TrainSmem& S = *reinterpret_cast<TrainSmem*>(smem_raw);
     const int lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3, wp = threadIdx.x >> 5;
@@ -344,9 +343,12 @@ __global__ void __launch_bounds__(kTrainWarps * 32, ACT == kRelu ? 3 : 1) k_mlp_
         t0 = v0 ? T[row0] : 0.f;
         t1 = v1 ? T[row1] : 0.f;
     };
+    // (the samples are no chained kernel's output: they are fetched while the
+    // previous step's reduction runs, 64 steps 2453 -> 2385 us)
     fetch(blockIdx.x);
-    stage_weights<NIN>(w, S.W1, S.W2, S.W2T, S.B1, S.B2, S.W3, &S.B3);
     for (int i = threadIdx.x; i < kTrainWarps * (3 * kH + 2); i += blockDim.x) (&S.G[0][0])[i] = 0.f;
+    after_previous();
+    stage_weights<NIN>(w, S.W1, S.W2, S.W2T, S.B1, S.B2, S.W3, &S.B3);
     __syncthreads();
 
     const float inv_b = 1.f / (float)batch;

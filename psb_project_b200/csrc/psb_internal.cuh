@@ -161,7 +161,8 @@ constexpr int kWallListMin = 131072;
 // placed while the stream's previous kernel still runs, once all of that one's
 // blocks have passed their own wait: its launch and block start-up overlap the
 // previous kernel's tail instead of following it. Such a kernel begins with
-// after_previous(), in every thread and before any access to memory: it waits
+// after_previous(), in every thread and before any access to memory that a
+// chained kernel ever writes: it waits
 // until the previous kernel has ended and its writes are visible -- so kernels
 // still run one after another, and a kernel's end implies the end of all
 // before it -- and then lets the next one be placed. (Letting it be placed
