@@ -172,7 +172,8 @@ __global__ void k_iso_weight(int n, double k_colour, const float2* __restrict__ 
 // by L1 wavefronts (93% of the data pipe with a node a thread, FP64 17%):
 // 128^3 nodes over 262,144 particles took 518 us in node order with every
 // candidate in FP64, 475 with the FP32 test, 412 with a warp's nodes in a
-// brick, 273 with 2 x 2 x 1 nodes a thread, 247 with 2 x 2 x 2. Nodes further
+// brick, 273 with 2 x 2 x 1 nodes a thread, 247 with 2 x 2 x 2, 215 with the
+// FP32 test axis by axis instead of over the eight nodes. Nodes further
 // apart than half a cell share too little and take a thread each, and so do
 // the nodes of grids too small to fill the chip with eighths (64^3: 77 us
 // with a node a thread, 112 with eight; 80^3: 85 with eight, 117 for the kernel
@@ -238,24 +239,16 @@ __global__ void __launch_bounds__(128) k_iso_field(IsoParams Q, Params P, const 
 #pragma unroll
                     for (uint32_t u = 0; u < 2; ++u) {
                         const float4 x = pos[lo + c + u];       // padded past the last particle
-                        float best = INFINITY;
+                        // the nearest node's distance: the nearest on each axis, as rounding is monotonic
+                        float dx = fabsf(fx[0] - x.x), dy = fabsf(fy[0] - x.y), dz = fabsf(fz[0] - x.z);
 #pragma unroll
-                        for (int g = 0; g < E; ++g) {
-                            const float dz = fz[g] - x.z;
-                            const float bz = __fmaf_rn(dz, dz, r2);
-#pragma unroll
-                            for (int f = 0; f < E; ++f) {
-                                const float dy = fy[f] - x.y;
-                                const float b = __fmaf_rn(dy, dy, bz);
-#pragma unroll
-                                for (int e = 0; e < E; ++e) {
-                                    const float dx = fx[e] - x.x;
-                                    const float d = __fmaf_rn(dx, dx, b);
-                                    best = E == 1 ? d : fminf(best, d);
-                                }
-                            }
+                        for (int e = 1; e < E; ++e) {
+                            dx = fminf(dx, fabsf(fx[e] - x.x));
+                            dy = fminf(dy, fabsf(fy[e] - x.y));
+                            dz = fminf(dz, fabsf(fz[e] - x.z));
                         }
-                        // a NaN position stays in, as in the FP64 test (fminf passes over it)
+                        const float best = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmaf_rn(dz, dz, r2)));
+                        // a NaN position stays in, as in the FP64 test
                         const bool in = !(best >= 0.f && best < INFINITY);
                         mask = mask << 1 | (in ? 1u : 0u);
                     }

@@ -162,15 +162,14 @@ constexpr int kWallListMin = 131072;
 // blocks have passed their own wait: its launch and block start-up overlap the
 // previous kernel's tail instead of following it. Such a kernel begins with
 // after_previous(), in every thread and before any access to memory that a
-// chained kernel ever writes: it waits
-// until the previous kernel has ended and its writes are visible -- so kernels
-// still run one after another, and a kernel's end implies the end of all
-// before it -- and then lets the next one be placed. (Letting it be placed
-// before the wait put several kernels' blocks on the chip at once: a 16k
-// particle WCSPH frame 843 us, 752 this way, 840 without.) Launched the usual
-// way the wait returns at once. Kernels that follow something other than a
-// kernel (a memset, a waited event, a loop node of a graph) are launched the
-// usual way.
+// chained kernel ever writes: it waits until the previous kernel has ended and
+// its writes are visible -- so kernels still run one after another, and a
+// kernel's end implies the end of all before it -- and then lets the next one
+// be placed. (Letting it be placed before the wait put several kernels' blocks
+// on the chip at once: a 16k particle WCSPH frame 843 us, 752 this way, 840
+// without.) Launched the usual way the wait returns at once. Kernels that
+// follow something other than a kernel (a memset, a waited event, a loop node
+// of a graph) are launched the usual way.
 __device__ __forceinline__ void after_previous() {
     cudaGridDependencySynchronize();
     cudaTriggerProgrammaticLaunchCompletion();
