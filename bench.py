@@ -51,6 +51,8 @@ UNIT = "particle-steps/s"
 ALG_BYTES = {
     "cell_keys": 24,          # pos 16 -> key + id 8
     "cell_sort": 16,          # keys and ranks in, sorted keys and slots out
+    "cell_place": 12,         # below 131,072 particles: keys and ranks in, (id, slot) in arrival order out ...
+    "rank_reorder": 93,       # ... then the sorted keys and slots and the whole state
     "radix_sort": 16,         # one read + write of the (key, value) pairs
     "reorder": 77,            # pos, vel, pressure 36 in + 36 out, cell ranges 5
     "reorder_pos": 53,        # after an upload: slot + key 8, pos + id 20 in and out, cell ranges 5
@@ -69,9 +71,9 @@ TUNE_KEYS = ("bucket", "nbr_block", "nbr_schedule", "density_block", "init_block
 
 
 # Kernels per timed group (radix_sort is 3 kernels per 8-bit pass, cell_sort
-# the scan, the placing and the ranking).
+# the scan, the placing and the ranking, cell_place the first two of them).
 def _kernels_per_group(name: str, sort_passes: int) -> int:
-    return 3 * sort_passes if name == "radix_sort" else 3 if name == "cell_sort" else 1
+    return {"radix_sort": 3 * sort_passes, "cell_sort": 3, "cell_place": 2}.get(name, 1)
 
 
 CORRECTOR_KERNELS = ("batch_begin", "pci_density", "batch_decide", "pci_force_predict")

@@ -575,36 +575,50 @@ int build(psb_ctx* c, bool keep_p = false, bool features = false) {
     // the counting sort clears the words itself
     if (!c->dense || n <= 0) cudaMemsetAsync(c->flags, 0, 8 * sizeof(int), st);
     int res = 0;
-    uint32_t* range_start = c->cell_start;      // the reorder records the cell ranges
-    if (c->dense) {
-        timed(c, "cell_keys", [&] {
-            psb::launch_cell_count(st, P, c->pos[c->cs], c->keys[0], c->vals[0], c->cell_count, c->tile_sum, &c->flags[6]);
-        });
-        // the predictor's x* buffer is free until the set-up sweep
-        timed(c, "cell_sort", [&] {
-            psb::launch_cell_sort(st, n, c->ncells, c->ids[c->cr], c->keys[0], c->vals[0], c->cell_count, c->tile_sum,
-                                  c->cell_start, c->flags, reinterpret_cast<uint2*>(c->xs[0].xy), c->keys[1], c->vals[1]);
-        });
-        res = 1;
-        range_start = nullptr;
-    } else {
-        timed(c, "cell_keys", [&] {
-            psb::launch_cell_keys(st, P, c->pos[c->cs], c->ids[c->cr], c->keys[0], c->vals[0], &c->flags[4]);
-        });
-        timed(c, "radix_sort", [&] { res = psb::radix_sort(st, n, c->key_bits, c->keys, c->vals, c->hist, c->hist_blocks); });
-    }
     const int os = c->cs, orr = c->cr, ns = os ^ 1, nr = orr ^ 1;
     // The first step after an upload gathers the positions first and the
     // rest of the state after its neighbour build, once the upload's copies
     // of it are in: they overlap the grid and the build. Other steps gather
-    // everything in one launch.
+    // everything in one launch, small ones in the sort's last.
     const bool split = capturing(st) ? c->capture_split : c->in_pending;
+    const bool fused = c->dense && !split && n < psb::kWallListMin;
+    uint32_t* range_start = c->cell_start;      // the reorder records the cell ranges
+    if (c->dense) {
+        timed(c, "cell_keys", [&] {
+            psb::launch_cell_count(st, P, c->pos[os], c->keys[0], c->vals[0], c->cell_count, c->tile_sum, &c->flags[6]);
+        });
+        // the predictor's x* buffer is free until the set-up sweep
+        uint2* placed = reinterpret_cast<uint2*>(c->xs[0].xy);
+        if (fused) {
+            timed(c, "cell_place", [&] {
+                psb::launch_cell_place(st, n, c->ncells, c->ids[orr], c->keys[0], c->vals[0], c->cell_count, c->tile_sum,
+                                       c->cell_start, c->flags, placed);
+            });
+            timed(c, "rank_reorder", [&] {
+                psb::launch_rank_reorder(st, P, c->keys[0], placed, c->cell_start, c->pos[os], c->vel[os], c->vap[os],
+                                         c->rp[orr], c->ids[orr], c->keys[1], c->vals[1], c->pos[ns], c->vel[ns],
+                                         c->vap[ns], c->rp[nr], c->ids[nr]);
+            });
+        } else {
+            timed(c, "cell_sort", [&] {
+                psb::launch_cell_sort(st, n, c->ncells, c->ids[orr], c->keys[0], c->vals[0], c->cell_count, c->tile_sum,
+                                      c->cell_start, c->flags, placed, c->keys[1], c->vals[1]);
+            });
+        }
+        res = 1;
+        range_start = nullptr;
+    } else {
+        timed(c, "cell_keys", [&] {
+            psb::launch_cell_keys(st, P, c->pos[os], c->ids[orr], c->keys[0], c->vals[0], &c->flags[4]);
+        });
+        timed(c, "radix_sort", [&] { res = psb::radix_sort(st, n, c->key_bits, c->keys, c->vals, c->hist, c->hist_blocks); });
+    }
     if (split) {
         timed(c, "reorder_pos", [&] {
             psb::launch_reorder_pos(st, P, c->keys[res], c->vals[res], c->pos[os], c->ids[orr], c->pos[ns], c->ids[nr],
                                     range_start, c->cell_end);
         });
-    } else {
+    } else if (!fused) {
         timed(c, "reorder", [&] {
             psb::launch_reorder(st, P, c->keys[res], c->vals[res], c->pos[os], c->vel[os], c->vap[os], c->rp[orr],
                                 c->ids[orr], c->pos[ns], c->vel[ns], c->vap[ns], c->rp[nr], c->ids[nr], range_start,

@@ -357,6 +357,15 @@ void launch_cell_count(cudaStream_t st, const Params& P, const float4* pos, uint
 void launch_cell_sort(cudaStream_t st, int n, size_t ncells, const int* ids, const uint32_t* keys, const uint32_t* ranks,
                       uint32_t* cell_count, uint32_t* tile_sum, uint32_t* cell_start, int* flags, uint2* placed,
                       uint32_t* keys_out, uint32_t* vals_out);
+// The same up to the arrival order in placed, and then the places and the
+// whole state into sorted order (scenes without a wall list).
+void launch_cell_place(cudaStream_t st, int n, size_t ncells, const int* ids, const uint32_t* keys,
+                       const uint32_t* ranks, uint32_t* cell_count, uint32_t* tile_sum, uint32_t* cell_start,
+                       int* flags, uint2* placed);
+void launch_rank_reorder(cudaStream_t st, const Params& P, const uint32_t* keys, const uint2* placed,
+                         const uint32_t* cell_start, const float4* pos, const float4* vel, const float4* vap,
+                         const float2* rp, const int* ids, uint32_t* keys_out, uint32_t* vals_out, float4* pos2,
+                         float4* vel2, float4* vap2, float2* rp2, int* ids2);
 // The whole state into sorted order, with the cell ranges; or in two
 // launches: positions, ids and cell ranges (what the neighbour build reads),
 // then the rest. cell_start null: the ranges are there already.
