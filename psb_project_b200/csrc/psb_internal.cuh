@@ -167,9 +167,9 @@ constexpr int kWallListMin = 131072;
 // kernel's end implies the end of all before it -- and then lets the next one
 // be placed. (Letting it be placed before the wait put several kernels' blocks
 // on the chip at once: a 16k particle WCSPH frame 843 us, 752 this way, 840
-// without.) Launched the usual way the wait returns at once. Kernels that
-// follow something other than a kernel (a memset, a waited event, a loop node
-// of a graph) are launched the usual way.
+// without.) Launched the usual way the wait returns at once. Only an order
+// between two kernels is loosened: behind a memset, a copy, a waited event or a
+// loop node of a graph a chained kernel starts as any other.
 __device__ __forceinline__ void after_previous() {
     cudaGridDependencySynchronize();
     cudaTriggerProgrammaticLaunchCompletion();
