@@ -89,6 +89,18 @@ __device__ __forceinline__ float4 at(const Soa3& a, int j) {
     const float2 xy = a.xy[j];
     return make_float4(xy.x, xy.y, a.z[j], 0.f);
 }
+// An 8-byte gather that stays one load where it is written, ahead of a pair's
+// tests: of a plain load of (z, pressure) the compiler moved the pressure
+// behind the tests, a second load there, and the pair waited for memory twice.
+// Pressure-force pass 97 -> 88 us at 1M particles, 294 -> 264 at 4M; set-up
+// sweep 146 -> 139 and 537 -> 504. (Velocities are better left to the compiler:
+// gathered this way the set-up sweep took 511 us at 4M, the density pass with
+// the network's inputs 132 against 124 at 1M.)
+__device__ __forceinline__ float2 gather2(const float2* p) {
+    float2 v;
+    asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(__cvta_generic_to_global(p)));
+    return v;
+}
 __device__ __forceinline__ void put(const Soa3& a, int t, float x, float y, float z) {
     a.xy[t] = make_float2(x, y);
     a.z[t] = z;
@@ -269,7 +281,7 @@ __device__ __forceinline__ void ghost_pressure(const Params& P, int t, float4 xi
     if (!near_faces(P, faces_of<BATCH>(P, t), xi, W)) return;
     const float ir0 = 1.f / __fmul_rn(P.rho0, P.rho0);
     for_each_nbr(list, P.n, t, cnt, [&](const int j) {
-        const float2 xy = P.x0.xy[j], zp = P.zp[j];
+        const float2 xy = gather2(P.x0.xy + j), zp = gather2(P.zp + j);
         ghost_pressure_pair(P, W, xi, make_float4(xy.x, xy.y, zp.x, 0.f), pVi, zp.y, ir0, ap);
     });
 }
@@ -606,8 +618,8 @@ __device__ __forceinline__ PairSums pair_sums(const Params& P, int t, float4 xi,
     const float pVi = WITH_PRESSURE ? pressure_volume<REF>(P, rpi) : 0.f;
     const int cnt = min(counts[t], P.cap);
     for_each_nbr(list, P.n, t, cnt, [&](const int j) {
-        // the pair's four 8-byte gathers, ahead of the tests
-        const float2 xy = P.x0.xy[j], zp = P.zp[j], vxy = P.v0.xy[j], vr = P.vr[j];
+        // the pair's four 8-byte gathers
+        const float2 xy = gather2(P.x0.xy + j), zp = gather2(P.zp + j), vxy = P.v0.xy[j], vr = P.vr[j];
         add_pair<REF, WITH_PRESSURE>(P, S, xi, vi, pVi, make_float4(xy.x, xy.y, zp.x, 0.f),
                                      make_float4(vxy.x, vxy.y, vr.x, 0.f), vr.y, zp.y);
     });
@@ -669,8 +681,9 @@ __global__ void __launch_bounds__(kBlock) k_wcsph_force(Params P, const float4* 
 // PCISPH set-up sweep: non-pressure forces at x (and, for a warm start, the
 // pressure acceleration of the carried pressure), then the first prediction.
 // Four 8-byte gathers a pair: bound by L1 wavefronts. With 1 / rho_j gathered
-// instead of rho_j (the division was ~10 of 79 instructions a pair) it takes
-// 147 us at 1M particles against 166, 538 at 4M against 613.
+// instead of rho_j (the division was ~10 of 79 instructions a pair) it took
+// 147 us at 1M particles against 166, 538 at 4M against 613; with gather2 139
+// and 504.
 template <bool REF, bool WARM, bool BATCH, int BS>
 __global__ void __launch_bounds__(BS, REF || !WARM ? 1 : kForceThreads / BS) k_pci_init(
     Params P, const float4* __restrict__ vap, const float2* __restrict__ rp, const int* __restrict__ counts,
@@ -883,7 +896,7 @@ __device__ __forceinline__ void pci_force_at(const Params& P, int t, const float
             const float2 rj = rpc[j];
             add_pressure_pair<REF>(P, xi, xj, pVi, rj, ir0, acc);
         } else {
-            const float2 xy = P.x0.xy[j], zp = P.zp[j];
+            const float2 xy = gather2(P.x0.xy + j), zp = gather2(P.zp + j);
             add_pressure_pair<REF>(P, xi, make_float4(xy.x, xy.y, zp.x, 0.f), pVi, zp, ir0, acc);
         }
     });
