@@ -295,10 +295,10 @@ __device__ __forceinline__ void ghost_pressure(const Params& P, int t, float4 xi
 // list ahead of the blocks over all slots, which skip the listed ones: full
 // warps of wall particles, started first. Each particle is summed by one
 // thread in the same order either way, so the results are the same bits.
-// Density pass / pressure-force pass with the list against without:
-// 78 / 86 against 88 / 96 us at 1,048,576 particles, 36 / 45 against 44 / 58
-// at 290,000; at 97,000, where the pass is one chain of loads and the list
-// adds two, 29 / 30 against 24 / 24 us.
+// Density pass / pressure-force pass (converged launches among the latter at
+// 1M) with the list against without: 71 / 69 against 79 / 78 us at 1,048,576
+// particles, 32 / 36 against 41 / 48 at 290,000; at 97,000, where the pass is
+// one chain of loads and the list adds two, 26 / 25 against 23 / 23 us.
 __device__ __forceinline__ bool in_wall_list(const Params& P, int t) {
     return P.wall_list && ((P.wall_bits[t >> 5] >> (t & 31)) & 1u);
 }
