@@ -167,8 +167,12 @@ __global__ void k_iso_weight(int n, double k_colour, const float2* __restrict__ 
 // FP32 test against the nearest of the thread's nodes, with a margin over its
 // own rounding (32 candidates to a mask), and only the rest, in order, see the
 // FP64 distances. Config profile: a particle within the radius lies in the
-// node's ring, so going over the union of several rings adds nothing to any
-// of them, and a candidate is loaded once for eight nodes. The field was bound
+// node's ring unless it was clamped into a border cell from outside the grid
+// (or has a NaN coordinate), so going over the union of several rings adds
+// nothing to any of them, and a candidate is loaded once for eight nodes. A
+// warp with a brick whose nodes lie in different cells and whose rings reach a
+// border cell adds a candidate to the nodes whose own ring holds it (OWN): the
+// field at a node does not depend on the nodes it is asked for with. The field was bound
 // by L1 wavefronts (93% of the data pipe with a node a thread, FP64 17%):
 // 128^3 nodes over 262,144 particles took 518 us in node order with every
 // candidate in FP64, 475 with the FP32 test, 412 with a warp's nodes in a
@@ -194,6 +198,7 @@ __global__ void __launch_bounds__(128) k_iso_field(IsoParams Q, Params P, const 
     if (ix >= Q.dims[0] || iy >= Q.dims[1] || iz >= Q.dims[2]) return;
     double px[E], py[E], pz[E];
     float fx[E], fy[E], fz[E];
+    int I[E], J[E], K[E];
     int lo_x = INT_MAX, hi_x = INT_MIN, lo_y = INT_MAX, hi_y = INT_MIN, lo_z = INT_MAX, hi_z = INT_MIN;
     // particle-grid cells of the nodes, as the reference computes them
     float far = 0.f;
@@ -201,13 +206,13 @@ __global__ void __launch_bounds__(128) k_iso_field(IsoParams Q, Params P, const 
     for (int e = 0; e < E; ++e) {
         px[e] = Q.origin[0] + (ix + e) * Q.spacing[0];
         py[e] = Q.origin[1] + (iy + e) * Q.spacing[1];
-        const int I = (int)floor((px[e] - (double)P.g.gx) / (double)P.g.cell);
-        const int J = (int)floor((py[e] - (double)P.g.gy) / (double)P.g.cell);
+        I[e] = (int)floor((px[e] - (double)P.g.gx) / (double)P.g.cell);
+        J[e] = (int)floor((py[e] - (double)P.g.gy) / (double)P.g.cell);
         pz[e] = Q.origin[2] + (iz + e) * Q.spacing[2];
-        const int K = (int)floor((pz[e] - (double)P.g.gz) / (double)P.g.cell);
-        lo_x = min(lo_x, I); hi_x = max(hi_x, I);
-        lo_y = min(lo_y, J); hi_y = max(hi_y, J);
-        lo_z = min(lo_z, K); hi_z = max(hi_z, K);
+        K[e] = (int)floor((pz[e] - (double)P.g.gz) / (double)P.g.cell);
+        lo_x = min(lo_x, I[e]); hi_x = max(hi_x, I[e]);
+        lo_y = min(lo_y, J[e]); hi_y = max(hi_y, J[e]);
+        lo_z = min(lo_z, K[e]); hi_z = max(hi_z, K[e]);
         fx[e] = (float)px[e];
         fy[e] = (float)py[e];
         fz[e] = (float)pz[e];
@@ -221,79 +226,103 @@ __global__ void __launch_bounds__(128) k_iso_field(IsoParams Q, Params P, const 
     far += (float)(ring + 1) * P.g.cell;
     const float reach = (float)Q.r * 1.0001f + far * 5e-7f;
     const float r2 = -(reach * reach);
+    const int k0 = max(lo_z - ring, 0), j0 = max(lo_y - ring, 0);
     const int k1 = min(hi_z + ring, P.g.nz - 1), j1 = min(hi_y + ring, P.g.ny - 1);
-    for (int k = max(lo_z - ring, 0); k <= k1 && a0 <= a1; ++k) {
-        for (int j = max(lo_y - ring, 0); j <= j1; ++j) {
-            const uint32_t row = (uint32_t)j * P.g.nx + (uint32_t)k * P.g.nx * P.g.ny;
-            uint32_t lo, hi;
-            if (P.dense_cells) {
-                lo = cell_start[row + a0];
-                hi = cell_end[row + a1];
-            } else {
-                row_range(cell_start, cell_end, row, a0, a1, lo, hi);
-            }
-            for (; lo < hi; lo += 32u) {
-                const uint32_t m = min(hi - lo, 32u);
-                uint32_t mask = 0u;
-                for (uint32_t c = 0; c < m; c += 2) {
+    // slots of cells i0..i1 of a row (none: i0 > i1)
+    auto slots = [&](uint32_t row, int i0, int i1, uint32_t& lo, uint32_t& hi) {
+        lo = hi = 0u;
+        if (i0 > i1) return;
+        if (P.dense_cells) {
+            lo = cell_start[row + i0];
+            hi = cell_end[row + i1];
+        } else {
+            row_range(cell_start, cell_end, row, i0, i1, lo, hi);
+        }
+    };
+    auto rows = [&](auto own) {
+        constexpr bool OWN = decltype(own)::value;
+        for (int k = k0; k <= k1 && a0 <= a1; ++k) {
+            for (int j = j0; j <= j1; ++j) {
+                const uint32_t row = (uint32_t)j * P.g.nx + (uint32_t)k * P.g.nx * P.g.ny;
+                uint32_t lo, hi, first[E], end[E];      // first, end: the part of the row in node e's own ring
+                bool in_y[E], in_z[E];
+                slots(row, a0, a1, lo, hi);
+                if (OWN) {
 #pragma unroll
-                    for (uint32_t u = 0; u < 2; ++u) {
-                        const float4 x = pos[lo + c + u];       // padded past the last particle
-                        // the nearest node's distance: the nearest on each axis, as rounding is monotonic
-                        float dx = fabsf(fx[0] - x.x), dy = fabsf(fy[0] - x.y), dz = fabsf(fz[0] - x.z);
-#pragma unroll
-                        for (int e = 1; e < E; ++e) {
-                            dx = fminf(dx, fabsf(fx[e] - x.x));
-                            dy = fminf(dy, fabsf(fy[e] - x.y));
-                            dz = fminf(dz, fabsf(fz[e] - x.z));
-                        }
-                        const float best = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmaf_rn(dz, dz, r2)));
-                        // a NaN position stays in, as in the FP64 test
-                        const bool in = !(best >= 0.f && best < INFINITY);
-                        mask = mask << 1 | (in ? 1u : 0u);
+                    for (int e = 0; e < E; ++e) {
+                        in_y[e] = abs(j - J[e]) <= ring;
+                        in_z[e] = abs(k - K[e]) <= ring;
+                        slots(row, max(I[e] - ring, 0), min(I[e] + ring, P.g.nx - 1), first[e], end[e]);
                     }
                 }
-                mask = (mask << (32u - ((m + 1u) & ~1u))) & (kEmpty << (32u - m));
-                uint32_t t = lo;
-                while (mask) {
-                    const int z = __clz((int)mask);
-                    mask = (mask << z) << 1;
-                    t += (uint32_t)z;
-                    const float4 x = pos[t];
-                    if (REF) {
-                        const double dx = px[0] - x.x, dy = py[0] - x.y, dz = pz[0] - x.z;
-                        const double d2 = dx * dx + dy * dy + dz * dz;
-                        // d = length(pos1 - pos2); (1/powf(r,6)) * powf(r*r - d*d, 3) in float
-                        const double d = sqrt(d2);
-                        if (d <= Q.r) {
-                            const float term = (1.f / powf((float)Q.r, 6.f)) * powf((float)(Q.r * Q.r - d * d), 3.f);
-                            acc[0][0][0] += (double)term;
+                for (; lo < hi; lo += 32u) {
+                    const uint32_t m = min(hi - lo, 32u);
+                    uint32_t mask = 0u;
+                    for (uint32_t c = 0; c < m; c += 2) {
+#pragma unroll
+                        for (uint32_t u = 0; u < 2; ++u) {
+                            const float4 x = pos[lo + c + u];       // padded past the last particle
+                            // the nearest node's distance: the nearest on each axis, as rounding is monotonic
+                            float dx = fabsf(fx[0] - x.x), dy = fabsf(fy[0] - x.y), dz = fabsf(fz[0] - x.z);
+#pragma unroll
+                            for (int e = 1; e < E; ++e) {
+                                dx = fminf(dx, fabsf(fx[e] - x.x));
+                                dy = fminf(dy, fabsf(fy[e] - x.y));
+                                dz = fminf(dz, fabsf(fz[e] - x.z));
+                            }
+                            const float best = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmaf_rn(dz, dz, r2)));
+                            // a NaN position stays in, as in the FP64 test
+                            const bool in = !(best >= 0.f && best < INFINITY);
+                            mask = mask << 1 | (in ? 1u : 0u);
                         }
-                    } else {
-                        const double wt = weight[t];
+                    }
+                    mask = (mask << (32u - ((m + 1u) & ~1u))) & (kEmpty << (32u - m));
+                    uint32_t t = lo;
+                    while (mask) {
+                        const int z = __clz((int)mask);
+                        mask = (mask << z) << 1;
+                        t += (uint32_t)z;
+                        const float4 x = pos[t];
+                        if (REF) {
+                            const double dx = px[0] - x.x, dy = py[0] - x.y, dz = pz[0] - x.z;
+                            const double d2 = dx * dx + dy * dy + dz * dz;
+                            // d = length(pos1 - pos2); (1/powf(r,6)) * powf(r*r - d*d, 3) in float
+                            const double d = sqrt(d2);
+                            if (d <= Q.r) {
+                                const float term = (1.f / powf((float)Q.r, 6.f)) * powf((float)(Q.r * Q.r - d * d), 3.f);
+                                acc[0][0][0] += (double)term;
+                            }
+                        } else {
+                            const double wt = weight[t];
 #pragma unroll
-                        for (int g = 0; g < E; ++g) {
-                            const double dz = pz[g] - x.z, dz2 = dz * dz;
+                            for (int g = 0; g < E; ++g) {
+                                const double dz = pz[g] - x.z, dz2 = dz * dz;
 #pragma unroll
-                            for (int f = 0; f < E; ++f) {
-                                const double dy = py[f] - x.y, dy2 = dy * dy + dz2;
+                                for (int f = 0; f < E; ++f) {
+                                    const double dy = py[f] - x.y, dy2 = dy * dy + dz2;
 #pragma unroll
-                                for (int e = 0; e < E; ++e) {
-                                    const double dx = px[e] - x.x;
-                                    const double q = (dx * dx + dy2) * Q.inv_r2;
-                                    if (!(q >= 1.0)) {
-                                        const double w = 1.0 - q;
-                                        acc[g][f][e] += w * w * w * wt;
+                                    for (int e = 0; e < E; ++e) {
+                                        const double dx = px[e] - x.x;
+                                        const double q = (dx * dx + dy2) * Q.inv_r2;
+                                        const bool mine = !OWN || (in_z[g] && in_y[f] && t >= first[e] && t < end[e]);
+                                        if (mine && !(q >= 1.0)) {
+                                            const double w = 1.0 - q;
+                                            acc[g][f][e] += w * w * w * wt;
+                                        }
                                     }
                                 }
                             }
                         }
+                        ++t;
                     }
-                    ++t;
                 }
             }
         }
-    }
+    };
+    const bool apart = lo_x != hi_x || lo_y != hi_y || lo_z != hi_z;
+    const bool border = a0 == 0 || a1 == P.g.nx - 1 || j0 == 0 || j1 == P.g.ny - 1 || k0 == 0 || k1 == P.g.nz - 1;
+    if (E > 1 && __any_sync(__activemask(), apart && border)) rows(std::true_type{});
+    else rows(std::false_type{});
 #pragma unroll
     for (int g = 0; g < E; ++g)
 #pragma unroll
