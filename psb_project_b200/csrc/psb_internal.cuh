@@ -214,16 +214,19 @@ inline size_t nbr_list_ints(size_t n, int cap) { return n * (size_t)((cap + 3) &
 // f(j) for the first cnt entries of slot t's list, in order. The next quad's
 // load is issued behind the current quad's gathers, so a quad costs one
 // latency, not two (density pass at 1M particles alone: 61 against 66 us).
-template <class F>
-__device__ __forceinline__ void for_each_nbr(const int* __restrict__ list, int n, int t, int cnt, F&& f) {
-    const int4* __restrict__ L = reinterpret_cast<const int4*>(list) + t;
+// FRESH: the kernel that calls it writes the lists, each thread its own, so
+// they are not loaded through the read-only path.
+template <bool FRESH = false, class F>
+__device__ __forceinline__ void for_each_nbr(const int* list, int n, int t, int cnt, F&& f) {
+    const int4* L = reinterpret_cast<const int4*>(list) + t;
+    auto load = [&] { return FRESH ? *L : __ldg(L); };
     int4 q = make_int4(0, 0, 0, 0);
-    if (cnt > 0) q = __ldg(L);
+    if (cnt > 0) q = load();
     int c = 0;
     for (; c + 4 <= cnt; c += 4) {
         int4 next = q;
         L += n;
-        if (c + 4 < cnt) next = __ldg(L);
+        if (c + 4 < cnt) next = load();
         f(q.x); f(q.y); f(q.z); f(q.w);
         q = next;
     }

@@ -265,12 +265,12 @@ __device__ __forceinline__ void ghost_pressure_pair(const Params& P, const NearF
 // particles within h of a face take (the walls are evaluated at xi). Kept
 // out of the main walk: a per-neighbour wall test there slows every
 // particle more than the separate walk costs the few near the faces.
-template <bool BATCH = false>
-__device__ __forceinline__ void ghost_density(const Params& P, int t, float4 xi, const Soa3& x,
-                                              const int* __restrict__ list, int cnt, Kahan& acc) {
+template <bool BATCH = false, bool FRESH = false>
+__device__ __forceinline__ void ghost_density(const Params& P, int t, float4 xi, const Soa3& x, const int* list,
+                                              int cnt, Kahan& acc) {
     NearFaces W;
     if (!near_faces(P, faces_of<BATCH>(P, t), xi, W)) return;
-    for_each_nbr(list, P.n, t, cnt, [&](const int j) { ghost_density_pair(P, W, xi, at(x, j), acc); });
+    for_each_nbr<FRESH>(list, P.n, t, cnt, [&](const int j) { ghost_density_pair(P, W, xi, at(x, j), acc); });
 }
 
 // The neighbours at the step's start positions with the pressures of P.zp.
@@ -457,12 +457,13 @@ struct DensityX {
     }
     // wall ghosts and boundary particles (config), then density, pressure
     // (EOS, or the carried / zeroed PCISPH pressure) and the features
-    template <bool BATCH>
-    __device__ __forceinline__ void finish(const Params& P, int t, float4 xi, const int* __restrict__ list, int cnt, int count, float2* __restrict__ rp,
-                                           float* __restrict__ rho_x, int zero_p, float p_scale,
-                                           float* __restrict__ feats) {
+    // (FRESH: over lists this kernel has written)
+    template <bool BATCH, bool FRESH = false>
+    __device__ __forceinline__ void finish(const Params& P, int t, float4 xi, const int* list, int cnt, int count,
+                                           float2* __restrict__ rp, float* __restrict__ rho_x, int zero_p,
+                                           float p_scale, float* __restrict__ feats) {
         if (!REF) {
-            ghost_density<BATCH>(P, t, xi, P.x0, list, cnt, acc);
+            ghost_density<BATCH, FRESH>(P, t, xi, P.x0, list, cnt, acc);
             if (!BATCH) boundary_density(P, t, xi, acc, P.bnd);
         }
         const float drho = density_deviation(P, acc);
@@ -560,7 +561,7 @@ __global__ void __launch_bounds__(BS) k_build_density(Params P, const float4* __
         });
         counts[t] = cnt;
         if (cnt > P.cap) atomicOr(&flags[0], 1);
-        D.template finish<false>(P, t, pi, list, min(cnt, P.cap), cnt, rp, rho_x, zero_p, p_scale, feats);
+        D.template finish<false, true>(P, t, pi, list, min(cnt, P.cap), cnt, rp, rho_x, zero_p, p_scale, feats);
     }
     nbr_flags(cnt, flags);
 }
