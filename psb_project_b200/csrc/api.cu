@@ -111,8 +111,10 @@ struct psb_ctx {
     uint32_t* cell_start = nullptr;
     uint32_t* cell_end = nullptr;
     size_t ncells = 0;
-    // the counting sort's words (dense_cells; grid.cu): cell_end is then
-    // cell_start + 1, and no cell is ever reset
+    // the counting sort (grid.cu): whether the context has its words, and
+    // whether the cell words are in its form: cell_end is then cell_start + 1,
+    // and no cell is ever reset
+    bool can_count = false;
     bool dense = false;
     uint32_t* cell_count = nullptr;
     uint32_t* tile_sum = nullptr;
@@ -546,13 +548,36 @@ int bits_for(size_t ncells) {
     return b;
 }
 
-// Whether a context of n particles sorts by counting over its ncells cells
-// (grid.cu) rather than by radix. Counting touches every cell (~12 B each,
-// little of it past L2: 15 us at 8.3M cells) and every particle about as often
-// as one radix pass of the 2-4 it replaces (28 us each at 1M). It is the
-// faster side up to a few million cells whatever n (the radix passes' launches
-// alone are ~40 us), and beyond that while the cells stay within 24 a particle.
-bool dense_cells(size_t ncells, size_t n) { return ncells <= std::max((size_t)4 << 20, 24 * n); }
+// Whether a context of up to n_max particles can sort by counting over its
+// ncells cells (grid.cu) and not only by radix: up to a few million cells
+// whatever n_max, and beyond that within 24 cells a particle.
+bool has_cell_counts(size_t ncells, size_t n_max) { return ncells <= std::max((size_t)4 << 20, 24 * n_max); }
+
+// Whether counting is the faster sort of the n particles a context holds.
+// Counting touches every cell and, in its scan, every earlier tile of cells;
+// radix only the particles, four times in grids this large. From keys to the
+// reorder's end, counting against radix: 86 against 104 us at 97M cells and
+// 20,000 particles, 273 / 344 at 97M and 4.0M, 160 / 96 at 200M and 20,000,
+// 209 / 144 at 200M and 1.0M, 343 / 344 at 200M and 4.0M, 570 / 103 at 475M
+// and 20,000, 746 / 345 at 475M and 4.0M, 1,493 / 1,650 at 475M and 20.4M. The
+// line between them, in us and millions; below ~98M cells it is always counting.
+bool counting_pays(size_t ncells, size_t n) {
+    const double cells = 1e-6 * (double)ncells;
+    return (0.66 + 0.001 * cells) * cells <= 75.0 + 27.0e-6 * (double)n;
+}
+
+// Puts the cell words into the form of one of the two sorts: no particles in
+// any cell. Only where the particle count has crossed counting_pays' line; a
+// step's graph is launched after a build of the same count, so it holds none.
+int set_sort(psb_ctx* c, cudaStream_t st, bool dense) {
+    c->dense = dense;
+    c->P.dense_cells = dense;
+    c->cell_end = dense ? c->cell_start + 1 : c->cell_count;
+    const size_t words = psb::cell_sort_cells(c->ncells) + psb::cell_sort_tiles(c->ncells);
+    const cudaError_t e = dense ? cudaMemsetAsync(c->cell_count, 0, sizeof(uint32_t) * words, st)
+                                : cudaMemsetAsync(c->cell_start, 0xFF, sizeof(uint32_t) * c->ncells, st);
+    return cuda_check(c, e, "cell words");
+}
 
 // Whether the density pass at x is folded into the neighbour build
 // (schedule 2): one config-profile PCISPH scene; batches, the reference
@@ -564,16 +589,21 @@ bool fused_density(const psb_ctx* c, const Params& P) { return can_fuse_density(
 // carried pressure in place even where the scene starts every step from 0.
 int build(psb_ctx* c, bool keep_p = false, bool features = false) {
     cudaStream_t st = c->stream;
-    Params P = c->P;
-    P.n = c->n;
     const int n = c->n;
-    const int rs = c->sorted >= 0 ? c->sorted : c->stale;       // cells occupied by the previous sort
+    int rs = c->sorted >= 0 ? c->sorted : c->stale;             // cells occupied by the previous sort
     const int rn = c->sorted >= 0 ? c->sorted_n : c->stale_n;
-    if (rs >= 0 && !c->dense)
+    const bool dense = c->can_count && counting_pays(c->ncells, (size_t)n);
+    if (dense != c->dense) {
+        PSB_TRY(set_sort(c, st, dense));
+        rs = -1;
+    }
+    Params P = c->P;
+    P.n = n;
+    if (rs >= 0 && !dense)
         timed(c, "reset_cells", [&] { psb::launch_reset_cells(st, rn, c->keys[rs], c->cell_start); });
     c->stale = -1;
     // the counting sort clears the words itself
-    if (!c->dense || n <= 0) cudaMemsetAsync(c->flags, 0, 8 * sizeof(int), st);
+    if (!dense || n <= 0) cudaMemsetAsync(c->flags, 0, 8 * sizeof(int), st);
     int res = 0;
     const int os = c->cs, orr = c->cr, ns = os ^ 1, nr = orr ^ 1;
     // The first step after an upload gathers the positions first and the
@@ -581,9 +611,9 @@ int build(psb_ctx* c, bool keep_p = false, bool features = false) {
     // of it are in: they overlap the grid and the build. Other steps gather
     // everything in one launch, small ones in the sort's last.
     const bool split = capturing(st) ? c->capture_split : c->in_pending;
-    const bool fused = c->dense && !split && n < psb::kWallListMin;
+    const bool fused = dense && !split && n < psb::kWallListMin;
     uint32_t* range_start = c->cell_start;      // the reorder records the cell ranges
-    if (c->dense) {
+    if (dense) {
         timed(c, "cell_keys", [&] {
             psb::launch_cell_count(st, P, c->pos[os], c->keys[0], c->vals[0], c->cell_count, c->tile_sum, &c->flags[6]);
         });
@@ -1076,7 +1106,7 @@ int create_impl(const psb_scene* scene, size_t ncells, int S, bool batch, psb_ct
     c->hist_blocks = psb::radix_blocks(c->n_max);
     cudaGetDevice(&c->device);
     const size_t n = (size_t)c->n_max, s_ = (size_t)S;
-    c->dense = dense_cells(c->ncells, n);
+    c->can_count = c->dense = has_cell_counts(c->ncells, n);
     c->P.dense_cells = c->dense;
     const bool ghosts = !c->P.ref && !c->P.dem;
     const size_t words = psb::cell_sort_cells(c->ncells), tiles = psb::cell_sort_tiles(c->ncells);
@@ -1095,13 +1125,13 @@ int create_impl(const psb_scene* scene, size_t ncells, int S, bool batch, psb_ct
             take(c->keys[i], n); take(c->vals[i], n);
             take(c->xs[i].xy, n); take(c->xs[i].z, n);
         }
-        if (c->dense) {
+        take(c->hist, (size_t)256 * c->hist_blocks + 256);
+        if (c->can_count) {
             take(c->cell_start, words);
             take(c->cell_count, words + tiles);
             c->cell_end = c->cell_start + 1;
             c->tile_sum = c->cell_count + words;
         } else {
-            take(c->hist, (size_t)256 * c->hist_blocks + 256);
             take(c->cell_start, c->ncells);
             take(c->cell_end, c->ncells);
         }
@@ -1154,7 +1184,7 @@ int create_impl(const psb_scene* scene, size_t ncells, int S, bool batch, psb_ct
         auto fill = [&](void* p, int v, size_t bytes) {
             if (!rc && cudaMemsetAsync(p, v, bytes, nullptr) != cudaSuccess) rc = PSB_ECUDA;
         };
-        if (c->dense) fill(c->cell_count, 0, sizeof(uint32_t) * (words + tiles));
+        if (c->can_count) fill(c->cell_count, 0, sizeof(uint32_t) * (words + tiles));
         else fill(c->cell_start, 0xFF, sizeof(uint32_t) * c->ncells);
         fill(c->mlp_w, 0, sizeof(float) * psb::kMlpParams);
         fill(c->mlp_wbf, 0, 2 * psb::kMlpParams);
