@@ -344,9 +344,12 @@ int psb_batch_stats(psb_ctx* ctx, int32_t* iters, int32_t* converged, double* er
  * commit. Graphs are captured on first use, one per state buffer parity,
  * recaptured after emissions change the particle count, and released by
  * psb_set_graph(ctx, 0) and psb_destroy. Steps that record training data,
- * emit particles or run with profiling on are launched kernel by kernel,
- * the corrector deciding on the device with one 4-byte read per pass; both
- * ways launch the same kernels in the same order. */
+ * emit particles or run with profiling on are launched kernel by kernel, the
+ * corrector deciding on the device and writing one word per pass into host
+ * memory; both ways launch the same kernels in the same order. The calling
+ * thread polls that word, unless the device is set to
+ * cudaDeviceScheduleBlockingSync (it sleeps until the pass is done) or
+ * cudaDeviceScheduleYield (it yields between looks). */
 int psb_set_graph(psb_ctx* ctx, int32_t on);
 
 /* The corrector loop of batches and config-profile PCISPH scenes (others

@@ -16,6 +16,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <thread>
 #include <vector>
 #include <algorithm>
 #include <map>
@@ -730,10 +731,14 @@ void move_boundary(psb_ctx* c, cudaStream_t st, const Params& P, int s, int r) {
 // 2 another pass. The pressure-force pass is still running then, so the next
 // pass is enqueued behind it; a copy and a wait for the stream at the end of
 // each pass left the device idle for ~12 us of ~100 (262k particles, 50 passes,
-// moving boundary). The stream is asked now and then, so that an error ends the wait.
-int await_decision(psb_ctx* c, cudaStream_t st) {
+// moving boundary). The stream is asked now and then, so that an error ends the
+// wait. A device set to cudaDeviceScheduleBlockingSync has its host threads
+// sleep while they wait: there the wait is for the stream.
+int await_decision(psb_ctx* c, cudaStream_t st, unsigned schedule) {
     const volatile int* word = c->h_go;
+    if (schedule == cudaDeviceScheduleBlockingSync) PSB_TRY(cuda_check(c, cudaStreamSynchronize(st), "sync"));
     for (unsigned turn = 1; *word == 0; ++turn) {
+        if (schedule == cudaDeviceScheduleYield) std::this_thread::yield();
         if (turn % 256) continue;
         const cudaError_t e = cudaStreamQuery(st);
         if (e == cudaErrorNotReady) {
@@ -792,11 +797,14 @@ int batch_corrector(psb_ctx* c, const Params& P, int s, int r, bool capture) {
         if (moving) move_boundary(c, bs, P, s, r);
     };
     if (!capture) {
+        unsigned schedule = 0;
+        cudaGetDeviceFlags(&schedule);
+        schedule &= cudaDeviceScheduleMask;
         for (int k = 0; k < max_it; ++k) {
             *c->h_go = 0;
             body(st, 0, 0);
             PSB_TRY(cuda_check(c, cudaGetLastError(), "launch"));
-            PSB_TRY(await_decision(c, st));
+            PSB_TRY(await_decision(c, st, schedule));
             if (*c->h_go == 1) break;
         }
         return PSB_OK;
