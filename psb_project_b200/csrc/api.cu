@@ -1626,7 +1626,7 @@ int psb_mlp_train(psb_ctx* c, int32_t iters, int32_t batch, float lr, uint64_t s
         ++c->mlp_step;
         timed(c, "mlp_train", [&] {
             psb::launch_mlp_step(st, c->mlp_arch, batch, c->ds_X, c->ds_T, rows, draw, c->mlp_part, c->mlp_grad,
-                                 c->mlp_loss, c->mlp_w, c->mlp_m1, c->mlp_m2, c->mlp_wbf, lr, c->mlp_step);
+                                 c->mlp_loss, c->mlp_w, c->mlp_m1, c->mlp_m2, c->mlp_wbf, lr, c->mlp_step, it > 0);
         });
     }
     if (loss) {

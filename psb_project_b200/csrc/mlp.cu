@@ -343,8 +343,9 @@ __global__ void __launch_bounds__(kTrainWarps * 32, ACT == kRelu ? 3 : 1) k_mlp_
         t0 = v0 ? T[row0] : 0.f;
         t1 = v1 ? T[row1] : 0.f;
     };
-    // (the samples are no chained kernel's output: they are fetched while the
-    // previous step's reduction runs, 64 steps 2453 -> 2385 us)
+    // (fetched while the previous step's reduction runs, 64 steps 2453 -> 2385
+    // us: nothing in a run of steps writes the samples, and the launches that
+    // may follow a kernel that does are not chained, see grad_launch)
     fetch(blockIdx.x);
     for (int i = threadIdx.x; i < kTrainWarps * (3 * kH + 2); i += blockDim.x) (&S.G[0][0])[i] = 0.f;
     after_previous();
@@ -639,15 +640,22 @@ void launch_mlp_forward(cudaStream_t st, int arch, int n, const float* X, const 
 }
 
 namespace {
+// after_step: the stream's last kernel is another step's reduction.
 void grad_launch(cudaStream_t st, int arch, int batch, const float* X, const float* T, uint64_t rows, uint64_t seed,
-                 const void* wbf, float* partial, float* grad, float* loss, const AdamStep& adam) {
+                 const void* wbf, float* partial, float* grad, float* loss, const AdamStep& adam, bool after_step) {
     const int tiles = (batch + kTrainRows - 1) / kTrainRows;
     const int blocks = std::min(tiles, kMlpGradBlocks);
     with_arch(arch, [&](auto nin, auto a) {
         auto kernel = k_mlp_train_mma<decltype(nin)::value, decltype(a)::value>;
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TrainSmem));
-        launch_chained(kernel, blocks, kTrainWarps * 32, sizeof(TrainSmem), st, batch, X, T, rows, seed,
-                       (const __nv_bfloat16*)wbf, partial);
+        const __nv_bfloat16* weights = (const __nv_bfloat16*)wbf;
+        // the kernel reads samples ahead of its wait: behind anything but a
+        // step (a recording of samples, say) it starts when that has ended
+        if (after_step)
+            launch_chained(kernel, blocks, kTrainWarps * 32, sizeof(TrainSmem), st, batch, X, T, rows, seed, weights,
+                           partial);
+        else
+            kernel<<<blocks, kTrainWarps * 32, sizeof(TrainSmem), st>>>(batch, X, T, rows, seed, weights, partial);
     });
     const int np = mlp_params(arch);
     launch_chained(k_grad_reduce, (np + 1 + 31) / 32, 256, 0, st, blocks, np, partial, grad, loss, adam);
@@ -661,16 +669,16 @@ void launch_mlp_grad(cudaStream_t st, int arch, int batch, const float* X, const
         cudaMemsetAsync(loss, 0, sizeof(float), st);
         return;
     }
-    grad_launch(st, arch, batch, X, T, 0, 0, wbf, partial, grad, loss, AdamStep{});
+    grad_launch(st, arch, batch, X, T, 0, 0, wbf, partial, grad, loss, AdamStep{}, false);
 }
 
 void launch_mlp_step(cudaStream_t st, int arch, int batch, const float* X, const float* T, uint64_t rows, uint64_t seed,
                      float* partial, float* grad, float* loss, float* w, float* m1, float* m2, void* wbf, float lr,
-                     int step) {
+                     int step, bool after_step) {
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - powf(b1, (float)step), c2 = 1.f - powf(b2, (float)step);
     grad_launch(st, arch, batch, X, T, rows, seed, wbf, partial, grad, loss,
-                AdamStep{w, m1, m2, (__nv_bfloat16*)wbf, lr, b1, b2, 1e-8f, c1, c2});
+                AdamStep{w, m1, m2, (__nv_bfloat16*)wbf, lr, b1, b2, 1e-8f, c1, c2}, after_step);
 }
 
 void launch_to_bf16(cudaStream_t st, int np, const float* w, void* wbf) {

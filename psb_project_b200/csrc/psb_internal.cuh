@@ -524,10 +524,11 @@ constexpr int kMlpGradBlocks = 148 * 4;
 constexpr size_t kMlpGradPartials = (size_t)kMlpGradBlocks * (kMlpParams + 1);
 void launch_mlp_grad(cudaStream_t st, int arch, int batch, const float* X, const float* T, const void* wbf,
                      float* partial, float* grad, float* loss);
-// One Adam step on a minibatch drawn from `rows` recorded rows (rows > 0).
+// One Adam step on a minibatch drawn from `rows` recorded rows (rows > 0);
+// after_step: enqueued directly behind another one.
 void launch_mlp_step(cudaStream_t st, int arch, int batch, const float* X, const float* T, uint64_t rows, uint64_t seed,
                      float* partial, float* grad, float* loss, float* w, float* m1, float* m2, void* wbf, float lr,
-                     int step);
+                     int step, bool after_step);
 void launch_to_bf16(cudaStream_t st, int np, const float* w, void* wbf);
 void launch_collect(cudaStream_t st, int n, int stride, int offset, uint64_t base, uint64_t cap, const float* feats,
                     const float2* rp, float p_scale, float* X, float* T);
