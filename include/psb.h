@@ -233,9 +233,10 @@ int psb_lattice(const int32_t nxyz[3], double spacing, const double origin[3], d
 /* Allocation-free sort. No counterpart in the reference: its launchers take
  * buffers the caller allocated up front and keep no scratch.
  *
- * Sorts n (key, value) pairs of device memory stably by key (the same LSD
- * radix sort psb_step uses for (cell, id) ordering), reading keys_in/vals_in
- * and writing keys_out/vals_out; key_bits (1..32) bounds the keys. For
+ * Sorts n (key, value) pairs of device memory stably by key (the LSD radix
+ * sort psb_step uses for (cell, id) ordering on sparse grids; up to 8,192 pairs
+ * in one block, without the array below), reading keys_in/vals_in and
+ * writing keys_out/vals_out; key_bits (1..32) bounds the keys. For
  * callers that cannot allocate device memory -- hosts that give the whole
  * GPU to their own memory pool and forbid libraries from allocating, and
  * per-frame loops that must not stall on cudaMalloc/cudaFree, which can

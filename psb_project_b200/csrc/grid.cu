@@ -1,5 +1,7 @@
-// grid.cu -- uniform-grid neighbour search: cell keys, stable radix sort by
-// (cell, id), cell-ordered reindexing with cell ranges, neighbour lists.
+// grid.cu -- uniform-grid neighbour search: cell keys, stable sort by (cell,
+// id), cell-ordered reindexing with cell ranges, neighbour lists. The sort is a
+// counting sort over the cells, or, where the grid is too sparse for the
+// particles, an LSD radix sort of the keys (api.cu, counting_pays).
 //
 // Replaces the reference's bucket grid (64 atomically filled slots per cell,
 // src/Utils/Neighborhood/UniformGrid/UniformGridKernel.cu:30-55) and its
@@ -9,8 +11,9 @@
 //     corner and cell edge (UniformGridKernel.cu:46-49), linearised as
 //     i + j*nx + k*nx*ny (:50);
 //   * the neighbour test length(x_i - x_j) <= h, self included (:81-82):
-//     decided in FP32 with a guard band and, inside the band, re-evaluated
-//     in FP64 with separately rounded operations in the reference's order.
+//     decided in FP32 (the sign of |d|^2 - h^2, collected per row of cells)
+//     and, within a band about h, re-evaluated in FP64 with separately rounded
+//     operations in the reference's order.
 // What differs by design: particles are sorted stably by (cell, id), so the
 // neighbour order is deterministic; particles outside the grid are clamped
 // into the border cells (the reference writes out of bounds there); lists
@@ -608,7 +611,8 @@ __global__ void k_reorder_state(Params P, const uint32_t* __restrict__ vals, con
 // over again with the reference's FP64 test. (A block of fluid started on a
 // lattice of spacing h/2 has candidates at exactly h in five of its nine rows;
 // going over the whole row took 198 us at 1M such particles and 26.9 at 16k,
-// the fours 184 and 23.0.) The masks of the nine rows wait in shared memory;
+// the fours 184 and 23.0.) Of a NaN coordinate e is the canonical NaN, whose
+// sign bit is clear: the particle is nobody's neighbour, as in a comparison. The masks of the nine rows wait in shared memory;
 // the list is then written quad by quad, every lane's k-th quad in the same
 // store (512 contiguous bytes a warp), where one 4-byte store per entry was a
 // sector write for each of 34M entries at 1M particles.

@@ -1,7 +1,7 @@
 // mc.cu -- iso field on a node grid and marching-cubes surface extraction.
 //
-// Iso field (one thread per node, gathered over the particle grid's cell
-// rings, FP64 accumulation):
+// Iso field (a thread per node or per brick of nodes, gathered over the
+// particle grid's cell rings, FP64 accumulation):
 //   reference profile: evaluateIso_Kernel (UniformGridKernel.cu:98-138):
 //     r = h / scale, ring = floor(1/scale) cells,
 //     iso(x) = sum_{|x - x_j| <= r} (1/r^6) (r^2 - d^2)^3, each term in float
@@ -14,9 +14,10 @@
 // iso(corner c) <= level, vertices on the edges by linear interpolation with
 // the reference's 1e-6 guards. The reference keeps 15 vertex slots per cell
 // and welds vertices on the host in O(V^2) (SurfaceSPH.cpp:120-186); here
-// every active grid edge owns one vertex (its index is the edge's rank in an
-// exclusive scan), so the mesh is welded by construction, and triangles are
-// written compacted through a second one.
+// every active grid edge owns one vertex, so the mesh is welded by
+// construction. Vertices and triangles are counted per block of nodes, one scan
+// over the blocks gives each block its first of both, and a second pass ranks
+// inside the block again and writes them compacted.
 //
 // The triangle table is generated here, not copied: for each of the 256
 // cases the active edges of every cube face are joined into segments (a face
@@ -179,9 +180,12 @@ __global__ void k_iso_weight(int n, double k_colour, const float2* __restrict__ 
 // brick, 273 with 2 x 2 x 1 nodes a thread, 247 with 2 x 2 x 2, 215 with the
 // FP32 test axis by axis instead of over the eight nodes. Nodes further
 // apart than half a cell share too little and take a thread each, and so do
-// the nodes of grids too small to fill the chip with eighths (64^3: 77 us
-// with a node a thread, 112 with eight; 80^3: 85 with eight, 117 for the kernel
-// before) and the reference profile's, whose ring may cut the radius off.
+// the nodes of grids too small to fill the chip with eighths, and the reference
+// profile's, whose ring may cut the radius off. A node a thread against eight,
+// spacing 0.3-0.5 / 0.15-0.4 of a cell: 48^3 nodes - / 56 against 72 us, 56^3 94 / 70
+// against 100 / 84, 64^3 119 / 91 against 91 / 87, 74^3 151 / 128 against 104 / 97,
+// 80^3 170 / 143 against 105 / 89: from 262,144 nodes on eight are the faster;
+// the line lies above that.
 constexpr long long kIsoBrickNodes = 393216;
 
 template <bool REF, int E>

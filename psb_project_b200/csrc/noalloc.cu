@@ -10,6 +10,9 @@
 // regular entry points allocate their buffers in psb_create; this one
 // allocates nothing, ever.
 //
+// Up to 8,192 pairs are sorted by one block in its shared memory (grid.cu,
+// small_sort): no scratch, and nothing shared between calls. Above that:
+//
 // The scratch: a file-scope static __device__ array sized for
 // PSB_NOALLOC_MAX_N elements. Every GPU that loads the library holds it
 // (about 2.1 MB) until the process exits. Host code cannot pass the array's
@@ -19,7 +22,7 @@
 // not caching it keeps the address right after the host application resets
 // the device and the runtime loads the module again.
 //
-// All calls share the one array and it keeps the last call's contents.
+// All such calls share the one array and it keeps the last call's contents.
 // Nothing in it needs clearing: every pass writes its histogram block by
 // block before the scan reads it, and the ping-pong half is fully written
 // before it is read. Calls that overlap on the GPU (different streams, or

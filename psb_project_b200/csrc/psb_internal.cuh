@@ -7,8 +7,9 @@
 //   vap   float4  leap-frog v+         16 B   (m_dVelInterAp)
 //   rp    float2  (density, pressure)   8 B   (pressure persists across steps)
 //   ids   int32   particle id           4 B
-// Per-step scratch: sort keys/values (2 x 2 x 4 B), cell_start/cell_end
-// (dense over the grid, only occupied cells are ever written or reset),
+// Per-step scratch: sort keys/values (2 x 2 x 4 B), the cells' slot ranges
+// (counting sort: every cell's, from the scan of the counts; radix sort: only
+// occupied cells are written, and reset before the next build),
 // neighbour lists (slot-major quads, see nbr_index; c < count[s]), and the
 // PCISPH predictor buffers xs[2] and vs (Soa3), rpc (float2),
 // fnp (float4 non-pressure force density), rho_x (float).
@@ -42,9 +43,11 @@ struct SceneGeom {
 
 // Launch configuration of the tunable kernels, the autotuner's choice for a
 // size bucket: block sizes (128, 256 or 512; 0 = 256) and the neighbour
-// build's schedule (0: each thread walks its own 27 cells; 1: the lanes of a
-// warp that share a grid row walk it together, staging candidates in shared
-// memory). Every choice computes the same result bit for bit.
+// build's schedule (0: each thread its own 27 cells, by sign masks; 1: the
+// lanes of a warp that share a grid row walk it together, staging candidates in
+// shared memory; 2: each thread's walk with the density pass at x folded in,
+// single config-profile PCISPH scenes, elsewhere as 0). Every choice computes
+// the same result bit for bit.
 struct Tune {
     int nbr_block, nbr_schedule, density_block, init_block, pci_density_block, force_block, xsph_block;
 };
@@ -152,8 +155,15 @@ struct Params {
 // Distance to a face, in h, up to which the reorder lists a particle: past
 // the h within which a face has ghosts, so that the corrector's predictions
 // (a CFL step moves a particle well under 0.1 h) rarely bring an unlisted
-// particle into range. The list is used from kWallListMin particles on
-// (sph.cu gives both sides' times).
+// particle into range. The list is used from kWallListMin particles on, where
+// a pass is no longer one chain of loads. A step (PCISPH with four
+// corrections, eager) with the list against without, blocks that fill their
+// box's floor: 306 / 276 us at 64,000 particles, 349 / 323 at 107,520, 365 /
+// 341 at 131,072, 411 / 386 at 184,320, 438 / 442 at 230,400, 462 / 506 at
+// 291,840, 671 / 760 at 522,240, 1,206 / 1,316 at 1,044,480: it pays from ~220,000
+// on. Scenes that are mostly wall lose by it further up, since the
+// list's blocks are sized for a quarter of the particles (four layers of
+// 65,536 between two faces: 873 / 512).
 constexpr float kWallReach = 1.1f;
 constexpr int kWallListMin = 131072;
 
@@ -177,8 +187,12 @@ __device__ __forceinline__ void after_previous() {
 
 // Threads up to which a launch is chained: a launch's start-up is worth ~2 us,
 // a part of the frame of 4k-290k particles (16 DEM steps 784 -> 600 us, four
-// PCISPH steps of 97k 1670 -> 1580, 50 corrections of 262k 5680 -> 5370), while
-// from 1M on the blocks placed early cost more than that (6570 -> 6630 us).
+// PCISPH steps of 97k 1670 -> 1580, 50 corrections of 262k 5680 -> 5370). In a
+// step's graph, as large scenes run, the blocks placed early cost as much from
+// ~350,000 particles on, chained against not: 503 / 504 us a step at 327,680,
+// 574 / 569 at 405,504, 692 / 690 at 524,160, 804 / 798 at 633,600, 1,031 / 1,019
+// at 860,160. Steps launched one by one still gain there (551 / 581, 670 / 702,
+// 781 / 818, 1,008 / 1,038); the line is where graphs still lose next to nothing.
 constexpr long long kChainThreads = 1 << 19;
 
 template <class... Params_, class... Args>
@@ -287,22 +301,20 @@ __device__ __forceinline__ void row_range(const uint32_t* __restrict__ cell_star
     if (lo == kEmpty) lo = 0u;
 }
 
-// The 27-cell walk of sorted particle t (one thread per particle): the three
-// cells of a grid row are adjacent in sorted order, so each of the nine rows
-// is one contiguous slot range, and accept(slot, position) runs for every
-// candidate within the list cut-off in increasing slot order, row by row --
-// the list order. In a batch the walk stays inside the particle's scene's
-// grid. Candidates beyond the FP32 window are out with one compare, those
-// below it in; inside it the reference's FP64 test decides.
-template <bool BATCH, class F>
+// The 27-cell walk of sorted particle t of a single scene (one thread per
+// particle; the build with the density folded in): the three cells of a grid
+// row are adjacent in sorted order, so each of the nine rows is one contiguous
+// slot range, and accept(slot, position) runs for every candidate within the
+// list cut-off in increasing slot order, row by row -- the list order.
+// Candidates beyond the FP32 window are out with one compare, those below it
+// in; inside it the reference's FP64 test decides.
+template <class F>
 __device__ __forceinline__ void walk_neighbours(const Params& P, int t, float4 pi, const float4* __restrict__ pos,
                                                 const uint32_t* __restrict__ keys,
                                                 const uint32_t* __restrict__ cell_start,
                                                 const uint32_t* __restrict__ cell_end, F&& accept) {
-    const Grid g = BATCH ? P.scenes[P.slot_scene[t]].g : P.g;
-    const uint32_t base = BATCH ? P.scenes[P.slot_scene[t]].cell_base : 0u;
-    const int nx = g.nx, ny = g.ny, nz = g.nz;
-    const uint32_t key = keys[t] - base;
+    const int nx = P.g.nx, ny = P.g.ny, nz = P.g.nz;
+    const uint32_t key = keys[t];
     const int ci = (int)(key % (uint32_t)nx);
     const int cj = (int)((key / (uint32_t)nx) % (uint32_t)ny);
     const int ck = (int)(key / ((uint32_t)nx * (uint32_t)ny));
@@ -313,7 +325,7 @@ __device__ __forceinline__ void walk_neighbours(const Params& P, int t, float4 p
     const int a0 = max(ci - 1, 0), a1 = min(ci + 1, nx - 1);
     for (int k = max(ck - 1, 0); k <= min(ck + 1, nz - 1); ++k) {
         for (int j = max(cj - 1, 0); j <= min(cj + 1, ny - 1); ++j) {
-            const uint32_t row = base + (uint32_t)j * (uint32_t)nx + (uint32_t)k * (uint32_t)nx * (uint32_t)ny;
+            const uint32_t row = (uint32_t)j * (uint32_t)nx + (uint32_t)k * (uint32_t)nx * (uint32_t)ny;
             uint32_t lo = kEmpty, hi = 0;
             for (int a = a0; a <= a1; ++a) {
                 const uint32_t s = cell_start[row + a];

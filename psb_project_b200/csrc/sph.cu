@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(BS) k_build_density(Params P, const float4* __
         D.begin(P, t);
         int* wq = list + nbr_index(0, P.n, t);
         const size_t qstride = (size_t)4 * (size_t)P.n;
-        walk_neighbours<false>(P, t, pi, pos, keys, cell_start, cell_end, [&](uint32_t q, float4 pj) {
+        walk_neighbours(P, t, pi, pos, keys, cell_start, cell_end, [&](uint32_t q, float4 pj) {
             if (cnt < P.cap) {
                 wq[cnt & 3] = (int)q;
                 D.pair(P, pi, pj, (int)q, rp);
