@@ -1133,7 +1133,6 @@ int create_impl(const psb_scene* scene, size_t ncells, int S, bool batch, psb_ct
             take(c->keys[i], n); take(c->vals[i], n);
             take(c->xs[i].xy, n); take(c->xs[i].z, n);
         }
-        take(c->hist, (size_t)256 * c->hist_blocks + 256);
         if (c->can_count) {
             take(c->cell_start, words);
             take(c->cell_count, words + tiles);
@@ -1170,6 +1169,7 @@ int create_impl(const psb_scene* scene, size_t ncells, int S, bool batch, psb_ct
         take(c->d_active, s_); take(c->d_err_scene, s_); take(c->d_err_sh, (PSB_MAX_ITERS + 1) * s_);
         take(c->d_loop, 2 + 4 * s_);
         if (batch) { take(c->d_scenes, s_); take(c->d_slot_scene, n); }
+        take(c->hist, (size_t)256 * c->hist_blocks + 256);
         dev_bytes = at;
         at = 0;
         auto pin = [&](auto& p, size_t count) {
